@@ -1,138 +1,392 @@
 // C[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) with plain 32-bit FMAs: the matrix product of the float32 path, and the
 // general fallback of the bfloat16 path for sizes the tensor-core kernel refuses.
 //
-// Every output element is one chain of fmaf over k = 0, 1, ..., K-1 in that order, started from zero, whatever M, N,
-// the tile or the thread it lands in. So a row's result has the same bits in every batch and every cutting of the
-// work, and no reduced-precision mode is involved (the reference's CUDA "float32" product is a 3xTF32 tensor-core
-// kernel, fusezap/device/cuda_kernels/tf32.py:1-12; its plain 32-bit product lives on its CPU device only).
+// Every output element is summed in one order that (N, K) alone fix, whatever M, the kernel, the tile or the thread it
+// lands in: K is cut into at most 32 chunks of equal length, a chunk is one chain of fmaf in rising k from zero, a group
+// of neighbouring chunks is added up in order, and the groups are added up in order. So a row's result has the same bits
+// in every batch and every cutting of the work, and no reduced-precision mode is involved (the reference's CUDA "float32"
+// product is a 3xTF32 tensor-core kernel, fusezap/device/cuda_kernels/tf32.py:1-12; its plain 32-bit product lives on its
+// CPU device only). The cuts are what lets a few rows use the whole chip: with one chain over all of K (the order before)
+// 4 x 4,864 -> 896 had 14 blocks to run in and took 215 us.
 //
-// Tiles of 64 x 64 outputs, 16 k per stage, 256 threads with 4 x 4 outputs each; operands are converted to float32
-// when staged in shared memory.
+// Few rows (M <= 16): `gemm_simt_few_kernel`, bound by reading W. More rows: `gemm_simt_tile_kernel`, bound by the FMA
+// pipes (a probe of independent fmaf chains reached 70 TFLOP/s; packed float32 x 2 forms reach no more).
 #include "common.cuh"
+#include <cooperative_groups.h>
+namespace cg = cooperative_groups;
 
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+// The order of an output's sum. `chunk` k (a multiple of 32) per chunk, `chunks` <= 32 of them, `per_group` chunks to a
+// group, `groups` <= 8 groups. A group is what one block of the tile kernel sums: at least 128 k, and the more groups the
+// fewer columns there are, so that a few hundred rows of a narrow product still give every SM work.
+struct Order { int chunk, chunks, per_group, groups; };
+Order order_of(int N, int K) {
+  Order o;
+  o.chunk = 32 * ((K + 1023) / 1024);
+  o.chunks = (K + o.chunk - 1) / o.chunk;
+  int g = K / 128 < 8 ? K / 128 : 8;
+  if (g > 16384 / N) g = 16384 / N;
+  if (g < 1) g = 1;
+  o.per_group = (o.chunks + g - 1) / g;
+  o.groups = (o.chunks + o.per_group - 1) / o.per_group;
+  return o;
+}
 
-template <typename TA, typename TC>
-__global__ void __launch_bounds__(256)
-gemm_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias,
-                 TC* __restrict__ C, int M, int N, int K) {
-  fz_grid_launch_dependents();
-  fz_grid_wait();
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Ws[BK][BN + 4];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  // staging: thread t loads row (t >> 2) and k offsets (t & 3) * 4 .. + 3 of both tiles
-  const int lr = tid >> 2, lk = (tid & 3) * 4;
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+__device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = ok ? 16 : 0;      // 0: the 16 bytes are filled with zeros and nothing is read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-  const TA* arow = A + (size_t)(m0 + lr) * K;
-  const TA* wrow = W + (size_t)(n0 + lr) * K;
-  const bool a_ok = m0 + lr < M, w_ok = n0 + lr < N;
-
-  for (int k0 = 0; k0 < K; k0 += BK) {
+// Four neighbouring k of one row into shared memory as float32; `k_end` is where the row's k stop, `row_ok` whether there
+// is such a row. VEC: rows start on 16-byte boundaries and K is a multiple of 4 (asynchronous copy); else one by one.
+template <typename T, bool VEC>
+__device__ __forceinline__ void stage4(float* dst, const T* base, long long row, int K, int k, int k_end, bool row_ok) {
+  if constexpr (VEC) {
+    const bool ok = row_ok && k < k_end;
+    cp16(dst, ok ? base + row * K + k : base, ok);
+  } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = k0 + lk + i;
-      As[lk + i][lr] = (a_ok && k < K) ? Cvt<TA>::to_f(arow[k]) : 0.f;
-      Ws[lk + i][lr] = (w_ok && k < K) ? Cvt<TA>::to_f(wrow[k]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[TM], b[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Ws[kk][tx * TN + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int m = m0 + ty * TM + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int n = n0 + tx * TN + j;
-      if (n >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[n];
-      C[(size_t)m * N + n] = Cvt<TC>::from_f(v);
-    }
+    for (int i = 0; i < 4; ++i) dst[i] = row_ok && k + i < k_end ? Cvt<T>::to_f(base[row * K + k + i]) : 0.f;
   }
 }
 
-// Few rows (M <= 16): 16 rows x 64 columns per block, 32 k per stage. A thread owns one column and four rows and walks
-// k alone (splitting k over lanes would change the order of the sum); W is staged through shared memory so that the
-// global reads stay coalesced.
-constexpr int SM_ROWS = 16, SN = 64, SK = 32;
-template <typename TA, typename TC>
+__device__ __forceinline__ void fma4(float& acc, float4 a, float4 w) {
+  acc = fmaf(a.x, w.x, acc);
+  acc = fmaf(a.y, w.y, acc);
+  acc = fmaf(a.z, w.z, acc);
+  acc = fmaf(a.w, w.w, acc);
+}
+
+// ---- few rows
+// A block owns 8 * RPL columns (rows of W) and all of K: warp w has chunks 4w .. 4w+3, eight lanes to a chunk, RPL columns
+// to a lane, MR rows of A to each. So N * 32 / RPL chains run at once, and a warp waits for no other until the end: it
+// streams its own 16 k of every (column, chunk) per stage through a ring of its own, 64 contiguous bytes each, rows padded
+// to 80 bytes (conflict-free 16-byte reads). The first stages of W, which no kernel of a step writes, are asked for ahead
+// of the wait on the kernel before. Blocks that stay and walk several tiles with the ring running on measured slower at
+// large N (896 -> 151,936 at 8 rows: 211 against 156 us): waiting at each tile's end for the slowest warp costs more than
+// a new block. Measured at 4 rows, weights from HBM: 4,864 -> 896 215 -> 10.1 us, 896 -> 9,728 75 -> 11.0 us, 896 ->
+// 151,936 417 -> 132 us (4.1 TB/s; 1 row 101 us, 5.4 TB/s: with more rows the reads of A from shared memory bind).
+constexpr int FEW_K = 16, FEW_ROW = FEW_K + 4;
+template <int MR, int RPL> struct Few {
+  static constexpr int W_FLOATS = 32 * RPL * FEW_ROW, A_SUB = MR * FEW_K + 4, STAGE = W_FLOATS + 4 * A_SUB;   // per warp
+  static constexpr int FIT = 112 * 1024 / (8 * STAGE * 4), STAGES = FIT < 2 ? 2 : FIT > 4 ? 4 : FIT;          // two blocks per SM where that leaves two stages
+};
+
+template <typename TA, typename TC, int MR, int RPL, bool VEC>
 __global__ void __launch_bounds__(256)
-gemm_simt_small_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias,
-                       TC* __restrict__ C, int M, int N, int K) {
+gemm_simt_few_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias,
+                     TC* __restrict__ C, int M, int N, int K, Order o, int slots) {
+  using F = Few<MR, RPL>;
+  constexpr int COLS = 8 * RPL;
+  extern __shared__ float4 few_smem[];
   fz_grid_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane & 7, sub = lane >> 3;
+  float* ring = reinterpret_cast<float*>(few_smem) + (size_t)warp * slots * F::STAGE;      // `slots`: STAGES, or the stages there are if fewer
+  const int n0 = blockIdx.x * COLS;
+  const int stages = o.chunk / FEW_K;
+
+  auto load_w = [&](int s) {
+    float* at = ring + (s % F::STAGES) * F::STAGE;
+#pragma unroll
+    for (int j = 0; j < 4 * RPL; ++j) {
+      const int e = lane + 32 * j, stream = e >> 2, q = (e & 3) * 4;
+      const int c = warp * 4 + stream / COLS, n = n0 + stream % COLS;
+      const int k = c * o.chunk + s * FEW_K + q, end = min(K, (c + 1) * o.chunk);
+      stage4<TA, VEC>(at + stream * FEW_ROW + q, W, n, K, k, end, n < N && c < o.chunks);
+    }
+  };
+  auto load_a = [&](int s) {
+    float* at = ring + (s % F::STAGES) * F::STAGE + F::W_FLOATS;
+#pragma unroll
+    for (int j = 0; j < (16 * MR + 31) / 32; ++j) {
+      const int e = lane + 32 * j;
+      if (16 * MR % 32 == 0 || e < 16 * MR) {
+        const int p = e / (4 * MR), m = e / 4 % MR, q = (e & 3) * 4, c = warp * 4 + p;
+        const int k = c * o.chunk + s * FEW_K + q, end = min(K, (c + 1) * o.chunk);
+        stage4<TA, VEC>(at + p * F::A_SUB + m * FEW_K + q, A, m, K, k, end, m < M && c < o.chunks);
+      }
+    }
+  };
+
+  float acc[RPL][MR];
+#pragma unroll
+  for (int i = 0; i < RPL; ++i)
+#pragma unroll
+    for (int m = 0; m < MR; ++m) acc[i][m] = 0.f;
+
+#pragma unroll
+  for (int s = 0; s < F::STAGES; ++s)
+    if (s < stages) load_w(s);
   fz_grid_wait();
-  __shared__ float As[SK][SM_ROWS + 1];
-  __shared__ float Ws[SK][SN + 1];
-  const int tid = threadIdx.x;
-  const int n0 = blockIdx.x * SN, m0 = blockIdx.y * SM_ROWS;
-  const int tn = tid & 63, tm = tid >> 6;   // 4 row groups x 64 columns; thread does rows tm, tm+4, tm+8, tm+12
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int k0 = 0; k0 < K; k0 += SK) {
-    // W tile: 64 rows x 32 k = 2048 elements, 8 per thread; consecutive threads read consecutive k
-    for (int e = tid; e < SN * SK; e += 256) {
-      const int r = e >> 5, k = e & 31;
-      Ws[k][r] = (n0 + r < N && k0 + k < K) ? Cvt<TA>::to_f(W[(size_t)(n0 + r) * K + k0 + k]) : 0.f;
-    }
-    for (int e = tid; e < SM_ROWS * SK; e += 256) {
-      const int r = e >> 5, k = e & 31;
-      As[k][r] = (m0 + r < M && k0 + k < K) ? Cvt<TA>::to_f(A[(size_t)(m0 + r) * K + k0 + k]) : 0.f;
-    }
-    __syncthreads();
 #pragma unroll
-    for (int kk = 0; kk < SK; ++kk) {
-      const float w = Ws[kk][tn];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i] = fmaf(As[kk][tm + 4 * i], w, acc[i]);
-    }
-    __syncthreads();
+  for (int s = 0; s < F::STAGES; ++s) {
+    if (s < stages) load_a(s);
+    cp_commit();
   }
-  const int n = n0 + tn;
-  if (n < N) {
+  for (int s = 0; s < stages; ++s) {
+    cp_wait<F::STAGES - 1>();
+    __syncwarp();
+    const float* at = ring + (s % F::STAGES) * F::STAGE;
+    const float* aw = at + F::W_FLOATS + sub * F::A_SUB;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int m = m0 + tm + 4 * i;
-      if (m < M) {
-        float v = acc[i];
+    for (int q = 0; q < FEW_K / 4; ++q) {
+      float4 w[RPL];
+#pragma unroll
+      for (int i = 0; i < RPL; ++i) w[i] = *reinterpret_cast<const float4*>(at + (sub * COLS + r + 8 * i) * FEW_ROW + 4 * q);
+#pragma unroll
+      for (int m = 0; m < MR; ++m) {
+        const float4 a = *reinterpret_cast<const float4*>(aw + m * FEW_K + 4 * q);
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) fma4(acc[i][m], a, w[i]);
+      }
+    }
+    __syncwarp();
+    if (s + F::STAGES < stages) {
+      load_w(s + F::STAGES);
+      load_a(s + F::STAGES);
+    }
+    cp_commit();
+  }
+  cp_wait<0>();
+  __syncthreads();      // the rings are done with: their memory takes the chunks' sums, [chunk][row of A][column]
+  float* sums = reinterpret_cast<float*>(few_smem);
+  const int c = warp * 4 + sub;
+  if (c < o.chunks) {
+#pragma unroll
+    for (int m = 0; m < MR; ++m)
+#pragma unroll
+      for (int i = 0; i < RPL; ++i) sums[(c * MR + m) * COLS + r + 8 * i] = acc[i][m];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < COLS * M; e += blockDim.x) {
+    const int n = n0 + e % COLS;
+    if (n >= N) continue;
+    float v = 0.f;
+    for (int g = 0, ch = 0; g < o.groups; ++g) {
+      float part = 0.f;
+      for (const int end = min(o.chunks, ch + o.per_group); ch < end; ++ch) part += sums[ch * MR * COLS + e];
+      v += part;
+    }
+    if (bias) v += bias[n];
+    C[(size_t)(e / COLS) * N + n] = Cvt<TC>::from_f(v);
+  }
+}
+
+// ---- more rows
+// Tiles of (8 TM) x (16 TN) outputs, 128 threads with TM x TN outputs each, 32 k per stage, three stages of asynchronous
+// copies; rows lie in shared memory as in memory, padded to 144 bytes, and are read 16 bytes (four k) at a time. With 8 x 4
+// outputs per thread 16 warps share an SM; 8 x 6 and 8 x 8 reach the same 40 TFLOP/s on large products and lose on small
+// ones (300 rows, 896 -> 9,728: 160, 174 and 208 us). A block sums one group of chunks (`acc` the chunk's chain, `tot` the group) and the blocks of a tile's groups, a cluster,
+// add their tiles up in order through distributed shared memory. Measured at 300 rows: 896 -> 9,728 265 -> 160 us, 4,864 ->
+// 896 215 -> 78 us, 896 -> 151,936 3,364 -> 2,031 us (40 TFLOP/s).
+constexpr int TN = 4, TILE_CTAS = 4, TILE_N = 16 * TN, TILE_K = 32, TILE_ROW = TILE_K + 4, TILE_STAGES = 3;
+template <typename TA, typename TC, int TM, bool VEC>
+__global__ void __launch_bounds__(128, TILE_CTAS)
+gemm_simt_tile_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias,
+                      TC* __restrict__ C, int M, int N, int K, Order o, int m_tiles) {
+  constexpr int BM = 8 * TM, STAGE = (BM + TILE_N) * TILE_ROW;
+  extern __shared__ float4 tile_smem[];
+  float* ring = reinterpret_cast<float*>(tile_smem);
+  fz_grid_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);      // 16 x 8 threads, a warp 8 x 4 of them
+  const int m0 = (blockIdx.x % m_tiles) * BM, n0 = (blockIdx.x / m_tiles) * TILE_N;
+  const int k_first = blockIdx.z * o.per_group * o.chunk, k_end = min(K, k_first + o.per_group * o.chunk);
+  const int stages = (k_end - k_first + TILE_K - 1) / TILE_K, per_chunk = o.chunk / TILE_K;
+
+  auto load = [&](int s, bool w_rows) {
+    float* at = ring + (s % TILE_STAGES) * STAGE + (w_rows ? BM * TILE_ROW : 0);
+    const int k = k_first + s * TILE_K + (tid & 7) * 4;
+    const int first = w_rows ? n0 : m0, limit = w_rows ? N : M;
+#pragma unroll
+    for (int i = 0; i < (w_rows ? TILE_N : BM) / 16; ++i) {
+      const int row = (tid >> 3) + 16 * i;
+      stage4<TA, VEC>(at + row * TILE_ROW + (tid & 7) * 4, w_rows ? W : A, first + row, K, k, k_end, first + row < limit);
+    }
+  };
+
+  float acc[TM][TN], tot[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = tot[i][j] = 0.f;
+
+#pragma unroll
+  for (int s = 0; s < TILE_STAGES - 1; ++s)
+    if (s < stages) load(s, true);
+  fz_grid_wait();
+#pragma unroll
+  for (int s = 0; s < TILE_STAGES - 1; ++s) {
+    if (s < stages) load(s, false);
+    cp_commit();
+  }
+  int left = per_chunk;
+  for (int s = 0; s < stages; ++s) {
+    cp_wait<TILE_STAGES - 2>();
+    __syncthreads();
+    if (s + TILE_STAGES - 1 < stages) {
+      load(s + TILE_STAGES - 1, true);
+      load(s + TILE_STAGES - 1, false);
+    }
+    cp_commit();
+    const float* as = ring + (s % TILE_STAGES) * STAGE + ty * TILE_ROW;
+    const float* ws = ring + (s % TILE_STAGES) * STAGE + (BM + tx) * TILE_ROW;
+#pragma unroll 2
+    for (int q = 0; q < TILE_K / 4; ++q) {
+      float4 w[TN];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const float4*>(ws + 16 * j * TILE_ROW + 4 * q);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(as + 8 * i * TILE_ROW + 4 * q);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.x, w[j].x, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.y, w[j].y, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.z, w[j].z, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a.w, w[j].w, acc[i][j]);
+      }
+    }
+    if (--left == 0 || s + 1 == stages) {
+      left = per_chunk;
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          tot[i][j] += acc[i][j];
+          acc[i][j] = 0.f;
+        }
+    }
+  }
+  cp_wait<0>();
+  if (o.groups == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      const int m = m0 + ty + 8 * i;
+      if (m >= M) continue;
+#pragma unroll
+      for (int j = 0; j < TN; ++j) {
+        const int n = n0 + tx + 16 * j;
+        if (n >= N) continue;
+        float v = tot[i][j];
         if (bias) v += bias[n];
         C[(size_t)m * N + n] = Cvt<TC>::from_f(v);
       }
     }
+    return;
   }
+  cg::cluster_group cluster = cg::this_cluster();
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) ring[(ty + 8 * i) * TILE_N + tx + 16 * j] = tot[i][j];
+  cluster.sync();
+  for (int e = blockIdx.z * 128 + tid; e < BM * TILE_N; e += 128 * o.groups) {      // the blocks share the tile
+    const int m = m0 + e / TILE_N, n = n0 + e % TILE_N;
+    if (m >= M || n >= N) continue;
+    float part[8];
+#pragma unroll
+    for (int g = 0; g < 8; ++g)
+      if (g < o.groups) part[g] = cluster.map_shared_rank(ring, g)[e];
+    float v = 0.f;
+#pragma unroll
+    for (int g = 0; g < 8; ++g)
+      if (g < o.groups) v += part[g];
+    if (bias) v += bias[n];
+    C[(size_t)m * N + n] = Cvt<TC>::from_f(v);
+  }
+  cluster.sync();      // nobody leaves while its tile may still be read
+}
+
+// Raises a kernel's shared-memory limit where it needs more than the default (once per instantiation and size, outside
+// any capture: a step is run once before it is captured).
+template <typename K> cudaError_t allow_smem(K kern, size_t smem, size_t& allowed) {
+  if (smem <= allowed) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) allowed = smem;
+  return e;
+}
+
+template <typename TA, typename TC, int MR, int RPL, bool VEC>
+int launch_few(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
+  using F = Few<MR, RPL>;
+  const int warps = (o.chunks + 3) / 4, stages = o.chunk / FEW_K, slots = stages < F::STAGES ? stages : F::STAGES;
+  const size_t ring = sizeof(float) * (size_t)warps * slots * F::STAGE, sums = sizeof(float) * (size_t)o.chunks * MR * 8 * RPL;
+  const size_t smem = ring > sums ? ring : sums;
+  auto kern = gemm_simt_few_kernel<TA, TC, MR, RPL, VEC>;
+  static size_t allowed = 48 * 1024;
+  const cudaError_t e = allow_smem(kern, smem, allowed);
+  if (e != cudaSuccess) return (int)e;
+  fz_launch(kern, dim3((N + 8 * RPL - 1) / (8 * RPL)), dim3(32 * warps), smem, stream, (const TA*)A, (const TA*)W, bias, (TC*)C, M, N, K, o, slots);
+  FZ_LAUNCH_CHECK();
+  return FZ_OK;
+}
+
+template <typename TA, typename TC, int TM, bool VEC>
+int launch_tile(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
+  const long long m_tiles = (M + 8 * TM - 1) / (8 * TM), tiles = m_tiles * ((N + TILE_N - 1) / TILE_N);
+  if (tiles > 2147483647LL) return FZ_TOO_LARGE;
+  // Blocks of a cluster may be put on one SM while others idle: few blocks ask for enough shared memory to be spread out.
+  const long long per_sm = (tiles * o.groups + 147) / 148;
+  size_t smem = sizeof(float) * TILE_STAGES * (size_t)(8 * TM + TILE_N) * TILE_ROW;
+  if (per_sm < TILE_CTAS && smem < 220 * 1024 / per_sm) smem = 220 * 1024 / per_sm / 1024 * 1024;
+  auto kern = gemm_simt_tile_kernel<TA, TC, TM, VEC>;
+  static size_t allowed = 48 * 1024;
+  const cudaError_t e = allow_smem(kern, smem, allowed);
+  if (e != cudaSuccess) return (int)e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)tiles, 1, o.groups);
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (o.groups > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = o.groups;
+  }
+  if (fz_pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  cudaLaunchKernelEx(&cfg, kern, (const TA*)A, (const TA*)W, bias, (TC*)C, M, N, K, o, (int)m_tiles);
+  FZ_LAUNCH_CHECK();
+  return FZ_OK;
+}
+
+// Two columns per lane (every value of A read once for both) where N still gives two blocks per SM.
+template <typename TA, typename TC, int MR, bool VEC>
+int launch_few_n(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
+    if (N >= 4096) return launch_few<TA, TC, MR, 2, VEC>(A, W, bias, C, M, N, K, o, stream);
+  return launch_few<TA, TC, MR, 1, VEC>(A, W, bias, C, M, N, K, o, stream);
+}
+
+template <typename TA, typename TC, bool VEC>
+int launch_rows(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, cudaStream_t stream) {
+  const Order o = order_of(N, K);
+  if (M <= 1) return launch_few_n<TA, TC, 1, VEC>(A, W, bias, C, M, N, K, o, stream);
+  if (M <= 2) return launch_few_n<TA, TC, 2, VEC>(A, W, bias, C, M, N, K, o, stream);
+  if (M <= 4) return launch_few_n<TA, TC, 4, VEC>(A, W, bias, C, M, N, K, o, stream);
+  if (M <= 8) return launch_few_n<TA, TC, 8, VEC>(A, W, bias, C, M, N, K, o, stream);
+  if (M <= 16) return launch_few_n<TA, TC, 16, VEC>(A, W, bias, C, M, N, K, o, stream);
+  if (M <= 32) return launch_tile<TA, TC, 4, VEC>(A, W, bias, C, M, N, K, o, stream);
+  return launch_tile<TA, TC, 8, VEC>(A, W, bias, C, M, N, K, o, stream);
 }
 
 template <typename TA, typename TC>
 int launch(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, cudaStream_t stream) {
-  if (M <= SM_ROWS) {
-    dim3 grid((N + SN - 1) / SN, (M + SM_ROWS - 1) / SM_ROWS);
-    fz_launch(gemm_simt_small_kernel<TA, TC>, grid, dim3(256), 0, stream, (const TA*)A, (const TA*)W, bias, (TC*)C, M, N, K);
-  } else {
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    fz_launch(gemm_simt_kernel<TA, TC>, grid, dim3(256), 0, stream, (const TA*)A, (const TA*)W, bias, (TC*)C, M, N, K);
-  }
-  FZ_LAUNCH_CHECK();
-  return FZ_OK;
+  if constexpr (sizeof(TA) == 4)
+    if (K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0) return launch_rows<TA, TC, true>(A, W, bias, C, M, N, K, stream);
+  return launch_rows<TA, TC, false>(A, W, bias, C, M, N, K, stream);
 }
 }  // namespace
 
