@@ -6,6 +6,8 @@
 // :317-427 rotation with cache write, :431-479 argmax, :547-575 step inputs); the residual stream is kept in float32
 // here, so the norm rounds once where the reference rounds x + d, y and w*y separately.
 #include "common.cuh"
+#include <cooperative_groups.h>
+namespace cg = cooperative_groups;
 #include <math.h>
 
 // ------------------------------------------------------------------------------------------------ embedding
@@ -960,7 +962,10 @@ FZ_API int fz_sample(const float* logits, const float* temperature, const double
 // The reference's host sampler on the device (fusezap/serve/sampling.py:25-45, 61-73): logits / T in float64; top-k keeps
 // everything not below the k-th largest value (ties stay); top-p keeps, in falling order of value (ties by rising
 // index), every token before which less than p of the probability lies; then one draw from the softmax of what is left:
-// the first index whose running sum in index order exceeds u times the total. One block of 1024 threads per row.
+// the first index whose running sum in index order exceeds u times the total. A cluster of SF_CLUSTER blocks of 1024
+// threads per row, a block for each SF_CLUSTER-th of its tokens (one block for short rows, SF_SHORT and less): bound by the instructions per
+// token and pass, so the blocks' number is what counts (8 rows of 151,936 with top-p, from the difference of whole steps:
+// 340 -> 70 us; 24 sampled tokens of 8 requests at Qwen2.5-0.5B sizes 32.2 -> 25.6 ms). The blocks add their bins and sums up through distributed shared memory in rank order; all then take the same decisions.
 // Nothing is sorted: the thresholds are found by radix selection over an order-preserving 32-bit key of the logit,
 // eight passes of 4 bits, with a histogram of counts for top-k and of probability mass (float64) for top-p. Each thread
 // fills 16 bins of its own in shared memory and the bins are then summed over the threads in a fixed order, so there
@@ -969,6 +974,7 @@ FZ_API int fz_sample(const float* logits, const float* temperature, const double
 constexpr int SF_THREADS = 1024;
 constexpr int SF_BINS = 16;
 constexpr size_t SF_SMEM = (size_t)SF_BINS * SF_THREADS * sizeof(double);
+constexpr int SF_CLUSTER = 8, SF_SHORT = 8192;
 
 __device__ __forceinline__ uint32_t falling_key(float x) {      // smaller key = larger value; -0 counts as +0
   const uint32_t u = __float_as_uint(x + 0.f);
@@ -1000,23 +1006,40 @@ __device__ __forceinline__ void sum_bins(const T* bins, T* s_part, T* total) {
   __syncthreads();
 }
 
-// f(i, key of row[i]) for every i this thread owns (i = tid, tid + 1024, ...), eight loads in flight at a time.
+// f(i, row[i], its key) for every i of [lo, hi) this thread owns (i = lo + tid, lo + tid + 1024, ...), eight loads in flight.
 template <typename F>
-__device__ __forceinline__ void for_each_key(const float* __restrict__ row, int V, F f) {
+__device__ __forceinline__ void for_each_key(const float* __restrict__ row, int lo, int hi, F f) {
   constexpr int U = 8;
-  for (int base = threadIdx.x; base < V; base += SF_THREADS * U) {
+  for (int base = lo + threadIdx.x; base < hi; base += SF_THREADS * U) {
     float x[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = base + u * SF_THREADS;
-      x[u] = i < V ? row[i] : 0.f;
+      x[u] = i < hi ? row[i] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = base + u * SF_THREADS;
-      if (i < V) f(i, x[u], falling_key(x[u]));
+      if (i < hi) f(i, x[u], falling_key(x[u]));
     }
   }
+}
+
+// The sum over the cluster's blocks, in rank order, of values[0..count) of each block; thread i < count gets sum i. Called
+// with the two halves of a pair of buffers in turn: a buffer is written again only after a cluster barrier that every
+// block reaches after it has read it.
+template <typename T>
+__device__ __forceinline__ T cluster_sum(const cg::cluster_group& cluster, T* values, int count) {
+  const int blocks = cluster.num_blocks();
+  if (blocks == 1) {
+    __syncthreads();
+    return threadIdx.x < count ? values[threadIdx.x] : T(0);
+  }
+  cluster.sync();
+  T v = 0;
+  if (threadIdx.x < count)
+    for (int b = 0; b < blocks; ++b) v += cluster.map_shared_rank(values, b)[threadIdx.x];
+  return v;
 }
 
 // Inclusive sum over the lanes below and this one, always in the same order.
@@ -1039,25 +1062,44 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
   unsigned int* bins_u = reinterpret_cast<unsigned int*>(sf_smem);
   __shared__ float s_val[32];
   __shared__ int s_idx[32];
-  __shared__ double s_part[32], s_mass[SF_BINS], s_wsum[32];
-  __shared__ unsigned int s_partu[32], s_count[SF_BINS];
+  __shared__ double s_part[32], s_mass[2][SF_BINS], s_wsum[32], s_all[SF_BINS], s_sum[2][1];
+  __shared__ unsigned int s_partu[32], s_count[2][SF_BINS], s_allu[SF_BINS];
+  __shared__ float s_best[1];
+  __shared__ int s_best_at[1], s_ties[1];
   __shared__ int s_wties[32];
   __shared__ uint32_t s_prefix;
   __shared__ unsigned int s_rank;
   __shared__ double s_need, s_target;
-  __shared__ int s_res, s_warp;
-  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ int s_warp;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int blocks = cluster.num_blocks(), rank = cluster.block_rank();
+  const int r = blockIdx.x / blocks, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slice = (V + blocks * 32 - 1) / (blocks * 32) * 32, lo = min(V, rank * slice), hi = min(V, lo + slice);
+  int turn = 0;      // which of a pair of buffers is next
   const float* row = logits + (size_t)r * V;
   double* e = scratch + (size_t)r * V;
   const float T = temperature[r];
   const int k = top_k[r];
-  const int amax = block_argmax(row, V, s_val, s_idx);
+  int amax = block_argmax(row + lo, hi - lo, s_val, s_idx);
+  if (tid == 0) {
+    s_best_at[0] = lo < hi ? lo + amax : 0x7fffffff;
+    s_best[0] = lo < hi ? row[lo + amax] : -INFINITY;
+  }
+  cluster.sync();
+  float top = -INFINITY;
+  amax = 0x7fffffff;
+  for (int b = 0; b < blocks; ++b) {      // slices in index order, as the row-split argmax does it
+    const float v = cluster.map_shared_rank(s_best, b)[0];
+    const int at = cluster.map_shared_rank(s_best_at, b)[0];
+    if (at != 0x7fffffff && (amax == 0x7fffffff || better(v, at, top, amax))) { top = v; amax = at; }
+  }
   if (!(T > 0.f) || k == 1) {
-    if (tid == 0) out[r] = amax;
+    if (rank == 0 && tid == 0) out[r] = amax;
+    cluster.sync();      // (nobody leaves while its shared memory may still be read)
     return;
   }
-  const double mx = (double)row[amax] / (double)T;
-  const uint32_t top_key = falling_key(row[amax]);
+  const double mx = (double)top / (double)T;
+  const uint32_t top_key = falling_key(top);
   // ---- top-k: the key of the k-th largest logit (x / T rises with x, so the selection runs on the logits themselves)
   uint32_t k_key = 0xffffffffu;                 // tokens with a key <= k_key stay
   if (k > 0 && k < V) {
@@ -1067,16 +1109,20 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
       __syncthreads();
       const uint32_t prefix = s_prefix;
       for (int b = 0; b < SF_BINS; ++b) bins_u[b * SF_THREADS + tid] = 0u;
-      for_each_key(row, V, [&](int, float, uint32_t key) {
+      for_each_key(row, lo, hi, [&](int, float, uint32_t key) {
         if (pass == 0 || (key >> (shift + 4)) == prefix) bins_u[((key >> shift) & 15u) * SF_THREADS + tid] += 1u;
       });
-      sum_bins(bins_u, s_partu, s_count);
+      sum_bins(bins_u, s_partu, s_count[turn]);
+      const unsigned int count = cluster_sum(cluster, s_count[turn], SF_BINS);
+      turn ^= 1;
+      if (tid < SF_BINS) s_allu[tid] = count;
+      __syncthreads();
       if (tid == 0) {
         unsigned int rank = s_rank, cum = 0;
         int b = 0;
         for (; b < SF_BINS - 1; ++b) {
-          if (cum + s_count[b] > rank) break;
-          cum += s_count[b];
+          if (cum + s_allu[b] > rank) break;
+          cum += s_allu[b];
         }
         s_prefix = (prefix << 4) | (uint32_t)b;
         s_rank = rank - cum;
@@ -1095,13 +1141,18 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
   double need_at_t = 0.0, total = 0.0;
   if (first == 8) {
     double local = 0.0;
-    for_each_key(row, V, [&](int i, float x, uint32_t key) {
+    for_each_key(row, lo, hi, [&](int i, float x, uint32_t key) {
       const double v = key <= k_key ? exp((double)x / (double)T - mx) : 0.0;
       e[i] = v;
       local += v;
     });
-    total = block_sum_fixed(local, s_part);
-    need_at_t = (double)pp * total;
+    local = block_sum_fixed(local, s_part);
+    if (tid == 0) s_sum[turn][0] = local;
+    total = cluster_sum(cluster, s_sum[turn], 1);      // (thread 0 has it; only thread 0 asks)
+    turn ^= 1;
+    if (tid == 0) s_need = (double)pp * total;
+    __syncthreads();
+    need_at_t = s_need;
   } else {
     if (tid == 0) s_prefix = first == 0 ? 0u : top_key >> (32 - 4 * first);
     for (int pass = first; pass < 8; ++pass) {
@@ -1111,20 +1162,27 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
       for (int b = 0; b < SF_BINS; ++b) bins_d[b * SF_THREADS + tid] = 0.0;
       if (pass == first) {
         double local = 0.0;
-        for_each_key(row, V, [&](int i, float x, uint32_t key) {
+        for_each_key(row, lo, hi, [&](int i, float x, uint32_t key) {
           const double v = key <= k_key ? exp((double)x / (double)T - mx) : 0.0;
           e[i] = v;
           local += v;
           if (key <= k_key) bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += v;
         });
-        total = block_sum_fixed(local, s_part);
+        local = block_sum_fixed(local, s_part);
+        if (tid == 0) s_sum[turn][0] = local;
+        total = cluster_sum(cluster, s_sum[turn], 1);
+        turn ^= 1;
         if (tid == 0) s_need = (double)pp * total;
       } else {
-        for_each_key(row, V, [&](int i, float, uint32_t key) {
+        for_each_key(row, lo, hi, [&](int i, float, uint32_t key) {
           if (key <= k_key && (key >> (shift + 4)) == prefix) bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += e[i];
         });
       }
-      sum_bins(bins_d, s_part, s_mass);
+      sum_bins(bins_d, s_part, s_mass[turn]);
+      const double mass = cluster_sum(cluster, s_mass[turn], SF_BINS);
+      turn ^= 1;
+      if (tid < SF_BINS) s_all[tid] = mass;
+      __syncthreads();
       if (tid == 0) {
         // bins run from the largest values down: the first one at whose end the mass reaches what is needed holds the
         // threshold; if rounding leaves the sum a hair short, the last bin with any mass does
@@ -1132,9 +1190,9 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
         double cum = 0.0, cum_last = 0.0;
         int b = 0, last = 0;
         for (; b < SF_BINS; ++b) {
-          if (s_mass[b] > 0.0) { last = b; cum_last = cum; }
-          if (cum + s_mass[b] >= need) break;
-          cum += s_mass[b];
+          if (s_all[b] > 0.0) { last = b; cum_last = cum; }
+          if (cum + s_all[b] >= need) break;
+          cum += s_all[b];
         }
         if (b == SF_BINS) { b = last; cum = cum_last; }
         s_prefix = (prefix << 4) | (uint32_t)b;
@@ -1145,11 +1203,11 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
     t_key = s_prefix;
     need_at_t = s_need;
   }
-  // ---- the draw. Warp w owns the contiguous range [w * span, (w + 1) * span) and walks it 32 tokens at a time, so that
-  // sums run in index order. Equal values at the threshold: the j-th of them in index order (j = 0, 1, ...) stays while
+  // ---- the draw. Warp w owns the contiguous range [w * span, (w + 1) * span) of its block's slice and walks it 32 tokens
+  // at a time, so that sums run in index order. Equal values at the threshold: the j-th of them in index order (j = 0, 1, ...) stays while
   // j * e < need_at_t.
-  const int span = ((V + 1023) / 1024) * 32;
-  const int w_lo = min(V, warp * span), w_hi = min(V, w_lo + span);
+  const int span = ((slice + 1023) / 1024) * 32;
+  const int w_lo = min(hi, lo + warp * span), w_hi = min(hi, w_lo + span);
   if (nucleus) {
     int ties = 0;
     for (int i = w_lo + lane; i < w_hi; i += 32) ties += falling_key(row[i]) == t_key ? 1 : 0;
@@ -1158,8 +1216,18 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
   }
   __syncthreads();
   int j0 = 0;
-  if (nucleus)
+  if (nucleus) {
+    if (blocks > 1) {
+      if (tid == 0) {
+        int all = 0;
+        for (int w = 0; w < 32; ++w) all += s_wties[w];
+        s_ties[0] = all;
+      }
+      cluster.sync();
+      for (int b = 0; b < rank; ++b) j0 += cluster.map_shared_rank(s_ties, b)[0];
+    }
     for (int w = 0; w < warp; ++w) j0 += s_wties[w];
+  }
   double run = 0.0;
   for (int base = w_lo; base < w_hi; base += 32) {
     const int i = base + lane;
@@ -1180,37 +1248,63 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
   if (lane == 0) s_wsum[warp] = run;
   __syncthreads();
   if (tid == 0) {
-    double before = 0.0;
-    for (int w = 0; w < 32; ++w) before += s_wsum[w];
-    const double target = uniform[r] * before;
-    before = 0.0;
-    int w = 0;
-    for (; w < 31; ++w) {
-      if (before + s_wsum[w] > target) break;
-      before += s_wsum[w];
+    double sum = 0.0;
+    for (int w = 0; w < 32; ++w) sum += s_wsum[w];
+    s_sum[turn][0] = sum;
+  }
+  if (blocks > 1) cluster.sync();
+  else __syncthreads();
+  if (tid == 0) {
+    double all = 0.0;
+    for (int b = 0; b < blocks; ++b) all += cluster.map_shared_rank(s_sum[turn], b)[0];
+    const double target = uniform[r] * all;
+    // the block, then the warp, whose tokens the draw falls into: the first at whose end the running sum exceeds the
+    // target. Where rounding leaves them all at or below it, the last one with any mass.
+    double before = 0.0, before_last = 0.0;
+    int b = 0, last = -1;
+    for (; b < blocks; ++b) {
+      const double sum = cluster.map_shared_rank(s_sum[turn], b)[0];
+      if (sum > 0.0) { last = b; before_last = before; }
+      if (before + sum > target) break;
+      before += sum;
+    }
+    if (b == blocks) { b = last; before = before_last; }
+    int w = -1;
+    if (b == rank) {
+      last = -1;
+      for (w = 0; w < 32; ++w) {
+        if (s_wsum[w] > 0.0) { last = w; before_last = before; }
+        if (before + s_wsum[w] > target) break;
+        before += s_wsum[w];
+      }
+      if (w == 32) { w = last; before = before_last; }
     }
     s_warp = w;
     s_need = before;
     s_target = target;
-    s_res = amax;   // stays only if rounding leaves every running sum at or below the target
+    if (b < 0 && rank == 0) out[r] = amax;      // no sum above zero: the largest logit is not a number
   }
   __syncthreads();
   if (warp == s_warp) {
     const double target = s_target;
     run = s_need;
+    int res = amax;
     for (int base = w_lo; base < w_hi; base += 32) {
       const int i = base + lane;
-      const double sc = warp_scan_fixed(i < w_hi ? e[i] : 0.0, lane);
+      const double v = i < w_hi ? e[i] : 0.0;
+      const unsigned int some = __ballot_sync(0xffffffffu, v > 0.0);
+      const double sc = warp_scan_fixed(v, lane);
       const unsigned int hit = __ballot_sync(0xffffffffu, run + sc > target);
       if (hit) {
-        if (lane == 0) s_res = base + __ffs(hit) - 1;
+        res = base + __ffs(hit) - 1;
         break;
       }
+      if (some) res = base + 31 - __clz(some);      // (stays only if rounding leaves every running sum at or below the target)
       run += __shfl_sync(0xffffffffu, sc, 31);
     }
+    if (lane == 0) out[r] = res;
   }
-  __syncthreads();
-  if (tid == 0) out[r] = s_res;
+  if (blocks > 1) cluster.sync();
 }
 
 // scratch: R * V doubles. top_k[r] <= 0 or >= V: no top-k; top_p[r] >= 1: no top-p; temperature[r] <= 0 or top_k[r]
@@ -1225,8 +1319,25 @@ FZ_API int fz_sample_filtered(const float* logits, const float* temperature, con
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
-  fz_launch(sample_filtered_kernel, dim3(R), dim3(SF_THREADS), SF_SMEM, stream, logits, temperature, top_k, top_p, uniform,
-            scratch, out, V);
+  const int blocks = V <= SF_SHORT ? 1 : SF_CLUSTER;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)R * blocks);
+  cfg.blockDim = dim3(SF_THREADS);
+  cfg.dynamicSmemBytes = SF_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  attr[n].id = cudaLaunchAttributeClusterDimension;
+  attr[n].val.clusterDim.x = blocks;
+  attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+  ++n;
+  if (fz_pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  cudaLaunchKernelEx(&cfg, sample_filtered_kernel, logits, temperature, top_k, top_p, uniform, scratch, out, V);
   FZ_LAUNCH_CHECK();
   return FZ_OK;
 }
