@@ -202,3 +202,14 @@ def test_decode_rows_without_tma(Hq, Hkv, hd, bs, monkeypatch):
     close(o, op, "decode without TMA")
     o, op, _ = run_both(Hq, Hkv, hd, bs, 300, lengths, rows)
     close(o, op, "decode without TMA, window")
+
+
+@pytest.mark.parametrize("Hq,Hkv,hd", [(8, 2, 128), (14, 2, 64)])
+def test_short_rows_beside_hundreds_of_prompt_rows(Hq, Hkv, hd):
+    """The kernel that merges the short rows' partial results looks for them among all rows of the step (64 blocks per head
+    at most, several rows to a block): short rows first, last and between portions, padding among them."""
+    lengths = [500, 700, 90, 1, 333, 64]
+    rows = [(2, 89, 1), (0, 100, 400), (-1, 0, 3), (3, 0, 1), (1, 3, 697), (4, 326, 7), (5, 63, 1), (-1, 0, 2)]
+    o, op, seq_row = run_both(Hq, Hkv, hd, 16, 0, lengths, rows)
+    close(o, op, "short rows beside portions")
+    assert float(o[torch.tensor(seq_row) < 0].abs().max()) == 0.0
