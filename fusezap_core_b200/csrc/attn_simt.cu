@@ -1,152 +1,468 @@
 // Paged attention with 32-bit arithmetic on CUDA cores: the attention of the float32 path (prompt portions and decoded
 // tokens alike), and the general fallback of the bfloat16 path.
 //
-// One block per (token row, kv head, slice of up to 32 query heads of that kv head's group); warp w serves the query
-// heads w, w + W, ... of the slice, so they share every key/value load. Any number of heads and any group size. Keys are walked in chunks of 32 whose boundaries are multiples of 32 in absolute
-// position: chunk c holds keys 32c .. 32c+31, lane j scores key 32c+j, and the running (max, sum, accumulator) is
-// updated chunk by chunk in rising c. The order of every sum therefore depends only on the row's own position and
-// window, never on the batch, the cut of the prompt or the pages used (the reference's general kernel stages 32-key
-// chunks in shared memory the same way: fusezap/device/cuda_kernels/attention.py:330-436).
+// Keys are walked in chunks of 32 whose boundaries are multiples of 32 in absolute position: chunk c holds keys 32c ..
+// 32c+31, lane j scores key 32c+j, and the running (max, sum, accumulator) is updated chunk by chunk in rising c. A row's
+// chunks are cut into at most eight spans of equal length (two chunks at least); a span starts afresh, and the spans'
+// results are merged in order. The order of every sum therefore depends only on the row's own position and window, never
+// on the batch, the cut of the prompt or the pages used (the reference's general kernel stages 32-key chunks in shared
+// memory the same way: fusezap/device/cuda_kernels/attention.py:330-436).
 //
 //   scores s_j = (q . k_j) * scale over keys max(0, p - window + 1) <= j <= p of the row's own request (window 0: all),
 //   out = sum_j exp(s_j - max) v_j / sum_j exp(s_j - max)                       (fusezap/serve/kv_cache.py:258-274)
+//
+// A block has a few neighbouring rows of the step, one kv head and up to 32 (row, query head) pairs, which share every
+// chunk's keys and values (copied to shared memory one chunk ahead); warp w has pairs w, w + W, ... Few rows: a row per
+// block, and the spans of a row go to the eight blocks of a cluster, merged through distributed shared memory. Bound by
+// latency at the path's sizes: a chain of chunks, each a copy, a dot product per lane and a walk over 32 values. Measured
+// at 14 heads of 64 over 2 kv heads, inside a step: 4 rows of 250 to 500 keys 8.4 us (one block per row and kv head, no spans,
+// copies element by element: 146), 300 rows of two prompts 35 us (61).
 #include "common.cuh"
+#include <cooperative_groups.h>
 #include <math.h>
+namespace cg = cooperative_groups;
 
 namespace {
 constexpr int CHUNK = 32;
 constexpr int MAX_WARPS = 8;
-constexpr int MAX_HPW = 4;   // query heads per warp -> up to 32 query heads per block; larger groups take more blocks
-constexpr int MAX_GROUP = MAX_WARPS * MAX_HPW;
 constexpr int MAX_HD = 512;
+constexpr int SPANS = 8, SPAN_CHUNKS = 2;      // most spans of a row; fewest chunks of a span
+constexpr int MAX_ROWS = 8;                    // rows of a block
 
-template <typename T, int DPL>   // DPL: output dims per lane = ceil(hd / 32)
-__global__ void attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool,
-                                 const int* __restrict__ pos, const int* __restrict__ seq_row,
-                                 const int* __restrict__ table, int mb, long long page_stride, int page_size,
-                                 T* __restrict__ out, int Hq, int Hkv, int hd, float scale, int window, int* err) {
+// (row, head) pairs per warp: what fits in registers beside DPL output dimensions per lane, twice
+template <int DPL> struct Pairs { static constexpr int PER_WARP = DPL <= 4 ? 4 : DPL <= 8 ? 2 : 1; };
+
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = ok ? 16 : 0;      // 0: the 16 bytes are filled with zeros and nothing is read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+__device__ __forceinline__ float4 four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 four(const __nv_bfloat16* p) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+
+// The merge of a span's (m, l, a) into what the spans before it gave; `keep` and `add` are the two weights.
+__device__ __forceinline__ void span_weights(float& M, float m, float& keep, float& add) {
+  const float mn = fmaxf(M, m);
+  keep = expf(M - mn);
+  add = expf(m - mn);
+  M = mn;
+}
+__device__ __forceinline__ float span_add(float total, float part, float keep, float add) { return __fmaf_rn(total, keep, __fmul_rn(part, add)); }
+
+__device__ __forceinline__ int span_length(int chunks) {
+  const int len = (chunks + SPANS - 1) / SPANS;
+  return len < SPAN_CHUNKS ? SPAN_CHUNKS : len;
+}
+
+struct Args {
+  const int *pos, *seq_row, *table;
+  long long page_stride;
+  int mb, page_size, N, Hq, Hkv, hd, hdp, G_all, GS, rows, window, buffers;
+  float scale;
+  int* err;
+};
+
+// VEC: rows of keys and values start on 16-byte boundaries and are whole 16-byte pieces (asynchronous copies).
+// SPLIT: one row per block, the blocks of a cluster along z take a span each.
+// PW: pairs per warp at most.
+template <typename T, int DPL, int PW, bool VEC, bool SPLIT>
+__global__ void __launch_bounds__(32 * MAX_WARPS)
+attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T* __restrict__ v_pool, T* __restrict__ out, Args A) {
+  constexpr int PAD = 16 / sizeof(T);
+  extern __shared__ float4 attn_smem[];
+  __shared__ int s_row[MAX_ROWS], s_pos[MAX_ROWS], s_lo[MAX_ROWS];
   fz_grid_launch_dependents();
-  fz_grid_wait();
-  extern __shared__ float smem[];
-  const int n = blockIdx.x, kvh = blockIdx.y;
-  const int G_all = Hq / Hkv, g_base = blockIdx.z * MAX_GROUP;
-  const int G = min(MAX_GROUP, G_all - g_base);           // the query heads of this block: g_base .. g_base + G - 1 of the group
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
-  const int kstride = hd + 1;
-  float* Ks = smem;                       // [CHUNK][hd + 1]
-  float* Vs = Ks + CHUNK * kstride;       // [CHUNK][hd]
-  float* Qs = Vs + CHUNK * hd;            // [G][hd]
-  T* orow = out + (size_t)n * Hq * hd + ((size_t)kvh * G_all + g_base) * hd;
-  const int row = seq_row[n];
-  if (row < 0) {
-    for (int i = threadIdx.x; i < G * hd; i += blockDim.x) orow[i] = Cvt<T>::from_f(0.f);
-    return;
-  }
-  const int p = pos[n];
-  const int lo = window > 0 ? max(0, p - window + 1) : 0;
-  const T* qrow = q + (size_t)n * Hq * hd + ((size_t)kvh * G_all + g_base) * hd;
-  for (int i = threadIdx.x; i < G * hd; i += blockDim.x) Qs[i] = Cvt<T>::to_f(qrow[i]);
+  const int hd = A.hd, hdp = A.hdp, ks = hdp + PAD;
+  const int kvh = blockIdx.y % A.Hkv, g_base = (blockIdx.y / A.Hkv) * A.GS, G = min(A.GS, A.G_all - g_base);
+  const int first = blockIdx.x * A.rows, rows = min(A.rows, A.N - first);
+  const int head0 = kvh * A.G_all + g_base;
+  // shared memory: per buffer keys [32][hdp + PAD] and values [32][hdp], then queries [pair][hdp] and weights [warp][PW][32] in float32
+  T* kv = reinterpret_cast<T*>(attn_smem);
+  const int kv_size = CHUNK * (ks + hdp);
+  float* Qs = reinterpret_cast<float*>(kv + A.buffers * kv_size);
+  float* Ps = Qs + A.rows * G * hdp + warp * PW * CHUNK;
 
-  float m[MAX_HPW], l[MAX_HPW], acc[MAX_HPW][DPL];
-#pragma unroll
-  for (int a = 0; a < MAX_HPW; ++a) {
-    m[a] = -INFINITY;
-    l[a] = 0.f;
-#pragma unroll
-    for (int i = 0; i < DPL; ++i) acc[a][i] = 0.f;
+  if (threadIdx.x < rows) {
+    const int n = first + threadIdx.x, row = A.seq_row[n], p = row < 0 ? -1 : A.pos[n];
+    s_row[threadIdx.x] = row;
+    s_pos[threadIdx.x] = p;
+    s_lo[threadIdx.x] = A.window > 0 ? max(0, p - A.window + 1) : 0;
   }
-  const int* trow = table + (size_t)row * mb;
-  const long long head_off = (long long)kvh * page_size * hd;
+  __syncthreads();
+  // Positions, rows and block tables are the step's metadata, which the host wrote before its first kernel: they are read
+  // ahead of the wait on the kernel before. Queries, keys and values are not.
+  bool waited = false;
+  auto queries = [&] {
+    for (int pair = warp; pair < rows * G; pair += W) {
+      const T* from = q + ((size_t)(first + pair / G) * A.Hq + head0 + pair % G) * hd;
+      for (int d = lane; d < hdp; d += 32) Qs[pair * hdp + d] = d < hd ? Cvt<T>::to_f(from[d]) : 0.f;
+    }
+  };
 
-  for (int c = lo / CHUNK; c <= p / CHUNK; ++c) {
-    __syncthreads();   // the previous chunk is consumed (and Qs is written, the first time)
-    for (int e = threadIdx.x; e < CHUNK * hd; e += blockDim.x) {
-      const int j = e / hd, d = e - j * hd;
-      const int key = c * CHUNK + j;
-      float kv = 0.f, vv = 0.f;
-      if (key >= lo && key <= p) {
-        const int page = trow[key / page_size];
-        if (page < 0) {
-          atomicOr(err, FZ_ERR_NO_PAGE);
+  for (int r0 = 0; r0 < rows;) {      // the block's rows in runs of one request (SPLIT: its one row)
+    const int row = s_row[r0];
+    int r1 = r0 + 1;
+    while (r1 < rows && s_row[r1] == row) ++r1;
+    if (row < 0) {      // padding rows give zeros
+      if (!waited) {
+        fz_grid_wait();
+        queries();
+        waited = true;
+      }
+      if (!SPLIT || blockIdx.z == 0)
+        for (int i = threadIdx.x; i < (r1 - r0) * G * hd; i += blockDim.x)
+          out[((size_t)(first + r0 + i / (G * hd)) * A.Hq + head0) * hd + i % (G * hd)] = Cvt<T>::from_f(0.f);
+      r0 = r1;
+      continue;
+    }
+    const int pairs = (r1 - r0) * G;
+    int at[PW];      // where a pair's query lies (a warp without one computes the last pair's scores and drops them)
+#pragma unroll
+    for (int a = 0; a < PW; ++a) at[a] = (r0 * G + min(warp + a * W, pairs - 1)) * hdp;
+    int c_first = 1 << 30, c_last = -1, lo_min = 1 << 30, p_max = -1;
+    for (int r = r0; r < r1; ++r) {
+      c_first = min(c_first, s_lo[r] / CHUNK);
+      c_last = max(c_last, s_pos[r] / CHUNK);
+      lo_min = min(lo_min, s_lo[r]);
+      p_max = max(p_max, s_pos[r]);
+    }
+    int spans = 1;
+    if constexpr (SPLIT) {
+      const int chunks = c_last - c_first + 1, len = span_length(chunks);
+      spans = (chunks + len - 1) / len;
+      c_first += blockIdx.z * len;
+      c_last = min(c_last, c_first + len - 1);
+    }
+    // per pair: the span being walked (m, l, acc), what the spans before it gave (M, L, tot), the chunk where the next span starts
+    float m[PW], l[PW], acc[PW][DPL], M[PW], L[PW], tot[PW][DPL];
+    int cut[PW];
+#pragma unroll
+    for (int a = 0; a < PW; ++a) {
+      m[a] = M[a] = -INFINITY;
+      l[a] = L[a] = 0.f;
+      cut[a] = -1;
+#pragma unroll
+      for (int i = 0; i < DPL; ++i) acc[a][i] = tot[a][i] = 0.f;
+    }
+    const int* trow = A.table + (size_t)row * A.mb;
+    const long long head_off = (long long)kvh * A.page_size * hd;
+
+    // Where the chunk's keys lie, a lane each (-1: not seen by any row, or without a page): asked for one chunk before the
+    // copies that need it.
+    auto find = [&](int c) {
+      const int key = c * CHUNK + lane;
+      long long off = -1;
+      if (c <= c_last && key >= lo_min && key <= p_max) {
+        const int page = trow[key / A.page_size];
+        if (page >= 0) off = (long long)page * A.page_stride + head_off + (long long)(key % A.page_size) * hd;
+        else atomicOr(A.err, FZ_ERR_NO_PAGE);
+      }
+      return off;
+    };
+    auto load = [&](int c, long long where) {
+      T* Ks = kv + (c & (A.buffers - 1)) * kv_size;
+      T* Vs = Ks + CHUNK * ks;
+      for (int j = warp; c <= c_last && j < CHUNK; j += W) {
+        long long off = __shfl_sync(0xffffffffu, where, j);
+        const bool ok = off >= 0;
+        if (!ok) off = 0;
+        if constexpr (VEC) {
+          for (int e = lane * PAD; e < 2 * hd; e += 32 * PAD) {
+            const bool is_k = e < hd;
+            const int d = is_k ? e : e - hd;
+            cp16(is_k ? Ks + j * ks + d : Vs + j * hdp + d, (is_k ? k_pool : v_pool) + off + d, ok);
+          }
         } else {
-          const long long off = (long long)page * page_stride + head_off + (long long)(key % page_size) * hd + d;
-          kv = Cvt<T>::to_f(k_pool[off]);
-          vv = Cvt<T>::to_f(v_pool[off]);
+          for (int d = lane; d < hdp; d += 32) {
+            const bool in = ok && d < hd;
+            Ks[j * ks + d] = in ? k_pool[off + d] : Cvt<T>::from_f(0.f);
+            Vs[j * hdp + d] = in ? v_pool[off + d] : Cvt<T>::from_f(0.f);
+          }
         }
       }
-      Ks[j * kstride + d] = kv;
-      Vs[j * hd + d] = vv;
+      if constexpr (VEC) asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    // The ring of `buffers` chunks (1, 2 or 4): all but one are filled here, the last in the loop, a chunk ahead.
+    const int ahead = A.buffers - 1;
+    long long early[3], next = -1;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) early[i] = i < ahead ? find(c_first + i) : -1;
+    next = find(c_first + ahead);
+    if (!waited) fz_grid_wait();
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (i < ahead) load(c_first + i, early[i]);
+    if (!waited) queries();
+    waited = true;
+    for (int c = c_first; c <= c_last; ++c) {
+      load(c + ahead, next);
+      next = find(c + ahead + 1);
+      if constexpr (VEC) {
+        if (ahead == 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
+        else if (ahead == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      __syncthreads();
+      const T* Ks = kv + (c & (A.buffers - 1)) * kv_size;
+      const T* Vs = Ks + CHUNK * ks;
+      // scores of the warp's pairs: four partial sums over d mod 4 each, added up as (0 + 1) + (2 + 3)
+      float s[PW][4];
+#pragma unroll
+      for (int a = 0; a < PW; ++a) s[a][0] = s[a][1] = s[a][2] = s[a][3] = 0.f;
+#pragma unroll 4
+      for (int d = 0; d < hdp; d += 4) {
+        const float4 k4 = four(Ks + lane * ks + d);
+#pragma unroll
+        for (int a = 0; a < PW; ++a) {
+          const float4 q4 = four(Qs + at[a] + d);
+          s[a][0] = fmaf(q4.x, k4.x, s[a][0]);
+          s[a][1] = fmaf(q4.y, k4.y, s[a][1]);
+          s[a][2] = fmaf(q4.z, k4.z, s[a][2]);
+          s[a][3] = fmaf(q4.w, k4.w, s[a][3]);
+        }
+      }
+      // j_from .. j_to: the chunk's keys that a pair's row sees (none: the chunk lies outside its row's range, and the pair
+      // stays as it is). The pairs' maxima, exponentials and sums run side by side.
+      int j_from[PW], j_to[PW];
+      float sc[PW], top[PW], sum[PW], corr[PW];
+      bool whole = true;
+#pragma unroll
+      for (int a = 0; a < PW; ++a) {
+        const int pair = warp + a * W;
+        j_from[a] = 0;
+        j_to[a] = -1;
+        if (pair < pairs) {
+          const int r = r0 + pair / G, p = s_pos[r], lo = s_lo[r];
+          j_from[a] = max(lo - c * CHUNK, 0);
+          j_to[a] = min(p - c * CHUNK, CHUNK - 1);
+          whole = whole && j_from[a] == 0 && j_to[a] == CHUNK - 1;
+          if constexpr (!SPLIT) {
+            if (j_from[a] <= j_to[a]) {
+              if (cut[a] < 0) cut[a] = lo / CHUNK + span_length(p / CHUNK - lo / CHUNK + 1);
+              if (c == cut[a]) {      // a new span: the last one joins the total
+                if (M[a] == -INFINITY && L[a] == 0.f) {
+                  M[a] = m[a];
+                  L[a] = l[a];
+#pragma unroll
+                  for (int i = 0; i < DPL; ++i) tot[a][i] = acc[a][i];
+                } else {
+                  float keep, add;
+                  span_weights(M[a], m[a], keep, add);
+                  L[a] = span_add(L[a], l[a], keep, add);
+#pragma unroll
+                  for (int i = 0; i < DPL; ++i) tot[a][i] = span_add(tot[a][i], acc[a][i], keep, add);
+                }
+                cut[a] += span_length(p / CHUNK - lo / CHUNK + 1);
+                m[a] = -INFINITY;
+                l[a] = 0.f;
+#pragma unroll
+                for (int i = 0; i < DPL; ++i) acc[a][i] = 0.f;
+              }
+            }
+          }
+        }
+        const bool valid = lane >= j_from[a] && lane <= j_to[a];
+        sc[a] = valid ? __fmul_rn((s[a][0] + s[a][1]) + (s[a][2] + s[a][3]), A.scale) : -INFINITY;
+        top[a] = sc[a];
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int a = 0; a < PW; ++a) top[a] = fmaxf(top[a], __shfl_xor_sync(0xffffffffu, top[a], o));
+#pragma unroll
+      for (int a = 0; a < PW; ++a) {
+        const bool live = j_from[a] <= j_to[a];
+        top[a] = fmaxf(m[a], top[a]);       // finite: every chunk walked holds at least one visible key
+        const float pj = lane >= j_from[a] && lane <= j_to[a] ? expf(sc[a] - top[a]) : 0.f;
+        corr[a] = live ? expf(m[a] - top[a]) : 1.f;               // 0 for the first chunk of a span (m = -inf)
+        sum[a] = pj;
+        Ps[a * CHUNK + lane] = pj;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int a = 0; a < PW; ++a) sum[a] += __shfl_xor_sync(0xffffffffu, sum[a], o);
+#pragma unroll
+      for (int a = 0; a < PW; ++a) {
+        if (j_from[a] <= j_to[a]) {
+          l[a] = __fmaf_rn(l[a], corr[a], sum[a]);
+          m[a] = top[a];
+        }
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) acc[a][i] *= corr[a];
+      }
+      __syncwarp();
+      for (int j = 0; j < CHUNK; j += 4) {
+        float v[4][DPL];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int i = 0; i < DPL; ++i) v[u][i] = lane + 32 * i < hdp ? Cvt<T>::to_f(Vs[(j + u) * hdp + lane + 32 * i]) : 0.f;
+#pragma unroll
+        for (int a = 0; a < PW; ++a) {
+          const float4 p4 = four(Ps + a * CHUNK + j);
+          const float pw[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            // (a key that the row does not see takes no part, whatever its value: 0 * inf)
+            const bool seen = whole || (j + u >= j_from[a] && j + u <= j_to[a]);
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) acc[a][i] = seen ? fmaf(pw[u], v[u][i], acc[a][i]) : acc[a][i];
+          }
+        }
+      }
+      __syncthreads();      // the chunk is consumed
     }
-    __syncthreads();
-    const int key = c * CHUNK + lane;
-    const bool valid = key >= lo && key <= p;
+
+    if constexpr (SPLIT) {
+      // a span's result per head: max, sum, accumulator; the cluster's blocks share the heads' values and merge in order
+      cg::cluster_group cluster = cg::this_cluster();
+      float* part = reinterpret_cast<float*>(kv);      // [head][2 + hd]
 #pragma unroll
-    for (int a = 0; a < MAX_HPW; ++a) {
-      const int g = warp + a * W;
-      if (g >= G) break;
-      const float* qh = Qs + g * hd;
-      const float* kr = Ks + lane * kstride;
-      float s = 0.f;
-      for (int d = 0; d < hd; ++d) s = fmaf(qh[d], kr[d], s);
-      s = valid ? s * scale : -INFINITY;
-      const float mn = fmaxf(m[a], warp_max(s));       // finite: every chunk walked holds at least one visible key
-      const float pj = valid ? expf(s - mn) : 0.f;
-      const float corr = expf(m[a] - mn);               // 0 for the first chunk (m = -inf)
-      l[a] = l[a] * corr + warp_sum(pj);
-      m[a] = mn;
+      for (int a = 0; a < PW; ++a) {
+        const int g = warp + a * W;
+        if (g >= G || (int)blockIdx.z >= spans) break;
+        if (lane == 0) {
+          part[g * (hd + 2)] = m[a];
+          part[g * (hd + 2) + 1] = l[a];
+        }
 #pragma unroll
-      for (int i = 0; i < DPL; ++i) acc[a][i] *= corr;
-      for (int j = 0; j < CHUNK; ++j) {
-        const float pv = __shfl_sync(0xffffffffu, pj, j);
+        for (int i = 0; i < DPL; ++i)
+          if (lane + 32 * i < hd) part[g * (hd + 2) + 2 + lane + 32 * i] = acc[a][i];
+      }
+      cluster.sync();
+      for (int e = blockIdx.z * blockDim.x + threadIdx.x; e < G * hd; e += gridDim.z * blockDim.x) {
+        const int g = e / hd, d = e - g * hd;
+        float sm[SPANS], sl[SPANS], sa[SPANS];
+#pragma unroll
+        for (int s = 0; s < SPANS; ++s) {
+          if (s < spans) {
+            const float* from = cluster.map_shared_rank(part, s) + g * (hd + 2);
+            sm[s] = from[0];
+            sl[s] = from[1];
+            sa[s] = from[2 + d];
+          }
+        }
+        float mm = sm[0], ll = sl[0], aa = sa[0];
+#pragma unroll
+        for (int s = 1; s < SPANS; ++s) {
+          if (s < spans) {
+            float keep, add;
+            span_weights(mm, sm[s], keep, add);
+            ll = span_add(ll, sl[s], keep, add);
+            aa = span_add(aa, sa[s], keep, add);
+          }
+        }
+        out[((size_t)(first + r0) * A.Hq + head0) * hd + e] = Cvt<T>::from_f(aa * (1.0f / ll));
+      }
+      cluster.sync();      // nobody leaves while its results may still be read
+    } else {
+#pragma unroll
+      for (int a = 0; a < PW; ++a) {
+        const int pair = warp + a * W;
+        if (pair >= pairs) break;
+        if (M[a] == -INFINITY && L[a] == 0.f) {      // one span
+          L[a] = l[a];
+#pragma unroll
+          for (int i = 0; i < DPL; ++i) tot[a][i] = acc[a][i];
+        } else {
+          float keep, add;
+          span_weights(M[a], m[a], keep, add);
+          L[a] = span_add(L[a], l[a], keep, add);
+#pragma unroll
+          for (int i = 0; i < DPL; ++i) tot[a][i] = span_add(tot[a][i], acc[a][i], keep, add);
+        }
+        const float inv = 1.0f / L[a];
+        T* orow = out + ((size_t)(first + r0 + pair / G) * A.Hq + head0 + pair % G) * hd;
 #pragma unroll
         for (int i = 0; i < DPL; ++i) {
           const int d = lane + 32 * i;
-          if (d < hd) acc[a][i] = fmaf(pv, Vs[j * hd + d], acc[a][i]);
+          if (d < hd) orow[d] = Cvt<T>::from_f(tot[a][i] * inv);
         }
       }
     }
-  }
-#pragma unroll
-  for (int a = 0; a < MAX_HPW; ++a) {
-    const int g = warp + a * W;
-    if (g >= G) break;
-    const float inv = 1.0f / l[a];
-#pragma unroll
-    for (int i = 0; i < DPL; ++i) {
-      const int d = lane + 32 * i;
-      if (d < hd) orow[g * hd + d] = Cvt<T>::from_f(acc[a][i] * inv);
-    }
+    r0 = r1;
   }
 }
 
-template <typename T, int DPL>
-int launch(const void* q, const void* k_pool, const void* v_pool, const int* pos, const int* seq_row, const int* table,
-           int mb, long long page_stride, int page_size, void* out, int N, int Hq, int Hkv, int hd, float scale,
-           int window, int* err, cudaStream_t stream) {
-  const int G_all = Hq / Hkv, G = G_all < MAX_GROUP ? G_all : MAX_GROUP;
-  const int W = G < MAX_WARPS ? G : MAX_WARPS;
-  const size_t smem = sizeof(float) * ((size_t)CHUNK * (hd + 1) + (size_t)CHUNK * hd + (size_t)G * hd);
-  auto kern = attn_simt_kernel<T, DPL>;
-  static size_t allowed = 48 * 1024;   // per instantiation: the attribute is raised once, outside any capture
+template <typename T, int DPL, int PW, bool VEC, bool SPLIT>
+int launch(const void* q, const void* k_pool, const void* v_pool, void* out, Args A, int slices, cudaStream_t stream) {
+  const int G = A.G_all < A.GS ? A.G_all : A.GS, pairs = A.rows * G;
+  const int W = pairs < MAX_WARPS ? pairs : MAX_WARPS;
+  const size_t kv = sizeof(T) * (size_t)CHUNK * (2 * A.hdp + 16 / sizeof(T)), rest = sizeof(float) * ((size_t)pairs * A.hdp + (size_t)W * PW * CHUNK);
+  A.buffers = 1;      // as many chunks as leave two blocks per SM, two if only one block fits
+  for (int b = 4; b > 1 && A.buffers == 1; b /= 2)
+    if (b * kv + rest <= (size_t)(b > 2 ? 100 : 200) * 1024) A.buffers = b;
+  size_t smem = A.buffers * kv + rest;
+  if (SPLIT) {      // (the spans' results reuse the keys and values)
+    const size_t part = sizeof(float) * (size_t)G * (A.hd + 2);
+    if (smem < part) smem = part;
+  }
+  auto kern = attn_simt_kernel<T, DPL, PW, VEC, SPLIT>;
+  static size_t allowed = 48 * 1024;   // per instantiation: the attribute is raised outside any capture (a step runs once before)
   if (smem > allowed) {
     if (smem > 227 * 1024) return FZ_TOO_LARGE;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     allowed = smem;
   }
-  dim3 grid(N, Hkv, (G_all + MAX_GROUP - 1) / MAX_GROUP);
-  fz_launch(kern, grid, dim3(32 * W), smem, stream, (const T*)q, (const T*)k_pool, (const T*)v_pool, pos, seq_row, table, mb,
-            page_stride, page_size, (T*)out, Hq, Hkv, hd, scale, window, err);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((A.N + A.rows - 1) / A.rows, A.Hkv * slices, SPLIT ? SPANS : 1);
+  cfg.blockDim = dim3(32 * W);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (SPLIT) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = SPANS;
+  }
+  if (fz_pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  cudaLaunchKernelEx(&cfg, kern, (const T*)q, (const T*)k_pool, (const T*)v_pool, (T*)out, A);
   FZ_LAUNCH_CHECK();
   return FZ_OK;
 }
 
+template <typename T, int DPL, bool VEC>
+int choose(const void* q, const void* k_pool, const void* v_pool, void* out, Args A, int max_context, cudaStream_t stream) {
+  constexpr int PAIRS = MAX_WARPS * Pairs<DPL>::PER_WARP;
+  A.GS = A.G_all < PAIRS ? A.G_all : PAIRS;
+  const int slices = (A.G_all + A.GS - 1) / A.GS;
+  if ((long long)A.Hkv * slices > 65535) return FZ_BAD_SHAPE;
+  const long long blocks = (long long)A.N * A.Hkv * slices;
+  // Spans of a row side by side: where rows, heads and slices alone are at most two blocks per SM, and rows may be long
+  // enough to have more than one span. (At 296 blocks of one span each the spans' blocks, eight times as many, still
+  // start within two rounds; beyond, sharing keys among rows gains more.)
+  A.rows = 1;
+  if (blocks <= 296 && max_context > SPAN_CHUNKS * CHUNK) {
+    if (A.GS <= MAX_WARPS) return launch<T, DPL, 1, VEC, true>(q, k_pool, v_pool, out, A, slices, stream);
+    return launch<T, DPL, PAIRS / MAX_WARPS, VEC, true>(q, k_pool, v_pool, out, A, slices, stream);
+  }
+  // Rows that share the keys of a block: as many as give it PAIRS pairs, while every SM keeps a block.
+  A.rows = PAIRS / A.GS < MAX_ROWS ? PAIRS / A.GS : MAX_ROWS;
+  while (A.rows > 1 && (blocks + A.rows - 1) / A.rows < 148) A.rows /= 2;
+  return launch<T, DPL, PAIRS / MAX_WARPS, VEC, false>(q, k_pool, v_pool, out, A, slices, stream);
+}
+
 template <typename T>
-int dispatch(const void* q, const void* k_pool, const void* v_pool, const int* pos, const int* seq_row,
-             const int* table, int mb, long long page_stride, int page_size, void* out, int N, int Hq, int Hkv,
-             int hd, float scale, int window, int* err, cudaStream_t stream) {
-#define FZ_GO(D) return launch<T, D>(q, k_pool, v_pool, pos, seq_row, table, mb, page_stride, page_size, out, N, Hq, Hkv, hd, scale, window, err, stream)
-  const int dpl = (hd + 31) / 32;
+int dispatch(const void* q, const void* k_pool, const void* v_pool, void* out, Args A, int max_context, cudaStream_t stream) {
+  const bool vec = A.hd * sizeof(T) % 16 == 0 && A.page_stride * sizeof(T) % 16 == 0 && (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0;
+  const int dpl = (A.hd + 31) / 32;
+#define FZ_GO(D)                                                                               \
+  return vec ? choose<T, D, true>(q, k_pool, v_pool, out, A, max_context, stream)              \
+             : choose<T, D, false>(q, k_pool, v_pool, out, A, max_context, stream)
   if (dpl <= 1) FZ_GO(1);
   if (dpl <= 2) FZ_GO(2);
   if (dpl <= 4) FZ_GO(4);
@@ -160,19 +476,35 @@ int dispatch(const void* q, const void* k_pool, const void* v_pool, const int* p
 // Sizes taken: any Hkv, Hq any multiple of Hkv, 0 < hd <= 512. Anything else returns FZ_BAD_SHAPE.
 FZ_API int fz_attn_simt_check(int Hq, int Hkv, int hd) {
   if (Hq <= 0 || Hkv <= 0 || hd <= 0 || Hq % Hkv) return FZ_BAD_SHAPE;
-  if (hd > MAX_HD || (Hq / Hkv + MAX_GROUP - 1) / MAX_GROUP > 65535) return FZ_BAD_SHAPE;
+  if (hd > MAX_HD || (Hq / Hkv + 31) / 32 > 65535) return FZ_BAD_SHAPE;
   return FZ_OK;
 }
 
+// max_context: the longest context among the rows, or more (it decides how the work is split, never the results).
 FZ_API int fz_attn_simt(const void* q, const void* k_pool, const void* v_pool, const int* pos, const int* seq_row,
                         const int* table, int mb, long long page_stride, int page_size, void* out, int dtype, int N,
-                        int Hq, int Hkv, int hd, float scale, int window, int* err, cudaStream_t stream) {
+                        int Hq, int Hkv, int hd, float scale, int window, int max_context, int* err, cudaStream_t stream) {
   if (N <= 0) return FZ_OK;
   if (fz_attn_simt_check(Hq, Hkv, hd) != FZ_OK || page_size <= 0 || Hkv > 65535) return FZ_BAD_SHAPE;
-  if (dtype == FZ_F32)
-    return dispatch<float>(q, k_pool, v_pool, pos, seq_row, table, mb, page_stride, page_size, out, N, Hq, Hkv, hd, scale, window, err, stream);
-  if (dtype == FZ_BF16)
-    return dispatch<__nv_bfloat16>(q, k_pool, v_pool, pos, seq_row, table, mb, page_stride, page_size, out, N, Hq, Hkv, hd, scale, window, err, stream);
+  Args A = {};
+  A.pos = pos;
+  A.seq_row = seq_row;
+  A.table = table;
+  A.page_stride = page_stride;
+  A.mb = mb;
+  A.page_size = page_size;
+  A.N = N;
+  A.Hq = Hq;
+  A.Hkv = Hkv;
+  A.hd = hd;
+  A.hdp = (hd + 3) / 4 * 4;
+  if (dtype == FZ_BF16) A.hdp = (hd + 7) / 8 * 8;
+  A.G_all = Hq / Hkv;
+  A.window = window;
+  A.scale = scale;
+  A.err = err;
+  if (dtype == FZ_F32) return dispatch<float>(q, k_pool, v_pool, out, A, max_context, stream);
+  if (dtype == FZ_BF16) return dispatch<__nv_bfloat16>(q, k_pool, v_pool, out, A, max_context, stream);
   return FZ_BAD_DTYPE;
 }
 

@@ -1,8 +1,12 @@
-"""The float32 path's product at the sizes where its rules change hands: few rows and tiles of rows, one chunk of k and
-many, one group of chunks and eight. Every result against 64-bit arithmetic within a bound from the order of the sums, and
-the same bits whoever computes it."""
+"""The float32 path's product and attention at the sizes where their rules change hands: few rows and tiles of rows, one
+chunk of k and many, one group of chunks and eight, a row's keys in one span and in eight, spans side by side and one
+after the other. Every result against 64-bit arithmetic within a bound from the order of the sums, and the same bits
+whoever computes it."""
+
 import pytest
 import torch
+
+from test_kernels_gpu import Meta, fill_cache, make_cache
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +49,60 @@ def test_linear(N, K):
     out = torch.empty(20, N, device="cuda")
     cu.linear(bad, w, bias, out)
     assert torch.equal(out[:3], full[:3]) and torch.equal(out[4:], full[4:20]) and not bool(out[3].isfinite().any())
+
+
+@pytest.mark.parametrize("Hq,Hkv,hd,bs,window", [(14, 2, 64, 16, 0), (3, 1, 32, 4, 0), (8, 8, 128, 8, 0), (40, 1, 48, 16, 0), (4, 2, 64, 16, 300),
+                                                 (2, 1, 512, 16, 0), (6, 2, 256, 1, 77), (2, 2, 20, 16, 0)])
+def test_attention_bits_do_not_depend_on_who_computes_them(Hq, Hkv, hd, bs, window):
+    cu = cuda()
+    lengths = [1100, 129, 31]
+    mb = -(-max(lengths) // bs)
+    g = torch.Generator().manual_seed(hd + window)
+    perm = torch.randperm(3 * mb + 2, generator=g).tolist()
+    table = [perm[r * mb:(r + 1) * mb] for r in range(3)]
+    cp = make_cache(3 * mb + 2, Hkv, bs, hd, torch.float32, "cpu")
+    fill_cache(cp, table, lengths, g)
+    cc = make_cache(3 * mb + 2, Hkv, bs, hd, torch.float32, "cuda")
+    cc.pool.copy_(cp.pool)
+    # a portion that ends at the longest context, one that starts a request, single tokens, a padding row
+    rows = [(0, p) for p in range(800, 1100)] + [(2, p) for p in range(31)] + [(-1, 0)] + [(1, 128), (0, 127), (0, 128)]
+    q = torch.randn(len(rows), Hq * hd, generator=g).cuda()
+    many = torch.full((len(rows), Hq * hd), float("nan"), device="cuda")
+    scale = hd ** -0.5
+
+    def attend(index, out, cache=cc):
+        cu.paged_attention(q[index].contiguous(), cache, Meta([rows[i][1] for i in index], [rows[i][0] for i in index], table, "cuda"), out,
+                           Hq, Hkv, hd, scale, window)
+
+    attend(list(range(len(rows))), many)
+    assert bool(many.isfinite().all()) and float(many[331].abs().max()) == 0.0
+    for index in ([0], [150], [299], [300], [330], [332], [333], [334], [299, 332, 331, 334], list(range(290, 335)), list(range(100, 300))):
+        few = torch.full((len(index), Hq * hd), float("nan"), device="cuda")
+        attend(index, few)
+        assert torch.equal(few, many[index]), f"rows {index[:4]}"
+    # against 64 bits: scores off by (hd + 2) roundings of at most sum |q||k| * scale, weights by that and an exponential,
+    # sums by the chunk, span and merge roundings (fewer than 200 for 1,100 keys) of values of at most max |v|
+    for i in (0, 299, 330, 332, 333):
+        r, p = rows[i]
+        lo = max(0, p - window + 1) if window else 0
+        at = torch.tensor([table[r][k // bs] for k in range(lo, p + 1)]), torch.tensor([k % bs for k in range(lo, p + 1)])
+        keys, values = (cp.pool[at[0], j][torch.arange(p + 1 - lo), :, at[1]].double() for j in (0, 1))      # (keys, Hkv, hd)
+        qi = q[i].cpu().double().view(Hkv, Hq // Hkv, hd)
+        s = torch.einsum("hgd,khd->hgk", qi, keys) * scale
+        ref = torch.einsum("hgk,khd->hgd", s.softmax(-1), values).reshape(-1)
+        s_err = (hd + 2) * 2.0 ** -24 * float(torch.einsum("hgd,khd->hgk", qi.abs(), keys.abs()).max()) * scale
+        bound = (2 * s_err + 210 * 2.0 ** -24) * float(values.abs().max())
+        assert float((many[i].cpu().double() - ref).abs().max()) <= bound
+    # keys and values that a row does not see yet take no part, whatever they hold
+    spoiled = make_cache(3 * mb + 2, Hkv, bs, hd, torch.float32, "cuda")
+    spoiled.pool.copy_(cp.pool)
+    for k in range(850, 1100):
+        spoiled.pool[table[0][k // bs], :, :, k % bs] = float("inf") if k % 2 else float("nan")
+    for index in ([0, 20, 49], list(range(0, 50)), [333, 334]):
+        few = torch.empty(len(index), Hq * hd, device="cuda")
+        attend(index, few, spoiled)
+        assert torch.equal(few, many[index])
+    whole = torch.empty(len(rows), Hq * hd, device="cuda")
+    attend(list(range(len(rows))), whole, spoiled)
+    assert torch.equal(whole[:50], many[:50]) and torch.equal(whole[300:], many[300:])
+    cu.check_errors()
