@@ -9,8 +9,9 @@
 // CPU device only). The cuts are what lets a few rows use the whole chip: with one chain over all of K (the order before)
 // 4 x 4,864 -> 896 had 14 blocks to run in and took 215 us.
 //
-// Few rows (M <= 16): `gemm_simt_few_kernel`, bound by reading W. More rows: `gemm_simt_tile_kernel`, bound by the FMA
-// pipes (a probe of independent fmaf chains reached 70 TFLOP/s; packed float32 x 2 forms reach no more).
+// Few rows (M <= 16): `gemm_simt_few_kernel`, bound by reading W. More rows: `gemm_simt_tile_kernel` and, where tiles are
+// many, `gemm_simt_wide_kernel`, bound by the FMA pipes (a probe of independent fmaf chains reached 70 TFLOP/s, of packed
+// pairs 71).
 #include "common.cuh"
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
@@ -304,6 +305,133 @@ gemm_simt_tile_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const 
   cluster.sync();      // nobody leaves while its tile may still be read
 }
 
+// ---- many rows and columns
+// Products of one group whose tiles of 64 x 128 outputs give every SM two blocks: 128 threads with 8 x 8 outputs each, 16 k
+// per stage. A stage is fetched into registers while the one before is multiplied and then lies in shared memory k by k, so
+// that a thread reads its 8 and 8 values of a k as 16-byte pieces and multiplies pairs of columns with `__ffma2_rn` (each
+// half rounds as fmaf, so the bits are the tile kernel's): half as many instructions, and fewer that wait for a register
+// bank, which held the tile kernel (0.39 cycles of dispatch stall per instruction) at 40 TFLOP/s. Measured: 300 x 896 ->
+// 9,728 160 -> 137 us, 300 x 896 -> 151,936 2,031 -> 1,750 us (47 TFLOP/s), 64 rows of it 435 -> 390; with one block per
+// SM (100 x 896 -> 9,728) it loses, 82 -> 92 us.
+constexpr int WIDE_N = 128, WIDE_K = 16;
+template <typename TA, typename TC, bool VEC>
+__global__ void __launch_bounds__(128, 2)
+gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias,
+                      TC* __restrict__ C, int M, int N, int K, Order o, int m_tiles) {
+  constexpr int TM = 8, BM = 8 * TM, STAGE = (BM + WIDE_N) * WIDE_K, A_PASSES = BM / 32, W_PASSES = WIDE_N / 32;
+  __shared__ __align__(16) float buf[2 * STAGE];      // two stages of [k][64 rows of A], [k][128 rows of W]
+  fz_grid_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);      // 16 x 8 threads, a warp 8 x 4 of them
+  const int m0 = (blockIdx.x % m_tiles) * BM, n0 = (blockIdx.x / m_tiles) * WIDE_N;
+  const int stages = (K + WIDE_K - 1) / WIDE_K, per_chunk = o.chunk / WIDE_K;
+  // staging: four lanes to a row (four k each), 32 rows a pass. Row r, k lies at [k][r ^ 8 (k / 4)]: the four lanes' rows
+  // then go to different banks, and pieces of eight rows stay whole.
+  const int lrow = tid >> 2, lk = (tid & 3) * 4, lswz = (tid & 3) * 8;
+
+  auto fetch = [&](const TA* base, int row, int limit, int s) {
+    const int k = s * WIDE_K + lk;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row < limit) {
+      const TA* at = base + (long long)row * K + k;
+      if constexpr (VEC) {
+        if (k < K) v = *reinterpret_cast<const float4*>(at);
+      } else {
+        if (k < K) v.x = Cvt<TA>::to_f(at[0]);
+        if (k + 1 < K) v.y = Cvt<TA>::to_f(at[1]);
+        if (k + 2 < K) v.z = Cvt<TA>::to_f(at[2]);
+        if (k + 3 < K) v.w = Cvt<TA>::to_f(at[3]);
+      }
+    }
+    return v;
+  };
+  auto put = [&](float* at, int width, int row, float4 v) {
+    at[lk * width + (row ^ lswz)] = v.x;
+    at[(lk + 1) * width + (row ^ lswz)] = v.y;
+    at[(lk + 2) * width + (row ^ lswz)] = v.z;
+    at[(lk + 3) * width + (row ^ lswz)] = v.w;
+  };
+  float4 fa[A_PASSES], fw[W_PASSES];
+  auto fetch_a = [&](int s) {
+#pragma unroll
+    for (int i = 0; i < A_PASSES; ++i) fa[i] = fetch(A, m0 + lrow + 32 * i, M, s);
+  };
+  auto fetch_w = [&](int s) {
+#pragma unroll
+    for (int i = 0; i < W_PASSES; ++i) fw[i] = fetch(W, n0 + lrow + 32 * i, N, s);
+  };
+  auto put_stage = [&](int which) {
+    float* at = buf + which * STAGE;
+#pragma unroll
+    for (int i = 0; i < A_PASSES; ++i) put(at, BM, lrow + 32 * i, fa[i]);
+#pragma unroll
+    for (int i = 0; i < W_PASSES; ++i) put(at + BM * WIDE_K, WIDE_N, lrow + 32 * i, fw[i]);
+  };
+
+  float2 acc[TM][4], tot[TM][4];      // columns tx * 4 + 0, 1 | 2, 3 and the same 64 further on
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = tot[i][j] = make_float2(0.f, 0.f);
+
+  fetch_w(0);      // (no kernel of a step writes weights)
+  fz_grid_wait();
+  fetch_a(0);
+  put_stage(0);
+  __syncthreads();
+  int left = per_chunk;
+  for (int s = 0; s < stages; ++s) {
+    const bool more = s + 1 < stages;
+    if (more) {
+      fetch_w(s + 1);
+      fetch_a(s + 1);
+    }
+    const float* as = buf + (s & 1) * STAGE;
+    const float* ws = as + BM * WIDE_K;
+#pragma unroll
+    for (int k = 0; k < WIDE_K; ++k) {
+      const int swz = (k >> 2) * 8;
+      alignas(16) float a[TM];
+#pragma unroll
+      for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4*>(a + i) = *reinterpret_cast<const float4*>(as + k * BM + ((ty * TM + i) ^ swz));
+      alignas(16) float2 w[4];
+      *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(ws + k * WIDE_N + ((tx * 4) ^ swz));
+      *reinterpret_cast<float4*>(w + 2) = *reinterpret_cast<const float4*>(ws + k * WIDE_N + ((tx * 4 + 64) ^ swz));
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const float2 aa = make_float2(a[i], a[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = __ffma2_rn(aa, w[j], acc[i][j]);
+      }
+    }
+    if (--left == 0 || !more) {
+      left = per_chunk;
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          tot[i][j] = __fadd2_rn(tot[i][j], acc[i][j]);
+          acc[i][j] = make_float2(0.f, 0.f);
+        }
+    }
+    if (more) put_stage((s + 1) & 1);      // (that buffer was last read a stage ago, before the barrier)
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + ty * TM + i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int n = n0 + tx * 4 + (j & 3) + (j >> 2) * 64;
+      if (n >= N) continue;
+      float v = j & 1 ? tot[i][j >> 1].y : tot[i][j >> 1].x;
+      if (bias) v += bias[n];
+      C[(size_t)m * N + n] = Cvt<TC>::from_f(v);
+    }
+  }
+}
+
 // Raises a kernel's shared-memory limit where it needs more than the default (once per instantiation and size, outside
 // any capture: a step is run once before it is captured).
 template <typename K> cudaError_t allow_smem(K kern, size_t smem, size_t& allowed) {
@@ -363,6 +491,16 @@ int launch_tile(const void* A, const void* W, const float* bias, void* C, int M,
   return FZ_OK;
 }
 
+template <typename TA, typename TC, bool VEC>
+int launch_wide(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
+  const int m_tiles = (M + 63) / 64;
+  const long long tiles = (long long)m_tiles * ((N + WIDE_N - 1) / WIDE_N);
+  if (tiles > 2147483647LL) return FZ_TOO_LARGE;
+  fz_launch(gemm_simt_wide_kernel<TA, TC, VEC>, dim3((unsigned)tiles), dim3(128), 0, stream, (const TA*)A, (const TA*)W, bias, (TC*)C, M, N, K, o, m_tiles);
+  FZ_LAUNCH_CHECK();
+  return FZ_OK;
+}
+
 // Two columns per lane (every value of A read once for both) where N still gives two blocks per SM.
 template <typename TA, typename TC, int MR, bool VEC>
 int launch_few_n(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
@@ -379,6 +517,8 @@ int launch_rows(const void* A, const void* W, const float* bias, void* C, int M,
   if (M <= 8) return launch_few_n<TA, TC, 8, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (M <= 16) return launch_few_n<TA, TC, 16, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (M <= 32) return launch_tile<TA, TC, 4, VEC>(A, W, bias, C, M, N, K, o, stream);
+  if (o.groups == 1 && (long long)((M + 63) / 64) * ((N + WIDE_N - 1) / WIDE_N) >= 296)
+    return launch_wide<TA, TC, VEC>(A, W, bias, C, M, N, K, o, stream);
   return launch_tile<TA, TC, 8, VEC>(A, W, bias, C, M, N, K, o, stream);
 }
 
