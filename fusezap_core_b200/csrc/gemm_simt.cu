@@ -64,23 +64,28 @@ __device__ __forceinline__ void fma4(float& acc, float4 a, float4 w) {
 // ---- few rows
 // A block owns 8 * RPL columns (rows of W) and all of K: warp w has chunks 4w .. 4w+3, eight lanes to a chunk, RPL columns
 // to a lane, MR rows of A to each. So N * 32 / RPL chains run at once, and a warp waits for no other until the end: it
-// streams its own 16 k of every (column, chunk) per stage through a ring of its own, 64 contiguous bytes each, rows padded
-// to 80 bytes (conflict-free 16-byte reads). The first stages of W, which no kernel of a step writes, are asked for ahead
+// streams its own 16 k of every (column, chunk) per stage through a ring of its own, 64 contiguous bytes each, whose 16-byte
+// pieces stand in an order that changes every two rows (conflict-free reads without padding, so that three blocks share an
+// SM at K = 896). Where the columns give every SM at most one block (DEEP) the ring takes all of its memory. The first stages of W, which no kernel of a step writes, are asked for ahead
 // of the wait on the kernel before. Blocks that stay and walk several tiles with the ring running on measured slower at
 // large N (896 -> 151,936 at 8 rows: 211 against 156 us): waiting at each tile's end for the slowest warp costs more than
-// a new block. Measured at 4 rows, weights from HBM: 4,864 -> 896 215 -> 10.1 us, 896 -> 9,728 75 -> 11.0 us, 896 ->
-// 151,936 417 -> 132 us (4.1 TB/s; 1 row 101 us, 5.4 TB/s: with more rows the reads of A from shared memory bind).
-constexpr int FEW_K = 16, FEW_ROW = FEW_K + 4;
-template <int MR, int RPL> struct Few {
-  static constexpr int W_FLOATS = 32 * RPL * FEW_ROW, A_SUB = MR * FEW_K + 4, STAGE = W_FLOATS + 4 * A_SUB;   // per warp
-  static constexpr int FIT = 112 * 1024 / (8 * STAGE * 4), STAGES = FIT < 2 ? 2 : FIT > 4 ? 4 : FIT;          // two blocks per SM where that leaves two stages
+// a new block. Measured at 4 rows, weights from HBM: 4,864 -> 896 7.1 us (rings two blocks could share: 10.1; one
+// chain of fmaf over all of K: 215), 896 -> 9,728 9.8 us (padded rows, two blocks per SM: 11.0; 75), 896 -> 151,936 113 us
+// (132; 417), 4.8 TB/s; 4,096 -> 28,672 75 us, 6.3 TB/s.
+constexpr int FEW_K = 16;
+template <int MR, int RPL, bool DEEP> struct Few {
+  static constexpr int W_FLOATS = 32 * RPL * FEW_K, A_SUB = MR * FEW_K + 4, STAGE = W_FLOATS + 4 * A_SUB;   // per warp
+  static constexpr int FIT = (DEEP ? 220 : 112) * 1024 / (8 * STAGE * 4), MOST = DEEP ? 8 : 4;
+  static constexpr int STAGES = FIT < 2 ? 2 : FIT > MOST ? MOST : FIT;      // two blocks per SM where that leaves two stages
 };
+// Where piece q (four k) of a stage's row lies within the row.
+__device__ __forceinline__ int few_piece(int row, int q) { return (q ^ ((row >> 1) & 3)) * 4; }
 
-template <typename TA, typename TC, int MR, int RPL, bool VEC>
+template <typename TA, typename TC, int MR, int RPL, bool VEC, bool DEEP>
 __global__ void __launch_bounds__(256)
 gemm_simt_few_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* __restrict__ bias,
                      TC* __restrict__ C, int M, int N, int K, Order o, int slots) {
-  using F = Few<MR, RPL>;
+  using F = Few<MR, RPL, DEEP>;
   constexpr int COLS = 8 * RPL;
   extern __shared__ float4 few_smem[];
   fz_grid_launch_dependents();
@@ -96,7 +101,7 @@ gemm_simt_few_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const f
       const int e = lane + 32 * j, stream = e >> 2, q = (e & 3) * 4;
       const int c = warp * 4 + stream / COLS, n = n0 + stream % COLS;
       const int k = c * o.chunk + s * FEW_K + q, end = min(K, (c + 1) * o.chunk);
-      stage4<TA, VEC>(at + stream * FEW_ROW + q, W, n, K, k, end, n < N && c < o.chunks);
+      stage4<TA, VEC>(at + stream * FEW_K + few_piece(stream, e & 3), W, n, K, k, end, n < N && c < o.chunks);
     }
   };
   auto load_a = [&](int s) {
@@ -136,7 +141,7 @@ gemm_simt_few_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const f
     for (int q = 0; q < FEW_K / 4; ++q) {
       float4 w[RPL];
 #pragma unroll
-      for (int i = 0; i < RPL; ++i) w[i] = *reinterpret_cast<const float4*>(at + (sub * COLS + r + 8 * i) * FEW_ROW + 4 * q);
+      for (int i = 0; i < RPL; ++i) w[i] = *reinterpret_cast<const float4*>(at + (sub * COLS + r + 8 * i) * FEW_K + few_piece(r, q));
 #pragma unroll
       for (int m = 0; m < MR; ++m) {
         const float4 a = *reinterpret_cast<const float4*>(aw + m * FEW_K + 4 * q);
@@ -441,13 +446,13 @@ template <typename K> cudaError_t allow_smem(K kern, size_t smem, size_t& allowe
   return e;
 }
 
-template <typename TA, typename TC, int MR, int RPL, bool VEC>
+template <typename TA, typename TC, int MR, int RPL, bool VEC, bool DEEP>
 int launch_few(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
-  using F = Few<MR, RPL>;
+  using F = Few<MR, RPL, DEEP>;
   const int warps = (o.chunks + 3) / 4, stages = o.chunk / FEW_K, slots = stages < F::STAGES ? stages : F::STAGES;
   const size_t ring = sizeof(float) * (size_t)warps * slots * F::STAGE, sums = sizeof(float) * (size_t)o.chunks * MR * 8 * RPL;
   const size_t smem = ring > sums ? ring : sums;
-  auto kern = gemm_simt_few_kernel<TA, TC, MR, RPL, VEC>;
+  auto kern = gemm_simt_few_kernel<TA, TC, MR, RPL, VEC, DEEP>;
   static size_t allowed = 48 * 1024;
   const cudaError_t e = allow_smem(kern, smem, allowed);
   if (e != cudaSuccess) return (int)e;
@@ -504,8 +509,10 @@ int launch_wide(const void* A, const void* W, const float* bias, void* C, int M,
 // Two columns per lane (every value of A read once for both) where N still gives two blocks per SM.
 template <typename TA, typename TC, int MR, bool VEC>
 int launch_few_n(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
-    if (N >= 4096) return launch_few<TA, TC, MR, 2, VEC>(A, W, bias, C, M, N, K, o, stream);
-  return launch_few<TA, TC, MR, 1, VEC>(A, W, bias, C, M, N, K, o, stream);
+    if (N >= 4096) return launch_few<TA, TC, MR, 2, VEC, false>(A, W, bias, C, M, N, K, o, stream);
+  if constexpr (VEC)      // (asynchronous copies alone gain from depth)
+    if ((N + 7) / 8 <= 148) return launch_few<TA, TC, MR, 1, VEC, true>(A, W, bias, C, M, N, K, o, stream);
+  return launch_few<TA, TC, MR, 1, VEC, false>(A, W, bias, C, M, N, K, o, stream);
 }
 
 template <typename TA, typename TC, bool VEC>
