@@ -38,7 +38,8 @@ constexpr int BM = 128;           // TMEM lanes = rows of the 128-row operand
 constexpr int BK = 64;            // k per stage: 64 bf16 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;  // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
-constexpr int PAIR_THREADS_G = 320;      // the many-token kernels: warps 2..9 epilogue (two per quarter of the tensor-memory lanes)
+constexpr int PAIR_PARTS = 4;            // the kernel with two SMs per tile: epilogue warps per quarter of the tensor-memory lanes
+constexpr int PAIR_THREADS_G = 64 + 128 * PAIR_PARTS;      // its threads: warps 2 and up are the epilogue
 
 // ---------------------------------------------------------------------------------------------- cluster helpers
 __device__ __forceinline__ void cluster_sync_all() {
@@ -487,17 +488,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // Rows mode: one thread's lane (token row `row`) of a finished accumulator of BN columns at `taddr`, with the bias added,
-// to the output's columns n0 .. n0 + BN - 1 (or, with the fused SwiGLU, to its packed half). Every lane of the warp takes
-// part in the loads from tensor memory whether or not its row exists.
-template <int BN>
-__device__ __forceinline__ void rows_store_tile(const Params& p, uint32_t taddr, int row, int n0) {
+// to the output's columns n0 .. n0 + BN - 1 (or, with the fused SwiGLU, to its packed half); of these the `part`-th of PARTS
+// equal shares. Every lane of the warp takes part in the loads from tensor memory whether or not its row exists.
+template <int BN, int PARTS>
+__device__ __forceinline__ void rows_store_tile(const Params& p, uint32_t taddr, int row, int n0, int part) {
   float v[16];
   if (p.swiglu) {
     // columns [128 b, 128 b + 64) are gate, [128 b + 64, 128 b + 128) up of output features 64 (n0 / 128 + b) ..
     float u[16];
+    constexpr int FEATS = BN / 2 / PARTS;        // features of a share
 #pragma unroll 1
-    for (int c = 0; c < BN; c += 16) {
-      if ((c & 64) != 0) continue;
+    for (int f = part * FEATS; f < (part + 1) * FEATS; f += 16) {
+      const int c = (f >> 6) * 128 + (f & 63);
       tmem_ld16(taddr + (uint32_t)c, v);
       tmem_ld16(taddr + (uint32_t)(c + 64), u);
       const int n = n0 + c;                       // packed index of the gate column
@@ -517,7 +519,7 @@ __device__ __forceinline__ void rows_store_tile(const Params& p, uint32_t taddr,
     return;
   }
 #pragma unroll 1
-  for (int c = 0; c < BN; c += 16) {
+  for (int c = part * (BN / PARTS); c < (part + 1) * (BN / PARTS); c += 16) {
     tmem_ld16(taddr + (uint32_t)c, v);
     if (row >= p.rows) continue;
     const int n = n0 + c;
@@ -662,7 +664,7 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       // (Four epilogue warps here. Eight, as in the two-SM kernel, were measured on this kernel and did not pay: the tiles
       // it gets are narrow or few, and 2,048 tokens at Qwen2.5-0.5B sizes took 3.94 ms with them against 3.77 ms.)
       const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quad * 32) << 16);
-      rows_store_tile<BN>(p, taddr, tm * BM + r, tn * BN);
+      rows_store_tile<BN, 1>(p, taddr, tm * BM + r, tn * BN, 0);
       tc_fence_before();
       mbar_arrive(&acc_empty[acc]);      // this thread has read its lane of the accumulator
     }
@@ -787,7 +789,7 @@ gemm_tc_rows_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 16); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8 * PAIR_PARTS); }
     flag[0] = 0;
     mbar_init_fence();
   }
@@ -871,12 +873,12 @@ gemm_tc_rows_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (j >> 1) & 1));
       if (!ok) { flag[0] = 1; break; }
       tc_fence_after();
-      // (warps 2..5 take the tile's first 128 columns, warps 6..9 the other 128: two warps per scheduler, so that one
-      // computes while the other waits; with four warps the epilogue of a tile took longer than the products of a tile
-      // with a short K: 13 us per tile at K = 896, where the products take 5)
-      const int col0 = warp >= 6 ? BN / 2 : 0;
-      const uint32_t taddr = tmem_base + (uint32_t)(acc * BN + col0) + ((uint32_t)(quad * 32) << 16);
-      rows_store_tile<BN / 2>(p, taddr, (2 * tm + (int)rank) * BM + r, tn * BN + col0);
+      // (PAIR_PARTS warps per quarter of the lanes, each with its share of the tile's columns, so that some compute while
+      // others wait: with one the epilogue of a tile took longer than the products of a tile with a short K, 13 us at
+      // K = 896, where the products take 5; with four instead of two a step of 2,101 rows at Qwen2.5-0.5B sizes takes 2.96
+      // ms instead of 3.12, and 2,048 rows at Llama-3.1-8B sizes, K = 4,096, the same as before)
+      const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quad * 32) << 16);
+      rows_store_tile<BN, PAIR_PARTS>(p, taddr, (2 * tm + (int)rank) * BM + r, tn * BN, (warp - 2) >> 2);
       tc_fence_before();
       __syncwarp();      // every lane of the warp has read its lane of the accumulator
       if (lane == 0) mbar_arrive_cluster(acc_empty0 + 8u * (uint32_t)acc);
@@ -1445,9 +1447,11 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
       if (p.stages > enough) p.stages = enough;
       // A matrix that the rings of all its CTAs hold whole (up to 24 MB of 148 x 227 KB): then every weight is on its way
       // before the wait on the kernel before, and what follows the wait is the activations, the sums and the store alone.
-      // Qwen2.5-0.5B sizes: a decode step of one row 757 -> 746 us, of 32 rows 1,072 -> 1,059 us. Larger ones would only keep the next kernels' blocks off the SMs.
+      // Qwen2.5-0.5B sizes: a decode step of one row 757 -> 746 us, of 32 rows 1,072 -> 1,059 us. Larger ones would only
+      // keep the next kernels' blocks off the SMs. (At least three stages: they also hold the sums of 128 columns and the
+      // exchange of the gated epilogue, 72 KB.)
       const long long ring = (long long)per_cta * (BM + bn) * BK * 2;
-      if (ring <= 200 * 1024 && ring * tiles * p.splits <= 24 << 20) p.stages = per_cta < 3 ? 3 : per_cta;      // (the sums of 128 columns and the exchange lie in three stages)
+      if (ring <= 200 * 1024 && ring * tiles * p.splits <= 24 << 20) p.stages = per_cta < 3 ? 3 : per_cta;
     }
     if ((st = get_map_bf16(w, N, K, BM, &ma)) != FZ_OK) return st;
     if ((st = get_map_bf16(x, M, K, bn, &mb)) != FZ_OK) return st;
