@@ -323,13 +323,19 @@ struct UnitCursor {
   bool valid;
 };
 
-template <int HD, int BOX, int NSTAGE, int MINB, bool SMALLG>
-__global__ void __launch_bounds__(THREADS, MINB)
+//
+// WHOLE (steps of single tokens whose contexts have at most WHOLE_UNITS units, rows x kv heads at most one block per SM): a
+// block has one (row, kv head) to itself, its eight warps share the row's units, leave their results in shared memory and
+// merge them there, in the order and with the arithmetic of the combine kernel, which is not launched. At these sizes both
+// kernels are a chain of latencies: a decode step of one row with 300 keys at Qwen2.5-0.5B sizes, 24 layers, 772 -> 691 us.
+constexpr int WHOLE_UNITS = 16;
+template <int HD, int BOX, int NSTAGE, int MINB, bool SMALLG, int WARPS = 4, bool WHOLE = false>
+__global__ void __launch_bounds__(32 * WARPS, MINB)
 attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_bfloat16* __restrict__ q,
                          const int* __restrict__ pos, const int* __restrict__ seq_row, const int* __restrict__ seg,
                          const int* __restrict__ table, int mb, int page_size, float* __restrict__ part_o,
                          float* __restrict__ part_ml, int N, int Hq, int Hkv, int NPU, float scale_log2, int window,
-                         int long_from, int single, int maps, int* err) {
+                         int long_from, int single, int maps, int* err, __nv_bfloat16* __restrict__ out) {
   // SMALLG (at most 8 query heads per kv head): the transposed products of `attend16_small`
   constexpr int KSTEPS = HD / 16, OB = SMALLG ? HD / 16 : HD / 8, QW = SMALLG ? 2 : 4, HALVES = HD / 64;
   constexpr int HALF_BYTES = 16 * 128;                 // one column half of a 16-key group
@@ -339,13 +345,13 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t s_base = smem_u32(smem);
-  uint64_t* bars = (uint64_t*)(smem + 4 * WARP_BYTES);                   // [4 warps][NSTAGE]
-  int* s_pre = (int*)(bars + 4 * NSTAGE);                                // [N + 1]: units before row n
+  uint64_t* bars = (uint64_t*)(smem + WARPS * WARP_BYTES);               // [WARPS][NSTAGE]
+  int* s_pre = (int*)(bars + WARPS * NSTAGE);                                // [N + 1]: units before row n
 
   // Prologue that depends on nothing another kernel writes: the barriers.
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int i = 0; i < 4 * NSTAGE; ++i) fztma::mbar_init(&bars[i], 1);
+    for (int i = 0; i < WARPS * NSTAGE; ++i) fztma::mbar_init(&bars[i], 1);
     fztma::mbar_init_fence();
   }
   __syncthreads();
@@ -354,8 +360,24 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
   // the step's first kernel started and no kernel changes it, so it may be read while the kernel before this one runs.
 
   const int G = Hq / Hkv;
+  // WHOLE: the block's row and kv head, and where the units' results go: [unit][head] (max, sum), then [unit][head][HD]
+  const int n_whole = WHOLE ? (int)blockIdx.x / Hkv : 0, kvh_whole = WHOLE ? (int)blockIdx.x - n_whole * Hkv : 0;
+  float2* s_ml = (float2*)(s_pre + 4);      // (16 bytes on: what follows is read in pieces of 16)
+  float* s_o = (float*)(s_ml + WHOLE_UNITS * 8);
+  if constexpr (WHOLE) {
+    const int row = seq_row[n_whole], p = pos[n_whole];
+    if (row < 0) {      // a padding row gives zeros
+      fz_grid_wait();
+      for (int i = tid; i < G * HD; i += 32 * WARPS) out[((size_t)n_whole * Hq + (size_t)kvh_whole * G) * HD + i] = __float2bfloat16_rn(0.f);
+      return;
+    }
+    if (tid == 0) {
+      s_pre[0] = 0;
+      s_pre[1] = unit_of(p) - unit_of(window > 0 ? max(0, p - window + 1) : 0) + 1;
+    }
+  }
   // units of every row (0 for padding rows and for rows of long portions), then their running sum
-  for (int n = tid; n < N; n += THREADS) {
+  for (int n = tid; !WHOLE && n < N; n += 32 * WARPS) {
     // `single`: every portion of the step is one token, so no row belongs to a long portion and the portion's record
     // need not be asked for (a load that could only start when the row number has arrived)
     const int row = seq_row[n];
@@ -367,9 +389,9 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
     }
     s_pre[n + 1] = cnt;
   }
-  if (tid == 0) s_pre[0] = 0;
+  if (!WHOLE && tid == 0) s_pre[0] = 0;
   __syncthreads();
-  if (warp == 0) {
+  if (!WHOLE && warp == 0) {
     int carry = 0;
     for (int base = 0; base < N; base += 32) {
       const int i = base + lane;
@@ -385,17 +407,17 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
   }
   __syncthreads();
   // from here on the warps go their own ways: no block-wide barrier below
-  const long long T = s_pre[N];
-  const long long gw = (long long)blockIdx.x * 4 + warp, W = (long long)gridDim.x * 4;
+  const long long T = WHOLE ? min(s_pre[1], WHOLE_UNITS) : s_pre[N];
+  const long long gw = WHOLE ? warp : (long long)blockIdx.x * 4 + warp, W = WHOLE ? WARPS : (long long)gridDim.x * 4;
   const int u_begin = (int)(T * gw / W), u_end = (int)(T * (gw + 1) / W);
-  if (u_begin >= u_end) { fz_grid_wait(); return; }
+  if (!WHOLE && u_begin >= u_end) { fz_grid_wait(); return; }
 
   auto load_unit = [&](UnitCursor& c, int u, int n_hint, bool with_pages) {
     c.u = u;
     c.valid = u < u_end;
     if (!c.valid) return;
-    int n = n_hint;
-    if (!(s_pre[n] <= u && u < s_pre[n + 1])) {      // the largest n with s_pre[n] <= u
+    int n = WHOLE ? n_whole : n_hint;
+    if (!WHOLE && !(s_pre[n] <= u && u < s_pre[n + 1])) {      // the largest n with s_pre[n] <= u
       int a = 0, b = N - 1;
       while (a < b) {
         const int mid = (a + b + 1) >> 1;
@@ -403,12 +425,12 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
       }
       n = a;
     }
-    const int r = u - s_pre[n], per_head = (s_pre[n + 1] - s_pre[n]) / Hkv;
+    const int r = WHOLE ? u : u - s_pre[n], per_head = WHOLE ? s_pre[1] : (s_pre[n + 1] - s_pre[n]) / Hkv;
     c.n = n;
-    c.kvh = r / per_head;
+    c.kvh = WHOLE ? kvh_whole : r / per_head;
     c.p = pos[n];
     c.lo = window > 0 ? max(0, c.p - window + 1) : 0;
-    c.unit = unit_of(c.lo) + (r - c.kvh * per_head);
+    c.unit = unit_of(c.lo) + (WHOLE ? u : r - c.kvh * per_head);
     c.key0 = unit_start(c.unit);
     c.g = c.lo > c.key0 ? (c.lo - c.key0) >> 4 : 0;
     c.g_end = min(unit_len(c.unit) >> 4, ((c.p - c.key0) >> 4) + 1);
@@ -543,6 +565,7 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
     const int stage = consumed % NSTAGE;
     if (!__all_sync(0xffffffffu, fztma::mbar_wait(&wbars[stage], (consumed / NSTAGE) & 1))) {
       if (lane == 0) atomicOr(err, FZ_ERR_WAIT_TIMEOUT);
+      if constexpr (WHOLE) break;
       return;
     }
     const uint32_t sk = s_warp + stage * STAGE_BYTES, sv = sk + KV_BYTES;
@@ -572,7 +595,7 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
       // partial result, marked by a negative sum, in the slot of its first unit.
       int write_unit = cc.unit;
       bool write = true;
-      if (cc.unit < SMALL_UNITS) {
+      if (!WHOLE && cc.unit < SMALL_UNITS) {
         const int bu0 = max(unit_of(cc.lo), cc.unit & ~3), bu1 = min(unit_of(cc.p), cc.unit | 3);
         if (bu1 > bu0 && cc.u - (cc.unit - bu0) >= u_begin && cc.u + (bu1 - cc.unit) < u_end) {
           if (cc.unit == bu0) {
@@ -600,7 +623,19 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
           }
         }
       }
-      if (write) {
+      if constexpr (WHOLE) {
+        static_assert(SMALLG, "at most eight heads");
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int g = 2 * (lane & 3) + j;
+          if (g < G) {
+            float* dst = s_o + (cc.u * G + g) * HD + (lane >> 2);
+#pragma unroll
+            for (int i = 0; i < OB; ++i) { dst[16 * i] = o[i][j]; dst[16 * i + 8] = o[i][2 + j]; }
+            if ((lane >> 2) == 0) s_ml[cc.u * G + g] = make_float2(m_run[j], l_run[j]);
+          }
+        }
+      } else if (write) {
         // unnormalised O and (max, sum), straight from the MMA fragments
         const size_t head0 = (size_t)cc.n * Hq + (size_t)cc.kvh * G;
         if constexpr (SMALLG) {
@@ -632,6 +667,42 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
       fresh = true;
     }
     if (++cc.g >= cc.g_end) load_unit(cc, cc.u + 1, cc.n, false);
+  }
+  if constexpr (WHOLE) {
+    __syncthreads();
+    const int p = pos[n_whole], lo = window > 0 ? max(0, p - window + 1) : 0, u0 = unit_of(lo), u1 = u0 + (int)T - 1;
+    for (int t = tid; t < G * (HD / 4); t += 32 * WARPS) {
+      const int g = t / (HD / 4), d4 = (t - g * (HD / 4)) * 4;
+      auto merge4 = [](float4& a, const float4& c, float fa, float fb) {
+        a.x = merge_unit_value(a.x, c.x, fa, fb); a.y = merge_unit_value(a.y, c.y, fa, fb);
+        a.z = merge_unit_value(a.z, c.z, fa, fb); a.w = merge_unit_value(a.w, c.w, fa, fb);
+      };
+      float M = 0.f, L = 0.f;
+      float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int b = u0 >> 2; b <= u1 >> 2; ++b) {      // (no more blocks than the combine kernel has chains: one to a chain)
+        const int i0 = max(u0, 4 * b) - u0, i1 = min(u1, 4 * b + 3) - u0;
+        float Mb = s_ml[i0 * G + g].x, Lb = s_ml[i0 * G + g].y, fa, fb;
+        float4 Ob = *(const float4*)(s_o + (i0 * G + g) * HD + d4);
+        for (int i = i0 + 1; i <= i1; ++i) {
+          const float2 next = s_ml[i * G + g];
+          merge_unit_scalars(Mb, Lb, next.x, next.y, fa, fb);
+          merge4(Ob, *(const float4*)(s_o + (i * G + g) * HD + d4), fa, fb);
+        }
+        float Mc = -INFINITY, Lc = 0.f;               // the block's chain
+        float4 Oc = make_float4(0.f, 0.f, 0.f, 0.f);
+        merge_unit_scalars(Mc, Lc, Mb, Lb, fa, fb);
+        merge4(Oc, Ob, fa, fb);
+        if (b == u0 >> 2) {
+          M = Mc; L = Lc; O = Oc;
+        } else {
+          merge_unit_scalars(M, L, Mc, Lc, fa, fb);
+          merge4(O, Oc, fa, fb);
+        }
+      }
+      const float inv = 1.0f / L;
+      const __nv_bfloat162 x = __floats2bfloat162_rn(O.x * inv, O.y * inv), y = __floats2bfloat162_rn(O.z * inv, O.w * inv);
+      *(uint2*)(out + ((size_t)n_whole * Hq + (size_t)kvh_whole * G + g) * HD + d4) = make_uint2(*(const uint32_t*)&x, *(const uint32_t*)&y);
+    }
   }
 }
 
@@ -844,7 +915,7 @@ int launch_units(const void* q, const void* k_pool, long long pool_rows, const i
   if (ctas > (long long)sms * MINB) ctas = (long long)sms * MINB;
   fz_launch(attn_decode_units_kernel<HD, BOX, NSTAGE, MINB, SMALLG>, dim3((unsigned)ctas), dim3(THREADS), smem, stream, map,
             (const __nv_bfloat16*)q, pos, seq_row, seg, table, mb, page_size, part_o, part_ml, N, Hq, Hkv, NPU,
-            scale * 1.4426950408889634f, window, long_from, single, maps, err);
+            scale * 1.4426950408889634f, window, long_from, single, maps, err, (__nv_bfloat16*)nullptr);
   FZ_LAUNCH_CHECK();
   const bool find = !single && N > 64;
   dim3 cgrid(Hq, find ? 64 : N);
@@ -868,10 +939,41 @@ inline int units_sms() {
   }
   return sms;
 }
+// Do blocks with a (row, kv head) to themselves take the step? Contexts of at most 1,024 keys: with more a warp's third unit
+// costs what the merge kernel's launch saves. One block per SM: with more rows the kernel that shares all units out evenly.
+bool whole_rows(int N, int Hq, int Hkv, int NPU, int single) {
+  return single && Hq / Hkv <= 8 && NPU <= WHOLE_UNITS && (long long)N * Hkv <= units_sms();
+}
+
+// A block per (row, kv head); see WHOLE at the kernel.
+template <int HD, int BOX>
+int launch_whole(const CUtensorMap& map, const void* q, const int* pos, const int* seq_row, const int* seg, const int* table, int mb,
+                 int page_size, void* out, int N, int Hq, int Hkv, float scale, int window, int long_from, int* err, cudaStream_t stream) {
+  constexpr int WARPS = 8, NSTAGE = HD == 64 ? 4 : 2;      // (128 KB of rings)
+  constexpr size_t smem = 1024 + WARPS * NSTAGE * (size_t)(2 * (HD / 64) * 16 * 128) + WARPS * NSTAGE * 8 + 16 + WHOLE_UNITS * 8 * 8 + (size_t)WHOLE_UNITS * 8 * HD * 4;
+  auto kern = attn_decode_units_kernel<HD, BOX, NSTAGE, 1, true, WARPS, true>;
+  static bool raised = false;
+  if (!raised) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    raised = true;
+  }
+  fz_launch(kern, dim3((unsigned)(N * Hkv)), dim3(32 * WARPS), smem, stream, map, (const __nv_bfloat16*)q, pos, seq_row, seg, table, mb,
+            page_size, (float*)nullptr, (float*)nullptr, N, Hq, Hkv, 0, scale * 1.4426950408889634f, window, long_from, 1, 1, err, (__nv_bfloat16*)out);
+  FZ_LAUNCH_CHECK();
+  return FZ_OK;
+}
+
 template <int HD, int BOX>
 int launch_tma(const void* q, const void* k_pool, long long pool_rows, const int* pos, const int* seq_row, const int* seg,
                const int* table, int mb, int page_size, void* out, float* part_o, float* part_ml, int N, int Hq, int Hkv,
                float scale, int window, int NPU, int long_from, int single, int maps, float* out32, int* err, cudaStream_t stream) {
+  if (whole_rows(N, Hq, Hkv, NPU, single) && maps == 1 && out32 == nullptr) {
+    CUtensorMap map;
+    const int st = fztma::get_map_bf16(k_pool, pool_rows, HD, BOX, &map);
+    if (st != FZ_OK) return st;
+    return launch_whole<HD, BOX>(map, q, pos, seq_row, seg, table, mb, page_size, out, N, Hq, Hkv, scale, window, long_from, err, stream);
+  }
 #define FZ_U(NS_, MB_, SG_) return launch_units<HD, BOX, NS_, MB_, SG_>(q, k_pool, pool_rows, pos, seq_row, seg, table, mb, page_size, out, part_o, part_ml, N, Hq, Hkv, scale, window, NPU, long_from, single, maps, out32, err, stream)
   // three stages of 16 keys per warp and two CTAs per SM (eight warps with 24 KB in flight each) measured best
   if (Hq / Hkv > 8) FZ_U(3, 2, false);
@@ -920,6 +1022,11 @@ FZ_API int fz_attn_decode_check(int Hq, int Hkv, int hd) {
 // Partial results per (row, head) the scratch must hold for contexts up to max_context: the units of the key axis
 // (never fewer than the 256-key partitions of the cp.async variant).
 FZ_API int fz_attn_partitions(int max_context) { return max_context <= 0 ? 1 : unit_of(max_context - 1) + 1; }
+
+// 1 if a step of single tokens runs without the merge kernel (for pages and pools that the TMA variant takes).
+FZ_API int fz_attn_decode_whole(int N, int Hq, int Hkv, int max_context, int single_tokens) {
+  return whole_rows(N, Hq, Hkv, fz_attn_partitions(max_context), single_tokens) ? 1 : 0;
+}
 
 // Float32 scratch the call needs: part_o N * Hq * NP * hd floats, part_ml N * Hq * NP * 2 floats.
 // maps 2: see the head of this file; out is not written, out32 (N * Hq * hd floats) is. maps 1: out32 null, or where the results

@@ -644,7 +644,10 @@ class CudaOps(Ops):
                     c_int(LONG_PORTION), c_int(1 if plan.single_tokens else 0), c_int(k.shape[0]), c_int(1), c_void_p(0), _p(self.err),
                     self._stream()),
                     "paged_attention (decode)", kv)
-                self.launches += 1    # the combine kernel
+                tma = cache.page_size == 8 or cache.page_size % 16 == 0
+                if not (tma and self.attn_tc.fz_attn_decode_whole(c_int(n), c_int(hq), c_int(hkv), c_int(meta.max_context),
+                                                                  c_int(1 if plan.single_tokens else 0))):
+                    self.launches += 1    # the combine kernel
             if plan.n_tiles > 0 and self.prefill_tcgen05 and \
                     self.attn_tc.fz_attn_prefill_tc_check(c_int(hq), c_int(hkv), c_int(hd), c_int(cache.page_size)) == 0:
                 # rows of long portions on the tcgen05 flash-attention kernel; the pieces of tiles that the plan cut along

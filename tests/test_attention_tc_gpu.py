@@ -213,3 +213,41 @@ def test_short_rows_beside_hundreds_of_prompt_rows(Hq, Hkv, hd):
     o, op, seq_row = run_both(Hq, Hkv, hd, 16, 0, lengths, rows)
     close(o, op, "short rows beside portions")
     assert float(o[torch.tensor(seq_row) < 0].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("Hq,Hkv,hd,bs,window", [(14, 2, 64, 16, 0), (8, 8, 64, 8, 0), (8, 2, 128, 16, 0), (16, 2, 128, 8, 300), (4, 4, 128, 16, 64), (7, 1, 64, 32, 500)])
+def test_short_contexts_without_the_merge_kernel(Hq, Hkv, hd, bs, window):
+    """Steps of few single tokens with contexts of at most 1,024 keys: a block has a row and kv head to itself and merges the
+    units' results itself. The same bits as the kernels that other steps run, at every number of units, padding included."""
+    from fusezap_core_b200.kernels import cuda_ops
+    cu, pl = cuda_ops("bfloat16"), PlainOps(BF)
+    g = torch.Generator().manual_seed(hd + window)
+    lengths = [1024, 1, 64, 65, 256, 257, 300, 513, 960, 1000]
+    mb = -(-1100 // bs)
+    table = [list(range(r * mb, (r + 1) * mb)) for r in range(len(lengths))]
+    cp = make_cache(len(lengths) * mb, Hkv, bs, hd, BF, "cpu")
+    fill_cache(cp, table, lengths, g)
+    cc = make_cache(len(lengths) * mb, Hkv, bs, hd, BF, "cuda")
+    cc.pool.copy_(cp.pool)
+    q = torch.randn(len(lengths) + 1, Hq * hd, generator=g).to(BF)
+    pos, seq = [n - 1 for n in lengths] + [0], list(range(len(lengths))) + [-1]
+
+    def attend(index, max_context):
+        meta = Meta([pos[i] for i in index], [seq[i] for i in index], table, "cuda")
+        meta.max_context = max_context
+        out = torch.full((len(index), Hq * hd), float("nan"), dtype=BF, device="cuda")
+        cu.paged_attention(q[index].cuda(), cc, meta, out, Hq, Hkv, hd, hd ** -0.5, window)
+        return out
+
+    every = list(range(len(lengths) + 1))
+    assert cu.attn_tc.fz_attn_decode_whole(len(every), Hq, Hkv, 1024, 1) == 1
+    assert cu.attn_tc.fz_attn_decode_whole(len(every), Hq, Hkv, 1025, 1) == 0
+    whole, shared = attend(every, 1024), attend(every, 1100)
+    assert torch.equal(whole, shared)
+    for i in every[:-1]:
+        assert torch.equal(attend([i], 1024)[0], shared[i])
+    ref = torch.empty(len(every), Hq * hd, dtype=BF)
+    pl.paged_attention(q, cp, Meta(pos, seq, table, "cpu"), ref, Hq, Hkv, hd, hd ** -0.5, window)
+    close(whole.float().cpu(), ref.float(), "short contexts")
+    assert float(whole[-1].float().abs().max()) == 0.0
+    cu.check_errors()
