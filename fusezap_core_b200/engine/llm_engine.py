@@ -74,23 +74,19 @@ class LLMEngine:
         self._next_id, self._clock = itertools.count(), itertools.count()
         pin = dev.type == "cuda"
         # per-step sampling inputs and outputs: pinned on the host, fixed buffers on the device
-        # (two of each host buffer: a step may be launched while the one before it is still in flight)
-        self._temp_h = torch.zeros(2, R, dtype=torch.float32, pin_memory=pin)
-        self._unif_h = torch.zeros(2, R, dtype=torch.float64, pin_memory=pin)
-        self._topk_h = torch.zeros(2, R, dtype=torch.int32, pin_memory=pin)
-        self._topp_h = torch.ones(2, R, dtype=torch.float32, pin_memory=pin)
-        # (numpy views of the same pinned memory: writing an element of a tensor costs microseconds, of an array not)
-        self._sampling_np = tuple(t.numpy() for t in (self._temp_h, self._unif_h, self._topk_h, self._topp_h))
+        # (two of each host buffer: a step may be launched while the one before it is still in flight). The inputs lie one
+        # after the other in one buffer, so that a step brings them up in one copy: [uniform | temperature | top_k | top_p].
+        self._sampling_h = torch.zeros(2, (20 * R + 15) // 16 * 16, dtype=torch.uint8, pin_memory=pin)
+        self._sampling_d = torch.zeros(self._sampling_h.shape[1], dtype=torch.uint8, device=dev)
+        # (numpy views of the pinned memory: writing an element of a tensor costs microseconds, of an array not)
+        self._sampling_np = [[v.numpy() for v in _sampling_views(h, R)] for h in self._sampling_h]
         self._ids_h = torch.zeros(2, R, dtype=torch.int32, pin_memory=pin)
         self._events = [torch.cuda.Event() for _ in range(2)] if pin else None
         self._slot = 0
         self._pending: _Launched | None = None
         self.profile = bool(cfg.profile) and pin and hasattr(model.ops, "start_profile")
         self.lookahead = bool(cfg.lookahead) and not self.profile
-        self._temp_d = torch.zeros(R, dtype=torch.float32, device=dev)
-        self._unif_d = torch.zeros(R, dtype=torch.float64, device=dev)
-        self._topk_d = torch.zeros(R, dtype=torch.int32, device=dev)
-        self._topp_d = torch.ones(R, dtype=torch.float32, device=dev)
+        self._unif_d, self._temp_d, self._topk_d, self._topp_d = _sampling_views(self._sampling_d, R)
         self._ids_d = torch.zeros(R, dtype=torch.int32, device=dev)
         self.runner.prev_ids = self._ids_d
         self.cuda_graphs = bool(cfg.cuda_graphs) and pin and model.graph_safe() and not self.profile
@@ -279,11 +275,10 @@ class LLMEngine:
         ids and the error word down. Does not wait for it."""
         runner, ops, st = self.runner, self.ops, self.stats
         slot = self._slot = (self._slot + 1) % 2
-        temp_h, unif_h, topk_h, topp_h = self._temp_h[slot], self._unif_h[slot], self._topk_h[slot], self._topp_h[slot]
         R = len(rows)
         filtered = False
-        temp_a, unif_a, topk_a, topp_a = (a[slot] for a in self._sampling_np)
-        temp_a[:R], unif_a[:R], topk_a[:R], topp_a[:R] = 0.0, 0.0, 0, 1.0      # greedy rows and rows sampled on the host
+        unif_a, temp_a, topk_a, topp_a = self._sampling_np[slot]
+        unif_a[:], temp_a[:], topk_a[:], topp_a[:] = 0.0, 0.0, 0, 1.0      # greedy rows, rows sampled on the host, padding
         for req, i in rows:
             p = req.params
             if p.on_device and not p.greedy:
@@ -317,16 +312,10 @@ class LLMEngine:
                 key = sig
                 m.max_context = covered
         n_w = runner.meta.n_wanted
-        if n_w:
-            temp_h[R:n_w] = 0.0
-            self._temp_d[:n_w].copy_(temp_h[:n_w], non_blocking=True)
-            self._unif_d[:n_w].copy_(unif_h[:n_w], non_blocking=True)
-            if filtered:
-                topk_h[R:n_w] = 0
-                topp_h[R:n_w] = 1.0
-                self._topk_d[:n_w].copy_(topk_h[:n_w], non_blocking=True)
-                self._topp_d[:n_w].copy_(topp_h[:n_w], non_blocking=True)
-        st["h2d_bytes"] += runner.meta.size * 4 + n_w * (20 if filtered else 12)
+        sampled = n_w > 0 and not self._greedy_step      # (the kernel that picks the largest logit reads none of them)
+        if sampled:
+            self._sampling_d.copy_(self._sampling_h[slot], non_blocking=True)
+        st["h2d_bytes"] += runner.meta.size * 4 + (self._sampling_d.shape[0] if sampled else 0)
         if key is not None:
             g = self._graphs.get(key)
             if g is None:
@@ -429,6 +418,12 @@ class LLMEngine:
         if not self.profile:
             raise RuntimeError("the engine was made without profile=True")
         return self.ops.profile_report()
+
+
+def _sampling_views(buffer: torch.Tensor, rows: int) -> tuple[torch.Tensor, ...]:
+    """A step's sampling inputs within their buffer of bytes: uniform (float64), temperature, top_k (int32), top_p."""
+    return (buffer[:8 * rows].view(torch.float64), buffer[8 * rows: 12 * rows].view(torch.float32),
+            buffer[12 * rows: 16 * rows].view(torch.int32), buffer[16 * rows: 20 * rows].view(torch.float32))
 
 
 def _config_from(config: EngineConfig | None, dtype, device, max_model_len, options: dict) -> EngineConfig:
