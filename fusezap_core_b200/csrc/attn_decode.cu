@@ -939,10 +939,14 @@ inline int units_sms() {
   }
   return sms;
 }
-// Do blocks with a (row, kv head) to themselves take the step? Contexts of at most 1,024 keys: with more a warp's third unit
-// costs what the merge kernel's launch saves. One block per SM: with more rows the kernel that shares all units out evenly.
+// Do blocks with a (row, kv head) to themselves take the step? Up to 512 keys, a unit per warp, always (a decode step at
+// Llama-3.1-8B sizes, 1 and 4 rows of 512 keys: 2,978 -> 2,918 us, 3,116 -> 2,956; at Qwen2.5-0.5B sizes 761 -> 683, 809 ->
+// 712). Up to 1,024 keys a warp has two units, which with few rows costs more than the merge kernel's launch (1 row of 600
+// keys: 2,970 -> 3,028 us, 754 -> 766; 4 rows: 3,107 -> 3,069, 808 -> 790; 16 rows of 1,024: 3,552 -> 3,346). Beyond, four units
+// a warp, most sizes lose (8 rows of 2,048: 3,440 -> 3,486). One block per SM: with more rows the kernel that shares all
+// units out evenly.
 bool whole_rows(int N, int Hq, int Hkv, int NPU, int single) {
-  return single && Hq / Hkv <= 8 && NPU <= WHOLE_UNITS && (long long)N * Hkv <= units_sms();
+  return single && Hq / Hkv <= 8 && NPU <= WHOLE_UNITS && (NPU <= WHOLE_UNITS / 2 || N >= 4) && (long long)N * Hkv <= units_sms();
 }
 
 // A block per (row, kv head); see WHOLE at the kernel.

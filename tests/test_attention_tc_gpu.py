@@ -244,8 +244,10 @@ def test_short_contexts_without_the_merge_kernel(Hq, Hkv, hd, bs, window):
     assert cu.attn_tc.fz_attn_decode_whole(len(every), Hq, Hkv, 1025, 1) == 0
     whole, shared = attend(every, 1024), attend(every, 1100)
     assert torch.equal(whole, shared)
+    assert [cu.attn_tc.fz_attn_decode_whole(n, Hq, Hkv, c, 1) for n, c in ((1, 512), (1, 513), (3, 1024), (4, 1024))] == [1, 0, 0, 1]
     for i in every[:-1]:
-        assert torch.equal(attend([i], 1024)[0], shared[i])
+        assert torch.equal(attend([i], 512 if lengths[i] <= 512 else 1024)[0], shared[i])
+    assert torch.equal(attend(every[1:7], 512), shared[1:7])
     ref = torch.empty(len(every), Hq * hd, dtype=BF)
     pl.paged_attention(q, cp, Meta(pos, seq, table, "cpu"), ref, Hq, Hkv, hd, hd ** -0.5, window)
     close(whole.float().cpu(), ref.float(), "short contexts")
