@@ -62,16 +62,17 @@ __device__ __forceinline__ void fma4(float& acc, float4 a, float4 w) {
 }
 
 // ---- few rows
-// A block owns 8 * RPL columns (rows of W) and all of K: warp w has chunks 4w .. 4w+3, eight lanes to a chunk, RPL columns
-// to a lane, MR rows of A to each. So N * 32 / RPL chains run at once, and a warp waits for no other until the end: it
-// streams its own 16 k of every (column, chunk) per stage through a ring of its own, 64 contiguous bytes each, whose 16-byte
-// pieces stand in an order that changes every two rows (conflict-free reads without padding, so that three blocks share an
-// SM at K = 896). Where the columns give every SM at most one block (DEEP) the ring takes all of its memory. The first stages of W, which no kernel of a step writes, are asked for ahead
-// of the wait on the kernel before. Blocks that stay and walk several tiles with the ring running on measured slower at
-// large N (896 -> 151,936 at 8 rows: 211 against 156 us): waiting at each tile's end for the slowest warp costs more than
-// a new block. Measured at 4 rows, weights from HBM: 4,864 -> 896 7.1 us (rings two blocks could share: 10.1; one
-// chain of fmaf over all of K: 215), 896 -> 9,728 9.8 us (padded rows, two blocks per SM: 11.0; 75), 896 -> 151,936 113 us
-// (132; 417), 4.8 TB/s; 4,096 -> 28,672 75 us, 6.3 TB/s.
+// A block owns 8 * RPL columns (rows of W) and all of K: warp w has chunks 4w .. 4w+3, eight lanes to a chunk, RPL
+// columns to a lane, MR rows of A to each. So N * 32 / RPL chains run at once, and a warp waits for no other until the
+// end: it streams its own 16 k of every (column, chunk) per stage through a ring of its own, 64 contiguous bytes each,
+// whose 16-byte pieces stand in an order that changes every two rows (conflict-free reads without padding, so that three
+// blocks share an SM at K = 896). Where the columns give every SM at most one block (DEEP) the ring takes all of its
+// memory. The first stages of W, which no kernel of a step writes, are asked for ahead of the wait on the kernel before.
+// Blocks that stay and walk several tiles with the ring running on measured slower at large N (896 -> 151,936 at 8 rows:
+// 211 against 156 us): waiting at each tile's end for the slowest warp costs more than a new block. Measured at 4 rows,
+// weights from HBM: 4,864 -> 896 7.1 us (rings two blocks could share: 10.1; one chain of fmaf over all of K: 215), 896
+// -> 9,728 9.8 us (padded rows, two blocks per SM: 11.0; 75), 896 -> 151,936 113 us (132; 417), 4.8 TB/s; 4,096 -> 28,672
+// 75 us, 6.3 TB/s.
 constexpr int FEW_K = 16;
 template <int MR, int RPL, bool DEEP> struct Few {
   static constexpr int W_FLOATS = 32 * RPL * FEW_K, A_SUB = MR * FEW_K + 4, STAGE = W_FLOATS + 4 * A_SUB;   // per warp
@@ -183,11 +184,12 @@ gemm_simt_few_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const f
 
 // ---- more rows
 // Tiles of (8 TM) x (16 TN) outputs, 128 threads with TM x TN outputs each, 32 k per stage, three stages of asynchronous
-// copies; rows lie in shared memory as in memory, padded to 144 bytes, and are read 16 bytes (four k) at a time. With 8 x 4
-// outputs per thread 16 warps share an SM; 8 x 6 and 8 x 8 reach the same 40 TFLOP/s on large products and lose on small
-// ones (300 rows, 896 -> 9,728: 160, 174 and 208 us). A block sums one group of chunks (`acc` the chunk's chain, `tot` the group) and the blocks of a tile's groups, a cluster,
-// add their tiles up in order through distributed shared memory. Measured at 300 rows: 896 -> 9,728 265 -> 160 us, 4,864 ->
-// 896 215 -> 78 us, 896 -> 151,936 3,364 -> 2,031 us (40 TFLOP/s).
+// copies; rows lie in shared memory as in memory, padded to 144 bytes, and are read 16 bytes (four k) at a time. With 8 x
+// 4 outputs per thread 16 warps share an SM; 8 x 6 and 8 x 8 reach the same 40 TFLOP/s on large products and lose on
+// small ones (300 rows, 896 -> 9,728: 160, 174 and 208 us). A block sums one group of chunks (`acc` the chunk's chain,
+// `tot` the group) and the blocks of a tile's groups, a cluster, add their tiles up in order through distributed shared
+// memory. Measured at 300 rows: 896 -> 9,728 265 -> 160 us, 4,864 -> 896 215 -> 78 us, 896 -> 151,936 3,364 -> 2,031 us
+// (40 TFLOP/s).
 constexpr int TN = 4, TILE_CTAS = 4, TILE_N = 16 * TN, TILE_K = 32, TILE_ROW = TILE_K + 4, TILE_STAGES = 3;
 template <typename TA, typename TC, int TM, bool VEC>
 __global__ void __launch_bounds__(128, TILE_CTAS)
@@ -518,6 +520,9 @@ int launch_few_n(const void* A, const void* W, const float* bias, void* C, int M
 template <typename TA, typename TC, bool VEC>
 int launch_rows(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, cudaStream_t stream) {
   const Order o = order_of(N, K);
+  // Few rows read W at memory's pace up to 8 and still beat tiles at 16 (896 -> 9,728: 13 us at 8 rows, 26 at 16, tiles 42 at
+  // 17; 896 -> 151,936: 148, 345 and 254 us, the one size measured where tiles would win at 16). Tiles of 32 rows waste less
+  // than tiles of 64 up to 32 (43 against 62 us). Wide tiles from two blocks per SM on (see there).
   if (M <= 1) return launch_few_n<TA, TC, 1, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (M <= 2) return launch_few_n<TA, TC, 2, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (M <= 4) return launch_few_n<TA, TC, 4, VEC>(A, W, bias, C, M, N, K, o, stream);
