@@ -111,7 +111,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const float* __restric
   }
 }
 
-// The same for D % 4 == 0 and D <= 4 * 512 * VPT: 512 threads, a thread keeps its VPT float4 groups of the row in
+// The same for D % 4 == 0 and D <= 4 * 512 * VPT: up to 512 threads, a thread keeps its VPT float4 groups of the row in
 // registers (all loads are issued before anything depends on them), so the row is read once.
 __device__ __forceinline__ float4 load4f(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ float4 load4f(const __nv_bfloat16* p) {
@@ -126,8 +126,8 @@ __device__ __forceinline__ void store4f(__nv_bfloat16* d, float a, float b, floa
 }
 
 // Rows of up to 2,048 values take as many threads as they have float4 (a multiple of 32) instead of 512, most of them idle:
-// a step of 2,101 prompt rows of 896, 49 norms, 3.228 -> 3.132 ms; steps of 1 and 32 rows unchanged. The block's size depends
-// on D alone, and so does the order of the sum.
+// a step of 2,101 prompt rows of 896, 49 norms, 3.228 -> 3.132 ms; steps of 1 and 32 rows unchanged. (Longer rows, VPT above 1,
+// have 512.) The block's size depends on D alone, and so does the order of the sum.
 template <typename TW, typename TH, int VPT, bool EARLY>
 __global__ void __launch_bounds__(512)
 add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, const TW* __restrict__ w,
@@ -144,7 +144,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, c
   if constexpr (EARLY) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * blockDim.x;
+      const int c = threadIdx.x + i * 512;
       g[i] = c < D4 ? load4f(w + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (rows != nullptr) src = rows[r];
@@ -166,14 +166,14 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, c
   float4 v[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int c = threadIdx.x + i * blockDim.x;
+    const int c = threadIdx.x + i * 512;
     v[i] = c < D4 ? xr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (dr) {
     float4 dv[VPT];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * blockDim.x;
+      const int c = threadIdx.x + i * 512;
       dv[i] = c < D4 ? dr[c] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
@@ -187,7 +187,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, c
   if (write_x) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int c = threadIdx.x + i * blockDim.x;
+      const int c = threadIdx.x + i * 512;
       if (c < D4) xr[c] = v[i];
     }
   }
@@ -195,7 +195,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ delta, c
   const float scale = 1.0f / sqrtf(ss * (1.0f / (float)D) + eps);
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int c = threadIdx.x + i * blockDim.x;
+    const int c = threadIdx.x + i * 512;
     if (c < D4) {
       const int d = c * 4;
       if constexpr (EARLY) {
@@ -963,8 +963,8 @@ FZ_API int fz_sample(const float* logits, const float* temperature, const double
 // everything not below the k-th largest value (ties stay); top-p keeps, in falling order of value (ties by rising
 // index), every token before which less than p of the probability lies; then one draw from the softmax of what is left:
 // the first index whose running sum in index order exceeds u times the total. A cluster of SF_CLUSTER blocks of 1024
-// threads per row, a block for each SF_CLUSTER-th of its tokens (one block for short rows, SF_SHORT and less): bound by the instructions per
-// token and pass, so the blocks' number is what counts (8 rows of 151,936 with top-p, from the difference of whole steps:
+// threads per row, a block for each SF_CLUSTER-th of its tokens (one block for rows of SF_SHORT tokens and less: the passes
+// over such a row cost less than the barriers between blocks; not measured in between): bound by the instructions per token and pass, so the blocks' number is what counts (8 rows of 151,936 with top-p, from the difference of whole steps:
 // 340 -> 70 us; 24 sampled tokens of 8 requests at Qwen2.5-0.5B sizes 32.2 -> 25.6 ms). The blocks add their bins and sums up through distributed shared memory in rank order; all then take the same decisions.
 // Nothing is sorted: the thresholds are found by radix selection over an order-preserving 32-bit key of the logit,
 // eight passes of 4 bits, with a histogram of counts for top-k and of probability mass (float64) for top-p. Each thread
@@ -1204,8 +1204,8 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
     need_at_t = s_need;
   }
   // ---- the draw. Warp w owns the contiguous range [w * span, (w + 1) * span) of its block's slice and walks it 32 tokens
-  // at a time, so that sums run in index order. Equal values at the threshold: the j-th of them in index order (j = 0, 1, ...) stays while
-  // j * e < need_at_t.
+  // at a time, so that sums run in index order. Equal values at the threshold: the j-th of them in index order (j = 0, 1,
+  // ...) stays while j * e < need_at_t.
   const int span = ((slice + 1023) / 1024) * 32;
   const int w_lo = min(hi, lo + warp * span), w_hi = min(hi, w_lo + span);
   if (nucleus) {
