@@ -61,7 +61,7 @@ __device__ __forceinline__ int span_length(int chunks) {
 struct Args {
   const int *pos, *seq_row, *table;
   long long page_stride;
-  int mb, page_size, N, Hq, Hkv, hd, hdp, G_all, GS, rows, window, buffers;
+  int mb, page_size, N, Hq, Hkv, hd, hdp, G_all, GS, slices, rows, window, buffers;
   float scale;
   int* err;
 };
@@ -78,8 +78,9 @@ attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T*
   fz_grid_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
   const int hd = A.hd, hdp = A.hdp, ks = hdp + PAD;
-  const int kvh = blockIdx.y % A.Hkv, g_base = (blockIdx.y / A.Hkv) * A.GS, G = min(A.GS, A.G_all - g_base);
-  const int first = blockIdx.x * A.rows, rows = min(A.rows, A.N - first);
+  // (a kv head's query heads beyond GS are another block's: slices along x, which has room for them beside any number of heads)
+  const int kvh = blockIdx.y, g_base = (blockIdx.x % A.slices) * A.GS, G = min(A.GS, A.G_all - g_base);
+  const int first = blockIdx.x / A.slices * A.rows, rows = min(A.rows, A.N - first);
   const int head0 = kvh * A.G_all + g_base;
   // shared memory: per buffer keys [32][hdp + PAD] and values [32][hdp], then queries [pair][hdp] and weights [warp][PW][32] in float32
   T* kv = reinterpret_cast<T*>(attn_smem);
@@ -392,7 +393,7 @@ attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T*
 }
 
 template <typename T, int DPL, int PW, bool VEC, bool SPLIT>
-int launch(const void* q, const void* k_pool, const void* v_pool, void* out, Args A, int slices, cudaStream_t stream) {
+int launch(const void* q, const void* k_pool, const void* v_pool, void* out, Args A, cudaStream_t stream) {
   const int G = A.G_all < A.GS ? A.G_all : A.GS, pairs = A.rows * G;
   const int W = pairs < MAX_WARPS ? pairs : MAX_WARPS;
   const size_t kv = sizeof(T) * (size_t)CHUNK * (2 * A.hdp + 16 / sizeof(T)), rest = sizeof(float) * ((size_t)pairs * A.hdp + (size_t)W * PW * CHUNK);
@@ -413,7 +414,9 @@ int launch(const void* q, const void* k_pool, const void* v_pool, void* out, Arg
     allowed = smem;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((A.N + A.rows - 1) / A.rows, A.Hkv * slices, SPLIT ? SPANS : 1);
+  const long long along_x = (long long)((A.N + A.rows - 1) / A.rows) * A.slices;
+  if (along_x > 2147483647LL) return FZ_TOO_LARGE;
+  cfg.gridDim = dim3((unsigned)along_x, A.Hkv, SPLIT ? SPANS : 1);
   cfg.blockDim = dim3(32 * W);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -439,21 +442,20 @@ template <typename T, int DPL, bool VEC>
 int choose(const void* q, const void* k_pool, const void* v_pool, void* out, Args A, int max_context, cudaStream_t stream) {
   constexpr int PAIRS = MAX_WARPS * Pairs<DPL>::PER_WARP;
   A.GS = A.G_all < PAIRS ? A.G_all : PAIRS;
-  const int slices = (A.G_all + A.GS - 1) / A.GS;
-  if ((long long)A.Hkv * slices > 65535) return FZ_BAD_SHAPE;
-  const long long blocks = (long long)A.N * A.Hkv * slices;
+  A.slices = (A.G_all + A.GS - 1) / A.GS;
+  const long long blocks = (long long)A.N * A.Hkv * A.slices;
   // Spans of a row side by side: where rows, heads and slices alone are at most two blocks per SM, and rows may be long
   // enough to have more than one span. (At 296 blocks of one span each the spans' blocks, eight times as many, still
   // start within two rounds; beyond, sharing keys among rows gains more.)
   A.rows = 1;
   if (blocks <= 296 && max_context > SPAN_CHUNKS * CHUNK) {
-    if (A.GS <= MAX_WARPS) return launch<T, DPL, 1, VEC, true>(q, k_pool, v_pool, out, A, slices, stream);
-    return launch<T, DPL, PAIRS / MAX_WARPS, VEC, true>(q, k_pool, v_pool, out, A, slices, stream);
+    if (A.GS <= MAX_WARPS) return launch<T, DPL, 1, VEC, true>(q, k_pool, v_pool, out, A, stream);
+    return launch<T, DPL, PAIRS / MAX_WARPS, VEC, true>(q, k_pool, v_pool, out, A, stream);
   }
   // Rows that share the keys of a block: as many as give it PAIRS pairs, while every SM keeps a block.
   A.rows = PAIRS / A.GS < MAX_ROWS ? PAIRS / A.GS : MAX_ROWS;
   while (A.rows > 1 && (blocks + A.rows - 1) / A.rows < 148) A.rows /= 2;
-  return launch<T, DPL, PAIRS / MAX_WARPS, VEC, false>(q, k_pool, v_pool, out, A, slices, stream);
+  return launch<T, DPL, PAIRS / MAX_WARPS, VEC, false>(q, k_pool, v_pool, out, A, stream);
 }
 
 template <typename T>

@@ -106,3 +106,24 @@ def test_attention_bits_do_not_depend_on_who_computes_them(Hq, Hkv, hd, bs, wind
     attend(list(range(len(rows))), whole, spoiled)
     assert torch.equal(whole[:50], many[:50]) and torch.equal(whole[300:], many[300:])
     cu.check_errors()
+
+
+def test_attention_with_more_heads_and_slices_than_a_grid_is_high():
+    """33,000 kv heads of nine query heads at a head size where a block takes eight: two slices of each kv head, 66,000 in
+    all, more than the 65,535 blocks that a grid's second dimension holds."""
+    from fusezap_core_b200.kernels import cuda_ops
+    cu = cuda_ops("bfloat16")
+    Hkv, G, hd, bs = 33000, 9, 264, 4
+    g = torch.Generator(device="cuda").manual_seed(1)
+    cache = make_cache(1, Hkv, bs, hd, torch.bfloat16, "cuda")
+    cache.pool.normal_(generator=g)
+    q = torch.randn(2, Hkv * G * hd, generator=g, device="cuda").bfloat16()
+    out = torch.empty_like(q)
+    cu.paged_attention(q, cache, Meta([0, 2], [0, 0], [[0]], "cuda"), out, Hkv * G, Hkv, hd, hd ** -0.5, 0)
+    cu.check_errors()
+    # the first row sees one key, whose value it returns; the second one's softmax has three
+    assert torch.equal(out[0].view(Hkv, G, hd), cache.values[0, :, 0][:, None].expand(Hkv, G, hd))
+    s = torch.einsum("hgd,hkd->hgk", q[1].view(Hkv, G, hd).float(), cache.keys[0, :, :3].float()) * hd ** -0.5
+    ref = torch.einsum("hgk,hkd->hgd", s.softmax(-1), cache.values[0, :, :3].float())
+    # half a bfloat16 step of the result, and the 32-bit sums
+    assert bool(((out[1].view(Hkv, G, hd).float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
