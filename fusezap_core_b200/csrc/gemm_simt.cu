@@ -439,14 +439,15 @@ gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const 
   }
 }
 
-// Raises a kernel's shared-memory limit where it needs more than the default (once per instantiation and size, outside
-// any capture: a step is run once before it is captured).
-template <typename K> cudaError_t allow_smem(K kern, size_t smem, size_t& allowed) {
-  if (smem <= allowed) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) allowed = smem;
-  return e;
-}
+// All the shared memory a block may have, as the limit of a kernel whose need differs from call to call: set once per
+// instantiation. (A limit raised step by step to each call's need can be lowered again by another thread's smaller call
+// between the check and the launch.)
+constexpr int MOST_SMEM = 227 * 1024;
+#define FZ_RAISE_SMEM(kern)                                                                                                  \
+  do {                                                                                                                       \
+    static const cudaError_t raised__ = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SMEM);  \
+    if (raised__ != cudaSuccess) return (int)raised__;                                                                       \
+  } while (0)
 
 template <typename TA, typename TC, int MR, int RPL, bool VEC, bool DEEP>
 int launch_few(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
@@ -455,9 +456,7 @@ int launch_few(const void* A, const void* W, const float* bias, void* C, int M, 
   const size_t ring = sizeof(float) * (size_t)warps * slots * F::STAGE, sums = sizeof(float) * (size_t)o.chunks * MR * 8 * RPL;
   const size_t smem = ring > sums ? ring : sums;
   auto kern = gemm_simt_few_kernel<TA, TC, MR, RPL, VEC, DEEP>;
-  static size_t allowed = 48 * 1024;
-  const cudaError_t e = allow_smem(kern, smem, allowed);
-  if (e != cudaSuccess) return (int)e;
+  FZ_RAISE_SMEM(kern);
   fz_launch(kern, dim3((N + 8 * RPL - 1) / (8 * RPL)), dim3(32 * warps), smem, stream, (const TA*)A, (const TA*)W, bias, (TC*)C, M, N, K, o, slots);
   FZ_LAUNCH_CHECK();
   return FZ_OK;
@@ -472,9 +471,7 @@ int launch_tile(const void* A, const void* W, const float* bias, void* C, int M,
   size_t smem = sizeof(float) * TILE_STAGES * (size_t)(8 * TM + TILE_N) * TILE_ROW;
   if (per_sm < TILE_CTAS && smem < 220 * 1024 / per_sm) smem = 220 * 1024 / per_sm / 1024 * 1024;
   auto kern = gemm_simt_tile_kernel<TA, TC, TM, VEC>;
-  static size_t allowed = 48 * 1024;
-  const cudaError_t e = allow_smem(kern, smem, allowed);
-  if (e != cudaSuccess) return (int)e;
+  FZ_RAISE_SMEM(kern);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)tiles, 1, o.groups);
   cfg.blockDim = dim3(128);

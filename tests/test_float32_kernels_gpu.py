@@ -3,6 +3,10 @@ chunk of k and many, one group of chunks and eight, a row's keys in one span and
 after the other. Every result against 64-bit arithmetic within a bound from the order of the sums, and the same bits
 whoever computes it."""
 
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -49,6 +53,41 @@ def test_linear(N, K):
     out = torch.empty(20, N, device="cuda")
     cu.linear(bad, w, bias, out)
     assert torch.equal(out[:3], full[:3]) and torch.equal(out[4:], full[4:20]) and not bool(out[3].isfinite().any())
+
+
+def test_linear_from_two_threads():
+    """Products whose blocks need different amounts of shared memory, first called by two threads at once in a process that
+    has launched none of them (the limit of a kernel's shared memory is set at its first call)."""
+    code = """
+import threading, torch
+from fusezap_core_b200.kernels.table import CudaOps
+from test_float32_kernels_gpu import thread_sizes
+torch.zeros(1, device="cuda")
+meet, bad = threading.Barrier(2), []
+def work(order):
+    ops = CudaOps("float32", "cuda:0")
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for m, n, k in order:
+            a, w, out = torch.ones(m, k, device="cuda"), torch.ones(n, k, device="cuda"), torch.empty(m, n, device="cuda")
+            meet.wait(60)
+            ops.linear(a, w, None, out)
+            if not bool((out == k).all()): bad.append((m, n, k))
+def guarded(order):
+    try: work(order)
+    except BaseException as e:
+        bad.append(repr(e)); meet.abort()
+sizes = thread_sizes()
+threads = [threading.Thread(target=guarded, args=(o,)) for o in (sizes, sizes[::-1])]
+for t in threads: t.start()
+for t in threads: t.join()
+assert not bad, bad
+"""
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join(p for p in sys.path if p))
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
+
+
+def thread_sizes():
+    return [(m, n, k) for m in (1, 3, 8, 16, 32, 64) for n, k in ((64, 64), (896, 896), (896, 4864), (9728, 896))]
 
 
 @pytest.mark.parametrize("Hq,Hkv,hd,bs,window", [(14, 2, 64, 16, 0), (3, 1, 32, 4, 0), (8, 8, 128, 8, 0), (40, 1, 48, 16, 0), (4, 2, 64, 16, 300),
