@@ -971,8 +971,9 @@ int launch_whole(const CUtensorMap& map, const void* q, const int* pos, const in
 template <int HD, int BOX>
 int launch_tma(const void* q, const void* k_pool, long long pool_rows, const int* pos, const int* seq_row, const int* seg,
                const int* table, int mb, int page_size, void* out, float* part_o, float* part_ml, int N, int Hq, int Hkv,
-               float scale, int window, int NPU, int long_from, int single, int maps, float* out32, int* err, cudaStream_t stream) {
+               float scale, int window, int NPU, int long_from, int single, int maps, float* out32, int* kernels, int* err, cudaStream_t stream) {
   if (whole_rows(N, Hq, Hkv, NPU, single) && maps == 1 && out32 == nullptr) {
+    *kernels = 1;
     CUtensorMap map;
     const int st = fztma::get_map_bf16(k_pool, pool_rows, HD, BOX, &map);
     if (st != FZ_OK) return st;
@@ -1027,7 +1028,7 @@ FZ_API int fz_attn_decode_check(int Hq, int Hkv, int hd) {
 // (never fewer than the 256-key partitions of the cp.async variant).
 FZ_API int fz_attn_partitions(int max_context) { return max_context <= 0 ? 1 : unit_of(max_context - 1) + 1; }
 
-// 1 if a step of single tokens runs without the merge kernel (for pages and pools that the TMA variant takes).
+// 1 if a step of single tokens runs without the merge kernel, for pages and pools that the TMA variant takes.
 FZ_API int fz_attn_decode_whole(int N, int Hq, int Hkv, int max_context, int single_tokens) {
   return whole_rows(N, Hq, Hkv, fz_attn_partitions(max_context), single_tokens) ? 1 : 0;
 }
@@ -1036,14 +1037,17 @@ FZ_API int fz_attn_decode_whole(int N, int Hq, int Hkv, int max_context, int sin
 // maps 2: see the head of this file; out is not written, out32 (N * Hq * hd floats) is. maps 1: out32 null, or where the results
 // go as float32 instead of out.
 // single_tokens != 0: every portion of the step is one token (the caller knows; the kernel then reads no portion records).
+// kernels: on the host, how many kernels the call launched.
 // num_pages > 0 and a pool laid out as (pages, 2, Hkv, page_size, hd) with v_pool = k_pool + Hkv * page_size * hd select
 // the TMA variant where the page size allows it (8, 16 or a multiple of 16); otherwise the cp.async variant runs.
 FZ_API int fz_attn_decode(const void* q, const void* k_pool, const void* v_pool, const int* pos, const int* seq_row,
                           const int* seg, const int* table, int mb, long long page_stride, int page_size, void* out,
                           float* part_o, float* part_ml, int N, int Hq, int Hkv, int hd, float scale, int window,
-                          int max_context, int long_from, int single_tokens, int num_pages, int maps, float* out32, int* err,
-                          cudaStream_t stream) {
+                          int max_context, int long_from, int single_tokens, int num_pages, int maps, float* out32, int* kernels,
+                          int* err, cudaStream_t stream) {
+  *kernels = 0;
   if (N <= 0) return FZ_OK;
+  *kernels = 2;      // the units and their merge, unless launch_tma below finds that one does both
   if ((maps != 1 && maps != 2) || (maps == 2 && (out32 == nullptr || (Hq / Hkv) % 2))) return FZ_BAD_SHAPE;
   const int single = single_tokens ? 1 : 0;
   if (fz_attn_decode_check(Hq, Hkv, hd) != FZ_OK || page_size <= 0) return FZ_BAD_SHAPE;
@@ -1057,7 +1061,7 @@ FZ_API int fz_attn_decode(const void* q, const void* k_pool, const void* v_pool,
                       (long long)N * Hkv * NPU < (1LL << 30) && (size_t)NPU * 8 < 40 * 1024 && !getenv("FZB200_NO_TMA_ATTN");
   if (tma_ok) {
     const long long pool_rows = (long long)num_pages * 2 * Hkv * page_size;
-#define FZ_T(HD_, BOX_) return launch_tma<HD_, BOX_>(q, k_pool, pool_rows, pos, seq_row, seg, table, mb, page_size, out, part_o, part_ml, N, Hq, Hkv, scale, window, NPU, long_from, single, maps, out32, err, stream)
+#define FZ_T(HD_, BOX_) return launch_tma<HD_, BOX_>(q, k_pool, pool_rows, pos, seq_row, seg, table, mb, page_size, out, part_o, part_ml, N, Hq, Hkv, scale, window, NPU, long_from, single, maps, out32, kernels, err, stream)
     if (hd == 64 && page_size == 8) FZ_T(64, 8);
     if (hd == 64) FZ_T(64, 16);
     if (page_size == 8) FZ_T(128, 8);

@@ -7,7 +7,7 @@ without a page) set a bit in a device error word instead of faulting; `check_err
 """
 from __future__ import annotations
 import ctypes
-from ctypes import c_int, c_void_p, c_float, c_longlong
+from ctypes import byref, c_int, c_void_p, c_float, c_longlong
 
 import torch
 
@@ -637,17 +637,15 @@ class CudaOps(Ops):
                 need = n * hq * parts * (hd + 2)
                 part_o = self._scratch("attention partials", need, torch.float32)
                 part_ml = part_o[n * hq * parts * hd:]
+                kernels = c_int(0)      # (one or two: the C side decides)
                 self._check(self.attn_tc.fz_attn_decode(
                     _p(q), _p(k), _p(v), _p(meta.pos), _p(meta.seq_row), _p(meta.seg), _p(table), c_int(table.shape[1]),
                     c_longlong(page_stride), c_int(cache.page_size), _p(out), _p(part_o), _p(part_ml), c_int(n),
                     c_int(hq), c_int(hkv), c_int(hd), c_float(scale), c_int(window), c_int(meta.max_context),
-                    c_int(LONG_PORTION), c_int(1 if plan.single_tokens else 0), c_int(k.shape[0]), c_int(1), c_void_p(0), _p(self.err),
-                    self._stream()),
+                    c_int(LONG_PORTION), c_int(1 if plan.single_tokens else 0), c_int(k.shape[0]), c_int(1), c_void_p(0), byref(kernels),
+                    _p(self.err), self._stream()),
                     "paged_attention (decode)", kv)
-                tma = cache.page_size == 8 or cache.page_size % 16 == 0
-                if not (tma and self.attn_tc.fz_attn_decode_whole(c_int(n), c_int(hq), c_int(hkv), c_int(meta.max_context),
-                                                                  c_int(1 if plan.single_tokens else 0))):
-                    self.launches += 1    # the combine kernel
+                self.launches += kernels.value - 1
             if plan.n_tiles > 0 and self.prefill_tcgen05 and \
                     self.attn_tc.fz_attn_prefill_tc_check(c_int(hq), c_int(hkv), c_int(hd), c_int(cache.page_size)) == 0:
                 # rows of long portions on the tcgen05 flash-attention kernel; the pieces of tiles that the plan cut along
@@ -1313,12 +1311,14 @@ class CudaOps(Ops):
             parts = self.attn_tc.fz_attn_partitions(c_int(meta.max_context))
             part_o = self._scratch("attention partials", n * heads * parts * (value_dim + 2), torch.float32)
             rows_out = self._scratch("attention maps", n * heads * value_dim, torch.float32)
+            kernels = c_int(0)
             self._check(self.attn_tc.fz_attn_decode(
                 _p(q), _p(k), _p(v), _p(meta.pos), _p(meta.seq_row), _p(meta.seg), _p(table), c_int(table.shape[1]),
                 c_longlong(page_stride), c_int(cache.page_size), c_void_p(0), _p(part_o), _p(part_o[n * heads * parts * value_dim:]), c_int(n),
                 c_int(heads), c_int(num_kv_heads), c_int(value_dim), c_float(scale), c_int(0), c_int(meta.max_context), c_int(LONG_PORTION),
-                c_int(1), c_int(k.shape[0]), c_int(2), _p(rows_out), _p(self.err), self._stream()), "differential_attention (decode)", nbytes)
-            self.launches += 1    # the kernel that merges the partial results
+                c_int(1), c_int(k.shape[0]), c_int(2), _p(rows_out), byref(kernels), _p(self.err), self._stream()),
+                "differential_attention (decode)", nbytes)
+            self.launches += kernels.value - 1
             self._combine_maps(rows_out, n, num_heads, value_dim, lam, eps, mult, meta, out)
             return
         self._sink_launch(q, k, v, cache, meta, out, num_heads, num_kv_heads, 2 * map_dim, value_dim, scale, 0, 0, None, 0.0,

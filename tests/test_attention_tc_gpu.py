@@ -253,3 +253,18 @@ def test_short_contexts_without_the_merge_kernel(Hq, Hkv, hd, bs, window):
     close(whole.float().cpu(), ref.float(), "short contexts")
     assert float(whole[-1].float().abs().max()) == 0.0
     cu.check_errors()
+
+
+@pytest.mark.parametrize("context,bs,tma,kernels", [(300, 16, True, 1), (300, 16, False, 2), (300, 4, True, 2), (1100, 16, True, 2)])
+def test_launches_of_a_decoded_row(context, bs, tma, kernels, monkeypatch):
+    """The launch count of a step of one token: one kernel for a short context on TMA loads, else a second that merges."""
+    from fusezap_core_b200.kernels import cuda_ops
+    if not tma:
+        monkeypatch.setenv("FZB200_NO_TMA_ATTN", "1")
+    cu, hd, pages = cuda_ops("bfloat16"), 64, -(-context // bs)
+    cache = make_cache(pages, 2, bs, hd, BF, "cuda")
+    q = torch.zeros(1, 14 * hd, dtype=BF, device="cuda")
+    before = cu.launches
+    cu.paged_attention(q, cache, Meta([context - 1], [0], [list(range(pages))], "cuda"), torch.empty_like(q), 14, 2, hd, hd ** -0.5, 0)
+    assert cu.launches - before == kernels
+    cu.check_errors()
