@@ -962,10 +962,12 @@ FZ_API int fz_sample(const float* logits, const float* temperature, const double
 // The reference's host sampler on the device (fusezap/serve/sampling.py:25-45, 61-73): logits / T in float64; top-k keeps
 // everything not below the k-th largest value (ties stay); top-p keeps, in falling order of value (ties by rising
 // index), every token before which less than p of the probability lies; then one draw from the softmax of what is left:
-// the first index whose running sum in index order exceeds u times the total. A cluster of SF_CLUSTER blocks of 1024
-// threads per row, a block for each SF_CLUSTER-th of its tokens (one block for rows of SF_SHORT tokens and less: the passes
-// over such a row cost less than the barriers between blocks; not measured in between): bound by the instructions per token and pass, so the blocks' number is what counts (8 rows of 151,936 with top-p, from the difference of whole steps:
-// 340 -> 70 us; 24 sampled tokens of 8 requests at Qwen2.5-0.5B sizes 32.2 -> 25.6 ms). The blocks add their bins and sums up through distributed shared memory in rank order; all then take the same decisions.
+// the first index whose running sum in index order exceeds u times the total. A row's tokens are cut into SLICES equal
+// slices (`sample_slices`), shared by the BLOCKS blocks of 1,024 threads of a cluster (`fz_sample_blocks`): bound by the
+// instructions per token and pass, so the SMs at work are what counts. Sums run over a slice first, then over the slices in
+// order, through distributed shared memory where they are several blocks', and all blocks then take the same decisions. us
+// with top-p, one block per row and slice (the kernel before) -> now: 151,936 tokens, 8 rows 378 -> 84, 32 rows 397 -> 141, 64
+// rows 569 -> 352, 96 rows 615 -> 448, 148 rows 665 -> 745; 32,000 tokens, 8 rows 98 -> 52, 64 rows 100 -> 82, 128 rows 101 -> 130.
 // Nothing is sorted: the thresholds are found by radix selection over an order-preserving 32-bit key of the logit,
 // eight passes of 4 bits, with a histogram of counts for top-k and of probability mass (float64) for top-p. Each thread
 // fills 16 bins of its own in shared memory and the bins are then summed over the threads in a fixed order, so there
@@ -974,7 +976,6 @@ FZ_API int fz_sample(const float* logits, const float* temperature, const double
 constexpr int SF_THREADS = 1024;
 constexpr int SF_BINS = 16;
 constexpr size_t SF_SMEM = (size_t)SF_BINS * SF_THREADS * sizeof(double);
-constexpr int SF_CLUSTER = 8, SF_SHORT = 8192;
 
 __device__ __forceinline__ uint32_t falling_key(float x) {      // smaller key = larger value; -0 counts as +0
   const uint32_t u = __float_as_uint(x + 0.f);
@@ -1025,20 +1026,27 @@ __device__ __forceinline__ void for_each_key(const float* __restrict__ row, int 
   }
 }
 
-// The sum over the cluster's blocks, in rank order, of values[0..count) of each block; thread i < count gets sum i. Called
-// with the two halves of a pair of buffers in turn: a buffer is written again only after a cluster barrier that every
-// block reaches after it has read it.
-template <typename T>
-__device__ __forceinline__ T cluster_sum(const cg::cluster_group& cluster, T* values, int count) {
-  const int blocks = cluster.num_blocks();
-  if (blocks == 1) {
-    __syncthreads();
-    return threadIdx.x < count ? values[threadIdx.x] : T(0);
-  }
-  cluster.sync();
+// The sum over a row's slices, in order, of values[slice][0..count): a block of the cluster has SLICES / BLOCKS neighbouring slices in
+// its shared memory. Thread i < count gets sum i. Called with the two halves of a pair of buffers in turn: a buffer is written
+// again only after a barrier that every block reaches after it has read it.
+template <int SLICES, int BLOCKS, typename T, int COUNT>
+__device__ __forceinline__ T slices_sum(T (*values)[COUNT]) {
+  constexpr int PER = SLICES / BLOCKS;
   T v = 0;
-  if (threadIdx.x < count)
-    for (int b = 0; b < blocks; ++b) v += cluster.map_shared_rank(values, b)[threadIdx.x];
+  if constexpr (BLOCKS == 1) {
+    __syncthreads();
+    if (threadIdx.x < COUNT) {
+#pragma unroll
+      for (int s = 0; s < SLICES; ++s) v += values[s][threadIdx.x];
+    }
+  } else {
+    const cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    if (threadIdx.x < COUNT) {
+#pragma unroll
+      for (int s = 0; s < SLICES; ++s) v += *cluster.map_shared_rank(&values[s % PER][threadIdx.x], s / PER);
+    }
+  }
   return v;
 }
 
@@ -1051,10 +1059,12 @@ __device__ __forceinline__ double warp_scan_fixed(double v, int lane) {
   return v;
 }
 
+template <int SLICES, int BLOCKS>
 __global__ void __launch_bounds__(SF_THREADS, 1)
 sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
                        const int* __restrict__ top_k, const float* __restrict__ top_p,
                        const double* __restrict__ uniform, double* __restrict__ scratch, int* __restrict__ out, int V) {
+  constexpr int PER = SLICES / BLOCKS;      // slices of a block
   fz_grid_launch_dependents();
   fz_grid_wait();
   extern __shared__ __align__(16) unsigned char sf_smem[];
@@ -1062,19 +1072,20 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
   unsigned int* bins_u = reinterpret_cast<unsigned int*>(sf_smem);
   __shared__ float s_val[32];
   __shared__ int s_idx[32];
-  __shared__ double s_part[32], s_mass[2][SF_BINS], s_wsum[32], s_all[SF_BINS], s_sum[2][1];
-  __shared__ unsigned int s_partu[32], s_count[2][SF_BINS], s_allu[SF_BINS];
+  __shared__ double s_part[32], s_mass[2][PER][SF_BINS], s_wsum[PER][32], s_all[SF_BINS], s_sum[2][PER][1], s_slices[SLICES];
+  __shared__ unsigned int s_partu[32], s_count[2][1][SF_BINS], s_allu[SF_BINS];
   __shared__ float s_best[1];
   __shared__ int s_best_at[1], s_ties[1];
-  __shared__ int s_wties[32];
+  __shared__ int s_wties[PER][32];
   __shared__ uint32_t s_prefix;
   __shared__ unsigned int s_rank;
   __shared__ double s_need, s_target;
-  __shared__ int s_warp;
+  __shared__ int s_warp, s_slice;
   const cg::cluster_group cluster = cg::this_cluster();
-  const int blocks = cluster.num_blocks(), rank = cluster.block_rank();
-  const int r = blockIdx.x / blocks, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int slice = (V + blocks * 32 - 1) / (blocks * 32) * 32, lo = min(V, rank * slice), hi = min(V, lo + slice);
+  const int rank = BLOCKS > 1 ? (int)cluster.block_rank() : 0;
+  const int r = blockIdx.x / BLOCKS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slice = (V + SLICES * 32 - 1) / (SLICES * 32) * 32;                   // tokens of a slice
+  const int lo = min(V, rank * PER * slice), hi = min(V, lo + PER * slice);       // the block's tokens
   int turn = 0;      // which of a pair of buffers is next
   const float* row = logits + (size_t)r * V;
   double* e = scratch + (size_t)r * V;
@@ -1085,17 +1096,19 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
     s_best_at[0] = lo < hi ? lo + amax : 0x7fffffff;
     s_best[0] = lo < hi ? row[lo + amax] : -INFINITY;
   }
-  cluster.sync();
+  if constexpr (BLOCKS > 1) cluster.sync();
+  else __syncthreads();
   float top = -INFINITY;
   amax = 0x7fffffff;
-  for (int b = 0; b < blocks; ++b) {      // slices in index order, as the row-split argmax does it
+#pragma unroll
+  for (int b = 0; b < BLOCKS; ++b) {      // slices in index order, as the row-split argmax does it
     const float v = cluster.map_shared_rank(s_best, b)[0];
     const int at = cluster.map_shared_rank(s_best_at, b)[0];
     if (at != 0x7fffffff && (amax == 0x7fffffff || better(v, at, top, amax))) { top = v; amax = at; }
   }
   if (!(T > 0.f) || k == 1) {
     if (rank == 0 && tid == 0) out[r] = amax;
-    cluster.sync();      // (nobody leaves while its shared memory may still be read)
+    if constexpr (BLOCKS > 1) cluster.sync();      // (nobody leaves while its shared memory may still be read)
     return;
   }
   const double mx = (double)top / (double)T;
@@ -1112,8 +1125,8 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
       for_each_key(row, lo, hi, [&](int, float, uint32_t key) {
         if (pass == 0 || (key >> (shift + 4)) == prefix) bins_u[((key >> shift) & 15u) * SF_THREADS + tid] += 1u;
       });
-      sum_bins(bins_u, s_partu, s_count[turn]);
-      const unsigned int count = cluster_sum(cluster, s_count[turn], SF_BINS);
+      sum_bins(bins_u, s_partu, s_count[turn][0]);
+      const unsigned int count = slices_sum<BLOCKS, BLOCKS>(s_count[turn]);      // (counts: the blocks' whole shares)
       turn ^= 1;
       if (tid < SF_BINS) s_allu[tid] = count;
       __syncthreads();
@@ -1140,15 +1153,18 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
   uint32_t t_key = nucleus ? top_key : 0xffffffffu;                         // (first == 8: one value stays)
   double need_at_t = 0.0, total = 0.0;
   if (first == 8) {
-    double local = 0.0;
-    for_each_key(row, lo, hi, [&](int i, float x, uint32_t key) {
-      const double v = key <= k_key ? exp((double)x / (double)T - mx) : 0.0;
-      e[i] = v;
-      local += v;
-    });
-    local = block_sum_fixed(local, s_part);
-    if (tid == 0) s_sum[turn][0] = local;
-    total = cluster_sum(cluster, s_sum[turn], 1);      // (thread 0 has it; only thread 0 asks)
+    for (int j = 0; j < PER; ++j) {
+      double local = 0.0;
+      const int s_lo = min(V, lo + j * slice);
+      for_each_key(row, s_lo, min(V, s_lo + slice), [&](int i, float x, uint32_t key) {
+        const double v = key <= k_key ? exp((double)x / (double)T - mx) : 0.0;
+        e[i] = v;
+        local += v;
+      });
+      local = block_sum_fixed(local, s_part);
+      if (tid == 0) s_sum[turn][j][0] = local;
+    }
+    total = slices_sum<SLICES, BLOCKS>(s_sum[turn]);      // (thread 0 has it; only thread 0 asks)
     turn ^= 1;
     if (tid == 0) s_need = (double)pp * total;
     __syncthreads();
@@ -1159,27 +1175,40 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
       const int shift = 28 - 4 * pass;
       __syncthreads();
       const uint32_t prefix = s_prefix;
-      for (int b = 0; b < SF_BINS; ++b) bins_d[b * SF_THREADS + tid] = 0.0;
-      if (pass == first) {
-        double local = 0.0;
-        for_each_key(row, lo, hi, [&](int i, float x, uint32_t key) {
-          const double v = key <= k_key ? exp((double)x / (double)T - mx) : 0.0;
-          e[i] = v;
-          local += v;
-          if (key <= k_key) bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += v;
-        });
-        local = block_sum_fixed(local, s_part);
-        if (tid == 0) s_sum[turn][0] = local;
-        total = cluster_sum(cluster, s_sum[turn], 1);
-        turn ^= 1;
-        if (tid == 0) s_need = (double)pp * total;
-      } else {
-        for_each_key(row, lo, hi, [&](int i, float, uint32_t key) {
-          if (key <= k_key && (key >> (shift + 4)) == prefix) bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += e[i];
-        });
+      bool zeroed = false;
+      for (int j = 0; j < PER; ++j) {
+        const int s_lo = min(V, lo + j * slice), s_hi = min(V, s_lo + slice);
+        if (!zeroed)
+          for (int b = 0; b < SF_BINS; ++b) bins_d[b * SF_THREADS + tid] = 0.0;
+        bool any = pass == first;
+        if (pass == first) {
+          double local = 0.0;
+          for_each_key(row, s_lo, s_hi, [&](int i, float x, uint32_t key) {
+            const double v = key <= k_key ? exp((double)x / (double)T - mx) : 0.0;
+            e[i] = v;
+            local += v;
+            if (key <= k_key) bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += v;
+          });
+          local = block_sum_fixed(local, s_part);
+          if (tid == 0) s_sum[turn][j][0] = local;
+        } else {
+          for_each_key(row, s_lo, s_hi, [&](int i, float, uint32_t key) {
+            if (key <= k_key && (key >> (shift + 4)) == prefix) {
+              bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += e[i];
+              any = true;
+            }
+          });
+        }
+        // (the last digits match in few slices: the bins of the others are all zero still)
+        zeroed = PER > 1 && !__syncthreads_or(any);
+        if (!zeroed) sum_bins(bins_d, s_part, s_mass[turn][j]);
+        else if (tid < SF_BINS) s_mass[turn][j][tid] = 0.0;
       }
-      sum_bins(bins_d, s_part, s_mass[turn]);
-      const double mass = cluster_sum(cluster, s_mass[turn], SF_BINS);
+      if (pass == first) {
+        total = slices_sum<SLICES, BLOCKS>(s_sum[turn]);
+        if (tid == 0) s_need = (double)pp * total;
+      }
+      const double mass = slices_sum<SLICES, BLOCKS>(s_mass[turn]);
       turn ^= 1;
       if (tid < SF_BINS) s_all[tid] = mass;
       __syncthreads();
@@ -1203,83 +1232,105 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
     t_key = s_prefix;
     need_at_t = s_need;
   }
-  // ---- the draw. Warp w owns the contiguous range [w * span, (w + 1) * span) of its block's slice and walks it 32 tokens
-  // at a time, so that sums run in index order. Equal values at the threshold: the j-th of them in index order (j = 0, 1,
-  // ...) stays while j * e < need_at_t.
+  // ---- the draw. Warp w owns the contiguous range [w * span, (w + 1) * span) of each slice and walks it 32 tokens at a time,
+  // so that sums run in index order. Equal values at the threshold: the j-th of them in index order (j = 0, 1, ...) stays
+  // while j * e < need_at_t.
   const int span = ((slice + 1023) / 1024) * 32;
-  const int w_lo = min(hi, lo + warp * span), w_hi = min(hi, w_lo + span);
-  if (nucleus) {
-    int ties = 0;
-    for (int i = w_lo + lane; i < w_hi; i += 32) ties += falling_key(row[i]) == t_key ? 1 : 0;
-    for (int o = 16; o; o >>= 1) ties += __shfl_xor_sync(0xffffffffu, ties, o);
-    if (lane == 0) s_wties[warp] = ties;
-  }
-  __syncthreads();
+  auto warp_range = [&](int j, int w, int& from, int& to) {
+    const int s_lo = min(V, lo + j * slice), s_hi = min(V, s_lo + slice);
+    from = min(s_hi, s_lo + w * span);
+    to = min(s_hi, from + span);
+  };
   int j0 = 0;
   if (nucleus) {
-    if (blocks > 1) {
-      if (tid == 0) {
+    for (int j = 0; j < PER; ++j) {
+      int from, to, ties = 0;
+      warp_range(j, warp, from, to);
+      for (int i = from + lane; i < to; i += 32) ties += falling_key(row[i]) == t_key ? 1 : 0;
+      for (int o = 16; o; o >>= 1) ties += __shfl_xor_sync(0xffffffffu, ties, o);
+      if (lane == 0) s_wties[j][warp] = ties;
+    }
+    __syncthreads();
+    if constexpr (BLOCKS > 1) {
+      if (warp == 0) {
         int all = 0;
-        for (int w = 0; w < 32; ++w) all += s_wties[w];
-        s_ties[0] = all;
+        for (int j = 0; j < PER; ++j) all += s_wties[j][lane];
+        all = __reduce_add_sync(0xffffffffu, all);
+        if (lane == 0) s_ties[0] = all;
       }
       cluster.sync();
       for (int b = 0; b < rank; ++b) j0 += cluster.map_shared_rank(s_ties, b)[0];
     }
-    for (int w = 0; w < warp; ++w) j0 += s_wties[w];
   }
-  double run = 0.0;
-  for (int base = w_lo; base < w_hi; base += 32) {
-    const int i = base + lane;
-    const bool in = i < w_hi;
-    double v = in ? e[i] : 0.0;
+  for (int j = 0; j < PER; ++j) {
+    int from, to;
+    warp_range(j, warp, from, to);
+    int nth = j0;      // of the equal values, how many lie before
     if (nucleus) {
-      const uint32_t key = in ? falling_key(row[i]) : 0u;
-      const bool tie = in && key == t_key;
-      const unsigned int tie_mask = __ballot_sync(0xffffffffu, tie);
-      bool drop = in && key > t_key;
-      if (tie) drop = !((double)(j0 + __popc(tie_mask & ((1u << lane) - 1u))) * v < need_at_t);
-      j0 += __popc(tie_mask);
-      if (drop && v != 0.0) e[i] = 0.0;
-      if (drop) v = 0.0;
+      const int ties = s_wties[j][lane];
+      nth += __reduce_add_sync(0xffffffffu, lane < warp ? ties : 0);
+      j0 += __reduce_add_sync(0xffffffffu, ties);
     }
-    run += __shfl_sync(0xffffffffu, warp_scan_fixed(v, lane), 31);
+    double run = 0.0;
+    for (int base = from; base < to; base += 32) {
+      const int i = base + lane;
+      const bool in = i < to;
+      double v = in ? e[i] : 0.0;
+      if (nucleus) {
+        const uint32_t key = in ? falling_key(row[i]) : 0u;
+        const bool tie = in && key == t_key;
+        const unsigned int tie_mask = __ballot_sync(0xffffffffu, tie);
+        bool drop = in && key > t_key;
+        if (tie) drop = !((double)(nth + __popc(tie_mask & ((1u << lane) - 1u))) * v < need_at_t);
+        nth += __popc(tie_mask);
+        if (drop && v != 0.0) e[i] = 0.0;
+        if (drop) v = 0.0;
+      }
+      run += __shfl_sync(0xffffffffu, warp_scan_fixed(v, lane), 31);
+    }
+    if (lane == 0) s_wsum[j][warp] = run;
   }
-  if (lane == 0) s_wsum[warp] = run;
+  __syncthreads();
+  if (tid < PER) {
+    double sum = 0.0;
+    for (int w = 0; w < 32; ++w) sum += s_wsum[tid][w];
+    s_sum[turn][tid][0] = sum;
+  }
+  if constexpr (BLOCKS > 1) {
+    cluster.sync();
+    if (tid < SLICES) s_slices[tid] = *cluster.map_shared_rank(&s_sum[turn][tid % PER][0], tid / PER);
+  } else {
+    if (tid < SLICES) s_slices[tid] = s_sum[turn][tid][0];
+  }
   __syncthreads();
   if (tid == 0) {
-    double sum = 0.0;
-    for (int w = 0; w < 32; ++w) sum += s_wsum[w];
-    s_sum[turn][0] = sum;
-  }
-  if (blocks > 1) cluster.sync();
-  else __syncthreads();
-  if (tid == 0) {
     double all = 0.0;
-    for (int b = 0; b < blocks; ++b) all += cluster.map_shared_rank(s_sum[turn], b)[0];
+    for (int s = 0; s < SLICES; ++s) all += s_slices[s];
     const double target = uniform[r] * all;
-    // the block, then the warp, whose tokens the draw falls into: the first at whose end the running sum exceeds the
+    // the slice, then the warp, whose tokens the draw falls into: the first at whose end the running sum exceeds the
     // target. Where rounding leaves them all at or below it, the last one with any mass.
     double before = 0.0, before_last = 0.0;
     int b = 0, last = -1;
-    for (; b < blocks; ++b) {
-      const double sum = cluster.map_shared_rank(s_sum[turn], b)[0];
+    for (; b < SLICES; ++b) {
+      const double sum = s_slices[b];
       if (sum > 0.0) { last = b; before_last = before; }
       if (before + sum > target) break;
       before += sum;
     }
-    if (b == blocks) { b = last; before = before_last; }
+    if (b == SLICES) { b = last; before = before_last; }
     int w = -1;
-    if (b == rank) {
+    if (b >= 0 && b / PER == rank) {
+      const double* wsum = s_wsum[b % PER];
       last = -1;
       for (w = 0; w < 32; ++w) {
-        if (s_wsum[w] > 0.0) { last = w; before_last = before; }
-        if (before + s_wsum[w] > target) break;
-        before += s_wsum[w];
+        if (wsum[w] > 0.0) { last = w; before_last = before; }
+        if (before + wsum[w] > target) break;
+        before += wsum[w];
       }
       if (w == 32) { w = last; before = before_last; }
     }
     s_warp = w;
+    s_slice = b < 0 ? 0 : b % PER;
     s_need = before;
     s_target = target;
     if (b < 0 && rank == 0) out[r] = amax;      // no sum above zero: the largest logit is not a number
@@ -1287,11 +1338,12 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
   __syncthreads();
   if (warp == s_warp) {
     const double target = s_target;
-    run = s_need;
-    int res = amax;
-    for (int base = w_lo; base < w_hi; base += 32) {
+    double run = s_need;
+    int res = amax, from, to;
+    warp_range(s_slice, warp, from, to);
+    for (int base = from; base < to; base += 32) {
       const int i = base + lane;
-      const double v = i < w_hi ? e[i] : 0.0;
+      const double v = i < to ? e[i] : 0.0;
       const unsigned int some = __ballot_sync(0xffffffffu, v > 0.0);
       const double sc = warp_scan_fixed(v, lane);
       const unsigned int hit = __ballot_sync(0xffffffffu, run + sc > target);
@@ -1304,7 +1356,52 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
     }
     if (lane == 0) out[r] = res;
   }
-  if (blocks > 1) cluster.sync();
+  if constexpr (BLOCKS > 1) cluster.sync();
+}
+
+// The slices that a row's sums are taken over: by V alone, so that a row's token does not depend on the rows beside it. As many
+// as few rows gain from while a block that has to walk all of them loses little. us for 14 and 128 rows, top-p, with one slice
+// and with more: 8,192 tokens 37, 37 | 2 slices 42, 53; 12,000 49, 51 | 2: 46, 62; 16,384 59, 61 | 2: 51, 71 | 4: 43, 97; 32,000 99,
+// 104 | 2: 71, 110 | 4: 52, 130 | 8: 45, 181; 65,536 2: 114, 242 | 4: 74, 264 | 8: 55, 306; 151,936 4: 131, 658 | 8: 85, 717.
+static int sample_slices(int V) { return V <= 12288 ? 1 : V <= 24576 ? 2 : V <= 98304 ? 4 : 8; }
+
+// Blocks per row (a cluster): a block has an SM to itself, and the rows should not queue for SMs. 14 clusters of eight, 32 of
+// four and 74 of two are on the chip at once (16 of eight and 36 of four take twice as long). With more rows one block
+// each, except that three rounds of fours still beat one of whole rows of eight slices: 96 rows of 151,936 448 against 686
+// us (top-k and top-p 463, 525), 128 rows 592, 718 (612, 541).
+FZ_API int fz_sample_blocks(int R, int V) {
+  const int slices = sample_slices(V), most = R <= 14 ? 8 : R <= 32 ? 4 : R <= 74 ? 2 : R <= 96 && slices == 8 ? 4 : 1;
+  return slices < most ? slices : most;
+}
+
+template <int SLICES, int BLOCKS>
+static int launch_sample(const float* logits, const float* temperature, const int* top_k, const float* top_p, const double* uniform,
+                         double* scratch, int* out, int R, int V, cudaStream_t stream) {
+  auto kern = sample_filtered_kernel<SLICES, BLOCKS>;
+  static const cudaError_t raised = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SF_SMEM);
+  if (raised != cudaSuccess) return (int)raised;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)R * BLOCKS);
+  cfg.blockDim = dim3(SF_THREADS);
+  cfg.dynamicSmemBytes = SF_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (BLOCKS > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = BLOCKS;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (fz_pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  cudaLaunchKernelEx(&cfg, kern, logits, temperature, top_k, top_p, uniform, scratch, out, V);
+  FZ_LAUNCH_CHECK();
+  return FZ_OK;
 }
 
 // scratch: R * V doubles. top_k[r] <= 0 or >= V: no top-k; top_p[r] >= 1: no top-p; temperature[r] <= 0 or top_k[r]
@@ -1313,33 +1410,14 @@ FZ_API int fz_sample_filtered(const float* logits, const float* temperature, con
                               const double* uniform, double* scratch, int* out, int R, int V, cudaStream_t stream) {
   if (R <= 0) return FZ_OK;
   if (V <= 0) return FZ_BAD_SHAPE;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(sample_filtered_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SF_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
-  const int blocks = V <= SF_SHORT ? 1 : SF_CLUSTER;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)R * blocks);
-  cfg.blockDim = dim3(SF_THREADS);
-  cfg.dynamicSmemBytes = SF_SMEM;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  int n = 0;
-  attr[n].id = cudaLaunchAttributeClusterDimension;
-  attr[n].val.clusterDim.x = blocks;
-  attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
-  ++n;
-  if (fz_pdl_enabled()) {
-    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n++].val.programmaticStreamSerializationAllowed = 1;
-  }
-  cfg.attrs = attr;
-  cfg.numAttrs = n;
-  cudaLaunchKernelEx(&cfg, sample_filtered_kernel, logits, temperature, top_k, top_p, uniform, scratch, out, V);
-  FZ_LAUNCH_CHECK();
-  return FZ_OK;
+  const int blocks = fz_sample_blocks(R, V);
+#define FZ_SF(S_, B_) if (sample_slices(V) == S_ && blocks == B_) return launch_sample<S_, B_>(logits, temperature, top_k, top_p, uniform, scratch, out, R, V, stream)
+  FZ_SF(1, 1);
+  FZ_SF(2, 1); FZ_SF(2, 2);
+  FZ_SF(4, 1); FZ_SF(4, 2); FZ_SF(4, 4);
+  FZ_SF(8, 1); FZ_SF(8, 2); FZ_SF(8, 4); FZ_SF(8, 8);
+#undef FZ_SF
+  return FZ_BAD_SHAPE;
 }
 
 // ------------------------------------------------------------------------------------------------ error word

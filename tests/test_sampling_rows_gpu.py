@@ -35,3 +35,36 @@ def test_rows_shared_by_blocks(V):
         one = torch.empty(1, dtype=torch.int32, device="cuda")
         cu.sample_filtered(lg[r:r + 1].cuda(), temp[r:r + 1].cuda(), top_k[r:r + 1].cuda(), top_p[r:r + 1].cuda(), u[r:r + 1].cuda(), one)
         assert int(one) == int(ref[r])
+
+
+@pytest.mark.parametrize("V", [12288, 12289, 24577, 98305])
+def test_a_token_does_not_depend_on_the_blocks_of_its_row(V):
+    """Rows of one vocabulary in steps of every size at which the blocks per row change: one token per row, whoever computes
+    it, with ties that cross slices, slices without mass and a row whose largest logit is not a number."""
+    cu, pl = ops_pair("float32")
+    blocks = [cu.core.fz_sample_blocks(r, V) for r in (1, 14, 15, 32, 33, 74, 75, 96, 97)]
+    assert blocks == {12288: [1] * 9, 12289: [2] * 6 + [1] * 3, 24577: [4] * 4 + [2] * 2 + [1] * 3,
+                      98305: [8, 8, 4, 4, 2, 2, 4, 4, 1]}[V]
+    g = torch.Generator().manual_seed(V)
+    R = 97
+    lg = torch.randn(R, V, generator=g) * 3
+    lg[1] = 1.0
+    lg[2] = (lg[2] / 3).round()
+    lg[3, 100:] = -float("inf")
+    lg[4, :V - 5] = -float("inf")
+    lg[5, V // 2] = float("nan")
+    temp = torch.full((R,), 0.9)
+    temp[6] = 0.0
+    top_k = torch.tensor([0, 0, 40, 0, 7, 0, 9] * 14, dtype=torch.int32)[:R]
+    top_p = torch.tensor([0.95, 0.6, 1.0, 0.9] * 25)[:R]
+    u = torch.rand(R, generator=g, dtype=torch.float64)
+    ref = torch.empty(R, dtype=torch.int32)
+    rest = [r for r in range(R) if r != 5]
+    part = torch.empty(len(rest), dtype=torch.int32)
+    pl.sample_filtered(lg[rest], temp[rest], top_k[rest], top_p[rest], u[rest], part)
+    ref[rest], ref[5] = part, V // 2
+    dev = [t.cuda() for t in (lg, temp, top_k, top_p, u)]
+    for n in (R, 96, 75, 74, 33, 32, 15, 14, 1):
+        out = torch.empty(n, dtype=torch.int32, device="cuda")
+        cu.sample_filtered(*(t[:n].contiguous() for t in dev), out)
+        assert out.cpu().tolist() == ref[:n].tolist(), f"{n} rows"
