@@ -674,7 +674,8 @@ class CudaOps(Ops):
         self._check(self.core.fz_attn_simt(
             _p(q), _p(k), _p(v), _p(meta.pos), _p(meta.seq_row), _p(table), c_int(table.shape[1]),
             c_longlong(page_stride), c_int(cache.page_size), _p(out), c_int(_CODE[self.dtype]), c_int(n), c_int(hq),
-            c_int(hkv), c_int(hd), c_float(scale), c_int(window), c_int(meta.max_context), _p(self.err), self._stream()), "paged_attention", kv)
+            c_int(hkv), c_int(hd), c_float(scale), c_int(window), c_int(meta.max_context),
+            c_int(int(getattr(meta, "max_portion", 0)) or n), _p(self.err), self._stream()), "paged_attention", kv)
 
     @staticmethod
     def _gate_kind(activation: str) -> int:

@@ -166,3 +166,58 @@ def test_attention_with_more_heads_and_slices_than_a_grid_is_high():
     ref = torch.einsum("hgk,hkd->hgd", s.softmax(-1), cache.values[0, :, :3].float())
     # half a bfloat16 step of the result, and the 32-bit sums
     assert bool(((out[1].view(Hkv, G, hd).float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
+
+
+def test_rows_of_different_requests_do_not_wait_for_each_other():
+    """Blocks hold several rows only where these can be of one portion."""
+    rows = cuda().core.fz_attn_simt_rows
+    # decoded tokens: a row's spans side by side while rows are few, then a row per block
+    assert [rows(n, 14, 2, 64, 300, 1) for n in (1, 64, 100, 300, 4000)] == [0, 0, 1, 1, 1]
+    assert [rows(n, 14, 2, 64, 2048, 1) for n in (1, 148, 300, 4000)] == [0, 0, 1, 1]
+    # portions: rows share keys, as many as they have and as leave blocks for every SM
+    assert [rows(n, 14, 2, 64, n, n) for n in (400, 2000)] == [2, 4]
+    assert rows(4000, 14, 2, 64, 300, 3) == 3 and rows(300, 8, 8, 64, 300, 300) == 8
+
+
+@pytest.mark.parametrize("dtype,Hq,Hkv,hd,bs,window", [("float32", 4, 4, 32, 16, 0), ("float32", 6, 2, 64, 8, 40), ("bfloat16", 3, 1, 48, 16, 0),
+                                                       ("bfloat16", 8, 8, 80, 8, 33), ("bfloat16", 4, 2, 36, 16, 0), ("bfloat16", 40, 1, 24, 16, 0)])
+def test_attention_rows_in_blocks(dtype, Hq, Hkv, hd, bs, window):
+    """Runs of rows that start and end off the multiples of eight at which blocks change hands, runs of two requests whose
+    positions continue, the same request at other positions, the same row twice, padding: every row has the bits that it
+    has alone, whatever the longest run is said to be, and is right."""
+    from fusezap_core_b200.kernels import cuda_ops
+    from plain_ops import PlainOps
+    dt = torch.float32 if dtype == "float32" else torch.bfloat16
+    cu, pl = cuda_ops(dtype), PlainOps(dt)
+    lengths = [700, 400, 90]
+    mb = -(-700 // bs)
+    g = torch.Generator().manual_seed(hd)
+    perm = torch.randperm(3 * mb, generator=g).tolist()
+    table = [perm[r * mb:(r + 1) * mb] for r in range(3)]
+    cp = make_cache(3 * mb, Hkv, bs, hd, dt, "cpu")
+    fill_cache(cp, table, lengths, g)
+    cc = make_cache(3 * mb, Hkv, bs, hd, dt, "cuda")
+    cc.pool.copy_(cp.pool)
+    rows = [(2, 5)] + [(0, p) for p in range(301, 330)] + [(1, p) for p in range(330, 347)] + [(-1, 0)] * 2 + [(0, p) for p in range(673, 700)] \
+        + [(0, 699), (0, 31), (0, 0), (1, 399)] + [(2, p) for p in range(60, 90)]
+    q = torch.randn(len(rows), Hq * hd, generator=g).to(dt)
+
+    def attend(index, longest):
+        out = torch.full((len(index), Hq * hd), float("nan"), dtype=dt, device="cuda")
+        meta = Meta([rows[i][1] for i in index], [rows[i][0] for i in index], table, "cuda")
+        meta.max_portion = longest
+        cu.paged_attention(q[index].cuda(), cc, meta, out, Hq, Hkv, hd, hd ** -0.5, window)
+        return out
+
+    every = list(range(len(rows))) * (6 if Hkv == 1 else 3)      # (enough rows for blocks of several)
+    full = attend(every, 30)
+    assert torch.equal(full, full[:len(rows)].repeat(len(every) // len(rows), 1))
+    for longest in (1, 2, 3, 5, 1000):
+        assert torch.equal(attend(every, longest), full), f"longest run {longest}"
+    for i in (0, 1, 2, 3, 11, 29, 30, 46, 47, 50, 75, 76, 77, 78, 79, 80, len(rows) - 1):
+        assert torch.equal(attend([i], 1)[0], full[i]), f"row {i}"
+    ref = torch.empty(len(rows), Hq * hd, dtype=dt)
+    pl.paged_attention(q, cp, Meta([p for _, p in rows], [r for r, _ in rows], table, "cpu"), ref, Hq, Hkv, hd, hd ** -0.5, window)
+    # float32: 700 keys' sums in two orders; bfloat16: the roundings of the two results
+    assert float((full[:len(rows)].float().cpu() - ref.float()).abs().max()) <= (1e-5 if dtype == "float32" else 2.0 ** -7) * float(ref.float().abs().max())
+    cu.check_errors()
