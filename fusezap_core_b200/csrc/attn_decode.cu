@@ -807,9 +807,9 @@ __device__ __forceinline__ void combine_units_row(const int n, const int h, cons
   *(uint2*)(orow + d4) = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&c);
 }
 
-// FIND false: one block per (head, row). true, in steps with long portions: a block looks at every gridDim.y-th row, a lane
-// each, and takes the short ones among them: a block per row, almost all of them with nothing to do, took
-// 22 us of a layer of a step of 500 prompt rows beside 7 decoded ones at 32 heads; the step of 32 layers 13.81 -> 13.33 ms.
+// FIND false: one block per (head, row). true, where most rows are of long portions (`combine_rows`): a block looks at every
+// gridDim.y-th row, a lane each, and takes the short ones among them: a block per row, almost all of them with nothing to do,
+// took 22 us of a layer of a step of 500 prompt rows beside 7 decoded ones at 32 heads; the step of 32 layers 13.81 -> 13.33 ms.
 template <bool FIND>
 __global__ void __launch_bounds__(256)
 attn_combine_units_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
@@ -886,10 +886,20 @@ __global__ void attn_combine_kernel(const float* __restrict__ part_o, const floa
   }
 }
 
+// Blocks per head of the merge kernel: one per row, or, where most rows are of long portions, fewer that look for the others
+// among gridDim.y-th rows: as many as there are short rows, 64 at least. us of the two kernels with a block per row, with 64
+// and with as many as the rule gives: 32 heads of 128, 500 prompt rows beside 7 of 300 keys 30.1, 14.4, 14.4, beside 200
+// 70.0, 57.1, 58; 512 rows in portions of four 39.9, 42.7, 39.9; 2 heads of 128, 500 beside 200 13.9, 18.9, 13.7, 300 portions of
+// seven 27, 71, 27.
+int combine_rows(int N, int single, int short_rows) {
+  if (single || N <= 64 || 2 * short_rows > N) return N;
+  return short_rows < 64 ? 64 : short_rows;
+}
+
 template <int HD, int BOX, int NSTAGE, int MINB, bool SMALLG>
 int launch_units(const void* q, const void* k_pool, long long pool_rows, const int* pos, const int* seq_row, const int* seg,
                  const int* table, int mb, int page_size, void* out, float* part_o, float* part_ml, int N, int Hq, int Hkv,
-                 float scale, int window, int NPU, int long_from, int single, int maps, float* out32, int* err, cudaStream_t stream) {
+                 float scale, int window, int NPU, int long_from, int single, int short_rows, int maps, float* out32, int* err, cudaStream_t stream) {
   CUtensorMap map;
   int st = fztma::get_map_bf16(k_pool, pool_rows, HD, BOX, &map);
   if (st != FZ_OK) return st;
@@ -917,14 +927,15 @@ int launch_units(const void* q, const void* k_pool, long long pool_rows, const i
             (const __nv_bfloat16*)q, pos, seq_row, seg, table, mb, page_size, part_o, part_ml, N, Hq, Hkv, NPU,
             scale * 1.4426950408889634f, window, long_from, single, maps, err, (__nv_bfloat16*)nullptr);
   FZ_LAUNCH_CHECK();
-  const bool find = !single && N > 64;
-  dim3 cgrid(Hq, find ? 64 : N);
+  const int rows_high = combine_rows(N, single, short_rows);
+  dim3 cgrid(Hq, rows_high);
   // shared memory: the row's (max, sum) pairs, then 256 float4 and up to 16 float2 of the chains' results
   // blocks of 256 threads (a chain per group) while there are fewer blocks than SMs, else of 128 (two chains per group):
   // two engines alternating in one process, a decode step of 32 layers at batch 1 3.100 -> 3.079 ms, batch 2 3.181 ->
   // 3.161, batch 4 3.369 -> 3.348; at batch 8 (256 blocks) 3.780 -> 3.789 and at batch 64 1.3 % slower
   const int ct = (long long)cgrid.y * Hq <= sms ? 256 : 128;
-  fz_launch(find ? attn_combine_units_kernel<true> : attn_combine_units_kernel<false>, cgrid, dim3(ct), (size_t)(NPU + 2) * 8 + 256 * 16 + 16 * 8, stream, (const float*)part_o,
+  fz_launch(rows_high < N ? attn_combine_units_kernel<true> : attn_combine_units_kernel<false>, cgrid, dim3(ct),
+            (size_t)(NPU + 2) * 8 + 256 * 16 + 16 * 8, stream, (const float*)part_o,
             (const float*)part_ml, pos, seq_row, seg, (__nv_bfloat16*)out, out32, N, Hq, HD, NPU, window, long_from);
   FZ_LAUNCH_CHECK();
   return FZ_OK;
@@ -971,7 +982,7 @@ int launch_whole(const CUtensorMap& map, const void* q, const int* pos, const in
 template <int HD, int BOX>
 int launch_tma(const void* q, const void* k_pool, long long pool_rows, const int* pos, const int* seq_row, const int* seg,
                const int* table, int mb, int page_size, void* out, float* part_o, float* part_ml, int N, int Hq, int Hkv,
-               float scale, int window, int NPU, int long_from, int single, int maps, float* out32, int* kernels, int* err, cudaStream_t stream) {
+               float scale, int window, int NPU, int long_from, int single, int short_rows, int maps, float* out32, int* kernels, int* err, cudaStream_t stream) {
   if (whole_rows(N, Hq, Hkv, NPU, single) && maps == 1 && out32 == nullptr) {
     *kernels = 1;
     CUtensorMap map;
@@ -979,7 +990,7 @@ int launch_tma(const void* q, const void* k_pool, long long pool_rows, const int
     if (st != FZ_OK) return st;
     return launch_whole<HD, BOX>(map, q, pos, seq_row, seg, table, mb, page_size, out, N, Hq, Hkv, scale, window, long_from, err, stream);
   }
-#define FZ_U(NS_, MB_, SG_) return launch_units<HD, BOX, NS_, MB_, SG_>(q, k_pool, pool_rows, pos, seq_row, seg, table, mb, page_size, out, part_o, part_ml, N, Hq, Hkv, scale, window, NPU, long_from, single, maps, out32, err, stream)
+#define FZ_U(NS_, MB_, SG_) return launch_units<HD, BOX, NS_, MB_, SG_>(q, k_pool, pool_rows, pos, seq_row, seg, table, mb, page_size, out, part_o, part_ml, N, Hq, Hkv, scale, window, NPU, long_from, single, short_rows, maps, out32, err, stream)
   // three stages of 16 keys per warp and two CTAs per SM (eight warps with 24 KB in flight each) measured best
   if (Hq / Hkv > 8) FZ_U(3, 2, false);
   // So few units that every warp of one CTA per SM gets at most one (a single row at 4,096 keys): four stages, so that
@@ -1033,17 +1044,20 @@ FZ_API int fz_attn_decode_whole(int N, int Hq, int Hkv, int max_context, int sin
   return whole_rows(N, Hq, Hkv, fz_attn_partitions(max_context), single_tokens) ? 1 : 0;
 }
 
+FZ_API int fz_attn_combine_rows(int N, int single_tokens, int short_rows) { return combine_rows(N, single_tokens, short_rows); }
+
 // Float32 scratch the call needs: part_o N * Hq * NP * hd floats, part_ml N * Hq * NP * 2 floats.
 // maps 2: see the head of this file; out is not written, out32 (N * Hq * hd floats) is. maps 1: out32 null, or where the results
 // go as float32 instead of out.
 // single_tokens != 0: every portion of the step is one token (the caller knows; the kernel then reads no portion records).
+// short_rows: the rows that are of no long portion (it decides how the merge is launched, never the results).
 // kernels: on the host, how many kernels the call launched.
 // num_pages > 0 and a pool laid out as (pages, 2, Hkv, page_size, hd) with v_pool = k_pool + Hkv * page_size * hd select
 // the TMA variant where the page size allows it (8, 16 or a multiple of 16); otherwise the cp.async variant runs.
 FZ_API int fz_attn_decode(const void* q, const void* k_pool, const void* v_pool, const int* pos, const int* seq_row,
                           const int* seg, const int* table, int mb, long long page_stride, int page_size, void* out,
                           float* part_o, float* part_ml, int N, int Hq, int Hkv, int hd, float scale, int window,
-                          int max_context, int long_from, int single_tokens, int num_pages, int maps, float* out32, int* kernels,
+                          int max_context, int long_from, int single_tokens, int short_rows, int num_pages, int maps, float* out32, int* kernels,
                           int* err, cudaStream_t stream) {
   *kernels = 0;
   if (N <= 0) return FZ_OK;
@@ -1061,7 +1075,7 @@ FZ_API int fz_attn_decode(const void* q, const void* k_pool, const void* v_pool,
                       (long long)N * Hkv * NPU < (1LL << 30) && (size_t)NPU * 8 < 40 * 1024 && !getenv("FZB200_NO_TMA_ATTN");
   if (tma_ok) {
     const long long pool_rows = (long long)num_pages * 2 * Hkv * page_size;
-#define FZ_T(HD_, BOX_) return launch_tma<HD_, BOX_>(q, k_pool, pool_rows, pos, seq_row, seg, table, mb, page_size, out, part_o, part_ml, N, Hq, Hkv, scale, window, NPU, long_from, single, maps, out32, kernels, err, stream)
+#define FZ_T(HD_, BOX_) return launch_tma<HD_, BOX_>(q, k_pool, pool_rows, pos, seq_row, seg, table, mb, page_size, out, part_o, part_ml, N, Hq, Hkv, scale, window, NPU, long_from, single, short_rows, maps, out32, kernels, err, stream)
     if (hd == 64 && page_size == 8) FZ_T(64, 8);
     if (hd == 64) FZ_T(64, 16);
     if (page_size == 8) FZ_T(128, 8);

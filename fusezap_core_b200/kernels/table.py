@@ -642,8 +642,8 @@ class CudaOps(Ops):
                     _p(q), _p(k), _p(v), _p(meta.pos), _p(meta.seq_row), _p(meta.seg), _p(table), c_int(table.shape[1]),
                     c_longlong(page_stride), c_int(cache.page_size), _p(out), _p(part_o), _p(part_ml), c_int(n),
                     c_int(hq), c_int(hkv), c_int(hd), c_float(scale), c_int(window), c_int(meta.max_context),
-                    c_int(LONG_PORTION), c_int(1 if plan.single_tokens else 0), c_int(k.shape[0]), c_int(1), c_void_p(0), byref(kernels),
-                    _p(self.err), self._stream()),
+                    c_int(LONG_PORTION), c_int(1 if plan.single_tokens else 0), c_int(plan.n_short_rows), c_int(k.shape[0]), c_int(1),
+                    c_void_p(0), byref(kernels), _p(self.err), self._stream()),
                     "paged_attention (decode)", kv)
                 self.launches += kernels.value - 1
             if plan.n_tiles > 0 and self.prefill_tcgen05 and \
@@ -1317,7 +1317,7 @@ class CudaOps(Ops):
                 _p(q), _p(k), _p(v), _p(meta.pos), _p(meta.seq_row), _p(meta.seg), _p(table), c_int(table.shape[1]),
                 c_longlong(page_stride), c_int(cache.page_size), c_void_p(0), _p(part_o), _p(part_o[n * heads * parts * value_dim:]), c_int(n),
                 c_int(heads), c_int(num_kv_heads), c_int(value_dim), c_float(scale), c_int(0), c_int(meta.max_context), c_int(LONG_PORTION),
-                c_int(1), c_int(k.shape[0]), c_int(2), _p(rows_out), byref(kernels), _p(self.err), self._stream()),
+                c_int(1), c_int(n), c_int(k.shape[0]), c_int(2), _p(rows_out), byref(kernels), _p(self.err), self._stream()),
                 "differential_attention (decode)", nbytes)
             self.launches += kernels.value - 1
             self._combine_maps(rows_out, n, num_heads, value_dim, lam, eps, mult, meta, out)

@@ -268,3 +268,16 @@ def test_launches_of_a_decoded_row(context, bs, tma, kernels, monkeypatch):
     cu.paged_attention(q, cache, Meta([context - 1], [0], [list(range(pages))], "cuda"), torch.empty_like(q), 14, 2, hd, hd ** -0.5, 0)
     assert cu.launches - before == kernels
     cu.check_errors()
+
+
+@pytest.mark.parametrize("Hq,Hkv,hd", [(8, 2, 128), (3, 1, 64)])
+@pytest.mark.parametrize("rows,blocks", [([(r, 90, 7) for r in range(18)], 126),
+                                         ([(0, 10, 90), (1, 0, 60), (-1, 0, 1)] + [(r, 60 + r % 40, 1) for r in range(2, 92)], 91),
+                                         ([(0, 10, 90), (1, 99, 1)], 64)])
+def test_blocks_of_the_merge_kernel(Hq, Hkv, hd, rows, blocks):
+    """Short rows alone, many beside prompt rows and one: a block per row where most rows are short, else as many as there
+    are short rows, 64 at least."""
+    from fusezap_core_b200.kernels import cuda_ops
+    o, op, _ = run_both(Hq, Hkv, hd, 16, 0, [100] * len(rows), rows)
+    close(o, op, "merged rows")
+    assert cuda_ops("bfloat16").attn_tc.fz_attn_combine_rows(len(o), 0, run_both.last_plan.n_short_rows) == blocks
