@@ -38,8 +38,6 @@ constexpr int BM = 128;           // TMEM lanes = rows of the 128-row operand
 constexpr int BK = 64;            // k per stage: 64 bf16 = 128 bytes = one swizzle row
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;  // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
-constexpr int PAIR_PARTS = 4;            // the kernel with two SMs per tile: epilogue warps per quarter of the tensor-memory lanes
-constexpr int PAIR_THREADS_G = 64 + 128 * PAIR_PARTS;      // its threads: warps 2 and up are the epilogue
 
 // ---------------------------------------------------------------------------------------------- cluster helpers
 __device__ __forceinline__ void cluster_sync_all() {
@@ -661,7 +659,7 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (j >> 1) & 1));
       if (!ok) { flag[0] = 1; break; }
       tc_fence_after();
-      // (Four epilogue warps here. Eight, as in the two-SM kernel, were measured on this kernel and did not pay: the tiles
+      // (Four epilogue warps here. Eight, as in the two-SM kernel's plain epilogue, were measured on this kernel and did not pay: the tiles
       // it gets are narrow or few, and 2,048 tokens at Qwen2.5-0.5B sizes took 3.94 ms with them against 3.77 ms.)
       const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quad * 32) << 16);
       rows_store_tile<BN, 1>(p, taddr, tm * BM + r, tn * BN, 0);
@@ -765,7 +763,13 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t addr, uint32_t cols) 
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
 
-__global__ void __launch_bounds__(PAIR_THREADS_G, 1)
+// PARTS epilogue warps (warps 2 and up) per quarter of the tensor-memory lanes, each with its share of the tile's columns, so
+// that some compute while others wait: with one the epilogue of a tile took longer than the products of a tile with a short
+// K, 13 us at K = 896, where the products take 5. The gated epilogue takes four (two: 2,048 x 896 -> 9,728 43.7 us, 34.2 with
+// four; 1,024 x 4,096 -> 28,672 177, 172), the plain one, which mostly stores, two (4,096 x 256 -> 8,192 61.7 us, 66.9 with
+// four; 2,048 x 512 -> 2,048 11.5, 12.0; others the same with both).
+template <int PARTS>
+__global__ void __launch_bounds__(64 + 128 * PARTS, 1)
 gemm_tc_rows_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const Params p,
                          int tiles_m, int tiles_n) {
   constexpr int BN = PAIR_BN;
@@ -789,7 +793,7 @@ gemm_tc_rows_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8 * PAIR_PARTS); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 8 * PARTS); }
     flag[0] = 0;
     mbar_init_fence();
   }
@@ -873,12 +877,8 @@ gemm_tc_rows_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (j >> 1) & 1));
       if (!ok) { flag[0] = 1; break; }
       tc_fence_after();
-      // (PAIR_PARTS warps per quarter of the lanes, each with its share of the tile's columns, so that some compute while
-      // others wait: with one the epilogue of a tile took longer than the products of a tile with a short K, 13 us at
-      // K = 896, where the products take 5; with four instead of two a step of 2,101 rows at Qwen2.5-0.5B sizes takes 2.96
-      // ms instead of 3.12, and 2,048 rows at Llama-3.1-8B sizes, K = 4,096, the same as before)
       const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quad * 32) << 16);
-      rows_store_tile<BN, PAIR_PARTS>(p, taddr, (2 * tm + (int)rank) * BM + r, tn * BN, (warp - 2) >> 2);
+      rows_store_tile<BN, PARTS>(p, taddr, (2 * tm + (int)rank) * BM + r, tn * BN, (warp - 2) >> 2);
       tc_fence_before();
       __syncwarp();      // every lane of the warp has read its lane of the accumulator
       if (lane == 0) mbar_arrive_cluster(acc_empty0 + 8u * (uint32_t)acc);
@@ -894,19 +894,20 @@ gemm_tc_rows_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   if (threadIdx.x == 0 && flag[0]) atomicOr(p.err, FZ_ERR_WAIT_TIMEOUT);
 }
 
+template <int PARTS>
 int launch_rows_pair(const CUtensorMap& mx, const CUtensorMap& mw, const Params& p, int tiles_m, int tiles_n, int sms, cudaStream_t stream) {
   constexpr int STAGE_BYTES = (BM + PAIR_BN / 2) * BK * 2;
   const size_t smem = (size_t)p.stages * STAGE_BYTES + 1024 + 8 * (2 * p.stages + 4) + 16;
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_rows_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_rows_pair_kernel<PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     allowed = smem;
   }
   const int total = tiles_m * tiles_n, most = sms / 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (unsigned)(total < most ? total : most));
-  cfg.blockDim = dim3(PAIR_THREADS_G);
+  cfg.blockDim = dim3(64 + 128 * PARTS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -923,7 +924,7 @@ int launch_rows_pair(const CUtensorMap& mx, const CUtensorMap& mw, const Params&
   ++na;
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_rows_pair_kernel, mx, mw, p, tiles_m, tiles_n);
+  cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_rows_pair_kernel<PARTS>, mx, mw, p, tiles_m, tiles_n);
   if (le != cudaSuccess) return (int)le;
   FZ_LAUNCH_CHECK();
   return FZ_OK;
@@ -1511,7 +1512,7 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
     p.stages = (200 * 1024) / ((BM + PAIR_BN / 2) * BK * 2);
     if ((st = get_map_bf16(x, M, K, BM, &ma)) != FZ_OK) return st;
     if ((st = get_map_bf16(w, N, K, PAIR_BN / 2, &mb)) != FZ_OK) return st;
-    return launch_rows_pair(ma, mb, p, (M + 2 * BM - 1) / (2 * BM), (N + PAIR_BN - 1) / PAIR_BN, device_sms(), stream);
+    return (p.swiglu ? launch_rows_pair<4> : launch_rows_pair<2>)(ma, mb, p, (M + 2 * BM - 1) / (2 * BM), (N + PAIR_BN - 1) / PAIR_BN, device_sms(), stream);
   }
   {
     const int stage = (BM + bn) * BK * 2;
