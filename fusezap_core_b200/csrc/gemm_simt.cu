@@ -505,10 +505,10 @@ int launch_wide(const void* A, const void* W, const float* bias, void* C, int M,
   return FZ_OK;
 }
 
-// Two columns per lane (every value of A read once for both) where N still gives two blocks per SM.
+// Two columns per lane (every value of A read once for both) from 256 blocks on.
 template <typename TA, typename TC, int MR, bool VEC>
 int launch_few_n(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
-    if (N >= 4096) return launch_few<TA, TC, MR, 2, VEC, false>(A, W, bias, C, M, N, K, o, stream);
+  if (N >= 4096) return launch_few<TA, TC, MR, 2, VEC, false>(A, W, bias, C, M, N, K, o, stream);
   if constexpr (VEC)      // (asynchronous copies alone gain from depth)
     if ((N + 7) / 8 <= 148) return launch_few<TA, TC, MR, 1, VEC, true>(A, W, bias, C, M, N, K, o, stream);
   return launch_few<TA, TC, MR, 1, VEC, false>(A, W, bias, C, M, N, K, o, stream);
@@ -517,15 +517,19 @@ int launch_few_n(const void* A, const void* W, const float* bias, void* C, int M
 template <typename TA, typename TC, bool VEC>
 int launch_rows(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, cudaStream_t stream) {
   const Order o = order_of(N, K);
-  // Few rows read W at memory's pace up to 8 and still beat tiles at 16 (896 -> 9,728: 13 us at 8 rows, 26 at 16, tiles 42 at
-  // 17; 896 -> 151,936: 148, 345 and 254 us, the one size measured where tiles would win at 16). Tiles of 32 rows waste less
-  // than tiles of 64 up to 32 (43 against 62 us). Wide tiles from two blocks per SM on (see there).
+  // Few rows read W at memory's pace up to 8 and still beat tiles at 16 (16 rows: 896 -> 9,728 26 us, tiles 42 at 17; 896 -> 151,936
+  // 230 us, 251 at 17). Wide tiles from two blocks per SM on (see there).
   if (M <= 1) return launch_few_n<TA, TC, 1, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (M <= 2) return launch_few_n<TA, TC, 2, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (M <= 4) return launch_few_n<TA, TC, 4, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (M <= 8) return launch_few_n<TA, TC, 8, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (M <= 16) return launch_few_n<TA, TC, 16, VEC>(A, W, bias, C, M, N, K, o, stream);
-  if (M <= 32) return launch_tile<TA, TC, 4, VEC>(A, W, bias, C, M, N, K, o, stream);
+  // Tiles of 32 rows waste less than tiles of 64 up to 32 (43 against 62 us) and are done in half the time where all of them
+  // start at once: 200 x 97 -> 384 in bfloat16 6.9 us, 10.9 with 64 rows, 300 x 256 -> 96 6.5, 10.0; operands that are read one by
+  // one gain up to three per SM (64 x 897 -> 9,728, 304 tiles, 92, 112; 128 x 897 -> 1,152, 504, loses 23, 30), the others lose
+  // in places (64 x 4,864 -> 896, 224 tiles, 32, 29).
+  const long long tiles32 = (long long)((M + 31) / 32) * ((N + TILE_N - 1) / TILE_N) * o.groups;
+  if (M <= 32 || tiles32 <= (VEC ? 148 : 444)) return launch_tile<TA, TC, 4, VEC>(A, W, bias, C, M, N, K, o, stream);
   if (o.groups == 1 && (long long)((M + 63) / 64) * ((N + WIDE_N - 1) / WIDE_N) >= 296)
     return launch_wide<TA, TC, VEC>(A, W, bias, C, M, N, K, o, stream);
   return launch_tile<TA, TC, 8, VEC>(A, W, bias, C, M, N, K, o, stream);

@@ -55,6 +55,36 @@ def test_linear(N, K):
     assert torch.equal(out[:3], full[:3]) and torch.equal(out[4:], full[4:20]) and not bool(out[3].isfinite().any())
 
 
+@pytest.mark.parametrize("dtype,N,K", [("float32", 16385, 1028), ("float32", 16385, 1030), ("float32", 9500, 33), ("float32", 384, 96),
+                                       ("bfloat16", 9500, 33), ("bfloat16", 9500, 1030), ("bfloat16", 384, 97), ("bfloat16", 100, 17)])
+def test_linear_bits_in_every_kernel(dtype, N, K):
+    """The bits of few rows from tiles of 32 and of 64 rows and from the wide tiles, with K off whole stages, chunks longer
+    than 32 and operands that are read one by one, misaligned ones among them."""
+    from fusezap_core_b200.kernels import cuda_ops
+    dt = torch.float32 if dtype == "float32" else torch.bfloat16
+    cu = cuda_ops(dtype)
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    rows = 400
+    a = torch.randn(rows, K, generator=g, device="cuda").to(dt)
+    w = torch.randn(N, K, generator=g, device="cuda").to(dt)
+    few = torch.empty(rows, N, device="cuda")
+    for r in range(0, rows, 16):
+        cu.linear(a[r:r + 16].contiguous(), w, None, few[r:r + 16])
+    steps = 32 * -(-K // 1024) + 41      # (as above)
+    bound = steps * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T)
+    assert bool(((few.double() - a.double() @ w.double().T).abs() <= bound).all())
+    for m in (33, 64, 200, 400):
+        out = torch.full((m + 1, N), float("nan"), device="cuda")
+        cu.linear(a[:m].contiguous(), w, None, out[:m])
+        assert torch.equal(out[:m], few[:m]) and bool(out[m].isnan().all()), f"{m} rows"
+    off_a, off_w = torch.empty(200 * K + 1, dtype=dt, device="cuda")[1:].view(200, K), torch.empty(N * K + 1, dtype=dt, device="cuda")[1:].view(N, K)
+    off_a.copy_(a[:200])
+    off_w.copy_(w)
+    out = torch.empty(200, N, device="cuda")
+    cu.linear(off_a, off_w, None, out)
+    assert torch.equal(out, few[:200])
+
+
 def test_linear_from_two_threads():
     """Products whose blocks need different amounts of shared memory, first called by two threads at once in a process that
     has launched none of them (the limit of a kernel's shared memory is set at its first call)."""
