@@ -284,7 +284,7 @@ attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T*
 #pragma unroll
     for (int a = 0; a < PW; ++a) {
       const bool live = j_from[a] <= j_to[a];
-      top[a] = fmaxf(m[a], top[a]);       // finite: every chunk walked holds at least one visible key
+      top[a] = fmaxf(m[a], top[a]);       // finite where the pair's row sees a key of the chunk; else nothing below uses it
       const float pj = lane >= j_from[a] && lane <= j_to[a] ? expf(sc[a] - top[a]) : 0.f;
       corr[a] = live ? expf(m[a] - top[a]) : 1.f;               // 0 for the first chunk of a span (m = -inf)
       sum[a] = pj;

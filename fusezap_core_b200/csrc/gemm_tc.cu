@@ -1448,8 +1448,8 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
       if (p.stages > enough) p.stages = enough;
       // A matrix that the rings of all its CTAs hold whole (up to 24 MB of 148 x 227 KB): then every weight is on its way
       // before the wait on the kernel before, and what follows the wait is the activations, the sums and the store alone.
-      // Qwen2.5-0.5B sizes: a decode step of one row 757 -> 746 us, of 32 rows 1,072 -> 1,059 us. Larger ones would only
-      // keep the next kernels' blocks off the SMs. (At least three stages: they also hold the sums of 128 columns and the
+      // Qwen2.5-0.5B sizes, 300 keys: a decode step of one row 684 -> 668 us, of 8 726 -> 722, of 32 905 -> 900, of 64 the same.
+      // Larger ones would only keep the next kernels' blocks off the SMs. (At least three stages: they also hold the sums of 128 columns and the
       // exchange of the gated epilogue, 72 KB.)
       const long long ring = (long long)per_cta * (BM + bn) * BK * 2;
       if (ring <= 200 * 1024 && ring * tiles * p.splits <= 24 << 20) p.stages = per_cta < 3 ? 3 : per_cta;
