@@ -421,13 +421,8 @@ int launch(const void* q, const void* k_pool, const void* v_pool, void* out, Arg
   const size_t smem = block.smem;
   A.buffers = block.buffers;
   auto kern = attn_simt_kernel<T, DPL, PW, VEC, SPLIT>;
-  static size_t allowed = 48 * 1024;   // per instantiation: the attribute is raised outside any capture (a step runs once before)
-  if (smem > allowed) {
-    if (smem > 227 * 1024) return FZ_TOO_LARGE;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    allowed = smem;
-  }
+  if (smem > (size_t)FZ_MOST_SMEM) return FZ_TOO_LARGE;
+  FZ_RAISE_SMEM(kern);
   cudaLaunchConfig_t cfg = {};
   const long long along_x = (long long)A.N * A.slices;
   if (along_x > 2147483647LL) return FZ_TOO_LARGE;

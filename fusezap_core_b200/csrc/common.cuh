@@ -119,6 +119,16 @@ inline cudaError_t fz_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// All the shared memory that a block may have, as the limit of a kernel without static shared memory whose need differs from
+// call to call: set once per kernel. (A limit raised step by step to each call's need can be lowered again by another thread's
+// smaller call between the check and the launch.)
+constexpr int FZ_MOST_SMEM = 227 * 1024;
+#define FZ_RAISE_SMEM(kern)                                                                                                    \
+  do {                                                                                                                         \
+    static const cudaError_t raised__ = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FZ_MOST_SMEM); \
+    if (raised__ != cudaSuccess) return (int)raised__;                                                                         \
+  } while (0)
+
 template <typename T> struct Cvt;
 template <> struct Cvt<float> {
   static __device__ __forceinline__ float to_f(float v) { return v; }

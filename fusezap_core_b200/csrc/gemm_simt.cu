@@ -439,16 +439,6 @@ gemm_simt_wide_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const 
   }
 }
 
-// All the shared memory a block may have, as the limit of a kernel whose need differs from call to call: set once per
-// instantiation. (A limit raised step by step to each call's need can be lowered again by another thread's smaller call
-// between the check and the launch.)
-constexpr int MOST_SMEM = 227 * 1024;
-#define FZ_RAISE_SMEM(kern)                                                                                                  \
-  do {                                                                                                                       \
-    static const cudaError_t raised__ = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SMEM);  \
-    if (raised__ != cudaSuccess) return (int)raised__;                                                                       \
-  } while (0)
-
 template <typename TA, typename TC, int MR, int RPL, bool VEC, bool DEEP>
 int launch_few(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, Order o, cudaStream_t stream) {
   using F = Few<MR, RPL, DEEP>;

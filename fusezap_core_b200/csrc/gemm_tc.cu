@@ -680,12 +680,7 @@ template <int BN>
 int launch_rows(const CUtensorMap& mx, const CUtensorMap& mw, const Params& p, int tiles_m, int tiles_n, cudaStream_t stream) {
   constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
   const size_t smem = (size_t)p.stages * STAGE_BYTES + 1024 + 8 * (2 * p.stages + 4) + 16;
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_rows_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    allowed = smem;
-  }
+  FZ_RAISE_SMEM(gemm_tc_rows_kernel<BN>);
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
@@ -898,12 +893,7 @@ template <int PARTS>
 int launch_rows_pair(const CUtensorMap& mx, const CUtensorMap& mw, const Params& p, int tiles_m, int tiles_n, int sms, cudaStream_t stream) {
   constexpr int STAGE_BYTES = (BM + PAIR_BN / 2) * BK * 2;
   const size_t smem = (size_t)p.stages * STAGE_BYTES + 1024 + 8 * (2 * p.stages + 4) + 16;
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_rows_pair_kernel<PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    allowed = smem;
-  }
+  FZ_RAISE_SMEM(gemm_tc_rows_pair_kernel<PARTS>);
   const int total = tiles_m * tiles_n, most = sms / 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (unsigned)(total < most ? total : most));
@@ -1146,12 +1136,7 @@ int launch_rows_split(const CUtensorMap& mx, const CUtensorMap& mw, const Params
   constexpr int STAGE_BYTES = (BM + (PAIR ? SPLIT_BN / 2 : SPLIT_BN)) * BK * 2;
   const size_t ring = (size_t)p.stages * STAGE_BYTES, partial = (size_t)BM * SPLIT_LD * 4;
   const size_t smem = (ring > partial ? ring : partial) + 1024 + 8 * (2 * p.stages + 1) + 16;
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_rows_split_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    allowed = smem;
-  }
+  FZ_RAISE_SMEM(gemm_tc_rows_split_kernel<PAIR>);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((PAIR ? 2 : 1) * tiles_m, tiles_n, p.splits);      // PAIR: tiles_m counts tiles of 256 rows
   cfg.blockDim = dim3(NUM_THREADS);
@@ -1182,12 +1167,7 @@ template <int BN>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, dim3 grid, cudaStream_t stream) {
   constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
   const size_t smem = (size_t)p.stages * STAGE_BYTES + 1024 + 8 * (2 * p.stages + 1) + 16;
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    allowed = smem;
-  }
+  FZ_RAISE_SMEM(gemm_tc_kernel<BN>);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(NUM_THREADS);

@@ -116,6 +116,55 @@ assert not bad, bad
     subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
 
 
+def test_attention_and_bfloat16_products_from_two_threads():
+    """The same of the 32-bit attention's kernels, whose blocks need more or less by head size, heads and rows, and of the
+    tensor-core products, whose rings are as deep as K asks for."""
+    code = """
+import threading, torch
+from fusezap_core_b200.kernels.table import CudaOps
+from test_float32_kernels_gpu import thread_calls
+torch.zeros(1, device="cuda")
+meet, bad = threading.Barrier(2), []
+def work(order):
+    ops = {t: CudaOps(t, "cuda:0") for t in ("float32", "bfloat16")}
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for call, args in order:
+            meet.wait(60)
+            if not call(ops, *args): bad.append((call.__name__, args))
+def guarded(order):
+    try: work(order)
+    except BaseException as e:
+        bad.append(repr(e)); meet.abort()
+calls = thread_calls()
+threads = [threading.Thread(target=guarded, args=(o,)) for o in (calls, calls[::-1])]
+for t in threads: t.start()
+for t in threads: t.join()
+assert not bad, bad
+"""
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join(p for p in sys.path if p))
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, timeout=300)
+
+
+def thread_calls():
+    def product(ops, m, n, k):
+        a, w = (torch.ones(r, k, dtype=torch.bfloat16, device="cuda") for r in (m, n))
+        out = torch.empty(m, n, dtype=torch.float32, device="cuda")
+        ops["bfloat16"].linear(a, w, None, out)
+        return bool((out == k).all())
+
+    def attention(ops, rows, heads, hd):
+        cache = make_cache(20, heads, 16, hd, torch.float32, "cuda")
+        cache.pool.fill_(1.0)
+        q = torch.ones(rows, 2 * heads * hd, device="cuda")
+        out = torch.empty_like(q)
+        ops["float32"].paged_attention(q, cache, Meta(list(range(300 - rows, 300)), [0] * rows, [list(range(20))], "cuda"), out,
+                                       2 * heads, heads, hd, hd ** -0.5, 0)
+        return bool(((out - 1.0).abs() < 1e-5).all())
+
+    return [(product, (m, n, k)) for m in (1, 20, 40, 100, 200) for n, k in ((256, 128), (896, 896), (896, 4864), (9728, 896))] \
+        + [(attention, (rows, heads, hd)) for rows in (1, 40, 300) for heads in (1, 4) for hd in (40, 48, 56, 64, 72, 96, 128, 160, 256)]
+
+
 def thread_sizes():
     return [(m, n, k) for m in (1, 3, 8, 16, 32, 64) for n, k in ((64, 64), (896, 896), (896, 4864), (9728, 896))]
 
