@@ -966,8 +966,8 @@ FZ_API int fz_sample(const float* logits, const float* temperature, const double
 // slices (`sample_slices`), shared by the BLOCKS blocks of 1,024 threads of a cluster (`fz_sample_blocks`): bound by the
 // instructions per token and pass, so the SMs at work are what counts. Sums run over a slice first, then over the slices in
 // order, through distributed shared memory where they are several blocks', and all blocks then take the same decisions. us
-// with top-p, one block per row and slice (the kernel before) -> now: 151,936 tokens, 8 rows 378 -> 84, 32 rows 397 -> 141, 64
-// rows 569 -> 352, 96 rows 615 -> 448, 148 rows 665 -> 745; 32,000 tokens, 8 rows 98 -> 52, 64 rows 100 -> 82, 128 rows 101 -> 130.
+// with top-p, one block per row and slice (the kernel before) -> now: 151,936 tokens, 8 rows 378 -> 83, 32 rows 395 -> 138, 64
+// rows 566 -> 350, 96 rows 613 -> 436, 148 rows 665 -> 736; 32,000 tokens, 8 rows 93 -> 49, 64 rows 100 -> 78, 128 rows 102 -> 122.
 // Nothing is sorted: the thresholds are found by radix selection over an order-preserving 32-bit key of the logit,
 // eight passes of 4 bits, with a histogram of counts for top-k and of probability mass (float64) for top-p. Each thread
 // fills 16 bins of its own in shared memory and the bins are then summed over the threads in a fixed order, so there
@@ -993,13 +993,15 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* s_part) {
   return run;
 }
 
-// bins[b * SF_THREADS + t]: thread t's share of bin b. Leaves the sums over the threads in total[0..15].
+// bins[b * SF_THREADS + t]: thread t's share of bin b. Leaves the sums over the threads in total[0..15]. used: in shared
+// memory, the bins in which any thread has something (the others' sums are zero); null: all.
 template <typename T>
-__device__ __forceinline__ void sum_bins(const T* bins, T* s_part, T* total) {
+__device__ __forceinline__ void sum_bins(const T* bins, T* s_part, T* total, const unsigned int* used = nullptr) {
   __syncthreads();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, b = w & (SF_BINS - 1), half = w >> 4;
   T acc = 0;
-  for (int j = 0; j < SF_THREADS / 64; ++j) acc += bins[b * SF_THREADS + half * (SF_THREADS / 2) + j * 32 + lane];
+  if (!used || (*used >> b & 1u))
+    for (int j = 0; j < SF_THREADS / 64; ++j) acc += bins[b * SF_THREADS + half * (SF_THREADS / 2) + j * 32 + lane];
   for (int o = 16; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if (lane == 0) s_part[w] = acc;
   __syncthreads();
@@ -1078,7 +1080,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
   __shared__ int s_best_at[1], s_ties[1];
   __shared__ int s_wties[PER][32];
   __shared__ uint32_t s_prefix;
-  __shared__ unsigned int s_rank;
+  __shared__ unsigned int s_rank, s_used[2];
   __shared__ double s_need, s_target;
   __shared__ int s_warp, s_slice;
   const cg::cluster_group cluster = cg::this_cluster();
@@ -1170,24 +1172,29 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
     __syncthreads();
     need_at_t = s_need;
   } else {
-    if (tid == 0) s_prefix = first == 0 ? 0u : top_key >> (32 - 4 * first);
+    if (tid == 0) {
+      s_prefix = first == 0 ? 0u : top_key >> (32 - 4 * first);
+      s_used[0] = 0u;
+    }
+    unsigned int mine = (1u << SF_BINS) - 1u;      // the bins in which this thread has, or may have, something
+    int side = 0;
     for (int pass = first; pass < 8; ++pass) {
       const int shift = 28 - 4 * pass;
       __syncthreads();
       const uint32_t prefix = s_prefix;
-      bool zeroed = false;
       for (int j = 0; j < PER; ++j) {
         const int s_lo = min(V, lo + j * slice), s_hi = min(V, s_lo + slice);
-        if (!zeroed)
-          for (int b = 0; b < SF_BINS; ++b) bins_d[b * SF_THREADS + tid] = 0.0;
-        bool any = pass == first;
+        for (; mine; mine &= mine - 1) bins_d[(__ffs(mine) - 1) * SF_THREADS + tid] = 0.0;
         if (pass == first) {
           double local = 0.0;
           for_each_key(row, s_lo, s_hi, [&](int i, float x, uint32_t key) {
             const double v = key <= k_key ? exp((double)x / (double)T - mx) : 0.0;
             e[i] = v;
             local += v;
-            if (key <= k_key) bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += v;
+            if (key <= k_key) {
+              bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += v;
+              mine |= 1u << ((key >> shift) & 15u);
+            }
           });
           local = block_sum_fixed(local, s_part);
           if (tid == 0) s_sum[turn][j][0] = local;
@@ -1195,14 +1202,16 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
           for_each_key(row, s_lo, s_hi, [&](int i, float, uint32_t key) {
             if (key <= k_key && (key >> (shift + 4)) == prefix) {
               bins_d[((key >> shift) & 15u) * SF_THREADS + tid] += e[i];
-              any = true;
+              mine |= 1u << ((key >> shift) & 15u);
             }
           });
         }
-        // (the last digits match in few slices: the bins of the others are all zero still)
-        zeroed = PER > 1 && !__syncthreads_or(any);
-        if (!zeroed) sum_bins(bins_d, s_part, s_mass[turn][j]);
-        else if (tid < SF_BINS) s_mass[turn][j][tid] = 0.0;
+        // (from the third digit on a slice has few bins with anything in them: only these are summed and cleared)
+        const unsigned int in_warp = __reduce_or_sync(0xffffffffu, mine);
+        if (lane == 0 && in_warp) atomicOr(&s_used[side], in_warp);
+        side ^= 1;
+        if (tid == 0) s_used[side] = 0u;      // (the next slice's; its last readers passed the last sum's barriers)
+        sum_bins(bins_d, s_part, s_mass[turn][j], &s_used[side ^ 1]);
       }
       if (pass == first) {
         total = slices_sum<SLICES, BLOCKS>(s_sum[turn]);
@@ -1361,14 +1370,14 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
 
 // The slices that a row's sums are taken over: by V alone, so that a row's token does not depend on the rows beside it. As many
 // as few rows gain from while a block that has to walk all of them loses little. us for 14 and 128 rows, top-p, with one slice
-// and with more: 8,192 tokens 37, 37 | 2 slices 42, 53; 12,000 49, 51 | 2: 46, 62; 16,384 59, 61 | 2: 51, 71 | 4: 43, 97; 32,000 99,
+// and with more (each slice beyond the first has cost a block about a quarter less since its bins are summed by use): 8,192 tokens 37, 37 | 2 slices 42, 53; 12,000 49, 51 | 2: 46, 62; 16,384 59, 61 | 2: 51, 71 | 4: 43, 97; 32,000 99,
 // 104 | 2: 71, 110 | 4: 52, 130 | 8: 45, 181; 65,536 2: 114, 242 | 4: 74, 264 | 8: 55, 306; 151,936 4: 131, 658 | 8: 85, 717.
 static int sample_slices(int V) { return V <= 12288 ? 1 : V <= 24576 ? 2 : V <= 98304 ? 4 : 8; }
 
 // Blocks per row (a cluster): a block has an SM to itself, and the rows should not queue for SMs. 14 clusters of eight, 32 of
 // four and 74 of two are on the chip at once (16 of eight and 36 of four take twice as long). With more rows one block
-// each, except that three rounds of fours still beat one of whole rows of eight slices: 96 rows of 151,936 448 against 686
-// us (top-k and top-p 463, 525), 128 rows 592, 718 (612, 541).
+// each, except that three rounds of fours still beat one of whole rows of eight slices: 96 rows of 151,936 436 against 686
+// us (top-k and top-p 448, 525), 128 rows 592, 712 (612, 539).
 FZ_API int fz_sample_blocks(int R, int V) {
   const int slices = sample_slices(V), most = R <= 14 ? 8 : R <= 32 ? 4 : R <= 74 ? 2 : R <= 96 && slices == 8 ? 4 : 1;
   return slices < most ? slices : most;
