@@ -32,12 +32,6 @@ constexpr int MAX_ROWS = 8;                    // rows of a block (a power of tw
 // (row, head) pairs per warp: what fits in registers beside DPL output dimensions per lane, twice
 template <int DPL> struct Pairs { static constexpr int PER_WARP = DPL <= 4 ? 4 : DPL <= 8 ? 2 : 1; };
 
-__device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = ok ? 16 : 0;      // 0: the 16 bytes are filled with zeros and nothing is read
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-
 __device__ __forceinline__ float4 four(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float4 four(const __nv_bfloat16* p) {
   const uint2 v = *reinterpret_cast<const uint2*>(p);
@@ -164,7 +158,7 @@ attn_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, const T*
         for (int e = lane * PAD; e < 2 * hd; e += 32 * PAD) {
           const bool is_k = e < hd;
           const int d = is_k ? e : e - hd;
-          cp16(is_k ? Ks + j * ks + d : Vs + j * hdp + d, (is_k ? k_pool : v_pool) + off + d, ok);
+          fz_copy16(is_k ? Ks + j * ks + d : Vs + j * hdp + d, (is_k ? k_pool : v_pool) + off + d, ok);
         }
       }
     } else if (c <= c_last) {

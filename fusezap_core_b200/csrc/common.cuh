@@ -119,6 +119,13 @@ inline cudaError_t fz_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// 16 bytes to shared memory, asynchronously; zeros and nothing read where not `ok`.
+__device__ __forceinline__ void fz_copy16(void* dst, const void* src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = ok ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
 // All the shared memory that a block may have, as the limit of a kernel without static shared memory whose need differs from
 // call to call: set once per kernel. (A limit raised step by step to each call's need can be lowered again by another thread's
 // smaller call between the check and the launch.)

@@ -33,11 +33,6 @@ Order order_of(int N, int K) {
   return o;
 }
 
-__device__ __forceinline__ void cp16(float* dst, const float* src, bool ok) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = ok ? 16 : 0;      // 0: the 16 bytes are filled with zeros and nothing is read
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -47,7 +42,7 @@ template <typename T, bool VEC>
 __device__ __forceinline__ void stage4(float* dst, const T* base, long long row, int K, int k, int k_end, bool row_ok) {
   if constexpr (VEC) {
     const bool ok = row_ok && k < k_end;
-    cp16(dst, ok ? base + row * K + k : base, ok);
+    fz_copy16(dst, ok ? base + row * K + k : base, ok);
   } else {
 #pragma unroll
     for (int i = 0; i < 4; ++i) dst[i] = row_ok && k + i < k_end ? Cvt<T>::to_f(base[row * K + k + i]) : 0.f;
@@ -538,7 +533,7 @@ FZ_API int fz_gemm_simt(const void* A, const void* W, const float* bias, void* C
                         int N, int K, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return FZ_OK;
   if (K <= 0) return FZ_BAD_SHAPE;
-  if ((long long)((N + 63) / 64) > 2147483647LL || (M + 15) / 16 > 65535) return FZ_TOO_LARGE;
+  if (M > 16 * 65535) return FZ_TOO_LARGE;      // (rows and their tiles are counted in int)
   if (in_dtype == FZ_F32 && out_dtype == FZ_F32) return launch<float, float>(A, W, bias, C, M, N, K, stream);
   if (in_dtype == FZ_BF16 && out_dtype == FZ_F32) return launch<__nv_bfloat16, float>(A, W, bias, C, M, N, K, stream);
   if (in_dtype == FZ_BF16 && out_dtype == FZ_BF16) return launch<__nv_bfloat16, __nv_bfloat16>(A, W, bias, C, M, N, K, stream);

@@ -1370,8 +1370,9 @@ sample_filtered_kernel(const float* __restrict__ logits, const float* __restrict
 
 // The slices that a row's sums are taken over: by V alone, so that a row's token does not depend on the rows beside it. As many
 // as few rows gain from while a block that has to walk all of them loses little. us for 14 and 128 rows, top-p, with one slice
-// and with more (each slice beyond the first has cost a block about a quarter less since its bins are summed by use): 8,192 tokens 37, 37 | 2 slices 42, 53; 12,000 49, 51 | 2: 46, 62; 16,384 59, 61 | 2: 51, 71 | 4: 43, 97; 32,000 99,
-// 104 | 2: 71, 110 | 4: 52, 130 | 8: 45, 181; 65,536 2: 114, 242 | 4: 74, 264 | 8: 55, 306; 151,936 4: 131, 658 | 8: 85, 717.
+// and with more (each slice beyond the first has cost a block about a quarter less since its bins are summed by use):
+// 8,192 tokens 37, 37 | 2 slices 42, 53; 12,000 49, 51 | 2: 46, 62; 16,384 59, 61 | 2: 51, 71 | 4: 43, 97; 32,000 99, 104 | 2: 71,
+// 110 | 4: 52, 130 | 8: 45, 181; 65,536 2: 114, 242 | 4: 74, 264 | 8: 55, 306; 151,936 4: 131, 658 | 8: 85, 717.
 static int sample_slices(int V) { return V <= 12288 ? 1 : V <= 24576 ? 2 : V <= 98304 ? 4 : 8; }
 
 // Blocks per row (a cluster): a block has an SM to itself, and the rows should not queue for SMs. 14 clusters of eight, 32 of
