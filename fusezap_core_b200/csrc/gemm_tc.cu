@@ -20,11 +20,12 @@
 //           stage's completion to its empty barrier, the last one to the accumulator-ready barrier;
 //   warps 2-5  read the accumulator with tcgen05.ld (each warp its own 32 lanes), add the bias and store.
 // Split K (swap mode; the count is chosen from N and K only, never from M): the splits of a tile form one thread-block
-// cluster. Each CTA leaves its float32 partial tile in its own shared memory; after a cluster barrier CTA r adds, for
-// the columns r, r + S, ..., the partials of all splits in split order 0, 1, 2, ... through distributed shared memory and
-// stores the result. The sum has one fixed order (as the reference's split-K has: wgmma.py:209-239) and no partial ever
-// goes to global memory. Waits on this CTA's own mbarriers are bounded by a time limit after which the kernel sets an
-// error bit and leaves; the cluster barriers are hardware barriers, not spins.
+// cluster. The tokens go in groups of one or four to the CTAs of the cluster: every CTA sends each CTA its float32
+// partial sums of that CTA's tokens (`st.async` from registers into the other's shared memory, the bytes counted on a
+// barrier there), and each CTA adds the splits' partials of its own tokens in split order 0, 1, 2, ... and stores the
+// result. The sum has one fixed order (as the reference's split-K has: wgmma.py:209-239) and no partial ever goes to
+// global memory. Waits on this CTA's own mbarriers are bounded by a time limit after which the kernel sets an error bit
+// and leaves; the cluster barriers are hardware barriers, not spins.
 // Epilogues besides bias + store: SwiGLU over weight rows packed as [64 gate | 64 up] blocks (both modes); for few
 // tokens the rotation of the q and k heads with the write of k and v into the paged cache, and a per-tile argmax that
 // stores no products at all (the lm_head of a greedy step).
@@ -49,20 +50,51 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// The float at shared-memory address `addr` of the cluster's CTA `rank`
-__device__ __forceinline__ float ld_dsmem(uint32_t addr, uint32_t rank) {
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// The cluster address of shared-memory address `addr` in the cluster's CTA `rank`
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
   uint32_t remote;
-  float v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-  // (volatile keeps it behind the cluster barrier, itself a volatile asm; no memory clobber, so that the loads of the
-  // next column may be issued before this column's result is stored)
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote));
-  return v;
+  return remote;
+}
+// VW floats to a cluster address, their bytes counted on the barrier at `bar` of the same CTA.
+template <int VW>
+__device__ __forceinline__ void send_floats(uint32_t to, uint32_t bar, const float* v) {
+  if constexpr (VW == 4)
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(to), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar) : "memory");
+  else
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];"
+                 ::"r"(to), "f"(v[0]), "r"(bar) : "memory");
+}
+// `mbar_wait` for bytes that other CTAs of the cluster send. They send whatever happens to their own waits, at the latest
+// when these have given up; this CTA waits longer than that, so that it is there when they do.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
+  const uint32_t addr = smem_u32(bar);
+  unsigned long long t0 = 0;
+  for (uint32_t spins = 0;; ++spins) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+    if (done) return true;
+    if ((spins & 1023u) == 1023u) {
+      const unsigned long long now = global_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > 5 * WAIT_LIMIT_NS) return false;
+    }
+  }
 }
 // The gated activation of the fused gate/up product. kind 1: silu(g) * u; 2: the tanh form of gelu,
 // 0.5 g (1 + tanh(sqrt(2 / pi) (g + 0.044715 g^3))) * u.
+__device__ __noinline__ float gelu_mul(float g, float u) {
+  return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
+}
 __device__ __forceinline__ float glu_mul(float g, float u, int kind) {
-  if (kind == 2) return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
+  if (kind == 2) return gelu_mul(g, u);
   return g / (1.0f + __expf(-g)) * u;
 }
 // (value, index) order of numpy.argmax: a NaN is the maximum, among equals the lower index wins; index 0x7fffffff: none
@@ -84,12 +116,12 @@ struct Params {
   int rows;                // token rows (M of the product)
   int feats;               // output features (N of the product)
   int K;
-  int swap;                // 1: lanes are features, columns are token rows
   int splits;
   int stages;
+  int parts_in_ring;       // few tokens: the partial sums arrive in the ring's memory (after a cluster barrier), not in memory of their own
   int vec_ok;              // rows mode: C rows are 16-byte aligned, so full groups of 16 columns go out as vectors
   int swiglu;              // W holds [64 gate rows | 64 up rows] blocks: store silu(gate) * up as bf16 [rows, feats / 2]
-  // rope != 0 (swap mode, hd divides 128): the features are [q heads | k heads | v heads] of size hd; q and k are rotated
+  // rope != 0 (few tokens, hd divides 128): the features are [q heads | k heads | v heads] of size hd; q and k are rotated
   // by the token's position, q goes to c_bf16 [rows, Hq * hd], k and v to the token's slot of the paged pool
   int rope;
   const float* cos_t;      // [max_len, hd / 2]
@@ -117,107 +149,179 @@ __device__ __forceinline__ float finished(const Params& p, float y) {
   return y * y;
 }
 
-template <int BN>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+// ---------------------------------------------------------------------------------------------- few tokens
+// Partial sums of a tile lie as [split][group of the receiving CTA][feature of the tile][token of the group]: group g of VW
+// tokens goes to rank g % splits, as its (g / splits)-th; 32 lanes of a warp, one feature each, send 128 VW neighbouring bytes.
+// Groups of four, of one where a cluster has a CTA for every token: the parts then take a quarter of the memory (with 16 KB of
+// parts the O product's CTAs at Llama-3.1-8B sizes do not all fit the SMs at once: 7.8 -> 11.9 us at one row).
+__host__ __device__ inline int parts_slots(int cols, int splits, int vw) { return ((cols + vw - 1) / vw + splits - 1) / splits; }
+__device__ __forceinline__ int parts_mine(int cols, int splits, int vw, int rank) { return ((cols + vw - 1) / vw - rank + splits - 1) / splits; }
+
+// Where a thread's pair of features of one token goes (null: nowhere) and the angle that it is turned by. `turn` 0: zeros, 1: as
+// it is, 2: turned.
+struct Place { __nv_bfloat16* dst; float cs, sn; int turn; };
+
+// The sums over the splits, in split order, of one, two or four neighbouring tokens of a group at one feature
+__device__ __forceinline__ void add(float& a, float b) { a += b; }
+__device__ __forceinline__ void add(float2& a, float2 b) { a.x += b.x; a.y += b.y; }
+__device__ __forceinline__ void add(float4& a, float4 b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+template <int NV> struct Vec;
+template <> struct Vec<1> { typedef float type; };
+template <> struct Vec<2> { typedef float2 type; };
+template <> struct Vec<4> { typedef float4 type; };
+template <int NV>
+__device__ __forceinline__ void sum_parts(const float* at, int splits, int step, float* out) {
+  typedef typename Vec<NV>::type V;
+  V v[8], acc{};
+#pragma unroll
+  for (int sp = 0; sp < 8; ++sp)
+    if (sp < splits) v[sp] = *(const V*)(at + sp * step);
+#pragma unroll
+  for (int sp = 0; sp < 8; ++sp)
+    if (sp < splits) add(acc, v[sp]);
+  *(V*)out = acc;
+}
+
+// The epilogue of a tile, as far as it is known when the kernel is compiled (a kernel that held all of them was 80 KB of
+// code and took its instructions from L2 on every launch of a decode step).
+enum { EP_PLAIN = 0, EP_GLU = 1, EP_ROPE = 2, EP_ARGMAX = 3 };
+
+// (Three or four CTAs to an SM as far as registers go. With 160 a thread, two CTAs took all of an SM's registers and the blocks of
+// the kernels after this one could not become resident beside them: a decode step of 64 rows at Llama-3.1-8B sizes 7,730 ->
+// 8,090 us.)
+template <int BN, int EP, int VW>
+__global__ void __launch_bounds__(NUM_THREADS, 4)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
   extern __shared__ uint8_t smem_raw[];
-  // stages of [A: 128 x 64 bf16][B: BN x 64 bf16], 1024-byte aligned for the swizzle
+  // stages of [A: 128 x 64 bf16][B: BN x 64 bf16], 1024-byte aligned for the swizzle; what the other CTAs send, unless it
+  // goes into the stages; the barriers
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
-  uint64_t* full = (uint64_t*)(smem + (size_t)p.stages * STAGE_BYTES);
+  constexpr bool PAIRS = EP == EP_GLU || EP == EP_ROPE;      // two features of a tile are finished together
+  const int cols = p.rows;      // token rows of the step: at most BN
+  const int tile = blockIdx.x, split = blockIdx.z;      // (the splits are the cluster: this CTA's rank is its split)
+  constexpr int PART_GROUP = BM * VW, CV = VW > 1 ? VW / 2 : 1;      // floats of a group; tokens of it that one of two threads finishes
+  const int slots = parts_slots(cols, p.splits, VW), mine = parts_mine(cols, p.splits, VW, split), part_step = slots * PART_GROUP;
+  float* parts = (float*)(smem + (p.parts_in_ring ? 0 : p.stages * STAGE_BYTES));
+  uint64_t* full = (uint64_t*)(smem + p.stages * STAGE_BYTES + (p.parts_in_ring ? 0 : p.splits * part_step * 4));
   uint64_t* empty = full + p.stages;
   uint64_t* acc_ready = empty + p.stages;
-  uint32_t* tmem_slot = (uint32_t*)(acc_ready + 1);
-  int* flag = (int*)(tmem_slot + 1);     // [0]: this CTA arrived last at its tile  [1]: a wait gave up
+  uint64_t* parts_here = acc_ready + 1;
+  uint32_t* tmem_slot = (uint32_t*)(parts_here + 1);
+  int* flag = (int*)(tmem_slot + 1);     // a wait gave up
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile_a = blockIdx.x, tile_b = blockIdx.y, split = blockIdx.z;
   const int kblocks = (p.K + BK - 1) / BK;
-  const int kb0 = (int)((long long)kblocks * split / p.splits), kb1 = (int)((long long)kblocks * (split + 1) / p.splits);
-  const int nkb = kb1 - kb0;
+  const int kb0 = kblocks * split / p.splits, nkb = kblocks * (split + 1) / p.splits - kb0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_ready, 1);
-    flag[0] = 0; flag[1] = 0;
+    mbar_init(parts_here, 1);
+    flag[0] = 0;
     mbar_init_fence();
+    if (p.splits > 1) mbar_expect_tx(parts_here, (uint32_t)(p.splits * mine * PART_GROUP * 4));
   }
   if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_d = *tmem_slot;
+  if (p.splits > 1) cluster_arrive();      // this CTA's barrier may be sent to; waited for before the first send
   fz_grid_launch_dependents();
-  // The rotation epilogue needs, of every token column this thread will finish, the request's row, the position, the
-  // page and the angles: loads that depend on one another and on nothing a kernel before this one writes (the host
-  // packed the step's metadata before the step began). They are asked for now, by the epilogue warps that would
-  // otherwise only wait, instead of column by column at the end. Measured with two engines alternating in one process:
-  // a batch-1 decode step of 32 layers 3.304 -> 3.210 ms; batch 8 and 32 unchanged (looking up eight columns ahead
-  // instead of two was no better there either, and slower at batch 4 and 32).
-  constexpr int PRE = 2;      // columns per thread that are looked up ahead; further ones are looked up in the loop
-  int pre_row[PRE], pre_ps[PRE], pre_page[PRE];
-  float pre_cos[PRE], pre_sin[PRE];
-  if (p.rope && warp >= 2) {
-    const int rank0 = p.splits > 1 ? (int)cluster_rank() : 0, cols0 = min(BN, p.rows - tile_b * BN);
-    const int feat = tile_a * BM + (warp & 3) * 32 + lane, head = feat / p.hd, j = feat - head * p.hd, half = p.hd >> 1;
-#pragma unroll
-    for (int i = 0; i < PRE; ++i) {
-      const int c = rank0 + i * p.splits;
-      pre_row[i] = c < cols0 ? p.seq_row[tile_b * BN + c] : -1;
-      pre_ps[i] = c < cols0 ? p.pos[tile_b * BN + c] : 0;
+
+  // An epilogue thread's lane of tensor memory is feature r of the tile. Where two features belong together (gate and up,
+  // the two values of a rotated pair) threads r and r + 64 finish features f1 and f2, each for half of a group's tokens.
+  const int r = (warp & 3) * 32 + lane, par = r >> 6, q = r & 63;
+  const int half = EP == EP_ROPE ? p.hd >> 1 : 64;
+  const int j = EP == EP_ROPE ? q % half : q, f1 = PAIRS ? (EP == EP_ROPE ? q / half * p.hd : 0) + j : r, f2 = f1 + half;
+  const int feat = tile * BM + f1;
+  const bool own = feat < p.feats;
+  float b1 = 0.f, b2 = 0.f;      // what no kernel of a step writes is asked for ahead of the wait on the kernel before
+  // The rotation needs, of every token this thread will finish, the request's row, the position, the page and the angles:
+  // loads that depend on one another and on nothing a kernel before this one writes (the host packed the step's metadata
+  // before the step began). They are asked for now, and the addresses computed, by the epilogue warps that would otherwise only
+  // wait, for the first group of tokens; those of further groups in the loop at the end. (With
+  // the addresses computed and the bias waited for at the end, what follows the sums took 2.2 us of the product at one row at
+  // Qwen2.5-0.5B sizes, 0.6 now: one warp per scheduler walks two hundred dependent instructions in a microsecond.)
+  Place ahead[CV];
+  const int head = EP == EP_ROPE ? feat / p.hd : 0;      // (a tile starts at a head's first feature: hd divides 128)
+  auto place = [&](int m, Place& at) {
+    at = Place{nullptr, 0.f, 0.f, 0};
+    if (m >= cols || !own) return;
+    const int row = p.seq_row[m], ps = p.pos[m];
+    const bool in_range = ps >= 0 && ps < p.max_len, there = row >= 0 && in_range;
+    if (row >= 0 && !in_range && q == 0) atomicOr(p.err, FZ_ERR_POS_RANGE);
+    if (head < p.Hq) {
+      at.dst = p.c_bf16 + ((size_t)m * p.Hq + head) * p.hd + j;
+    } else if (there && p.write) {
+      const int page = p.table[(size_t)row * p.mb + ps / p.page_size];
+      if (page < 0) {
+        if (j == 0 && head == p.Hq) atomicOr(p.err, FZ_ERR_NO_PAGE);
+      } else {
+        __nv_bfloat16* pool = head < p.Hq + p.Hkv ? p.k_pool : p.v_pool;
+        const int h = head - p.Hq - (head < p.Hq + p.Hkv ? 0 : p.Hkv);
+        at.dst = pool + (long long)page * p.page_stride + ((long long)h * p.page_size + ps % p.page_size) * p.hd + j;
+      }
     }
-#pragma unroll
-    for (int i = 0; i < PRE; ++i) {
-      const bool live = pre_row[i] >= 0 && pre_ps[i] >= 0 && pre_ps[i] < p.max_len && feat < p.feats;
-      pre_page[i] = (live && p.write && head >= p.Hq) ? p.table[(size_t)pre_row[i] * p.mb + pre_ps[i] / p.page_size] : -1;
-      const bool turn = live && head < p.Hq + p.Hkv && j < half;
-      pre_cos[i] = turn ? p.cos_t[(size_t)pre_ps[i] * half + j] : 0.f;
-      pre_sin[i] = turn ? p.sin_t[(size_t)pre_ps[i] * half + j] : 0.f;
+    if (head >= p.Hq + p.Hkv) at.turn = 1;
+    else if (there) {
+      at.turn = 2;
+      at.cs = p.cos_t[(size_t)ps * half + j];
+      at.sn = p.sin_t[(size_t)ps * half + j];
     }
+  };
+  if (warp >= 2) {
+    if (p.bias && own) {
+      b1 = p.bias[feat];
+      if constexpr (PAIRS) b2 = p.bias[feat + half];
+    }
+    if constexpr (EP == EP_ROPE) {
+#pragma unroll
+      for (int e = 0; e < CV; ++e)
+        if (VW > 1 || par == 0) place(split * VW + par * CV + e, ahead[e]);
+    }
+    // (Used here, so that the loads cannot be put off to the end: 0.9 us of the q/k/v product with a bias.)
+    asm volatile("" ::"f"(b1), "f"(b2) : "memory");
   }
   if (warp != 0) fz_grid_wait();    // warp 0 waits after it has requested the first weight stages
 
   if (warp == 0) {
     if (lane == 0) {
-      // The weight operand does not depend on the kernel before this one: its first stages are requested before the
-      // wait on that kernel, so the weights stream in while it finishes. (swap mode: A holds the weights; rows mode: B.)
+      // The weights (A) do not depend on the kernel before this one: their first stages are requested before the wait on
+      // that kernel, so they stream in while it finishes. Every weight is read once per step: it should leave L2 before
+      // the activations, which are read again.
       const uint64_t stream_once = l2_evict_first();
       auto load_weights = [&](int i, int s) {
-        uint8_t* sa = smem + (size_t)s * STAGE_BYTES;
-        // swap mode streams every weight once per step: it should leave L2 before the activations, which are read again
-        if (p.swap) tma_load_2d_u32_hint(smem_u32(sa), &map_a, smem_u32(&full[s]), (kb0 + i) * BK, tile_a * BM, stream_once);
-        else tma_load_2d(sa + A_BYTES, &map_b, &full[s], (kb0 + i) * BK, tile_b * BN);
-      };
-      auto load_activations = [&](int i, int s) {
-        uint8_t* sa = smem + (size_t)s * STAGE_BYTES;
-        if (p.swap) tma_load_2d(sa + A_BYTES, &map_b, &full[s], (kb0 + i) * BK, tile_b * BN);
-        else tma_load_2d(sa, &map_a, &full[s], (kb0 + i) * BK, tile_a * BM);
+        tma_load_2d_u32_hint(smem_u32(smem + s * STAGE_BYTES), &map_a, smem_u32(&full[s]), (kb0 + i) * BK, tile * BM, stream_once);
       };
       const int early = nkb < p.stages ? nkb : p.stages;
+#pragma unroll 1
       for (int i = 0; i < early; ++i) {
         mbar_expect_tx(&full[i], STAGE_BYTES);
         load_weights(i, i);
       }
       fz_grid_wait();
+#pragma unroll 1
       for (int i = 0, s = 0, round = 0; i < nkb; ++i) {
         if (round > 0) {
-          if (!mbar_wait(&empty[s], (round - 1) & 1)) { flag[1] = 1; break; }
+          if (!mbar_wait(&empty[s], (round - 1) & 1)) { flag[0] = 1; break; }
           mbar_expect_tx(&full[s], STAGE_BYTES);
           load_weights(i, s);
         }
-        load_activations(i, s);
+        tma_load_2d(smem + s * STAGE_BYTES + A_BYTES, &map_b, &full[s], (kb0 + i) * BK, 0);
         if (++s == p.stages) { s = 0; ++round; }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc(BM, BN);
-      bool ok = true;
-      for (int i = 0, s = 0, round = 0; i < nkb && ok; ++i) {
-        if (!mbar_wait(&full[s], round & 1)) { flag[1] = 1; ok = false; break; }
+#pragma unroll 1
+      for (int i = 0, s = 0, round = 0; i < nkb; ++i) {
+        if (!mbar_wait(&full[s], round & 1)) { flag[0] = 1; break; }
         tc_fence_after();
-        const uint8_t* sa = smem + (size_t)s * STAGE_BYTES;
+        const uint8_t* sa = smem + s * STAGE_BYTES;
         const uint64_t da = desc_k_major(smem_u32(sa)), db = desc_k_major(smem_u32(sa + A_BYTES));
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k)   // 32 bytes further along the swizzled row per 16 k
@@ -228,253 +332,159 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
       umma_commit(acc_ready);   // arrives when every MMA issued so far has finished (at once if none was issued)
     }
-  } else {
-    // ---- epilogue: 4 warps, warp w reads TMEM lanes 32 * (w % 4) ..
-    const int quad = warp & 3;
-    const int r = quad * 32 + lane;          // TMEM lane = row of the 128-row operand
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_ready, 0));   // warp-uniform: tcgen05.ld is warp-wide
-    if (!ok) flag[1] = 1;
-    tc_fence_after();
-    const int a_row = tile_a * BM + r;       // rows mode: token row; swap mode: output feature
-    const int a_limit = p.swap ? p.feats : p.rows;
-    const int b_limit = p.swap ? p.rows : p.feats;
-    const int b0 = tile_b * BN;
-    const uint32_t taddr = tmem_d + ((uint32_t)(quad * 32) << 16);
-    const bool direct = p.splits == 1 && !p.swiglu && !p.rope;
-    float* part = (float*)smem + r;          // split K: partial tile as [column][row] in the (now idle) stage buffers
-    float v[16];
-    auto store16 = [&](const float* x, int c) {   // columns c..c+15 of this thread's row, final values
-      if (a_row >= a_limit) return;
-      if (p.swap) {
-        const float bv = p.bias ? p.bias[a_row] : 0.f;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int m = b0 + c + j;
-          if (m < b_limit) {
-            const float y = finished(p, x[j] + bv);
-            if (p.c_f32) p.c_f32[(size_t)m * p.feats + a_row] = y;
-            else p.c_bf16[(size_t)m * p.feats + a_row] = __float2bfloat16_rn(y);
-          }
-        }
-      } else if (p.vec_ok && b0 + c + 16 <= b_limit) {
-        const int n = b0 + c;
-        float y[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) y[j] = finished(p, x[j] + (p.bias ? p.bias[n + j] : 0.f));
-        if (p.c_f32) {
-          float4* dst = (float4*)(p.c_f32 + (size_t)a_row * p.feats + n);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dst[j] = make_float4(y[4 * j], y[4 * j + 1], y[4 * j + 2], y[4 * j + 3]);
-        } else {
-          uint32_t w[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(y[2 * j], y[2 * j + 1]);
-            w[j] = *(const uint32_t*)&h;
-          }
-          uint4* dst = (uint4*)(p.c_bf16 + (size_t)a_row * p.feats + n);
-          dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-          dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int n = b0 + c + j;
-          if (n < b_limit) {
-            const float y = finished(p, x[j] + (p.bias ? p.bias[n] : 0.f));
-            if (p.c_f32) p.c_f32[(size_t)a_row * p.feats + n] = y;
-            else p.c_bf16[(size_t)a_row * p.feats + n] = __float2bfloat16_rn(y);
-          }
-        }
-      }
-    };
-    if (ok) {
-      for (int c = 0; c < BN; c += 16) {
-        if (nkb > 0) tmem_ld16(taddr + (uint32_t)c, v);
-        else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = 0.f;
-        }
-        if (p.argmax) {
-          // the tile's logits go to the (idle) stage buffers as [token][feature], rows one float apart from a multiple of
-          // the bank count, and are searched below
-          const float bv = (p.bias && a_row < a_limit) ? p.bias[a_row] : 0.f;
-          float* am = (float*)smem;                   // [BN][BM + 1]
-#pragma unroll
-          for (int j = 0; j < 16; ++j) am[(c + j) * (BM + 1) + r] = v[j] + bv;
-        } else if (direct) store16(v, c);
-        else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) part[(c + j) * BM] = v[j];
-        }
-      }
-      if (p.argmax) {
-        // 128 / BN threads share a token: each scans its part of the tile's 128 features in rising order (so the lower
-        // index wins among equals), then the parts are merged in rising order
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        constexpr int TPC = BM / BN < 1 ? 1 : BM / BN;          // threads per token
-        constexpr int SEG = BM / TPC;                            // features per thread
-        const float* am = (const float*)smem;
-        float* best_v = (float*)smem + BN * (BM + 1);            // [BN][TPC]
-        int* best_i = (int*)(best_v + BN * TPC);
-        const int col = r % BN, seg = r / BN;                    // (for BN = 128 every thread has a token of its own)
-        float x = 0.f;
-        int ix = 0x7fffffff;
-        if (seg < TPC) {
-          for (int i = 0; i < SEG; ++i) {
-            const int f = seg * SEG + i, feat = tile_a * BM + f;
-            if (feat < a_limit && am_better(am[col * (BM + 1) + f], feat, x, ix)) { x = am[col * (BM + 1) + f]; ix = feat; }
-          }
-          best_v[col * TPC + seg] = x;
-          best_i[col * TPC + seg] = ix;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        const int m = b0 + col;
-        if (seg == 0 && m < b_limit) {
-          for (int sgm = 1; sgm < TPC; ++sgm)
-            if (am_better(best_v[col * TPC + sgm], best_i[col * TPC + sgm], x, ix)) { x = best_v[col * TPC + sgm]; ix = best_i[col * TPC + sgm]; }
-          p.am_val[(size_t)m * gridDim.x + tile_a] = x;
-          p.am_idx[(size_t)m * gridDim.x + tile_a] = ix;
-        }
-      }
-    }
   }
-  if (p.splits > 1 || p.swiglu || p.rope) {
-    // split K: every thread of every CTA of the cluster passes both cluster barriers; only the epilogue warps work
-    // between them. Without a split (fused SwiGLU only) the epilogue warps synchronise among themselves.
-    if (p.splits > 1) cluster_sync_all();
-    if (warp >= 2) {
-      if (p.splits == 1) asm volatile("bar.sync 1, 128;" ::: "memory");
-      const int r = (warp & 3) * 32 + lane;
-      const int feat = tile_a * BM + r;
-      const uint32_t rank = p.splits > 1 ? cluster_rank() : 0u;
-      const int cols = min(BN, p.rows - tile_b * BN);
-      const float bv = (p.bias && feat < p.feats) ? p.bias[feat] : 0.f;
-      const uint32_t base = smem_u32(smem) + (uint32_t)r * 4u;
-      float* ex = (float*)smem + BN * BM;            // [16][128]: a group of columns, for the gate / up exchange
-      int n_my = cols > (int)rank ? (cols - (int)rank + p.splits - 1) / p.splits : 0;   // columns rank, rank + S, ...
-      if (p.swiglu && p.splits == 1) {
-        // K not split: the tile is complete in this CTA's shared memory as [token][feature]. Thread r and thread r + 64
-        // share feature r of the tile's 64 (gate in row r, up in row r + 64) and take every other token; the loop is
-        // unrolled so that the loads, exponentials and divisions of eight tokens are in flight together (two of the
-        // four warps walking the tokens one by one took 14 us of a 58 us product at 64 tokens).
-        const int f = r & 63, par = r >> 6, gate_feat = tile_a * BM + f;
-        if (gate_feat < p.feats) {
-          const float bg = p.bias ? p.bias[gate_feat] : 0.f, bu = p.bias ? p.bias[gate_feat + 64] : 0.f;
-          const float* tile = (const float*)smem;
-          __nv_bfloat16* dst = p.c_bf16 + (size_t)(tile_b * BN) * (p.feats >> 1) + tile_a * 64 + f;
-#pragma unroll 8
-          for (int c = par; c < cols; c += 2)
-            dst[(size_t)c * (p.feats >> 1)] = __float2bfloat16_rn(glu_mul(tile[c * BM + f] + bg, tile[c * BM + f + 64] + bu, p.swiglu));
-        }
-        n_my = 0;
+  bool ok = true;
+  if (warp >= 2) {      // the epilogue: 4 warps, warp w reads TMEM lanes 32 * (w % 4) ..
+    ok = __all_sync(0xffffffffu, mbar_wait(acc_ready, 0));   // warp-uniform: tcgen05.ld is warp-wide
+    if (!ok) flag[0] = 1;
+    tc_fence_after();
+  }
+  if (p.splits > 1) {
+    // Every CTA sends, whatever became of its waits, and nobody leaves before all that it is sent has arrived: no CTA's
+    // memory goes away under a sender. In the ring's memory the parts may arrive once every CTA of the cluster has consumed
+    // its stages. (Fetched column by column from the other CTAs' shared memory, with a cluster barrier before and one behind,
+    // what follows the accumulator took 2.0 to 2.6 us of each of a layer's products at Qwen2.5-0.5B sizes at one row and 3.0 to
+    // 5.7 at 32; 0.9 to 1.2 and 1.3 to 3.4 now. Decode steps: 1 row of 300 keys 674 -> 592 us, 32 of 1,280 1,057 -> 879; at
+    // Llama-3.1-8B sizes 1, 8 and 64 rows of 4,096 keys 3,085 -> 2,957, 3,604 -> 3,455, 7,752 -> 7,643.)
+    cluster_wait();
+    if (p.parts_in_ring) cluster_sync_all();
+  }
+  if (warp >= 2) {
+    const uint32_t taddr = tmem_d + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool live = ok && nkb > 0;
+    const uint32_t bar = smem_u32(parts_here);
+    uint32_t at = smem_u32(parts) + (uint32_t)(split * part_step + r * VW) * 4u, to = 0;
+#pragma unroll 1
+    for (int c = 0; c < cols; c += 16) {
+      float v[16];
+      if (live) tmem_ld16(taddr + (uint32_t)c, v);
+      else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = 0.f;
       }
-      if (p.splits > 1 && !p.swiglu && !p.rope) {
-        // the plain sum over the splits: four columns' partial results asked for before the first is added up
-#pragma unroll 4
-        for (int i = 0; i < n_my; ++i) {
-          const int c = (int)rank + i * p.splits;
-          float v[8];
+      if (p.splits > 1) {
 #pragma unroll
-          for (int sp = 0; sp < 8; ++sp) v[sp] = sp < p.splits ? ld_dsmem(base + (uint32_t)(c * BM) * 4u, (uint32_t)sp) : 0.f;
-          float acc = 0.f;
+        for (int e = 0; e < 16; e += VW) {
+          if (c + e >= cols) break;
+          send_floats<VW>(map_to_cta(at, to), map_to_cta(bar, to), v + e);
+          if (++to == (uint32_t)p.splits) { to = 0; at += PART_GROUP * 4; }
+        }
+      } else if (EP == EP_ARGMAX) {
+        // the tile's logits go to the (idle) stage buffers as [token][feature], rows one float apart from a multiple of
+        // the bank count, and are searched below
 #pragma unroll
-          for (int sp = 0; sp < 8; ++sp) acc += v[sp];
-          if (feat < p.feats) {
-            const int m = tile_b * BN + c;
-            const float y = finished(p, acc + bv);
+        for (int e = 0; e < 16; ++e) ((float*)smem)[(c + e) * (BM + 1) + r] = v[e] + b1;
+      } else if (EP == EP_GLU) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) ((float*)smem)[(c + e) * BM + r] = v[e];      // [token][feature]
+      } else if (EP == EP_ROPE) {
+#pragma unroll
+        for (int e = 0; e < 16; e += 4) ((float4*)smem)[((c + e) >> 2) * BM + r] = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+      } else if (own) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const int m = c + e;
+          if (m < cols) {
+            const float y = finished(p, v[e] + b1);
             if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = y;
             else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(y);
           }
-        }
-        n_my = 0;
-      }
-      for (int i0 = 0; i0 < n_my; i0 += 16) {
-        const int ni = min(16, n_my - i0);
-#pragma unroll 2
-        for (int i = 0; i < ni; ++i) {
-          const int c = (int)rank + (i0 + i) * p.splits;
-          float acc = 0.f;
-          if (p.splits > 1) {
-            // all splits' partials are asked for before the first is used (a cluster holds at most 8 CTAs); the sum
-            // runs in split order
-            float v[8];
-#pragma unroll
-            for (int sp = 0; sp < 8; ++sp) v[sp] = sp < p.splits ? ld_dsmem(base + (uint32_t)(c * BM) * 4u, (uint32_t)sp) : 0.f;
-#pragma unroll
-            for (int sp = 0; sp < 8; ++sp) acc += v[sp];
-          } else {
-            acc = ((const float*)smem)[c * BM + r];
-          }
-          const float y = acc + bv;
-          if (p.swiglu || p.rope) {
-            ex[i * BM + r] = y;
-          } else if (feat < p.feats) {
-            const int m = tile_b * BN + c;
-            if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = y;
-            else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(y);
-          }
-        }
-        if (p.swiglu) {
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (r < 64) {
-            const int half = p.feats >> 1;
-            for (int i = 0; i < ni; ++i) {
-              const int m = tile_b * BN + (int)rank + (i0 + i) * p.splits;
-              p.c_bf16[(size_t)m * half + tile_a * 64 + r] = __float2bfloat16_rn(glu_mul(ex[i * BM + r], ex[i * BM + r + 64], p.swiglu));
-            }
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
-        if (p.rope) {
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          const int hd = p.hd, half = hd >> 1;
-          const int head = feat / hd, j = feat - head * hd;      // (a tile starts at a head's first feature: hd divides 128)
-          if (feat < p.feats) {
-            for (int i = 0; i < ni; ++i) {
-              const int m = tile_b * BN + (int)rank + (i0 + i) * p.splits;
-              // (columns 0 .. PRE - 1 of this thread were looked up at the kernel's start; i0 is 0 for them)
-              const bool ahead = i0 + i < PRE;
-              int row = 0, ps = 0, page_ahead = -1;
-              float cs = 0.f, sn = 0.f;
-#pragma unroll
-              for (int q = 0; q < PRE; ++q)
-                if (i0 + i == q) { row = pre_row[q]; ps = pre_ps[q]; page_ahead = pre_page[q]; cs = pre_cos[q]; sn = pre_sin[q]; }
-              if (!ahead) { row = p.seq_row[m]; ps = p.pos[m]; }
-              const bool in_range = ps >= 0 && ps < p.max_len;
-              if (row >= 0 && !in_range && r == 0) atomicOr(p.err, FZ_ERR_POS_RANGE);
-              const bool live = row >= 0 && in_range;
-              __nv_bfloat16* dst = nullptr;
-              if (head < p.Hq) {
-                dst = p.c_bf16 + ((size_t)m * p.Hq + head) * hd;
-              } else if (live && p.write) {
-                const int page = ahead ? page_ahead : p.table[(size_t)row * p.mb + ps / p.page_size];
-                if (page < 0) {
-                  if (j == 0 && head == p.Hq) atomicOr(p.err, FZ_ERR_NO_PAGE);
-                } else {
-                  const long long slot = (long long)page * p.page_stride + (long long)(ps % p.page_size) * hd;
-                  const long long head_stride = (long long)p.page_size * hd;
-                  dst = head < p.Hq + p.Hkv ? p.k_pool + slot + (long long)(head - p.Hq) * head_stride
-                                            : p.v_pool + slot + (long long)(head - p.Hq - p.Hkv) * head_stride;
-                }
-              }
-              if (dst == nullptr) continue;
-              if (head >= p.Hq + p.Hkv) {
-                dst[j] = __float2bfloat16_rn(ex[i * BM + r]);
-              } else if (j < half) {
-                float o1 = 0.f, o2 = 0.f;
-                if (live && !ahead) { cs = p.cos_t[(size_t)ps * half + j]; sn = p.sin_t[(size_t)ps * half + j]; }
-                if (live) fz_rope_pair(ex[i * BM + r], ex[i * BM + r + half], cs, sn, o1, o2);
-                dst[j] = __float2bfloat16_rn(o1);
-                dst[j + half] = __float2bfloat16_rn(o2);
-              }
-            }
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
         }
       }
     }
-    if (p.splits > 1) cluster_sync_all();    // nobody leaves while its shared memory may still be read
+    bool summed = true;      // this thread's tokens are complete in `parts`
+    if (p.splits > 1) {
+      summed = mbar_wait_cluster(parts_here, 0);
+      if (!summed) flag[0] = 1;
+    } else if (EP != EP_PLAIN) asm volatile("bar.sync 1, 128;" ::: "memory");
+
+    if (EP == EP_GLU && p.splits == 1) {
+      // K not split: the tile is complete in this CTA's shared memory. A warp takes every fourth token, a lane two
+      // neighbouring features of the 64.
+      const int f = 2 * lane, g0 = tile * BM + f;
+      if (ok && g0 < p.feats) {
+        float2 bg = make_float2(0.f, 0.f), bu = bg;
+        if (p.bias) { bg = make_float2(p.bias[g0], p.bias[g0 + 1]); bu = make_float2(p.bias[g0 + 64], p.bias[g0 + 65]); }
+        const float* t = (const float*)smem + f;
+        __nv_bfloat16* dst = p.c_bf16 + tile * 64 + f;
+#pragma unroll 4
+        for (int c = warp & 3; c < cols; c += 4) {
+          const float2 g = *(const float2*)(t + c * BM), u = *(const float2*)(t + c * BM + 64);
+          const __nv_bfloat162 y = __floats2bfloat162_rn(glu_mul(g.x + bg.x, u.x + bu.x, p.swiglu), glu_mul(g.y + bg.y, u.y + bu.y, p.swiglu));
+          *(__nv_bfloat162*)(dst + (size_t)c * (p.feats >> 1)) = y;
+        }
+      }
+    } else if (EP == EP_ARGMAX) {
+      // 128 / BN threads share a token: each scans its part of the tile's 128 features in rising order (so the lower
+      // index wins among equals), then the parts are merged in rising order
+      constexpr int TPC = BM / BN < 1 ? 1 : BM / BN;          // threads per token
+      constexpr int SEG = BM / TPC;                            // features per thread
+      const float* am = (const float*)smem;
+      float* best_v = (float*)smem + BN * (BM + 1);            // [BN][TPC]
+      int* best_i = (int*)(best_v + BN * TPC);
+      const int col = r % BN, seg = r / BN;                    // (for BN = 128 every thread has a token of its own)
+      float x = 0.f;
+      int ix = 0x7fffffff;
+      if (seg < TPC) {
+#pragma unroll 4
+        for (int i = 0; i < SEG; ++i) {
+          const int f = seg * SEG + i, ft = tile * BM + f;
+          if (ft < p.feats && am_better(am[col * (BM + 1) + f], ft, x, ix)) { x = am[col * (BM + 1) + f]; ix = ft; }
+        }
+        best_v[col * TPC + seg] = x;
+        best_i[col * TPC + seg] = ix;
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (seg == 0 && col < cols) {
+#pragma unroll 1
+        for (int sgm = 1; sgm < TPC; ++sgm)
+          if (am_better(best_v[col * TPC + sgm], best_i[col * TPC + sgm], x, ix)) { x = best_v[col * TPC + sgm]; ix = best_i[col * TPC + sgm]; }
+        p.am_val[(size_t)col * gridDim.x + tile] = x;
+        p.am_idx[(size_t)col * gridDim.x + tile] = ix;
+      }
+    } else if constexpr (EP == EP_PLAIN) {
+      if (p.splits > 1 && summed && own) {
+#pragma unroll 1
+        for (int i = 0; i < mine; ++i) {
+          alignas(16) float y[VW];
+          sum_parts<VW>(parts + i * PART_GROUP + r * VW, p.splits, part_step, y);
+#pragma unroll
+          for (int e = 0; e < VW; ++e) {
+            const int m = (split + i * p.splits) * VW + e;
+            if (m >= cols) break;
+            const float v = finished(p, y[e] + b1);
+            if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = v;
+            else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(v);
+          }
+        }
+      }
+    } else if (summed && ok && own && (VW > 1 || par == 0)) {
+#pragma unroll (EP == EP_GLU ? 2 : 1)
+      for (int i = 0; i < mine; ++i) {
+        const float* at = parts + i * PART_GROUP + par * CV;
+        alignas(8) float s1[CV], s2[CV];
+        sum_parts<CV>(at + f1 * VW, p.splits, part_step, s1);
+        sum_parts<CV>(at + f2 * VW, p.splits, part_step, s2);
+#pragma unroll
+        for (int e = 0; e < CV; ++e) {
+          const int m = (split + i * p.splits) * VW + par * CV + e;
+          if (m >= cols) break;
+          const float v1 = s1[e] + b1, v2 = s2[e] + b2;
+          if constexpr (EP == EP_GLU) {
+            p.c_bf16[(size_t)m * (p.feats >> 1) + tile * 64 + q] = __float2bfloat16_rn(glu_mul(v1, v2, p.swiglu));
+          } else {
+            Place& at = ahead[e];
+            if (VW > 1 && i > 0) place(m, at);
+            if (at.dst == nullptr) continue;
+            float o1 = 0.f, o2 = 0.f;
+            if (at.turn == 2) fz_rope_pair(v1, v2, at.cs, at.sn, o1, o2);
+            else if (at.turn == 1) { o1 = v1; o2 = v2; }
+            at.dst[0] = __float2bfloat16_rn(o1);
+            at.dst[half] = __float2bfloat16_rn(o2);
+          }
+        }
+      }
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -482,7 +492,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem_d, TMEM_COLS);
   }
-  if (threadIdx.x == 0 && flag[1]) atomicOr(p.err, FZ_ERR_WAIT_TIMEOUT);
+  if (threadIdx.x == 0 && flag[0]) atomicOr(p.err, FZ_ERR_WAIT_TIMEOUT);
 }
 
 // Rows mode: one thread's lane (token row `row`) of a finished accumulator of BN columns at `taddr`, with the bias added,
@@ -711,11 +721,6 @@ int launch_rows(const CUtensorMap& mx, const CUtensorMap& mw, const Params& p, i
 // both CTAs pass a cluster barrier after the barriers' initialisation and before they leave.
 constexpr int PAIR_BN = 256;
 
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-  return remote;
-}
 __device__ __forceinline__ uint32_t ld_dsmem_u32(uint32_t cluster_addr) {
   uint32_t v;
   asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
@@ -1163,11 +1168,34 @@ int launch_rows_split(const CUtensorMap& mx, const CUtensorMap& mw, const Params
 }
 
 // ---------------------------------------------------------------------------------------------- host side
-template <int BN>
-int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, dim3 grid, cudaStream_t stream) {
+int device_sms() {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+      sms = 148;
+  }
+  return sms;
+}
+
+template <int BN, int EP, int VW>
+int launch_few(const CUtensorMap& ma, const CUtensorMap& mb, Params p, dim3 grid, cudaStream_t stream) {
   constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
-  const size_t smem = (size_t)p.stages * STAGE_BYTES + 1024 + 8 * (2 * p.stages + 1) + 16;
-  FZ_RAISE_SMEM(gemm_tc_kernel<BN>);
+  const size_t region = (size_t)p.splits * parts_slots(p.rows, p.splits, VW) * VW * BM * 4;
+  size_t smem = (size_t)p.stages * STAGE_BYTES + 1024 + 8 * (2 * p.stages + 2) + 16;
+  p.parts_in_ring = 1;
+  if (p.splits > 1) {
+    // The parts have memory of their own where as many CTAs fit an SM with it as without, or there are no more CTAs than SMs.
+    // (The O product at Llama-3.1-8B sizes, 256 CTAs in clusters of eight, three to an SM: with 4 KB more, two to an SM, the
+    // last cluster started only when others had left, 7.8 -> 11.3 us.)
+    constexpr size_t sm = 228 * 1024, reserved = 1024;
+    if (smem + region <= FZ_MOST_SMEM && (sm / (smem + region + reserved) == sm / (smem + reserved) || (int)grid.x * p.splits <= device_sms())) {
+      p.parts_in_ring = 0;
+      smem += region;
+    } else if (region > (size_t)p.stages * STAGE_BYTES) return FZ_BAD_SHAPE;
+  }
+  const auto kern = gemm_tc_kernel<BN, EP, VW>;
+  FZ_RAISE_SMEM(kern);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(NUM_THREADS);
@@ -1189,10 +1217,24 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, dim3 g
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN>, ma, mb, p);
+  cudaError_t le = cudaLaunchKernelEx(&cfg, kern, ma, mb, p);
   if (le != cudaSuccess) return (int)le;
   FZ_LAUNCH_CHECK();
   return FZ_OK;
+}
+template <int BN, int VW>
+int launch_few_ep(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, dim3 grid, cudaStream_t stream) {
+  if (p.swiglu) return launch_few<BN, EP_GLU, VW>(ma, mb, p, grid, stream);
+  if constexpr (BN <= 32)
+    if (p.rope) return launch_few<BN, EP_ROPE, VW>(ma, mb, p, grid, stream);
+  return launch_few<BN, EP_PLAIN, VW>(ma, mb, p, grid, stream);
+}
+template <int BN>
+int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, dim3 grid, cudaStream_t stream) {
+  if (p.argmax) return launch_few<BN, EP_ARGMAX, 4>(ma, mb, p, grid, stream);
+  if constexpr (BN == 16)
+    if (p.rows <= p.splits && p.splits > 1) return launch_few_ep<16, 1>(ma, mb, p, grid, stream);
+  return launch_few_ep<BN, 4>(ma, mb, p, grid, stream);
 }
 
 int pick_stages(int bn) {
@@ -1245,16 +1287,6 @@ FZ_API int fz_gemm_tc_rows_splits(int M, int N, int K) {
   for (int s = 8; s >= 2; s >>= 1)
     if (tiles * s <= (s == 2 ? sms : 128) && kblocks / 8 >= s) return s;
   return 1;
-}
-
-static int device_sms() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      sms = 148;
-  }
-  return sms;
 }
 
 // Which many-token kernel takes a product: 0 by the rule below, 1 always one SM per tile, 2 a pair of SMs per tile
@@ -1414,7 +1446,6 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
   if (M <= 128) {
     // swap mode: W rows are the 128 lanes, the token rows are the instruction's N
     const int bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
-    p.swap = 1;
     p.stages = pick_stages(bn);
     const int tiles = (N + BM - 1) / BM;
     p.splits = fz_gemm_tc_splits(N, K);
@@ -1429,8 +1460,8 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
       // A matrix that the rings of all its CTAs hold whole (up to 24 MB of 148 x 227 KB): then every weight is on its way
       // before the wait on the kernel before, and what follows the wait is the activations, the sums and the store alone.
       // Qwen2.5-0.5B sizes, 300 keys: a decode step of one row 684 -> 668 us, of 8 726 -> 722, of 32 905 -> 900, of 64 the same.
-      // Larger ones would only keep the next kernels' blocks off the SMs. (At least three stages: they also hold the sums of 128 columns and the
-      // exchange of the gated epilogue, 72 KB.)
+      // Larger ones would only keep the next kernels' blocks off the SMs. (At least three stages: they also hold the parts of 128
+      // tokens, 72 KB.)
       const long long ring = (long long)per_cta * (BM + bn) * BK * 2;
       if (ring <= 200 * 1024 && ring * tiles * p.splits <= 24 << 20) p.stages = per_cta < 3 ? 3 : per_cta;
     }
@@ -1445,7 +1476,6 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
     }
   }
   // rows mode: token rows are the 128 lanes; persistent CTAs with two accumulators
-  p.swap = 0;
   int bn = N >= 256 ? 256 : N >= 128 ? 128 : 64;     // with the fused SwiGLU N = 2 I >= 128, so a tile holds whole blocks
   if (bn == 256 && !p.swiglu) {
     // So few 128 x 256 tiles that the SMs are not half used, and a K worth cutting: the tiles' K ranges are cut so that

@@ -145,6 +145,33 @@ def test_a_row_does_not_depend_on_the_other_rows():
     ops.check_errors()
 
 
+@pytest.mark.parametrize("tiles,splits", [(7, 8), (36, 7), (42, 6), (48, 5), (64, 4), (76, 3), (128, 2), (130, 1)])
+def test_tokens_dealt_out_to_the_splits(tiles, splits):
+    """Few rows: the tokens go in groups to the CTAs that share a tile, one by one or four by four, into memory of their own
+    or the ring's; for every number of CTAs, at rows around the groups' and the instruction's sizes, the last tile ragged."""
+    from fusezap_core_b200.kernels import cuda_ops
+    ops = cuda_ops("bfloat16")
+    N, K = tiles * 128 - 40, 1024
+    assert ops.tc.fz_gemm_tc_splits(N, K) == splits
+    g = torch.Generator(device="cuda").manual_seed(tiles)
+    a = torch.randn(128, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, generator=g, device="cuda")
+    ref = a.double() @ w.double().T + b.double()
+    # K exact products, each addition off by at most 2^-23 of a partial sum (the tensor cores may cut off), at most the magnitudes' sum
+    bound = (K + 8) * 2.0 ** -23 * (a.abs().double() @ w.abs().double().T + b.abs().double())
+    full = torch.empty(128, N, device="cuda")
+    ops.linear(a, w, b, full)
+    assert bool(((full.double() - ref).abs() <= bound).all())
+    for rows in (1, 2, 3, splits, splits + 1, 4 * splits, 4 * splits + 1, 9, 16, 17, 31, 33, 64, 65, 127):
+        if rows > 128:
+            continue
+        part = torch.full((rows + 1, N), float("nan"), device="cuda")
+        ops.linear(a[:rows].contiguous(), w, b, part[:rows])
+        assert torch.equal(part[:rows], full[:rows]) and bool(part[rows].isnan().all()), f"{rows} rows"
+    ops.check_errors()
+
+
 def test_refused_shapes_fall_back_to_the_plain_kernel():
     from fusezap_core_b200.kernels import cuda_ops
     ops = cuda_ops("bfloat16")
