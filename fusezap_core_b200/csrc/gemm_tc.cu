@@ -141,6 +141,20 @@ struct Params {
   int argmax;
   float* am_val;           // [rows][tiles]
   int* am_idx;
+  // x set (few tokens): the product ends in the residual stream and the norm that follows it: x[row] += product + bias (float32),
+  // h = x * norm_w in bfloat16, and per row the sums of squares of the new x over the features that one warp finishes, as
+  // `ss_parts` numbers. The row's factor 1 / sqrt(mean of squares + eps) is left to the products that read h. (A norm's kernel of
+  // its own is 1.5 to 3 us of a chain of dependent kernels, two a layer; h has one rounding either way. Decode steps at
+  // Llama-3.1-8B sizes, 1, 8 and 64 rows of 4,096 keys: 2,957 -> 2,847 us, 3,455 -> 3,392, 7,643 -> 7,631; at Qwen2.5-0.5B sizes,
+  // 1 row of 300 and 32 of 1,280: 592 -> 545, 879 -> 843.)
+  float* x;
+  const float* norm_w;
+  __nv_bfloat16* h;
+  float* ss_out;           // [rows][ss_parts]
+  // ss set: the rows of X are such an h; each output is the product times its row's factor, plus the bias
+  const float* ss;         // [rows][ss_parts]
+  int ss_parts;
+  float ss_mean, ss_eps;   // 1 / the size of a row, and what is added to the mean
 };
 
 __device__ __forceinline__ float finished(const Params& p, float y) {
@@ -184,7 +198,7 @@ __device__ __forceinline__ void sum_parts(const float* at, int splits, int step,
 
 // The epilogue of a tile, as far as it is known when the kernel is compiled (a kernel that held all of them was 80 KB of
 // code and took its instructions from L2 on every launch of a decode step).
-enum { EP_PLAIN = 0, EP_GLU = 1, EP_ROPE = 2, EP_ARGMAX = 3 };
+enum { EP_PLAIN = 0, EP_GLU = 1, EP_ROPE = 2, EP_ARGMAX = 3, EP_NORM = 4 };      // EP_NORM: see Params::x
 
 // (Three or four CTAs to an SM as far as registers go. With 160 a thread, two CTAs took all of an SM's registers and the blocks of
 // the kernels after this one could not become resident beside them: a decode step of 64 rows at Llama-3.1-8B sizes 7,730 ->
@@ -210,6 +224,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint64_t* parts_here = acc_ready + 1;
   uint32_t* tmem_slot = (uint32_t*)(parts_here + 1);
   int* flag = (int*)(tmem_slot + 1);     // a wait gave up
+  float* factor = (float*)(flag + 1);    // [BN] of the tokens that this CTA finishes
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kblocks = (p.K + BK - 1) / BK;
@@ -238,7 +253,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int j = EP == EP_ROPE ? q % half : q, f1 = PAIRS ? (EP == EP_ROPE ? q / half * p.hd : 0) + j : r, f2 = f1 + half;
   const int feat = tile * BM + f1;
   const bool own = feat < p.feats;
-  float b1 = 0.f, b2 = 0.f;      // what no kernel of a step writes is asked for ahead of the wait on the kernel before
+  float nw = 0.f, b1 = 0.f, b2 = 0.f;      // what no kernel of a step writes is asked for ahead of the wait on the kernel before
   // The rotation needs, of every token this thread will finish, the request's row, the position, the page and the angles:
   // loads that depend on one another and on nothing a kernel before this one writes (the host packed the step's metadata
   // before the step began). They are asked for now, and the addresses computed, by the epilogue warps that would otherwise only
@@ -277,15 +292,37 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       b1 = p.bias[feat];
       if constexpr (PAIRS) b2 = p.bias[feat + half];
     }
+    if constexpr (EP == EP_NORM)
+      if (own) nw = p.norm_w[feat];
     if constexpr (EP == EP_ROPE) {
 #pragma unroll
       for (int e = 0; e < CV; ++e)
         if (VW > 1 || par == 0) place(split * VW + par * CV + e, ahead[e]);
     }
     // (Used here, so that the loads cannot be put off to the end: 0.9 us of the q/k/v product with a bias.)
-    asm volatile("" ::"f"(b1), "f"(b2) : "memory");
+    asm volatile("" ::"f"(b1), "f"(b2), "f"(nw) : "memory");
   }
   if (warp != 0) fz_grid_wait();    // warp 0 waits after it has requested the first weight stages
+  float xs[VW] = {};      // EP_NORM: the stream's values of the tokens that this thread finishes next
+  if (warp >= 2) {
+    if constexpr (EP == EP_NORM) {
+#pragma unroll
+      for (int e = 0; e < VW; ++e)
+        if (own && split * VW + e < cols) xs[e] = p.x[(size_t)(split * VW + e) * p.feats + feat];
+    } else if (p.ss != nullptr) {      // (while the products are under way)
+      const int tokens = p.splits > 1 ? mine * VW : cols;
+#pragma unroll 4
+      for (int t = warp & 3; t < tokens; t += 4) {
+        const int m = p.splits > 1 ? (split + t / VW * p.splits) * VW + t % VW : t;
+        float sum = 0.f;
+        if (m < cols)
+          for (int i = lane; i < p.ss_parts; i += 32) sum += p.ss[(size_t)m * p.ss_parts + i];
+        sum = warp_sum(sum);
+        if (lane == 0) factor[t] = 1.0f / sqrtf(sum * p.ss_mean + p.ss_eps);
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    }
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -385,7 +422,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int e = 0; e < 16; ++e) {
           const int m = c + e;
           if (m < cols) {
-            const float y = finished(p, v[e] + b1);
+            const float y = finished(p, fmaf(v[e], p.ss ? factor[m] : 1.f, b1));
             if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = y;
             else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(y);
           }
@@ -410,7 +447,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll 4
         for (int c = warp & 3; c < cols; c += 4) {
           const float2 g = *(const float2*)(t + c * BM), u = *(const float2*)(t + c * BM + 64);
-          const __nv_bfloat162 y = __floats2bfloat162_rn(glu_mul(g.x + bg.x, u.x + bu.x, p.swiglu), glu_mul(g.y + bg.y, u.y + bu.y, p.swiglu));
+          const float sc = p.ss ? factor[c] : 1.f;      // (times one: the sum's bits)
+          const __nv_bfloat162 y = __floats2bfloat162_rn(glu_mul(fmaf(g.x, sc, bg.x), fmaf(u.x, sc, bu.x), p.swiglu), glu_mul(fmaf(g.y, sc, bg.y), fmaf(u.y, sc, bu.y), p.swiglu));
           *(__nv_bfloat162*)(dst + (size_t)c * (p.feats >> 1)) = y;
         }
       }
@@ -442,6 +480,41 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         p.am_val[(size_t)col * gridDim.x + tile] = x;
         p.am_idx[(size_t)col * gridDim.x + tile] = ix;
       }
+    } else if constexpr (EP == EP_NORM) {
+      summed = __all_sync(0xffffffffu, summed);
+#pragma unroll 1
+      for (int i = 0; i < mine && summed; ++i) {      // (a warp's lanes stay together: they add up their squares)
+        alignas(16) float y[VW];
+        float sq[VW], old[VW];
+#pragma unroll
+        for (int e = 0; e < VW; ++e) {
+          old[e] = xs[e];
+          const int m = (split + (i + 1) * p.splits) * VW + e;
+          if (own && m < cols) xs[e] = p.x[(size_t)m * p.feats + feat];
+        }
+        sum_parts<VW>(parts + i * PART_GROUP + r * VW, p.splits, part_step, y);
+#pragma unroll
+        for (int e = 0; e < VW; ++e) {
+          const int m = (split + i * p.splits) * VW + e;
+          sq[e] = 0.f;
+          if (own && m < cols) {
+            const size_t at = (size_t)m * p.feats + feat;
+            const float v = old[e] + (y[e] + b1);
+            p.x[at] = v;
+            p.h[at] = __float2bfloat16_rn(v * nw);
+            sq[e] = v * v;
+          }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int e = 0; e < VW; ++e) sq[e] += __shfl_xor_sync(0xffffffffu, sq[e], o);
+#pragma unroll
+        for (int e = 0; e < VW; ++e) {
+          const int m = (split + i * p.splits) * VW + e;
+          if (lane == e && m < cols) p.ss_out[(size_t)m * p.ss_parts + tile * 4 + (warp & 3)] = sq[e];
+        }
+      }
     } else if constexpr (EP == EP_PLAIN) {
       if (p.splits > 1 && summed && own) {
 #pragma unroll 1
@@ -452,7 +525,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           for (int e = 0; e < VW; ++e) {
             const int m = (split + i * p.splits) * VW + e;
             if (m >= cols) break;
-            const float v = finished(p, y[e] + b1);
+            const float v = finished(p, fmaf(y[e], p.ss ? factor[i * VW + e] : 1.f, b1));
             if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = v;
             else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(v);
           }
@@ -469,7 +542,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int e = 0; e < CV; ++e) {
           const int m = (split + i * p.splits) * VW + par * CV + e;
           if (m >= cols) break;
-          const float v1 = s1[e] + b1, v2 = s2[e] + b2;
+          const float sc = p.ss ? factor[i * VW + par * CV + e] : 1.f;
+          const float v1 = fmaf(s1[e], sc, b1), v2 = fmaf(s2[e], sc, b2);
           if constexpr (EP == EP_GLU) {
             p.c_bf16[(size_t)m * (p.feats >> 1) + tile * 64 + q] = __float2bfloat16_rn(glu_mul(v1, v2, p.swiglu));
           } else {
@@ -1182,7 +1256,7 @@ template <int BN, int EP, int VW>
 int launch_few(const CUtensorMap& ma, const CUtensorMap& mb, Params p, dim3 grid, cudaStream_t stream) {
   constexpr int STAGE_BYTES = (BM + BN) * BK * 2;
   const size_t region = (size_t)p.splits * parts_slots(p.rows, p.splits, VW) * VW * BM * 4;
-  size_t smem = (size_t)p.stages * STAGE_BYTES + 1024 + 8 * (2 * p.stages + 2) + 16;
+  size_t smem = (size_t)p.stages * STAGE_BYTES + 1024 + 8 * (2 * p.stages + 2) + 16 + (p.ss ? BN * 4 : 0);
   p.parts_in_ring = 1;
   if (p.splits > 1) {
     // The parts have memory of their own where as many CTAs fit an SM with it as without, or there are no more CTAs than SMs.
@@ -1225,6 +1299,7 @@ int launch_few(const CUtensorMap& ma, const CUtensorMap& mb, Params p, dim3 grid
 template <int BN, int VW>
 int launch_few_ep(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, dim3 grid, cudaStream_t stream) {
   if (p.swiglu) return launch_few<BN, EP_GLU, VW>(ma, mb, p, grid, stream);
+  if (p.x) return p.splits > 1 ? launch_few<BN, EP_NORM, VW>(ma, mb, p, grid, stream) : FZ_BAD_SHAPE;
   if constexpr (BN <= 32)
     if (p.rope) return launch_few<BN, EP_ROPE, VW>(ma, mb, p, grid, stream);
   return launch_few<BN, EP_PLAIN, VW>(ma, mb, p, grid, stream);
@@ -1318,6 +1393,35 @@ FZ_API int fz_gemm_tc_rows_pair_splits(int M, int N, int K) {
   return tiles * 4 <= 128 ? 2 : 1;
 }
 
+// Which kernel takes a product of M > 128 token rows, and in what tiles.
+struct RowsPlan {
+  enum Kernel { ROWS, PAIR, SPLIT, SPLIT_PAIR } kernel;
+  int bn, splits, parts;      // width of a tile; pieces of K; PAIR: groups of four epilogue warps
+};
+static RowsPlan rows_plan(int M, int N, int K, bool swiglu) {
+  int bn = N >= 256 ? 256 : N >= 128 ? 128 : 64;     // with the fused SwiGLU N = 2 I >= 128, so a tile holds whole blocks
+  if (bn == 256 && !swiglu) {
+    // So few 128 x 256 tiles that the SMs are not half used, and a K worth cutting: the tiles' K ranges are cut so that
+    // about one CTA per SM works (see `gemm_tc_rows_split_kernel`). The count follows from (M, N, K) of the product.
+    const int pair_splits = fz_gemm_tc_rows_pair_splits(M, N, K), splits = fz_gemm_tc_rows_splits(M, N, K);
+    if (pair_splits > 1) return {RowsPlan::SPLIT_PAIR, SPLIT_BN, pair_splits, 1};
+    if (splits > 1) return {RowsPlan::SPLIT, SPLIT_BN, splits, 1};
+    // Few token rows: when the 256-wide tiles do not fill the SMs even once, the narrowest width that still fits one
+    // round is the fastest (256 x 4096 x 4096 is 32 tiles of 256 columns for 148 SMs, but 52 of 160). Not below 160:
+    // a 128-wide instruction reads its operands from shared memory at the rate the tensor core consumes them and runs
+    // at about half speed. With more than one round the widest tile stays: measured at 2,048 rows, 160-wide tiles in
+    // three rounds (60 -> 72 us) lose against 256-wide ones in two, whatever the count of rounds says.
+    const long long tm = (M + BM - 1) / BM;
+    if (tm * ((N + 255) / 256) < device_sms()) {
+      for (int cand : {224, 192, 160})
+        if (tm * ((N + cand - 1) / cand) <= device_sms()) bn = cand;
+    }
+  }
+  // many token rows: a pair of SMs on every 256 x 256 tile (see `gemm_tc_rows_pair_kernel`)
+  if (bn == 256 && fz_gemm_tc_rows_pairs(M, N, K)) return {RowsPlan::PAIR, PAIR_BN, 1, swiglu ? 4 : 2};
+  return {RowsPlan::ROWS, bn, 1, 1};
+}
+
 // x: [M, K] bf16, w: [N, K] bf16, bias: [N] float32 or null, c: [M, N] float32 (out_dtype 0) or bf16 (1).
 static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c, int out_dtype, int M, int N, int K,
                         const Params& fused, int* err, cudaStream_t stream);
@@ -1325,6 +1429,45 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
 FZ_API int fz_gemm_tc(const void* x, const void* w, const float* bias, void* c, int out_dtype, int M, int N, int K,
                       int* err, cudaStream_t stream) {
   return gemm_tc_impl(x, w, bias, c, out_dtype, M, N, K, Params{}, err, stream);
+}
+
+// How many partial sums of squares per row a product that ends in the residual stream and the norm behind it leaves (0: such
+// a product is refused). Few rows alone, K cut (up to 16,384 features, K from 72 on), and rows that the next product can read: the sums of squares are 0.2 us beside
+// the partial sums that are in shared memory anyway. With many rows a thread finishes a row's piece, 64 bytes here and there of
+// the stream, and every tile of the next product needs its rows' factors: 2,048 rows at Llama-3.1-8B sizes 26.9 -> 29.7 ms, 2,100
+// rows at Qwen2.5-0.5B sizes 2.96 -> 3.14, so those keep the norm's kernel.
+FZ_API int fz_gemm_tc_norm_parts(int M, int N, int K) {
+  if (M <= 0 || M > 128 || N <= 0 || N % 8 || K <= 0 || K % 8 || fz_gemm_tc_splits(N, K) == 1) return 0;
+  return (N + BM - 1) / BM * 4;
+}
+
+// stream [M, N] float32 += x . w^T + bias; h [M, N] bf16 = the new stream * norm_w; ss [M, fz_gemm_tc_norm_parts(M, N, K)]: partial
+// sums of the new stream's squares.
+FZ_API int fz_gemm_tc_add_norm(const void* x, const void* w, const float* bias, float* stream_x, const float* norm_w, void* h, float* ss,
+                               int M, int N, int K, int* err, cudaStream_t stream) {
+  Params f{};
+  f.ss_parts = fz_gemm_tc_norm_parts(M, N, K);
+  if (f.ss_parts == 0) return FZ_BAD_SHAPE;
+  if ((uintptr_t)h & 15) return FZ_BAD_ALIGNMENT;      // (the next product reads it)
+  f.x = stream_x; f.norm_w = norm_w; f.h = (__nv_bfloat16*)h; f.ss_out = ss;
+  return gemm_tc_impl(x, w, bias, h, FZ_BF16, M, N, K, f, err, stream);
+}
+
+static void set_factors(Params& f, const float* ss, int ss_parts, float eps, int K) {
+  f.ss = ss; f.ss_parts = ss_parts; f.ss_mean = 1.0f / (float)K; f.ss_eps = eps;
+}
+
+// `fz_gemm_tc` and `fz_gemm_tc_swiglu` (kind 0, 1, 2) of rows that `fz_gemm_tc_add_norm` left: x is its h, ss and ss_parts its
+// partial sums; each row of the product is multiplied by 1 / sqrt(mean of squares + eps).
+FZ_API int fz_gemm_tc_normed(const void* x, const float* ss, int ss_parts, float eps, const void* w, const float* bias, void* c, int out_dtype,
+                             int M, int N, int K, int kind, int* err, cudaStream_t stream) {
+  if (ss == nullptr || ss_parts <= 0 || kind < 0 || kind > 2) return FZ_BAD_SHAPE;
+  if (kind && (N % 128 || out_dtype != FZ_BF16)) return FZ_BAD_SHAPE;
+  if (kind && ((uintptr_t)c & 15)) return FZ_BAD_ALIGNMENT;
+  Params f{};
+  f.swiglu = kind;
+  set_factors(f, ss, ss_parts, eps, K);
+  return gemm_tc_impl(x, w, bias, c, out_dtype, M, N, K, f, err, stream);
 }
 
 // Can the query/key/value product of M token rows with heads of size hd end in the rotation and the cache write?
@@ -1337,13 +1480,15 @@ FZ_API int fz_gemm_tc_qkv_rope_check(int M, int hd) {
 // x: [M, K] bf16; w: [(Hq + 2 Hkv) hd, K] bf16, rows [q heads | k heads | v heads]; bias float32 or null. Rotates the q
 // and k heads of every token by its position (pairs j, j + hd / 2; angles from cos_t / sin_t [max_len, hd / 2]) and
 // writes q to q_out [M, Hq hd] bf16 and, if `write`, k and v to the token's slot of the paged pools (as the separate
-// rotation kernel does, with the same roundings). seq_row < 0: a padding row (q zeros, nothing stored).
-FZ_API int fz_gemm_tc_qkv_rope(const void* x, const void* w, const float* bias, int M, int K, const float* cos_t,
+// rotation kernel does, with the same roundings). seq_row < 0: a padding row (q zeros, nothing stored). ss: null, or as in
+// `fz_gemm_tc_normed`.
+FZ_API int fz_gemm_tc_qkv_rope(const void* x, const float* ss, int ss_parts, float eps, const void* w, const float* bias, int M, int K, const float* cos_t,
                                const float* sin_t, const int* pos, const int* seq_row, const int* table, int mb,
                                void* k_pool, void* v_pool, long long page_stride, int page_size, int write, void* q_out,
                                int Hq, int Hkv, int hd, int max_len, int* err, cudaStream_t stream) {
   if (fz_gemm_tc_qkv_rope_check(M, hd) != FZ_OK || Hq <= 0 || Hkv <= 0 || page_size <= 0) return FZ_BAD_SHAPE;
   Params f{};
+  if (ss) set_factors(f, ss, ss_parts, eps, K);
   f.rope = 1;
   f.cos_t = cos_t; f.sin_t = sin_t; f.pos = pos; f.seq_row = seq_row; f.table = table; f.mb = mb;
   f.k_pool = (__nv_bfloat16*)k_pool; f.v_pool = (__nv_bfloat16*)v_pool; f.page_stride = page_stride;
@@ -1476,63 +1621,23 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
     }
   }
   // rows mode: token rows are the 128 lanes; persistent CTAs with two accumulators
-  int bn = N >= 256 ? 256 : N >= 128 ? 128 : 64;     // with the fused SwiGLU N = 2 I >= 128, so a tile holds whole blocks
-  if (bn == 256 && !p.swiglu) {
-    // So few 128 x 256 tiles that the SMs are not half used, and a K worth cutting: the tiles' K ranges are cut so that
-    // about one CTA per SM works (see `gemm_tc_rows_split_kernel`). The count follows from (M, N, K) of the product.
-    const int pair_splits = fz_gemm_tc_rows_pair_splits(M, N, K);
-    if (pair_splits > 1) {      // the same with a pair of SMs on each 256 x 256 tile
-      p.splits = pair_splits;
-      p.stages = (200 * 1024) / ((BM + SPLIT_BN / 2) * BK * 2);
-      if ((st = get_map_bf16(x, M, K, BM, &ma)) != FZ_OK) return st;
-      if ((st = get_map_bf16(w, N, K, SPLIT_BN / 2, &mb)) != FZ_OK) return st;
-      return launch_rows_split<true>(ma, mb, p, (M + 2 * BM - 1) / (2 * BM), (N + SPLIT_BN - 1) / SPLIT_BN, stream);
-    }
-    const int splits = fz_gemm_tc_rows_splits(M, N, K);
-    if (splits > 1) {
-      p.splits = splits;
-      const int stage = (BM + SPLIT_BN) * BK * 2;
-      p.stages = (200 * 1024) / stage;
-      if ((st = get_map_bf16(x, M, K, BM, &ma)) != FZ_OK) return st;
-      if ((st = get_map_bf16(w, N, K, SPLIT_BN, &mb)) != FZ_OK) return st;
-      return launch_rows_split<false>(ma, mb, p, (M + BM - 1) / BM, (N + SPLIT_BN - 1) / SPLIT_BN, stream);
-    }
-  }
-  if (bn == 256 && !p.swiglu) {
-    // Few token rows: when the 256-wide tiles do not fill the SMs even once, the narrowest width that still fits one
-    // round is the fastest (256 x 4096 x 4096 is 32 tiles of 256 columns for 148 SMs, but 52 of 160). Not below 160:
-    // a 128-wide instruction reads its operands from shared memory at the rate the tensor core consumes them and runs
-    // at about half speed. With more than one round the widest tile stays: measured at 2,048 rows, 160-wide tiles in
-    // three rounds (60 -> 72 us) lose against 256-wide ones in two, whatever the count of rounds says.
-    static int sms = 0;
-    if (sms == 0) {
-      int dev = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      if (sms <= 0) sms = 148;
-    }
-    const long long tm = (M + BM - 1) / BM;
-    if (tm * ((N + 255) / 256) < sms) {
-      for (int cand : {224, 192, 160})
-        if (tm * ((N + cand - 1) / cand) <= sms) bn = cand;
-    }
-  }
-  if (bn == 256 && fz_gemm_tc_rows_pairs(M, N, K)) {
-    // many token rows: a pair of SMs on every 256 x 256 tile (see `gemm_tc_rows_pair_kernel`)
-    p.stages = (200 * 1024) / ((BM + PAIR_BN / 2) * BK * 2);
-    if ((st = get_map_bf16(x, M, K, BM, &ma)) != FZ_OK) return st;
-    if ((st = get_map_bf16(w, N, K, PAIR_BN / 2, &mb)) != FZ_OK) return st;
-    return (p.swiglu ? launch_rows_pair<4> : launch_rows_pair<2>)(ma, mb, p, (M + 2 * BM - 1) / (2 * BM), (N + PAIR_BN - 1) / PAIR_BN, device_sms(), stream);
-  }
-  {
-    const int stage = (BM + bn) * BK * 2;
-    const int st_n = (200 * 1024) / stage;
-    p.stages = st_n < 2 ? 2 : (st_n > 8 ? 8 : st_n);
-  }
+  if (p.x || p.ss) return FZ_BAD_SHAPE;
+  const RowsPlan plan = rows_plan(M, N, K, p.swiglu != 0);
+  p.splits = plan.splits;
+  const bool pair = plan.kernel == RowsPlan::PAIR || plan.kernel == RowsPlan::SPLIT_PAIR;
+  const int box = pair ? plan.bn / 2 : plan.bn, st_n = (200 * 1024) / ((BM + box) * BK * 2);
+  p.stages = st_n < 2 || pair ? st_n : st_n > 8 ? 8 : st_n;
+  if (p.stages < 2) p.stages = 2;
   if ((st = get_map_bf16(x, M, K, BM, &ma)) != FZ_OK) return st;
-  if ((st = get_map_bf16(w, N, K, bn, &mb)) != FZ_OK) return st;
-  const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + bn - 1) / bn;
-  switch (bn) {
+  if ((st = get_map_bf16(w, N, K, box, &mb)) != FZ_OK) return st;
+  const int tiles_m = (M + BM - 1) / BM, pairs_m = (M + 2 * BM - 1) / (2 * BM), tiles_n = (N + plan.bn - 1) / plan.bn;
+  switch (plan.kernel) {
+    case RowsPlan::SPLIT_PAIR: return launch_rows_split<true>(ma, mb, p, pairs_m, tiles_n, stream);
+    case RowsPlan::SPLIT: return launch_rows_split<false>(ma, mb, p, tiles_m, tiles_n, stream);
+    case RowsPlan::PAIR: return (plan.parts == 4 ? launch_rows_pair<4> : launch_rows_pair<2>)(ma, mb, p, pairs_m, tiles_n, device_sms(), stream);
+    default: break;
+  }
+  switch (plan.bn) {
     case 256: return launch_rows<256>(ma, mb, p, tiles_m, tiles_n, stream);
     case 224: return launch_rows<224>(ma, mb, p, tiles_m, tiles_n, stream);
     case 192: return launch_rows<192>(ma, mb, p, tiles_m, tiles_n, stream);

@@ -85,6 +85,14 @@ class DecoderModel:
             pn = self.layers[e.layer].mixer.position_name()
             if pn is not None and pn not in self.positions:
                 raise ValueError(f"layer {e.layer} names position encoding {pn!r}, the model has {sorted(self.positions)}")
+        # a block whose every successor's first norm takes products leaves its last one to it
+        behind: dict[int, list[bool]] = {}
+        for e, then in zip(spec.schedule, [*spec.schedule[1:], None]):
+            behind.setdefault(e.layer, []).append(getattr(self.final_norm, "takes_products", False) if then is None else
+                                                  not then.add_embedding and getattr(self.layers[then.layer], "scaled1", False))
+        for layer, takes in behind.items():
+            if hasattr(self.layers[layer], "product_left"):
+                self.layers[layer].product_left = all(takes)
         self.embed: torch.Tensor | None = None
         self.lm_head: torch.Tensor | None = None
         self.dtype: str | None = None

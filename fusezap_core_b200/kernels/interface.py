@@ -11,9 +11,23 @@ and store nothing in the cache. All sums over a row, a head or a key range are i
 on the row's own data, never on the other rows of the step.
 """
 from __future__ import annotations
+from dataclasses import dataclass
 from typing import Any
 
 import torch
+
+
+@dataclass
+class ScaledRows:
+    """The rows of an RMS norm without each row's factor (see `Ops.linear_add_norm`): rows (M, N) T, squares (M, parts) float32.
+    `linear`, `linear_swiglu` and `linear_rope_kv_write` of a table that makes them take them in place of their first operand."""
+    rows: torch.Tensor
+    squares: torch.Tensor
+    eps: float
+
+    @property
+    def shape(self) -> torch.Size:
+        return self.rows.shape
 
 
 class Ops:
@@ -366,6 +380,19 @@ class Ops:
         """out[m, n] = sum_k a[m, k] * w[n, k] (+ bias[n]); a: (M, K) T, w: (N, K) T, bias float32, out float32 or T;
         accumulation in float32, one rounding into out."""
         raise NotImplementedError
+
+    def norm_parts(self, m: int, n: int, k: int) -> int:
+        """How many partial sums of squares per row `linear_add_norm` leaves for a product of these sizes; 0 if this table has
+        no such kernel for them."""
+        return 0
+
+    def linear_add_norm(self, a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, x: torch.Tensor, weight: torch.Tensor,
+                        h: torch.Tensor, squares: torch.Tensor) -> bool:
+        """x += a . w^T + bias (x (M, N) float32), h = T(x * weight) and, in squares (M, `norm_parts(M, N, K)`) float32, partial
+        sums of the new x's squares: an RMS norm but for each row's factor 1 / sqrt(mean(x^2) + eps), which the products that
+        read h apply to their float32 sums (they take `ScaledRows` for their first operand). Returns False, having done
+        nothing, if this table cannot take the operands; the caller then runs `linear` and `add_rmsnorm`."""
+        return False
 
     def pack_gate_up(self, gate: torch.Tensor, up: torch.Tensor, gate_bias: torch.Tensor | None = None,
                      up_bias: torch.Tensor | None = None):

@@ -12,7 +12,7 @@ from ctypes import byref, c_int, c_void_p, c_float, c_longlong
 import torch
 
 from .build import load
-from .interface import Ops
+from .interface import Ops, ScaledRows
 from .profile import contexts, ideal_linear_bytes
 
 F32, BF16 = 0, 1
@@ -130,6 +130,7 @@ class CudaOps(Ops):
         self._attn_tc = self._mix = self._mix_tc = self._latent = self._latent_tc = self._seq = self._seq_tc = self._rows = self._ssd = self._ssd_tc = self._gla = self._scan_tc = None   # libraries loaded (and built) when a part first asks for their kernels
         self.prefill_tcgen05 = True        # False: long portions on the mma.sync flash-attention kernel
         self.fuse_swiglu = True            # gate/up product and SwiGLU in one kernel where the sizes allow it
+        self.fuse_norm = True              # a sublayer's last product, the residual add and the norm behind it in one kernel
         self.fuse_argmax = True            # lm_head product and argmax in one pass where no logits are asked for
         self.sink_max_runs = 64            # single-token steps over all earlier keys: a row's keys are cut into at most this many runs
         self.fuse_depth_norm = True        # the depth average of a layer's result and the norm that follows in one kernel
@@ -480,7 +481,46 @@ class CudaOps(Ops):
                     ideal_linear_bytes(m, n, k, 2, 2, out.element_size()))
         return True
 
+    @staticmethod
+    def _factors(a):
+        """The first operand's tensor, and the pointer, parts and eps of its rows' factors."""
+        if isinstance(a, ScaledRows):
+            if a.squares.dtype != torch.float32 or not a.squares.is_contiguous() or a.squares.shape[0] != a.rows.shape[0]:
+                raise KernelError(f"sums of squares {tuple(a.squares.shape)} {a.squares.dtype} for rows {tuple(a.rows.shape)}")
+            return a.rows, (_p(a.squares), c_int(a.squares.shape[1]), c_float(a.eps))
+        return a, None
+
+    def norm_parts(self, m: int, n: int, k: int) -> int:
+        if m > 128 or not (self.use_tensor_cores and self.fuse_norm and self.dtype == torch.bfloat16):
+            return 0
+        return int(self.tc.fz_gemm_tc_norm_parts(c_int(m), c_int(n), c_int(k)))
+
+    def linear_add_norm(self, a, w, bias, x, weight, h, squares) -> bool:
+        m, k = a.shape
+        n = w.shape[0]
+        parts = self.norm_parts(m, n, k)
+        if parts == 0 or weight.dtype != torch.float32 or self.tc.fz_gemm_tc_check(_p(a), _p(w), c_int(m), c_int(n), c_int(k)) != 0 or \
+                h.data_ptr() % 16:
+            return False
+        self._want(a, "linear input", (torch.bfloat16,), 2)
+        self._want(w, "linear weight", (torch.bfloat16,), 2)
+        self._want(x, "x", (torch.float32,), 2)
+        self._want(weight, "norm weight", (torch.float32,), 1)
+        self._want(h, "h", (torch.bfloat16,), 2)
+        self._want(squares, "sums of squares", (torch.float32,), 2)
+        if bias is not None:
+            self._want(bias, "linear bias", (torch.float32,), 1)
+        if w.shape[1] != k or x.shape != (m, n) or h.shape != (m, n) or weight.shape[0] != n or squares.shape != (m, parts) or \
+                (bias is not None and bias.shape[0] != n):
+            raise KernelError(f"linear_add_norm: a {tuple(a.shape)}, w {tuple(w.shape)}, x {tuple(x.shape)}, h {tuple(h.shape)}, "
+                              f"squares {tuple(squares.shape)}")
+        self._check(self.tc.fz_gemm_tc_add_norm(_p(a), _p(w), _p(bias), _p(x), _p(weight), _p(h), _p(squares), c_int(m), c_int(n), c_int(k),
+                                                _p(self.err), self._stream()), "linear_add_norm (tensor cores)",
+                    ideal_linear_bytes(m, n, k, 2, 2, 10))
+        return True
+
     def linear(self, a, w, bias, out) -> None:
+        a, factors = self._factors(a)
         self._want(a, "linear input", (self.dtype,), 2)
         self._want(w, "linear weight", (self.dtype,), 2)
         self._want(out, "linear output", (torch.float32, self.dtype), 2)
@@ -490,7 +530,14 @@ class CudaOps(Ops):
         n = w.shape[0]
         if w.shape[1] != k or out.shape != (m, n) or (bias is not None and bias.shape[0] != n):
             raise KernelError(f"linear: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+        if factors is not None:
+            self._normed(a, factors, w, bias, out, m, n, k, 0, "linear (tensor cores)", ideal_linear_bytes(m, n, k, 2, 2, out.element_size()))
+            return
         self._gemm(a, w, bias, out, m, n, k)
+
+    def _normed(self, a, factors, w, bias, out, m, n, k, kind, what, nbytes) -> None:
+        self._check(self.tc.fz_gemm_tc_normed(_p(a), *factors, _p(w), _p(bias), _p(out), c_int(_CODE[out.dtype]), c_int(m), c_int(n),
+                                              c_int(k), c_int(kind), _p(self.err), self._stream()), what, nbytes)
 
     def _gemm(self, a, w, bias, out, m, n, k) -> None:
         if self.use_tensor_cores and self.tc.fz_gemm_tc_check(_p(a), _p(w), c_int(m), c_int(n), c_int(k)) == 0:
@@ -517,11 +564,16 @@ class CudaOps(Ops):
 
     def linear_swiglu(self, a, packed, out, activation: str = "silu") -> None:
         w, b, i = packed
+        a, factors = self._factors(a)
         self._want(a, "linear input", (torch.bfloat16,), 2)
         self._want(out, "swiglu output", (torch.bfloat16,), 2)
         m, k = a.shape
         if w.shape != (2 * i, k) or out.shape != (m, i):
             raise KernelError(f"linear_swiglu: a {tuple(a.shape)}, packed {tuple(w.shape)}, out {tuple(out.shape)}")
+        if factors is not None:
+            self._normed(a, factors, w, b, out, m, 2 * i, k, self._gate_kind(activation), "linear_swiglu (tensor cores)",
+                         ideal_linear_bytes(m, 2 * i, k, 2, 2, 1))
+            return
         self._check(self.tc.fz_gemm_tc_swiglu(_p(a), _p(w), _p(b), _p(out), c_int(m), c_int(i), c_int(k),
                                               c_int(self._gate_kind(activation)), _p(self.err),
                                               self._stream()), "linear_swiglu (tensor cores)",
@@ -558,6 +610,7 @@ class CudaOps(Ops):
             c_int(cos.shape[0]), _p(self.err), self._stream()), "rope_kv_write")
 
     def linear_rope_kv_write(self, a, w, bias, cos, sin, meta, cache, q_out, num_heads, num_kv_heads, head_dim) -> bool:
+        a, factors = self._factors(a)
         m, k = a.shape
         if not (self.use_tensor_cores and self.fuse_rope and self.dtype == torch.bfloat16) or \
                 self.tc.fz_gemm_tc_qkv_rope_check(c_int(m), c_int(head_dim)) != 0 or \
@@ -578,8 +631,8 @@ class CudaOps(Ops):
         kp, vp, page_stride = self._pool(cache, num_kv_heads, head_dim)
         table = meta.table(cache.group)
         self._check(self.tc.fz_gemm_tc_qkv_rope(
-            _p(a), _p(w), _p(bias), c_int(m), c_int(k), _p(cos), _p(sin), _p(meta.pos), _p(meta.seq_row), _p(table),
-            c_int(table.shape[1]), _p(kp), _p(vp), c_longlong(page_stride), c_int(cache.page_size),
+            _p(a), *(factors or (_p(None), c_int(0), c_float(0.0))), _p(w), _p(bias), c_int(m), c_int(k), _p(cos), _p(sin), _p(meta.pos),
+            _p(meta.seq_row), _p(table), c_int(table.shape[1]), _p(kp), _p(vp), c_longlong(page_stride), c_int(cache.page_size),
             c_int(1 if cache.write else 0), _p(q_out), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim),
             c_int(cos.shape[0]), _p(self.err), self._stream()), "linear_rope_kv_write (tensor cores)",
             ideal_linear_bytes(m, n, k, 2, 2, 2))

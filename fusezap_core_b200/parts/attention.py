@@ -13,7 +13,7 @@ import torch
 
 from ..cache import KVNeed
 from ..weights import ParamSpec
-from .base import LayerCache, Mixer, register_mixer
+from .base import LayerCache, Mixer, PendingProduct, register_mixer
 
 
 @register_mixer("gqa_attention")
@@ -57,7 +57,13 @@ class GQAttention(Mixer):
     def step_needs(self) -> tuple[str, ...]:
         return ("attention",)
 
+    takes_scaled = True      # h may be `ScaledRows`
+
     def forward(self, ctx, h: torch.Tensor, cache: LayerCache) -> torch.Tensor:
+        return self.forward_pending(ctx, h, cache).resolve(ctx, None)
+
+    def forward_pending(self, ctx, h, cache: LayerCache) -> PendingProduct:
+        """`forward` with the output product left to the norm behind it."""
         n, ops, ws = h.shape[0], ctx.ops, ctx.ws
         Hq, Hkv, hd = self.Hq, self.Hkv, self.hd
         q = ws.get("q", (n, Hq * hd), ops.dtype)
@@ -68,6 +74,4 @@ class GQAttention(Mixer):
             position.rotate_and_store(ctx, qkv, q, cache, Hq, Hkv, hd)
         o = ws.get("attn_out", (n, Hq * hd), ops.dtype)
         ops.paged_attention(q, cache, ctx.meta, o, Hq, Hkv, hd, self.scale, self.window)
-        delta = ws.get("delta", (n, self.D), torch.float32)
-        ops.linear(o, self.wo, self.bo, delta)
-        return delta
+        return PendingProduct(o, self.wo, self.bo)

@@ -111,6 +111,20 @@ class PendingNorm:
         return out
 
 
+@dataclass
+class PendingProduct:
+    """A pending residual term that is still to be computed, rows . weight^T + bias, with nothing read or written in between: what a
+    sublayer hands to a norm with `takes_products`, which can have the product end in the stream and the norm."""
+    rows: torch.Tensor
+    weight: torch.Tensor
+    bias: torch.Tensor | None
+
+    def resolve(self, ctx, x) -> torch.Tensor:
+        out = ctx.ws.get("delta", (self.rows.shape[0], self.weight.shape[0]), torch.float32)
+        ctx.ops.linear(self.rows, self.weight, self.bias, out)
+        return out
+
+
 class Part:
     # False for a part whose forward depends on the step's host-side metadata (for instance a Python loop over
     # `ctx.meta.segments`): such a step cannot be replayed from a captured CUDA graph, and the engine then runs every

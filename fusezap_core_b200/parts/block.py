@@ -25,6 +25,10 @@ class PreNormBlock(Block):
         self.norm2 = None
         if ffn is not None:
             self.norm2 = make_norm(norms[1]) if norms[1] is not None else make_norm()
+        # Which of its norms may hand `ScaledRows` on (see `Ops.linear_add_norm`), and so take a sublayer's last product unlaunched.
+        self.scaled1, self.scaled2 = (getattr(norm, "takes_products", False) and getattr(part, "takes_scaled", False)
+                                      for norm, part in ((self.norm1, mixer), (self.norm2, ffn)))
+        self.product_left = False      # the model says whether the norm behind the block takes the feed-forward's
 
     def children(self):
         n1, mx, n2, ff = self.names
@@ -47,13 +51,16 @@ class PreNormBlock(Block):
             part.bind(own, ops)
 
     def forward(self, ctx, x, delta, cache: LayerCache):
-        h = self.norm1.forward(ctx, x, delta)
-        delta = self.mixer.forward(ctx, h, cache)
+        h = self.norm1.forward(ctx, x, delta, scaled=True) if self.scaled1 else self.norm1.forward(ctx, x, delta)
         if self.ffn is None:
-            return x, delta
-        h = self.norm2.forward(ctx, x, delta)
-        delta = self.ffn.forward(ctx, h)
-        return x, delta
+            return x, self.mixer.forward(ctx, h, cache)
+        if self.scaled2 and hasattr(self.mixer, "forward_pending"):
+            h = self.norm2.forward(ctx, x, self.mixer.forward_pending(ctx, h, cache), scaled=True)
+        else:
+            h = self.norm2.forward(ctx, x, self.mixer.forward(ctx, h, cache))
+        if self.product_left and hasattr(self.ffn, "forward_pending"):
+            return x, self.ffn.forward_pending(ctx, h)
+        return x, self.ffn.forward(ctx, h)
 
 
 @register_block("sandwich_norm")

@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 
 from ..weights import ParamSpec
-from .base import FeedForward, register_feed_forward
+from .base import FeedForward, PendingProduct, register_feed_forward
 
 
 @register_feed_forward("swiglu")
@@ -50,8 +50,9 @@ class SwiGLU(FeedForward):
         self.wd = tensors[f"{d}{sx}"]
         self.bd = tensors[f"{d}.bias"].float() if f"{d}.bias" in tensors else None
 
-    def forward(self, ctx, h: torch.Tensor, tag: str = "") -> torch.Tensor:
-        """tag: a prefix for the names of its scratch buffers (a feed-forward that runs inside another one)."""
+    takes_scaled = True      # h may be `ScaledRows`
+
+    def _act(self, ctx, h, tag: str = "") -> torch.Tensor:
         n, ops, ws = h.shape[0], ctx.ops, ctx.ws
         a = ws.get(tag + "act", (n, self.I), ops.dtype)
         other = {} if self.activation == "silu" else {"activation": self.activation}
@@ -61,9 +62,18 @@ class SwiGLU(FeedForward):
             gu = ws.get(tag + "gate_up", (n, 2 * self.I), ops.dtype)
             ops.linear(h, self.wgu, self.bgu, gu)
             ops.swiglu(gu, a, **other)
-        delta = ws.get(tag + "delta", (n, self.D), torch.float32)
-        ops.linear(a, self.wd, self.bd, delta)
+        return a
+
+    def forward(self, ctx, h: torch.Tensor, tag: str = "") -> torch.Tensor:
+        """tag: a prefix for the names of its scratch buffers (a feed-forward that runs inside another one)."""
+        a = self._act(ctx, h, tag)
+        delta = ctx.ws.get(tag + "delta", (a.shape[0], self.D), torch.float32)
+        ctx.ops.linear(a, self.wd, self.bd, delta)
         return delta
+
+    def forward_pending(self, ctx, h) -> PendingProduct:
+        """`forward` with the down product left to the norm behind it."""
+        return PendingProduct(self._act(ctx, h), self.wd, self.bd)
 
 
 @register_feed_forward("ungated")

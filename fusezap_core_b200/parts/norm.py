@@ -15,7 +15,8 @@ from __future__ import annotations
 import torch
 
 from ..weights import ParamSpec
-from .base import Norm, PendingNorm, PendingSum, register_norm
+from ..kernels.interface import ScaledRows
+from .base import Norm, PendingNorm, PendingProduct, PendingSum, register_norm
 
 
 @register_norm("rmsnorm")
@@ -31,6 +32,12 @@ class RMSNorm(Norm):
         self.size, self.eps, self.groups, self.name, self.scalar = size, float(eps), int(groups), name, bool(scalar)
         self.offset = float(offset)
         self.weight: torch.Tensor | None = None
+        self.weight32: torch.Tensor | None = None
+
+    @property
+    def takes_products(self) -> bool:
+        """Whether the pending term may be a `PendingProduct`."""
+        return True
 
     def tensors(self) -> dict[str, ParamSpec]:
         return {self.name: ParamSpec(() if self.scalar else (self.size,), role="vector", init="normal" if self.offset else "ones")}
@@ -41,10 +48,21 @@ class RMSNorm(Norm):
             self.weight = (self.weight.float() + self.offset).contiguous()
         if self.scalar:      # the kernels take a weight per coordinate
             self.weight = self.weight.float().reshape(1).expand(self.size).contiguous()
+        self.weight32 = self.weight.float()      # (the product that ends in the norm takes float32)
 
-    def forward(self, ctx, x, delta, rows=None, n_rows=None):
+    def forward(self, ctx, x, delta, rows=None, n_rows=None, scaled: bool = False):
+        """scaled: the caller's next part takes `ScaledRows`; it gets them where the pending term is a product whose kernel can
+        end in the norm."""
         n = x.shape[0] if rows is None else (n_rows if n_rows is not None else rows.shape[0])
         h = ctx.ws.get("norm_h" if rows is None else "norm_h_rows", (n, self.size), ctx.ops.dtype)
+        if isinstance(delta, PendingProduct):
+            count = getattr(ctx.ops, "norm_parts", None)      # an optional entry of the kernel table
+            parts = count(n, self.size, delta.rows.shape[1]) if count is not None and scaled and rows is None and self.groups == 1 else 0
+            if parts:
+                squares = ctx.ws.get("norm_squares", (n, parts), torch.float32)
+                if ctx.ops.linear_add_norm(delta.rows, delta.weight, delta.bias, x, self.weight32, h, squares):
+                    return ScaledRows(h, squares, self.eps)
+            delta = delta.resolve(ctx, x)
         self._run(ctx, x, delta, h, rows)
         return h
 

@@ -172,6 +172,64 @@ def test_tokens_dealt_out_to_the_splits(tiles, splits):
     ops.check_errors()
 
 
+@pytest.mark.parametrize("D,K", [(896, 4864), (4096, 4096), (136, 72), (1000, 200), (16384, 128)])
+def test_product_that_ends_in_the_norm(D, K):
+    """x += a . w^T + bias and the norm behind it in the product's kernel, then the products that read its rows: the stream has
+    the bits of the product followed by an addition, h those of x * weight, and what reads them is the product of the normed
+    rows; at rows around the groups that the tokens are dealt out in."""
+    from fusezap_core_b200.kernels import cuda_ops
+    from fusezap_core_b200.kernels.interface import ScaledRows
+    from test_kernels_gpu import Meta, make_cache
+    ops, eps = cuda_ops("bfloat16"), 1e-5
+    g = torch.Generator(device="cuda").manual_seed(D + K)
+    a, w = (torch.randn(n, K, generator=g, device="cuda").to(torch.bfloat16) for n in (128, D))
+    x0 = 30 * torch.randn(128, D, generator=g, device="cuda")
+    bias, weight = torch.randn(D, generator=g, device="cuda"), 1 + 0.1 * torch.randn(D, generator=g, device="cuda")
+    Hq, Hkv, hd, inner = 3, 1, 64, 192
+    wq = (torch.randn((Hq + 2 * Hkv) * hd, D, generator=g, device="cuda") * D ** -0.5).to(torch.bfloat16)
+    bq = torch.randn(wq.shape[0], generator=g, device="cuda")
+    gate, up = ((torch.randn(inner, D, generator=g, device="cuda") * D ** -0.5).to(torch.bfloat16) for _ in range(2))
+    packed = ops.pack_gate_up(gate, up)
+    ang = torch.rand(200, hd // 2, generator=g, device="cuda") * 6.28
+    for rows in (1, 2, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128):
+        parts = ops.norm_parts(rows, D, K)
+        assert parts == -(-D // 128) * 4
+        x, h = x0[:rows].clone(), torch.empty(rows, D, dtype=torch.bfloat16, device="cuda")
+        squares = torch.full((rows, parts), float("nan"), device="cuda")
+        assert ops.linear_add_norm(a[:rows].contiguous(), w, bias, x, weight, h, squares)
+        delta = torch.empty(rows, D, device="cuda")
+        ops.linear(a[:rows].contiguous(), w, bias, delta)
+        assert torch.equal(x, x0[:rows] + delta) and torch.equal(h, (x * weight).to(torch.bfloat16)), f"{rows} rows"
+        mean = x.double().square().mean(1)
+        # at most 5 additions of 32 squares each, rounding each by 2^-24 of a partial sum of one sign
+        assert bool(((squares.double().sum(1) / D - mean).abs() <= 8 * 2.0 ** -24 * mean).all())
+        factor = (mean + eps).rsqrt()[:, None]
+        normed, scaled = factor * h.double(), ScaledRows(h, squares, eps)
+        out = torch.empty(rows, wq.shape[0], device="cuda")
+        ops.linear(scaled, wq, bq, out)
+        # (D exact products, each addition off by at most 2^-23 of the magnitudes' sum, and the factor's own 40 roundings)
+        bound = (D + 48) * 2.0 ** -23 * (normed.abs() @ wq.abs().double().T + bq.abs().double())
+        assert bool(((out.double() - (normed @ wq.double().T + bq.double())).abs() <= bound).all()), f"{rows} rows"
+        act = torch.empty(rows, inner, dtype=torch.bfloat16, device="cuda")
+        ops.linear_swiglu(scaled, packed, act)
+        z = normed @ gate.double().T
+        ref = z / (1 + torch.exp(-z)) * (normed @ up.double().T)
+        assert float((act.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()) * 1.01, f"{rows} rows"
+        if rows <= 32:      # the rotated product against the plain one and the rotation's kernel
+            meta = Meta([3 * i % 200 for i in range(rows)], [i % 2 for i in range(rows)], [list(range(13)), list(range(13, 26))], "cuda")
+            res = []
+            for fused in (True, False):
+                cache, q = make_cache(26, Hkv, 16, hd, torch.bfloat16, "cuda"), torch.empty(rows, Hq * hd, dtype=torch.bfloat16, device="cuda")
+                if fused:
+                    assert ops.linear_rope_kv_write(scaled, wq, bq, ang.cos(), ang.sin(), meta, cache, q, Hq, Hkv, hd)
+                else:
+                    ops.rope_kv_write(out, ang.cos(), ang.sin(), meta, cache, q, Hq, Hkv, hd)
+                res.append((q, cache.pool.clone()))
+            assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1]), f"{rows} rows"
+    ops.check_errors()
+    assert ops.norm_parts(129, D, K) == 0 and ops.norm_parts(1, D, 64) == 0 and ops.norm_parts(1, 129 * 128, K) == 0 and ops.norm_parts(1, D + 4, K) == 0
+
+
 def test_refused_shapes_fall_back_to_the_plain_kernel():
     from fusezap_core_b200.kernels import cuda_ops
     ops = cuda_ops("bfloat16")
