@@ -302,28 +302,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // (Used here, so that the loads cannot be put off to the end: 0.9 us of the q/k/v product with a bias.)
     asm volatile("" ::"f"(b1), "f"(b2), "f"(nw) : "memory");
   }
-  if (warp != 0) fz_grid_wait();    // warp 0 waits after it has requested the first weight stages
-  float xs[VW] = {};      // EP_NORM: the stream's values of the tokens that this thread finishes next
-  if (warp >= 2) {
-    if constexpr (EP == EP_NORM) {
-#pragma unroll
-      for (int e = 0; e < VW; ++e)
-        if (own && split * VW + e < cols) xs[e] = p.x[(size_t)(split * VW + e) * p.feats + feat];
-    } else if (p.ss != nullptr) {      // (while the products are under way)
-      const int tokens = p.splits > 1 ? mine * VW : cols;
-#pragma unroll 4
-      for (int t = warp & 3; t < tokens; t += 4) {
-        const int m = p.splits > 1 ? (split + t / VW * p.splits) * VW + t % VW : t;
-        float sum = 0.f;
-        if (m < cols)
-          for (int i = lane; i < p.ss_parts; i += 32) sum += p.ss[(size_t)m * p.ss_parts + i];
-        sum = warp_sum(sum);
-        if (lane == 0) factor[t] = 1.0f / sqrtf(sum * p.ss_mean + p.ss_eps);
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-    }
-  }
-
+  if (warp == 1) fz_grid_wait();      // (warp 0 waits after it has requested the first weight stages)
   if (warp == 0) {
     if (lane == 0) {
       // The weights (A) do not depend on the kernel before this one: their first stages are requested before the wait on
@@ -370,191 +349,235 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       umma_commit(acc_ready);   // arrives when every MMA issued so far has finished (at once if none was issued)
     }
   }
-  bool ok = true;
-  if (warp >= 2) {      // the epilogue: 4 warps, warp w reads TMEM lanes 32 * (w % 4) ..
-    ok = __all_sync(0xffffffffu, mbar_wait(acc_ready, 0));   // warp-uniform: tcgen05.ld is warp-wide
-    if (!ok) flag[0] = 1;
-    tc_fence_after();
-  }
-  if (p.splits > 1) {
-    // Every CTA sends, whatever became of its waits, and nobody leaves before all that it is sent has arrived: no CTA's
-    // memory goes away under a sender. In the ring's memory the parts may arrive once every CTA of the cluster has consumed
-    // its stages. (Fetched column by column from the other CTAs' shared memory, with a cluster barrier before and one behind,
-    // what follows the accumulator took 2.0 to 2.6 us of each of a layer's products at Qwen2.5-0.5B sizes at one row and 3.0 to
-    // 5.7 at 32; 0.9 to 1.2 and 1.3 to 3.4 now. Decode steps: 1 row of 300 keys 674 -> 592 us, 32 of 1,280 1,057 -> 879; at
-    // Llama-3.1-8B sizes 1, 8 and 64 rows of 4,096 keys 3,085 -> 2,957, 3,604 -> 3,455, 7,752 -> 7,643.)
-    cluster_wait();
-    if (p.parts_in_ring) cluster_sync_all();
-  }
-  if (warp >= 2) {
-    const uint32_t taddr = tmem_d + ((uint32_t)((warp & 3) * 32) << 16);
-    const bool live = ok && nkb > 0;
-    const uint32_t bar = smem_u32(parts_here);
-    uint32_t at = smem_u32(parts) + (uint32_t)(split * part_step + r * VW) * 4u, to = 0;
+  if (warp < 2) {
+    if (p.splits > 1) {
+      cluster_wait();
+      if (p.parts_in_ring) cluster_sync_all();
+    }
+  } else {
+    // The epilogue: 4 warps, warp w reads TMEM lanes 32 * (w % 4) ... With a token at most for each CTA of a cluster they walk
+    // through what they will do once before they wait, with nothing loaded, sent or stored: its instructions then are in the SM's
+    // cache instead of on their way from L2, line by line, at the end of a chain of a few microseconds. Decode steps at
+    // Qwen2.5-0.5B sizes, 1 row of 300 keys and 8 of 224, 552 -> 535 us, 618 -> 595; at Llama-3.1-8B sizes, 8 rows of 4,096, 3,415 ->
+    // 3,375. With groups of four tokens the code for both passes costs more than it saves (32 rows of 1,280 keys 832 -> 868 us).
+    float xs[VW] = {};      // EP_NORM: the stream's values of the tokens that this thread finishes next
+    int pass = 1;
+    if constexpr (VW == 1) {
+      pass = p.splits > 1 ? 0 : 1;
+      asm volatile("" : "+r"(pass));      // (two passes through the same code, not two copies of it)
+    }
 #pragma unroll 1
-    for (int c = 0; c < cols; c += 16) {
-      float v[16];
-      if (live) tmem_ld16(taddr + (uint32_t)c, v);
-      else {
+    for (; pass < 2; ++pass) {
+      const bool real = VW > 1 || pass == 1;
+      bool ok = true;
+      if (real) {
+        fz_grid_wait();
+        if constexpr (EP == EP_NORM) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) v[e] = 0.f;
+          for (int e = 0; e < VW; ++e)
+            if (own && split * VW + e < cols) xs[e] = p.x[(size_t)(split * VW + e) * p.feats + feat];
+        } else if (p.ss != nullptr) {      // (while the products are under way)
+          const int tokens = p.splits > 1 ? mine * VW : cols;
+#pragma unroll 4
+          for (int t = warp & 3; t < tokens; t += 4) {
+            const int m = p.splits > 1 ? (split + t / VW * p.splits) * VW + t % VW : t;
+            float sum = 0.f;
+            if (m < cols)
+              for (int i = lane; i < p.ss_parts; i += 32) sum += p.ss[(size_t)m * p.ss_parts + i];
+            sum = warp_sum(sum);
+            if (lane == 0) factor[t] = 1.0f / sqrtf(sum * p.ss_mean + p.ss_eps);
+          }
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
+        ok = __all_sync(0xffffffffu, mbar_wait(acc_ready, 0));   // warp-uniform: tcgen05.ld is warp-wide
+        if (!ok) flag[0] = 1;
+        tc_fence_after();
+        if (p.splits > 1) {
+          // Every CTA sends, whatever became of its waits, and nobody leaves before all that it is sent has arrived: no CTA's
+          // memory goes away under a sender. In the ring's memory the parts may arrive once every CTA of the cluster has consumed
+          // its stages. (Fetched column by column from the other CTAs' shared memory, with a cluster barrier before and one behind,
+          // what follows the accumulator took 2.0 to 2.6 us of each of a layer's products at Qwen2.5-0.5B sizes at one row and 3.0 to
+          // 5.7 at 32; 0.9 to 1.2 and 1.3 to 3.4 now. Decode steps: 1 row of 300 keys 674 -> 592 us, 32 of 1,280 1,057 -> 879; at
+          // Llama-3.1-8B sizes 1, 8 and 64 rows of 4,096 keys 3,085 -> 2,957, 3,604 -> 3,455, 7,752 -> 7,643.)
+          cluster_wait();
+          if (p.parts_in_ring) cluster_sync_all();
+        }
       }
-      if (p.splits > 1) {
+      const uint32_t taddr = tmem_d + ((uint32_t)((warp & 3) * 32) << 16);
+      const bool live = ok && nkb > 0;
+      const uint32_t bar = smem_u32(parts_here);
+      uint32_t at = smem_u32(parts) + (uint32_t)(split * part_step + r * VW) * 4u, to = 0;
+#pragma unroll 1
+      for (int c = 0; c < cols; c += 16) {
+        float v[16];
+        if (live && real) tmem_ld16(taddr + (uint32_t)c, v);
+        else {
 #pragma unroll
-        for (int e = 0; e < 16; e += VW) {
-          if (c + e >= cols) break;
-          send_floats<VW>(map_to_cta(at, to), map_to_cta(bar, to), v + e);
-          if (++to == (uint32_t)p.splits) { to = 0; at += PART_GROUP * 4; }
+          for (int e = 0; e < 16; ++e) v[e] = 0.f;
+        }
+        if (p.splits > 1) {
+#pragma unroll
+          for (int e = 0; e < 16; e += VW) {
+            if (c + e >= cols) break;
+            if (real) send_floats<VW>(map_to_cta(at, to), map_to_cta(bar, to), v + e);
+            if (++to == (uint32_t)p.splits) { to = 0; at += PART_GROUP * 4; }
+          }
+        } else if (EP == EP_ARGMAX) {
+          // the tile's logits go to the (idle) stage buffers as [token][feature], rows one float apart from a multiple of
+          // the bank count, and are searched below
+#pragma unroll
+          for (int e = 0; e < 16; ++e) ((float*)smem)[(c + e) * (BM + 1) + r] = v[e] + b1;
+        } else if (EP == EP_GLU) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) ((float*)smem)[(c + e) * BM + r] = v[e];      // [token][feature]
+        } else if (EP == EP_ROPE) {
+#pragma unroll
+          for (int e = 0; e < 16; e += 4) ((float4*)smem)[((c + e) >> 2) * BM + r] = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+        } else if (own) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const int m = c + e;
+            if (m < cols) {
+              const float y = finished(p, fmaf(v[e], p.ss ? factor[m] : 1.f, b1));
+              if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = y;
+              else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(y);
+            }
+          }
+        }
+      }
+      bool summed = true;      // this thread's tokens are complete in `parts`
+      if (p.splits > 1) {
+        if (real) summed = mbar_wait_cluster(parts_here, 0);
+        if (!summed) flag[0] = 1;
+      } else if (EP != EP_PLAIN) asm volatile("bar.sync 1, 128;" ::: "memory");
+
+      if (EP == EP_GLU && p.splits == 1) {
+        // K not split: the tile is complete in this CTA's shared memory. A warp takes every fourth token, a lane two
+        // neighbouring features of the 64.
+        const int f = 2 * lane, g0 = tile * BM + f;
+        if (ok && g0 < p.feats) {
+          float2 bg = make_float2(0.f, 0.f), bu = bg;
+          if (p.bias) { bg = make_float2(p.bias[g0], p.bias[g0 + 1]); bu = make_float2(p.bias[g0 + 64], p.bias[g0 + 65]); }
+          const float* t = (const float*)smem + f;
+          __nv_bfloat16* dst = p.c_bf16 + tile * 64 + f;
+#pragma unroll 4
+          for (int c = warp & 3; c < cols; c += 4) {
+            const float2 g = *(const float2*)(t + c * BM), u = *(const float2*)(t + c * BM + 64);
+            const float sc = p.ss ? factor[c] : 1.f;      // (times one: the sum's bits)
+            const __nv_bfloat162 y = __floats2bfloat162_rn(glu_mul(fmaf(g.x, sc, bg.x), fmaf(u.x, sc, bu.x), p.swiglu), glu_mul(fmaf(g.y, sc, bg.y), fmaf(u.y, sc, bu.y), p.swiglu));
+            *(__nv_bfloat162*)(dst + (size_t)c * (p.feats >> 1)) = y;
+          }
         }
       } else if (EP == EP_ARGMAX) {
-        // the tile's logits go to the (idle) stage buffers as [token][feature], rows one float apart from a multiple of
-        // the bank count, and are searched below
-#pragma unroll
-        for (int e = 0; e < 16; ++e) ((float*)smem)[(c + e) * (BM + 1) + r] = v[e] + b1;
-      } else if (EP == EP_GLU) {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) ((float*)smem)[(c + e) * BM + r] = v[e];      // [token][feature]
-      } else if (EP == EP_ROPE) {
-#pragma unroll
-        for (int e = 0; e < 16; e += 4) ((float4*)smem)[((c + e) >> 2) * BM + r] = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
-      } else if (own) {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int m = c + e;
-          if (m < cols) {
-            const float y = finished(p, fmaf(v[e], p.ss ? factor[m] : 1.f, b1));
-            if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = y;
-            else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(y);
-          }
-        }
-      }
-    }
-    bool summed = true;      // this thread's tokens are complete in `parts`
-    if (p.splits > 1) {
-      summed = mbar_wait_cluster(parts_here, 0);
-      if (!summed) flag[0] = 1;
-    } else if (EP != EP_PLAIN) asm volatile("bar.sync 1, 128;" ::: "memory");
-
-    if (EP == EP_GLU && p.splits == 1) {
-      // K not split: the tile is complete in this CTA's shared memory. A warp takes every fourth token, a lane two
-      // neighbouring features of the 64.
-      const int f = 2 * lane, g0 = tile * BM + f;
-      if (ok && g0 < p.feats) {
-        float2 bg = make_float2(0.f, 0.f), bu = bg;
-        if (p.bias) { bg = make_float2(p.bias[g0], p.bias[g0 + 1]); bu = make_float2(p.bias[g0 + 64], p.bias[g0 + 65]); }
-        const float* t = (const float*)smem + f;
-        __nv_bfloat16* dst = p.c_bf16 + tile * 64 + f;
+        // 128 / BN threads share a token: each scans its part of the tile's 128 features in rising order (so the lower
+        // index wins among equals), then the parts are merged in rising order
+        constexpr int TPC = BM / BN < 1 ? 1 : BM / BN;          // threads per token
+        constexpr int SEG = BM / TPC;                            // features per thread
+        const float* am = (const float*)smem;
+        float* best_v = (float*)smem + BN * (BM + 1);            // [BN][TPC]
+        int* best_i = (int*)(best_v + BN * TPC);
+        const int col = r % BN, seg = r / BN;                    // (for BN = 128 every thread has a token of its own)
+        float x = 0.f;
+        int ix = 0x7fffffff;
+        if (seg < TPC) {
 #pragma unroll 4
-        for (int c = warp & 3; c < cols; c += 4) {
-          const float2 g = *(const float2*)(t + c * BM), u = *(const float2*)(t + c * BM + 64);
-          const float sc = p.ss ? factor[c] : 1.f;      // (times one: the sum's bits)
-          const __nv_bfloat162 y = __floats2bfloat162_rn(glu_mul(fmaf(g.x, sc, bg.x), fmaf(u.x, sc, bu.x), p.swiglu), glu_mul(fmaf(g.y, sc, bg.y), fmaf(u.y, sc, bu.y), p.swiglu));
-          *(__nv_bfloat162*)(dst + (size_t)c * (p.feats >> 1)) = y;
-        }
-      }
-    } else if (EP == EP_ARGMAX) {
-      // 128 / BN threads share a token: each scans its part of the tile's 128 features in rising order (so the lower
-      // index wins among equals), then the parts are merged in rising order
-      constexpr int TPC = BM / BN < 1 ? 1 : BM / BN;          // threads per token
-      constexpr int SEG = BM / TPC;                            // features per thread
-      const float* am = (const float*)smem;
-      float* best_v = (float*)smem + BN * (BM + 1);            // [BN][TPC]
-      int* best_i = (int*)(best_v + BN * TPC);
-      const int col = r % BN, seg = r / BN;                    // (for BN = 128 every thread has a token of its own)
-      float x = 0.f;
-      int ix = 0x7fffffff;
-      if (seg < TPC) {
-#pragma unroll 4
-        for (int i = 0; i < SEG; ++i) {
-          const int f = seg * SEG + i, ft = tile * BM + f;
-          if (ft < p.feats && am_better(am[col * (BM + 1) + f], ft, x, ix)) { x = am[col * (BM + 1) + f]; ix = ft; }
-        }
-        best_v[col * TPC + seg] = x;
-        best_i[col * TPC + seg] = ix;
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (seg == 0 && col < cols) {
-#pragma unroll 1
-        for (int sgm = 1; sgm < TPC; ++sgm)
-          if (am_better(best_v[col * TPC + sgm], best_i[col * TPC + sgm], x, ix)) { x = best_v[col * TPC + sgm]; ix = best_i[col * TPC + sgm]; }
-        p.am_val[(size_t)col * gridDim.x + tile] = x;
-        p.am_idx[(size_t)col * gridDim.x + tile] = ix;
-      }
-    } else if constexpr (EP == EP_NORM) {
-      summed = __all_sync(0xffffffffu, summed);
-#pragma unroll 1
-      for (int i = 0; i < mine && summed; ++i) {      // (a warp's lanes stay together: they add up their squares)
-        alignas(16) float y[VW];
-        float sq[VW], old[VW];
-#pragma unroll
-        for (int e = 0; e < VW; ++e) {
-          old[e] = xs[e];
-          const int m = (split + (i + 1) * p.splits) * VW + e;
-          if (own && m < cols) xs[e] = p.x[(size_t)m * p.feats + feat];
-        }
-        sum_parts<VW>(parts + i * PART_GROUP + r * VW, p.splits, part_step, y);
-#pragma unroll
-        for (int e = 0; e < VW; ++e) {
-          const int m = (split + i * p.splits) * VW + e;
-          sq[e] = 0.f;
-          if (own && m < cols) {
-            const size_t at = (size_t)m * p.feats + feat;
-            const float v = old[e] + (y[e] + b1);
-            p.x[at] = v;
-            p.h[at] = __float2bfloat16_rn(v * nw);
-            sq[e] = v * v;
+          for (int i = 0; i < SEG; ++i) {
+            const int f = seg * SEG + i, ft = tile * BM + f;
+            if (ft < p.feats && am_better(am[col * (BM + 1) + f], ft, x, ix)) { x = am[col * (BM + 1) + f]; ix = ft; }
           }
+          best_v[col * TPC + seg] = x;
+          best_i[col * TPC + seg] = ix;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-          for (int e = 0; e < VW; ++e) sq[e] += __shfl_xor_sync(0xffffffffu, sq[e], o);
-#pragma unroll
-        for (int e = 0; e < VW; ++e) {
-          const int m = (split + i * p.splits) * VW + e;
-          if (lane == e && m < cols) p.ss_out[(size_t)m * p.ss_parts + tile * 4 + (warp & 3)] = sq[e];
-        }
-      }
-    } else if constexpr (EP == EP_PLAIN) {
-      if (p.splits > 1 && summed && own) {
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (seg == 0 && col < cols) {
 #pragma unroll 1
-        for (int i = 0; i < mine; ++i) {
+          for (int sgm = 1; sgm < TPC; ++sgm)
+            if (am_better(best_v[col * TPC + sgm], best_i[col * TPC + sgm], x, ix)) { x = best_v[col * TPC + sgm]; ix = best_i[col * TPC + sgm]; }
+          p.am_val[(size_t)col * gridDim.x + tile] = x;
+          p.am_idx[(size_t)col * gridDim.x + tile] = ix;
+        }
+      } else if constexpr (EP == EP_NORM) {
+        summed = __all_sync(0xffffffffu, summed);
+#pragma unroll 1
+        for (int i = 0; i < mine && summed; ++i) {      // (a warp's lanes stay together: they add up their squares)
           alignas(16) float y[VW];
+          float sq[VW], old[VW];
+#pragma unroll
+          for (int e = 0; e < VW; ++e) {
+            old[e] = xs[e];
+            const int m = (split + (i + 1) * p.splits) * VW + e;
+            if (real && own && m < cols) xs[e] = p.x[(size_t)m * p.feats + feat];
+          }
           sum_parts<VW>(parts + i * PART_GROUP + r * VW, p.splits, part_step, y);
 #pragma unroll
           for (int e = 0; e < VW; ++e) {
             const int m = (split + i * p.splits) * VW + e;
-            if (m >= cols) break;
-            const float v = finished(p, fmaf(y[e], p.ss ? factor[i * VW + e] : 1.f, b1));
-            if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = v;
-            else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(v);
+            sq[e] = 0.f;
+            if (own && m < cols) {
+              const size_t at = (size_t)m * p.feats + feat;
+              const float v = old[e] + (y[e] + b1);
+              if (real) {
+                p.x[at] = v;
+                p.h[at] = __float2bfloat16_rn(v * nw);
+              }
+              sq[e] = v * v;
+            }
+          }
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int e = 0; e < VW; ++e) sq[e] += __shfl_xor_sync(0xffffffffu, sq[e], o);
+#pragma unroll
+          for (int e = 0; e < VW; ++e) {
+            const int m = (split + i * p.splits) * VW + e;
+            if (real && lane == e && m < cols) p.ss_out[(size_t)m * p.ss_parts + tile * 4 + (warp & 3)] = sq[e];
           }
         }
-      }
-    } else if (summed && ok && own && (VW > 1 || par == 0)) {
-#pragma unroll (EP == EP_GLU ? 2 : 1)
-      for (int i = 0; i < mine; ++i) {
-        const float* at = parts + i * PART_GROUP + par * CV;
-        alignas(8) float s1[CV], s2[CV];
-        sum_parts<CV>(at + f1 * VW, p.splits, part_step, s1);
-        sum_parts<CV>(at + f2 * VW, p.splits, part_step, s2);
+      } else if constexpr (EP == EP_PLAIN) {
+        if (p.splits > 1 && summed && own) {
+#pragma unroll 1
+          for (int i = 0; i < mine; ++i) {
+            alignas(16) float y[VW];
+            sum_parts<VW>(parts + i * PART_GROUP + r * VW, p.splits, part_step, y);
 #pragma unroll
-        for (int e = 0; e < CV; ++e) {
-          const int m = (split + i * p.splits) * VW + par * CV + e;
-          if (m >= cols) break;
-          const float sc = p.ss ? factor[i * VW + par * CV + e] : 1.f;
-          const float v1 = fmaf(s1[e], sc, b1), v2 = fmaf(s2[e], sc, b2);
-          if constexpr (EP == EP_GLU) {
-            p.c_bf16[(size_t)m * (p.feats >> 1) + tile * 64 + q] = __float2bfloat16_rn(glu_mul(v1, v2, p.swiglu));
-          } else {
-            Place& at = ahead[e];
-            if (VW > 1 && i > 0) place(m, at);
-            if (at.dst == nullptr) continue;
-            float o1 = 0.f, o2 = 0.f;
-            if (at.turn == 2) fz_rope_pair(v1, v2, at.cs, at.sn, o1, o2);
-            else if (at.turn == 1) { o1 = v1; o2 = v2; }
-            at.dst[0] = __float2bfloat16_rn(o1);
-            at.dst[half] = __float2bfloat16_rn(o2);
+            for (int e = 0; e < VW; ++e) {
+              const int m = (split + i * p.splits) * VW + e;
+              if (m >= cols) break;
+              const float v = finished(p, fmaf(y[e], p.ss ? factor[i * VW + e] : 1.f, b1));
+              if (!real) continue;
+              if (p.c_f32) p.c_f32[(size_t)m * p.feats + feat] = v;
+              else p.c_bf16[(size_t)m * p.feats + feat] = __float2bfloat16_rn(v);
+            }
+          }
+        }
+      } else if (summed && ok && own && (VW > 1 || par == 0)) {
+#pragma unroll (EP == EP_GLU ? 2 : 1)
+        for (int i = 0; i < mine; ++i) {
+          const float* at = parts + i * PART_GROUP + par * CV;
+          alignas(8) float s1[CV], s2[CV];
+          sum_parts<CV>(at + f1 * VW, p.splits, part_step, s1);
+          sum_parts<CV>(at + f2 * VW, p.splits, part_step, s2);
+#pragma unroll
+          for (int e = 0; e < CV; ++e) {
+            const int m = (split + i * p.splits) * VW + par * CV + e;
+            if (m >= cols) break;
+            const float sc = p.ss ? factor[i * VW + par * CV + e] : 1.f;
+            const float v1 = fmaf(s1[e], sc, b1), v2 = fmaf(s2[e], sc, b2);
+            if constexpr (EP == EP_GLU) {
+              const __nv_bfloat16 y = __float2bfloat16_rn(glu_mul(v1, v2, p.swiglu));
+              if (real) p.c_bf16[(size_t)m * (p.feats >> 1) + tile * 64 + q] = y;
+            } else {
+              Place& at = ahead[e];
+              if (VW > 1 && i > 0) place(m, at);
+              float o1 = 0.f, o2 = 0.f;
+              if (at.turn == 2) fz_rope_pair(v1, v2, at.cs, at.sn, o1, o2);
+              else if (at.turn == 1) { o1 = v1; o2 = v2; }
+              const __nv_bfloat16 y1 = __float2bfloat16_rn(o1), y2 = __float2bfloat16_rn(o2);
+              if (real && at.dst != nullptr) {
+                at.dst[0] = y1;
+                at.dst[half] = y2;
+              }
+            }
           }
         }
       }
