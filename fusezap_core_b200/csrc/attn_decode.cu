@@ -715,7 +715,7 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
 // from its position and the window alone, as in the kernel above.
 __device__ __forceinline__ void combine_units_row(const int n, const int h, const int row, const int p, const float* __restrict__ part_o,
                                                   const float* __restrict__ part_ml, __nv_bfloat16* __restrict__ out,
-                                                  float* __restrict__ out32, int Hq, int HD, int NPU, int window, float2* s_ml) {
+                                                  float* __restrict__ out32, int Hq, int HD, int NPU, int window, float2* s_ml, bool real = true) {
   const int tid = threadIdx.x, CT = blockDim.x;
   const int per_row = HD >> 2, groups = CT / per_row;           // threads per row, groups per block
   const int grp = tid / per_row, d4 = (tid - grp * per_row) * 4;
@@ -799,6 +799,7 @@ __device__ __forceinline__ void combine_units_row(const int n, const int h, cons
     merge4(O, s_o[k * per_row + tid], fa, fb);
   }
   const float inv = 1.0f / L;
+  if (!real) return;
   if (out32 != nullptr) {
     *(float4*)(orow32 + d4) = make_float4(O.x * inv, O.y * inv, O.z * inv, O.w * inv);
     return;
@@ -810,7 +811,7 @@ __device__ __forceinline__ void combine_units_row(const int n, const int h, cons
 // FIND false: one block per (head, row). true, where most rows are of long portions (`combine_rows`): a block looks at every
 // gridDim.y-th row, a lane each, and takes the short ones among them: a block per row, almost all of them with nothing to do,
 // took 22 us of a layer of a step of 500 prompt rows beside 7 decoded ones at 32 heads; the step of 32 layers 13.81 -> 13.33 ms.
-template <bool FIND>
+template <bool FIND, bool TWICE>
 __global__ void __launch_bounds__(256)
 attn_combine_units_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                           const int* __restrict__ pos, const int* __restrict__ seq_row, const int* __restrict__ seg,
@@ -822,8 +823,17 @@ attn_combine_units_kernel(const float* __restrict__ part_o, const float* __restr
   if constexpr (!FIND) {
     const int n = blockIdx.y, row = seq_row[n], p = pos[n];
     const bool skip = row >= 0 && seg[row * 4 + 1] >= long_from;
-    fz_grid_wait();
-    if (!skip) combine_units_row(n, h, row, p, part_o, part_ml, out, out32, Hq, HD, NPU, window, s_ml);
+    int pass = 1;
+    if constexpr (TWICE) {
+      pass = !skip && row >= 0 ? 0 : 1;
+      asm volatile("" : "+r"(pass));      // (two passes through the same code, not two copies of it)
+    }
+#pragma unroll 1
+    for (; pass < 2; ++pass) {
+      if (!TWICE || pass == 1) fz_grid_wait();
+      if (!skip) combine_units_row(n, h, row, p, part_o, part_ml, out, out32, Hq, HD, NPU, window, s_ml, !TWICE || pass == 1);
+      if constexpr (TWICE) __syncthreads();
+    }
     return;
   }
   const int lane = threadIdx.x & 31;
@@ -934,7 +944,12 @@ int launch_units(const void* q, const void* k_pool, long long pool_rows, const i
   // two engines alternating in one process, a decode step of 32 layers at batch 1 3.100 -> 3.079 ms, batch 2 3.181 ->
   // 3.161, batch 4 3.369 -> 3.348; at batch 8 (256 blocks) 3.780 -> 3.789 and at batch 64 1.3 % slower
   const int ct = (long long)cgrid.y * Hq <= sms ? 256 : 128;
-  fz_launch(rows_high < N ? attn_combine_units_kernel<true> : attn_combine_units_kernel<false>, cgrid, dim3(ct),
+  // Few blocks merge twice: once before they wait, whatever the scratch holds and with nothing stored, so that the instructions are in
+  // the SMs' caches when the partial results are there. Where all blocks are resident at once and have little to read (4 MB): 32 rows
+  // of 1,280 keys and 4 of 2,000 at Qwen2.5-0.5B sizes 832 -> 800 us a step, 674 -> 653, one of 4,096 at Llama-3.1-8B sizes 2,834
+  // -> 2,809; 8 of 4,096 there, 8 MB, 3,375 -> 3,407.
+  const bool twice = (long long)cgrid.y * Hq <= 4 * sms && (long long)cgrid.y * Hq * NPU * HD <= 1 << 20;
+  fz_launch(rows_high < N ? attn_combine_units_kernel<true, false> : twice ? attn_combine_units_kernel<false, true> : attn_combine_units_kernel<false, false>, cgrid, dim3(ct),
             (size_t)(NPU + 2) * 8 + 256 * 16 + 16 * 8, stream, (const float*)part_o,
             (const float*)part_ml, pos, seq_row, seg, (__nv_bfloat16*)out, out32, N, Hq, HD, NPU, window, long_from);
   FZ_LAUNCH_CHECK();
