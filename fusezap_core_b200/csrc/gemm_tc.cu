@@ -595,9 +595,88 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // Rows mode: one thread's lane (token row `row`) of a finished accumulator of BN columns at `taddr`, with the bias added,
 // to the output's columns n0 .. n0 + BN - 1 (or, with the fused SwiGLU, to its packed half); of these the `part`-th of PARTS
 // equal shares. Every lane of the warp takes part in the loads from tensor memory whether or not its row exists.
+//
+// With p.rope the columns are whole heads [q | k | v] (the head size divides a share): q and k are rotated by the row's position, q
+// goes to c_bf16, k and v to the token's slot of the paged pools, as the rotation's kernel does from the product's float32 output,
+// with the same roundings. `RowPlace`: what a row's rotation needs, looked up while the tile is being computed.
+// (The rotation's kernel read the product from L2 and wrote half of it again: 16.7 us of a layer of 2,048 rows at Llama-3.1-8B sizes
+// beside 94 of the product; 88 together now, 27.5 -> 26.5 ms a prompt. 2,100 rows at Qwen2.5-0.5B sizes 14.0 + 4.5 -> 15.6, 507 rows at
+// the former 31.4 + 13.0 -> 34.4.)
+struct RowPlace { int there, ps; long long slot; };      // slot: of the row's key in a page's first head, negative: not stored
+__device__ __forceinline__ RowPlace row_place(const Params& p, int row, bool first) {
+  RowPlace at{0, 0, -1};
+  if (!p.rope || row >= p.rows) return at;
+  const int seq = p.seq_row[row];
+  at.ps = p.pos[row];
+  const bool in_range = at.ps >= 0 && at.ps < p.max_len;
+  if (seq >= 0 && !in_range && first) atomicOr(p.err, FZ_ERR_POS_RANGE);
+  at.there = seq >= 0 && in_range;
+  if (at.there && p.write) {
+    const int page = p.table[(size_t)seq * p.mb + at.ps / p.page_size];
+    if (page >= 0) at.slot = (long long)page * p.page_stride + (long long)(at.ps % p.page_size) * p.hd;
+    else if (first) atomicOr(p.err, FZ_ERR_NO_PAGE);
+  }
+  return at;
+}
+__device__ __forceinline__ void store16_bf16(__nv_bfloat16* dst, const float* v) {
+  uint32_t w[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    w[i] = *(const uint32_t*)&h;
+  }
+  ((uint4*)dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  ((uint4*)dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
 template <int BN, int PARTS>
-__device__ __forceinline__ void rows_store_tile(const Params& p, uint32_t taddr, int row, int n0, int part) {
+__device__ __forceinline__ void rows_store_tile(const Params& p, uint32_t taddr, int row, int n0, int part, const RowPlace& at) {
   float v[16];
+  if (p.rope) {
+    float u[16];
+    const int half = p.hd >> 1, hq = p.Hq * p.hd, hk = hq + p.Hkv * p.hd;
+    const float* cs = p.cos_t + (size_t)(at.there ? at.ps : 0) * half;
+    const float* sn = p.sin_t + (size_t)(at.there ? at.ps : 0) * half;
+#pragma unroll 1
+    for (int c = part * (BN / PARTS); c < (part + 1) * (BN / PARTS); c += 16) {
+      if ((c & (p.hd - 1)) >= half) continue;      // (the second values of the pairs go with the first)
+      const int n = n0 + c, j = n & (p.hd - 1);
+      const bool turn = at.there && n < hk && row < p.rows;
+      float4 co[4], si[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        co[i] = turn ? *(const float4*)(cs + j + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        si[i] = turn ? *(const float4*)(sn + j + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      tmem_ld16(taddr + (uint32_t)c, v);
+      tmem_ld16(taddr + (uint32_t)(c + half), u);
+      if (row >= p.rows || n >= p.feats) continue;
+      if (p.bias) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { v[i] += p.bias[n + i]; u[i] += p.bias[n + half + i]; }
+      }
+      __nv_bfloat16* dst;
+      if (n < hq) dst = p.c_bf16 + (size_t)row * hq + n;
+      else if (at.slot < 0) continue;
+      else {
+        const int head = (n - (n < hk ? hq : hk)) / p.hd;
+        dst = (n < hk ? p.k_pool : p.v_pool) + at.slot + (long long)head * p.page_size * p.hd + j;
+      }
+      if (n < hk) {
+        const float* cf = (const float*)co;
+        const float* sf = (const float*)si;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float o1 = 0.f, o2 = 0.f;
+          if (at.there) fz_rope_pair(v[i], u[i], cf[i], sf[i], o1, o2);
+          v[i] = o1;
+          u[i] = o2;
+        }
+      }
+      store16_bf16(dst, v);
+      store16_bf16(dst + half, u);
+    }
+    return;
+  }
   if (p.swiglu) {
     // columns [128 b, 128 b + 64) are gate, [128 b + 64, 128 b + 128) up of output features 64 (n0 / 128 + b) ..
     float u[16];
@@ -763,13 +842,14 @@ gemm_tc_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       const int tile = (int)blockIdx.x + j * (int)gridDim.x;
       const int tm = tile % tiles_m, tn = tile / tiles_m;
       const int acc = j & 1;
+      const RowPlace at = row_place(p, tm * BM + r, tn == 0);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (j >> 1) & 1));
       if (!ok) { flag[0] = 1; break; }
       tc_fence_after();
       // (Four epilogue warps here. Eight, as in the two-SM kernel's plain epilogue, were measured on this kernel and did not pay: the tiles
       // it gets are narrow or few, and 2,048 tokens at Qwen2.5-0.5B sizes took 3.94 ms with them against 3.77 ms.)
       const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quad * 32) << 16);
-      rows_store_tile<BN, 1>(p, taddr, tm * BM + r, tn * BN, 0);
+      rows_store_tile<BN, 1>(p, taddr, tm * BM + r, tn * BN, 0, at);
       tc_fence_before();
       mbar_arrive(&acc_empty[acc]);      // this thread has read its lane of the accumulator
     }
@@ -971,11 +1051,12 @@ gemm_tc_rows_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       const int tile = pair + j * pairs;
       const int tm = tile % tiles_m, tn = tile / tiles_m;
       const int acc = j & 1;
+      const RowPlace at = row_place(p, (2 * tm + (int)rank) * BM + r, tn == 0 && warp < 6);
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (j >> 1) & 1));
       if (!ok) { flag[0] = 1; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + (uint32_t)(acc * BN) + ((uint32_t)(quad * 32) << 16);
-      rows_store_tile<BN, PARTS>(p, taddr, (2 * tm + (int)rank) * BM + r, tn * BN, (warp - 2) >> 2);
+      rows_store_tile<BN, PARTS>(p, taddr, (2 * tm + (int)rank) * BM + r, tn * BN, (warp - 2) >> 2, at);
       tc_fence_before();
       __syncwarp();      // every lane of the warp has read its lane of the accumulator
       if (lane == 0) mbar_arrive_cluster(acc_empty0 + 8u * (uint32_t)acc);
@@ -1421,7 +1502,7 @@ struct RowsPlan {
   enum Kernel { ROWS, PAIR, SPLIT, SPLIT_PAIR } kernel;
   int bn, splits, parts;      // width of a tile; pieces of K; PAIR: groups of four epilogue warps
 };
-static RowsPlan rows_plan(int M, int N, int K, bool swiglu) {
+static RowsPlan rows_plan(int M, int N, int K, bool swiglu, int hd = 0) {      // hd: the tile must hold whole heads
   int bn = N >= 256 ? 256 : N >= 128 ? 128 : 64;     // with the fused SwiGLU N = 2 I >= 128, so a tile holds whole blocks
   if (bn == 256 && !swiglu) {
     // So few 128 x 256 tiles that the SMs are not half used, and a K worth cutting: the tiles' K ranges are cut so that
@@ -1437,7 +1518,7 @@ static RowsPlan rows_plan(int M, int N, int K, bool swiglu) {
     const long long tm = (M + BM - 1) / BM;
     if (tm * ((N + 255) / 256) < device_sms()) {
       for (int cand : {224, 192, 160})
-        if (tm * ((N + cand - 1) / cand) <= device_sms()) bn = cand;
+        if (tm * ((N + cand - 1) / cand) <= device_sms() && (hd == 0 || cand % hd == 0)) bn = cand;
     }
   }
   // many token rows: a pair of SMs on every 256 x 256 tile (see `gemm_tc_rows_pair_kernel`)
@@ -1446,6 +1527,7 @@ static RowsPlan rows_plan(int M, int N, int K, bool swiglu) {
 }
 
 // x: [M, K] bf16, w: [N, K] bf16, bias: [N] float32 or null, c: [M, N] float32 (out_dtype 0) or bf16 (1).
+FZ_API int fz_gemm_tc_qkv_rope_rows(int M, int N, int K, int hd);
 static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c, int out_dtype, int M, int N, int K,
                         const Params& fused, int* err, cudaStream_t stream);
 
@@ -1500,6 +1582,13 @@ FZ_API int fz_gemm_tc_qkv_rope_check(int M, int hd) {
   return (M >= 1 && M <= 32 && hd >= 2 && hd % 2 == 0 && 128 % hd == 0) ? FZ_OK : FZ_BAD_SHAPE;
 }
 
+// The same for many rows (1 or 0): heads of 64 or 128, three tiles of rows and more, and a product whose K is not cut.
+FZ_API int fz_gemm_tc_qkv_rope_rows(int M, int N, int K, int hd) {
+  if (M <= 2 * BM || N < 256 || (hd != 64 && hd != 128)) return 0;
+  const RowsPlan plan = rows_plan(M, N, K, false, hd);
+  return plan.splits == 1 && plan.bn / plan.parts % hd == 0 ? 1 : 0;
+}
+
 // x: [M, K] bf16; w: [(Hq + 2 Hkv) hd, K] bf16, rows [q heads | k heads | v heads]; bias float32 or null. Rotates the q
 // and k heads of every token by its position (pairs j, j + hd / 2; angles from cos_t / sin_t [max_len, hd / 2]) and
 // writes q to q_out [M, Hq hd] bf16 and, if `write`, k and v to the token's slot of the paged pools (as the separate
@@ -1509,7 +1598,11 @@ FZ_API int fz_gemm_tc_qkv_rope(const void* x, const float* ss, int ss_parts, flo
                                const float* sin_t, const int* pos, const int* seq_row, const int* table, int mb,
                                void* k_pool, void* v_pool, long long page_stride, int page_size, int write, void* q_out,
                                int Hq, int Hkv, int hd, int max_len, int* err, cudaStream_t stream) {
-  if (fz_gemm_tc_qkv_rope_check(M, hd) != FZ_OK || Hq <= 0 || Hkv <= 0 || page_size <= 0) return FZ_BAD_SHAPE;
+  if (Hq <= 0 || Hkv <= 0 || page_size <= 0) return FZ_BAD_SHAPE;
+  if (fz_gemm_tc_qkv_rope_check(M, hd) != FZ_OK) {
+    if (ss || !fz_gemm_tc_qkv_rope_rows(M, (Hq + 2 * Hkv) * hd, K, hd)) return FZ_BAD_SHAPE;
+    if (((uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15 || page_stride % 8) return FZ_BAD_ALIGNMENT;
+  }
   Params f{};
   if (ss) set_factors(f, ss, ss_parts, eps, K);
   f.rope = 1;
@@ -1603,7 +1696,7 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
   int st = fz_gemm_tc_check(x, w, M, N, K);
   if (st != FZ_OK) return st;
   if (out_dtype != FZ_F32 && out_dtype != FZ_BF16) return FZ_BAD_DTYPE;
-  if (fused.rope && M > 32) return FZ_BAD_SHAPE;
+  if (fused.rope && M > 32 && !fz_gemm_tc_qkv_rope_rows(M, N, K, fused.hd)) return FZ_BAD_SHAPE;
   Params p = fused;
   p.c_f32 = out_dtype == FZ_F32 ? (float*)c : nullptr;
   p.c_bf16 = out_dtype == FZ_BF16 ? (__nv_bfloat16*)c : nullptr;
@@ -1645,7 +1738,7 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
   }
   // rows mode: token rows are the 128 lanes; persistent CTAs with two accumulators
   if (p.x || p.ss) return FZ_BAD_SHAPE;
-  const RowsPlan plan = rows_plan(M, N, K, p.swiglu != 0);
+  const RowsPlan plan = rows_plan(M, N, K, p.swiglu != 0, p.rope ? p.hd : 0);
   p.splits = plan.splits;
   const bool pair = plan.kernel == RowsPlan::PAIR || plan.kernel == RowsPlan::SPLIT_PAIR;
   const int box = pair ? plan.bn / 2 : plan.bn, st_n = (200 * 1024) / ((BM + box) * BK * 2);

@@ -612,9 +612,15 @@ class CudaOps(Ops):
     def linear_rope_kv_write(self, a, w, bias, cos, sin, meta, cache, q_out, num_heads, num_kv_heads, head_dim) -> bool:
         a, factors = self._factors(a)
         m, k = a.shape
-        if not (self.use_tensor_cores and self.fuse_rope and self.dtype == torch.bfloat16) or \
-                self.tc.fz_gemm_tc_qkv_rope_check(c_int(m), c_int(head_dim)) != 0 or \
-                self.tc.fz_gemm_tc_check(_p(a), _p(w), c_int(m), c_int(w.shape[0]), c_int(k)) != 0:
+        if not (self.use_tensor_cores and self.fuse_rope and self.dtype == torch.bfloat16):
+            return False
+        if self.tc.fz_gemm_tc_qkv_rope_check(c_int(m), c_int(head_dim)) != 0:
+            # many rows: 16 bytes at a time
+            if factors is not None or not self.tc.fz_gemm_tc_qkv_rope_rows(c_int(m), c_int(w.shape[0]), c_int(k), c_int(head_dim)) or \
+                    (q_out.data_ptr() | cache.keys.data_ptr() | cache.values.data_ptr() | cos.data_ptr() | sin.data_ptr()) % 16 or \
+                    cache.keys.stride(0) % 8:
+                return False
+        if self.tc.fz_gemm_tc_check(_p(a), _p(w), c_int(m), c_int(w.shape[0]), c_int(k)) != 0:
             return False
         self._want(a, "linear input", (torch.bfloat16,), 2)
         self._want(w, "linear weight", (torch.bfloat16,), 2)

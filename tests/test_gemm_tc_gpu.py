@@ -331,6 +331,50 @@ def test_qkv_product_with_rotation_and_cache_write(Hq, Hkv, hd, K, bs, M):
     assert ops.linear_rope_kv_write(big, w, b, cos, sin, meta, cache, q, Hq, Hkv, hd) is False
 
 
+@pytest.mark.parametrize("Hq,Hkv,hd,K,M", [(32, 8, 128, 512, 300), (32, 8, 128, 512, 1100), (14, 2, 64, 896, 257), (14, 2, 64, 896, 2101),
+                                           (2, 1, 128, 200, 600), (6, 6, 64, 72, 1000)])
+@pytest.mark.parametrize("bias,write", [(True, True), (False, False)])
+def test_qkv_product_of_many_rows_with_rotation_and_cache_write(Hq, Hkv, hd, K, M, bias, write):
+    """The same for prompts, on one SM per tile and on pairs: the bits of the product followed by the rotation's kernel, with padding
+    rows, a row without a page (flagged by both), ragged last tiles of rows and features."""
+    from fusezap_core_b200.kernels import cuda_ops
+    from fusezap_core_b200.kernels.table import KernelError
+    from test_kernels_gpu import Meta, make_cache
+    ops, bs = cuda_ops("bfloat16"), 16
+    N = (Hq + 2 * Hkv) * hd
+    assert ops.tc.fz_gemm_tc_qkv_rope_rows(M, N, K, hd) == 1
+    assert ops.tc.fz_gemm_tc_qkv_rope_rows(256, N, K, hd) == 0 and ops.tc.fz_gemm_tc_qkv_rope_rows(M, N, K, 32) == 0
+    g = torch.Generator(device="cuda").manual_seed(M + hd)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    b = torch.randn(N, generator=g, device="cuda") if bias else None
+    ang = torch.rand(1500, hd // 2, generator=g, device="cuda") * 6.28
+    pages = -(-M // bs)
+    table = [list(range(pages)), list(range(pages, 2 * pages))]
+    table[1][0] = -1 if write else table[1][0]
+    pos, seq = [i % 1500 if i < M // 2 else i - M // 2 for i in range(M)], [0] * (M // 2) + [1] * (M - M // 2)
+    seq[5] = seq[M - 1] = -1
+    meta, res, flagged = Meta(pos, seq, table, "cuda"), [], []
+    for fused in (True, False):
+        cache = make_cache(2 * pages, Hkv, bs, hd, torch.bfloat16, "cuda", write=write)
+        cache.pool.copy_(torch.randn(cache.pool.shape, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16))
+        q = torch.full((M, Hq * hd), float("nan"), dtype=torch.bfloat16, device="cuda")
+        if fused:
+            assert ops.linear_rope_kv_write(a, w, b, ang.cos(), ang.sin(), meta, cache, q, Hq, Hkv, hd)
+        else:
+            qkv = torch.empty(M, N, device="cuda")
+            ops.linear(a, w, b, qkv)
+            ops.rope_kv_write(qkv, ang.cos(), ang.sin(), meta, cache, q, Hq, Hkv, hd)
+        try:
+            ops.check_errors()
+            flagged.append("")
+        except KernelError as e:
+            flagged.append(str(e))
+        res.append((q, cache.pool.clone()))
+    assert torch.isfinite(res[0][0].float()).all() and torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    assert flagged[0] == flagged[1] and bool(flagged[0]) == write
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 20000, 256), (8, 33333, 128), (37, 17000, 64), (128, 16512, 72)])
 def test_product_that_keeps_only_the_largest_of_each_row(M, N, K):
     """`linear_argmax` gives the ids that `argmax` finds in the logits `linear` writes, with the numpy rule for ties (the
