@@ -1724,7 +1724,11 @@ static int gemm_tc_impl(const void* x, const void* w, const float* bias, void* c
       // Larger ones would only keep the next kernels' blocks off the SMs. (At least three stages: they also hold the parts of 128
       // tokens, 72 KB.)
       const long long ring = (long long)per_cta * (BM + bn) * BK * 2;
-      if (ring <= 200 * 1024 && ring * tiles * p.splits <= 24 << 20) p.stages = per_cta < 3 ? 3 : per_cta;
+      // With up to 16 tokens only where two CTAs could share an SM: a CTA that takes an SM's whole memory starts when the kernel before
+      // has left it, a smaller one beside that kernel, its first stages then on their way. (The down product at Qwen2.5-0.5B sizes,
+      // 56 CTAs of ten k-blocks, in rings of 10, 7, 5 and 4: a decode step of 1 row of 300 keys 532, 535, 507, 517 us, of 8 of 224 593,
+      // 584, 580, 585, of 32 of 1,280, where it gains nothing, 794, 798, 806, 812.)
+      if (ring <= (bn == 16 ? 100 : 200) * 1024 && ring * tiles * p.splits <= 24 << 20) p.stages = per_cta < 3 ? 3 : per_cta;
     }
     if ((st = get_map_bf16(w, N, K, BM, &ma)) != FZ_OK) return st;
     if ((st = get_map_bf16(x, M, K, bn, &mb)) != FZ_OK) return st;
