@@ -54,8 +54,13 @@ class Workspace:
         self.device, self.row_capacity = device, row_capacity
         self._bufs: dict[tuple, torch.Tensor] = {}
         self._retired: list[torch.Tensor] = []      # outgrown buffers: a captured step may still point at them
+        # what was handed out, by exactly what was asked for: a step asks for some 200 views, 2 us of Python each
+        self._views: dict[tuple, torch.Tensor] = {}
 
     def get(self, tag: str, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        view = self._views.get((tag, shape, dtype))
+        if view is not None:
+            return view
         key = (tag, tuple(shape[1:]), dtype)
         buf = self._bufs.get(key)
         if buf is None or buf.shape[0] < shape[0]:
@@ -63,7 +68,11 @@ class Workspace:
                 self._retired.append(buf)
             buf = torch.empty((max(self.row_capacity, shape[0]), *shape[1:]), dtype=dtype, device=self.device)
             self._bufs[key] = buf
-        return buf[:shape[0]]
+            self._views.clear()
+        if len(self._views) >= 1024:      # (steps of many sizes)
+            self._views.clear()
+        view = self._views[tag, tuple(shape), dtype] = buf[:shape[0]]
+        return view
 
     def bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._bufs.values())
@@ -96,6 +105,7 @@ class StepMeta:
         self.host = self._hosts[0]
         self.np = self.host.numpy()
         self.dev = torch.zeros(self.size, dtype=torch.int32, device=device)
+        self._views: dict[tuple, torch.Tensor] = {}      # slices of `dev` by offset and length: a step asks for each many times
         # filled per step
         self.n_rows = self.n_wanted = self.n_segments = 0
         self.segments: list[Segment] = []
@@ -106,25 +116,33 @@ class StepMeta:
         self.latent_extra = 0     # kernel table: how many blocks beyond rows x heads / 64 the latent attention launches
 
     # device views (static addresses; sliced to the step's sizes)
+    def _view(self, offset: int, length: int, columns: int = 0) -> torch.Tensor:
+        view = self._views.get((offset, length, columns))
+        if view is None:
+            if len(self._views) >= 1024:      # (steps of many sizes)
+                self._views.clear()
+            view = self.dev[offset: offset + length]
+            view = self._views[offset, length, columns] = view.view(self.max_segments, columns) if columns else view
+        return view
     @property
-    def tokens(self) -> torch.Tensor: return self.dev[self.o_tokens: self.o_tokens + self.n_rows]
+    def tokens(self) -> torch.Tensor: return self._view(self.o_tokens, self.n_rows)
     @property
-    def pos(self) -> torch.Tensor: return self.dev[self.o_pos: self.o_pos + self.n_rows]
+    def pos(self) -> torch.Tensor: return self._view(self.o_pos, self.n_rows)
     @property
-    def seq_row(self) -> torch.Tensor: return self.dev[self.o_row: self.o_row + self.n_rows]
+    def seq_row(self) -> torch.Tensor: return self._view(self.o_row, self.n_rows)
     @property
-    def src(self) -> torch.Tensor: return self.dev[self.o_src: self.o_src + self.n_rows]
+    def src(self) -> torch.Tensor: return self._view(self.o_src, self.n_rows)
     @property
-    def sel(self) -> torch.Tensor: return self.dev[self.o_sel: self.o_sel + self.n_wanted]
+    def sel(self) -> torch.Tensor: return self._view(self.o_sel, self.n_wanted)
     @property
-    def seg(self) -> torch.Tensor: return self.dev[self.o_seg: self.o_seg + 4 * self.max_segments].view(self.max_segments, 4)
+    def seg(self) -> torch.Tensor: return self._view(self.o_seg, 4 * self.max_segments, 4)
     @property
     def extra(self) -> torch.Tensor: return self.dev[self.o_extra: self.o_extra + self.extra_ints]
     @property
     def extra_host(self) -> np.ndarray: return self.np[self.o_extra: self.o_extra + self.extra_ints]
     def table(self, group: int) -> torch.Tensor:
         n = self.max_segments * self.mb
-        return self.dev[self.o_tab + group * n: self.o_tab + (group + 1) * n].view(self.max_segments, self.mb)
+        return self._view(self.o_tab + group * n, n, self.mb)
 
     def fill(self, cache: CacheManager, portions: Sequence[Portion], starts: Sequence[int], pad_rows: int = 0,
              pad_wanted: int = 0, ops: Any = None, needs: tuple = ()) -> None:

@@ -284,6 +284,8 @@ class CudaOps(Ops):
             self._profile.note(what, ideal_bytes)
 
     def _want(self, t: torch.Tensor, name: str, dtypes: tuple, dims: int | None = None) -> None:
+        if t.is_cuda and t.dtype in dtypes and t.is_contiguous() and (dims is None or t.dim() == dims):
+            return
         if not t.is_cuda:
             raise KernelError(f"{name} is on {t.device}; the kernels take CUDA tensors only")
         if t.dtype not in dtypes:
