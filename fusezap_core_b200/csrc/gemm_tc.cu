@@ -26,9 +26,9 @@
 // result. The sum has one fixed order (as the reference's split-K has: wgmma.py:209-239) and no partial ever goes to
 // global memory. Waits on this CTA's own mbarriers are bounded by a time limit after which the kernel sets an error bit
 // and leaves; the cluster barriers are hardware barriers, not spins.
-// Epilogues besides bias + store: SwiGLU over weight rows packed as [64 gate | 64 up] blocks (both modes); for few
-// tokens the rotation of the q and k heads with the write of k and v into the paged cache, and a per-tile argmax that
-// stores no products at all (the lm_head of a greedy step).
+// Epilogues besides bias + store: SwiGLU over weight rows packed as [64 gate | 64 up] blocks and the rotation of the q and k
+// heads with the write of k and v into the paged cache (both modes); for few tokens the residual add with the norm behind
+// it, and a per-tile argmax that stores no products at all (the lm_head of a greedy step).
 #include "umma.cuh"
 
 namespace {
@@ -121,7 +121,7 @@ struct Params {
   int parts_in_ring;       // few tokens: the partial sums arrive in the ring's memory (after a cluster barrier), not in memory of their own
   int vec_ok;              // rows mode: C rows are 16-byte aligned, so full groups of 16 columns go out as vectors
   int swiglu;              // W holds [64 gate rows | 64 up rows] blocks: store silu(gate) * up as bf16 [rows, feats / 2]
-  // rope != 0 (few tokens, hd divides 128): the features are [q heads | k heads | v heads] of size hd; q and k are rotated
+  // rope != 0 (few tokens: hd divides 128; many: a share of a tile's columns holds whole heads): the features are [q heads | k heads | v heads] of size hd; q and k are rotated
   // by the token's position, q goes to c_bf16 [rows, Hq * hd], k and v to the token's slot of the paged pool
   int rope;
   const float* cos_t;      // [max_len, hd / 2]
