@@ -712,7 +712,9 @@ attn_decode_units_kernel(const __grid_constant__ CUtensorMap kv_map, const __nv_
 // merged by the unit kernel or merged here in rising order with the same arithmetic; a 256-key unit above). The groups'
 // results are merged in group order, normalised and rounded to bf16. All (max, sum) pairs of the row are brought into
 // shared memory first, so that what a thread loads next never waits on a load before it. Which units a row has follows
-// from its position and the window alone, as in the kernel above.
+// from its position and the window alone, as in the kernel above. `real` false: a walk through the same instructions that reads
+// nothing of the partial results, which another grid may be writing: a thread's own zeros in shared memory stand in their place.
+// It stores nothing.
 __device__ __forceinline__ void combine_units_row(const int n, const int h, const int row, const int p, const float* __restrict__ part_o,
                                                   const float* __restrict__ part_ml, __nv_bfloat16* __restrict__ out,
                                                   float* __restrict__ out32, int Hq, int HD, int NPU, int window, float2* s_ml, bool real = true) {
@@ -729,8 +731,7 @@ __device__ __forceinline__ void combine_units_row(const int n, const int h, cons
   const int lo = window > 0 ? max(0, p - window + 1) : 0;
   const int u0 = unit_of(lo), u1 = unit_of(p), cnt = u1 - u0 + 1;
   const float2* ml = (const float2*)part_ml + ((size_t)n * Hq + h) * NPU + u0;
-  const float* po = part_o + (((size_t)n * Hq + h) * NPU + u0) * HD + d4;
-  for (int i = tid; i < cnt; i += CT) s_ml[i] = ml[i];
+  for (int i = tid; i < cnt; i += CT) s_ml[i] = real ? ml[i] : make_float2(0.f, 1.f);
   __syncthreads();
   // The row's blocks are merged in VG chains (chain v: blocks v, v + VG, ...), and the chains then in rising order: VG
   // is the group count of a block of 256 threads, and a block of 128 threads walks two chains per group, so the order
@@ -738,6 +739,14 @@ __device__ __forceinline__ void combine_units_row(const int n, const int h, cons
   const int VG = 256 / per_row, lane_in = tid - grp * per_row;
   float4* s_o = (float4*)(s_ml + cnt + (cnt & 1));              // [VG][per_row]
   float2* s_g = (float2*)(s_o + VG * per_row);                  // [VG]: (max, sum)
+  const float* po = part_o + (((size_t)n * Hq + h) * NPU + u0) * HD + d4;
+  size_t step = HD;
+  if (!real) {
+    s_o[tid] = make_float4(0.f, 0.f, 0.f, 0.f);      // (this thread's until it leaves its chain's result there)
+    po = (const float*)(s_o + tid);
+    step = 0;
+  }
+  auto unit = [&](int i) { return *(const float4*)(po + i * step); };
   const int n_small = u0 < SMALL_UNITS ? (min(u1, SMALL_UNITS - 1) >> 2) - (u0 >> 2) + 1 : 0;
   const int big0 = max(u0, SMALL_UNITS);
   const int n_items = n_small + (u1 >= SMALL_UNITS ? u1 - big0 + 1 : 0);
@@ -757,12 +766,12 @@ __device__ __forceinline__ void combine_units_row(const int n, const int h, cons
         const float2 first = s_ml[i0];
         Mb = first.x; Lb = fabsf(first.y);
         if (first.y < 0.f || i1 == i0) {
-          Ob = *(const float4*)(po + (size_t)i0 * HD);
+          Ob = unit(i0);
         } else {                        // not merged by the unit kernel: the block's units one by one, loads first
           float4 v[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            if (i0 + j <= i1) v[j] = *(const float4*)(po + (size_t)(i0 + j) * HD);
+            if (i0 + j <= i1) v[j] = unit(i0 + j);
           Ob = v[0];
 #pragma unroll
           for (int j = 1; j < 4; ++j) {
@@ -778,7 +787,7 @@ __device__ __forceinline__ void combine_units_row(const int n, const int h, cons
         const int i = big0 + (k - n_small) - u0;
         const float2 v = s_ml[i];
         Mb = v.x; Lb = v.y;
-        Ob = *(const float4*)(po + (size_t)i * HD);
+        Ob = unit(i);
       }
       float fa, fb;
       merge_unit_scalars(M, L, Mb, Lb, fa, fb);
@@ -944,10 +953,12 @@ int launch_units(const void* q, const void* k_pool, long long pool_rows, const i
   // two engines alternating in one process, a decode step of 32 layers at batch 1 3.100 -> 3.079 ms, batch 2 3.181 ->
   // 3.161, batch 4 3.369 -> 3.348; at batch 8 (256 blocks) 3.780 -> 3.789 and at batch 64 1.3 % slower
   const int ct = (long long)cgrid.y * Hq <= sms ? 256 : 128;
-  // Few blocks merge twice: once before they wait, whatever the scratch holds and with nothing stored, so that the instructions are in
-  // the SMs' caches when the partial results are there. Where all blocks are resident at once and have little to read (4 MB): 32 rows
-  // of 1,280 keys and 4 of 2,000 at Qwen2.5-0.5B sizes 832 -> 800 us a step, 674 -> 653, one of 4,096 at Llama-3.1-8B sizes 2,834
-  // -> 2,809; 8 of 4,096 there, 8 MB, 3,375 -> 3,407.
+  // Few blocks merge twice: once before they wait, with nothing read of the scratch and nothing stored, so that the instructions are
+  // in the SMs' caches when the partial results are there. Where all blocks are resident at once and have little to read (4 MB):
+  // 32 rows of 1,280 keys and 4 of 2,000 at Qwen2.5-0.5B sizes 825 -> 787 us a step, 666 -> 641, one of 4,096 at Llama-3.1-8B sizes
+  // 2,818 -> 2,793. 8 of 4,096 there have 8 MB: 3,375 -> 3,407 with a first walk that also read the scratch. Reading the scratch
+  // ahead of the wait gained nothing over the zeros in shared memory; a branch around every load of the first walk lost 9 us of the
+  // 32 rows' gain, prefetches of the scratch 12.
   const bool twice = (long long)cgrid.y * Hq <= 4 * sms && (long long)cgrid.y * Hq * NPU * HD <= 1 << 20;
   fz_launch(rows_high < N ? attn_combine_units_kernel<true, false> : twice ? attn_combine_units_kernel<false, true> : attn_combine_units_kernel<false, false>, cgrid, dim3(ct),
             (size_t)(NPU + 2) * 8 + 256 * 16 + 16 * 8, stream, (const float*)part_o,

@@ -281,3 +281,46 @@ def test_blocks_of_the_merge_kernel(Hq, Hkv, hd, rows, blocks):
     o, op, _ = run_both(Hq, Hkv, hd, 16, 0, [100] * len(rows), rows)
     close(o, op, "merged rows")
     assert cuda_ops("bfloat16").attn_tc.fz_attn_combine_rows(len(o), 0, run_both.last_plan.n_short_rows) == blocks
+
+
+@pytest.mark.parametrize("Hq,Hkv,hd,rows,context,window", [(14, 2, 64, 32, 1280, 0), (8, 2, 128, 4, 1500, 0), (8, 8, 64, 9, 1400, 300), (4, 1, 128, 1, 5000, 0)])
+def test_steps_behind_one_another_on_one_scratch(Hq, Hkv, hd, rows, context, window):
+    """Few blocks of the merge kernel walk through their code before the kernel before them has ended. Two attentions with other
+    queries and other keys, queued behind one another on one scratch without a synchronisation, and each behind partial results
+    that are all NaN or infinite: the bits of each alone."""
+    from fusezap_core_b200.kernels import cuda_ops
+    cu, bs = cuda_ops("bfloat16"), 16
+    g = torch.Generator().manual_seed(rows + hd)
+    lengths = [context - 17 * i for i in range(rows)]
+    mb = -(-context // bs)
+    table = [list(range(r * mb, (r + 1) * mb)) for r in range(rows)]
+    meta = Meta([n - 1 for n in lengths], list(range(rows)), table, "cuda")
+    steps = []
+    for _ in range(2):
+        cp, cc = (make_cache(rows * mb, Hkv, bs, hd, BF, device) for device in ("cpu", "cuda"))
+        fill_cache(cp, table, lengths, g)
+        cc.pool.copy_(cp.pool)
+        q = torch.randn(rows, Hq * hd, generator=g).to(BF)
+        ref = torch.empty(rows, Hq * hd, dtype=BF)
+        PlainOps(BF).paged_attention(q, cp, Meta([n - 1 for n in lengths], list(range(rows)), table, "cpu"), ref, Hq, Hkv, hd, hd ** -0.5, window)
+        steps.append((q.cuda(), cc, ref))
+
+    def attend(step):
+        out = torch.full((rows, Hq * hd), float("nan"), dtype=BF, device="cuda")
+        cu.paged_attention(step[0], step[1], meta, out, Hq, Hkv, hd, hd ** -0.5, window)
+        return out
+
+    before = cu.launches
+    alone = [attend(step) for step in steps]
+    assert cu.launches - before == 4      # (the kernel of the units and the merge, twice)
+    torch.cuda.synchronize()
+    for out, (_, _, ref) in zip(alone, steps):
+        close(out.float().cpu(), ref.float(), "alone")
+    for fill in (float("nan"), float("inf"), -float("inf")):
+        for i in (0, 1):
+            cu._scratch_bufs["attention partials"].fill_(fill)
+            assert torch.equal(attend(steps[i]), alone[i]), f"behind a scratch of {fill}"
+    queued = [attend(steps[i % 2]) for i in range(8)]
+    for i, out in enumerate(queued):
+        assert torch.equal(out, alone[i % 2]), f"{i}-th in the queue"
+    cu.check_errors()
