@@ -594,7 +594,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
 // Rows mode: one thread's lane (token row `row`) of a finished accumulator of BN columns at `taddr`, with the bias added,
 // to the output's columns n0 .. n0 + BN - 1 (or, with the fused SwiGLU, to its packed half); of these the `part`-th of PARTS
-// equal shares. Every lane of the warp takes part in the loads from tensor memory whether or not its row exists.
+// equal shares. Every lane of the warp takes part in the loads from tensor memory whether or not its row exists or is stored: the
+// loads are warp-wide instructions, so no lane leaves an iteration early (what follows a load is guarded instead) and the lanes
+// meet at the head of every iteration.
 //
 // With p.rope the columns are whole heads [q | k | v] (the head size divides a share): q and k are rotated by the row's position, q
 // goes to c_bf16, k and v to the token's slot of the paged pools, as the rotation's kernel does from the product's float32 output,
@@ -647,33 +649,34 @@ __device__ __forceinline__ void rows_store_tile(const Params& p, uint32_t taddr,
         co[i] = turn ? *(const float4*)(cs + j + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
         si[i] = turn ? *(const float4*)(sn + j + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
+      __syncwarp();
       tmem_ld16(taddr + (uint32_t)c, v);
       tmem_ld16(taddr + (uint32_t)(c + half), u);
-      if (row >= p.rows || n >= p.feats) continue;
-      if (p.bias) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { v[i] += p.bias[n + i]; u[i] += p.bias[n + half + i]; }
-      }
-      __nv_bfloat16* dst;
-      if (n < hq) dst = p.c_bf16 + (size_t)row * hq + n;
-      else if (at.slot < 0) continue;
-      else {
+      __nv_bfloat16* dst = nullptr;
+      if (row < p.rows && n < p.feats) {
         const int head = (n - (n < hk ? hq : hk)) / p.hd;
-        dst = (n < hk ? p.k_pool : p.v_pool) + at.slot + (long long)head * p.page_size * p.hd + j;
+        if (n < hq) dst = p.c_bf16 + (size_t)row * hq + n;
+        else if (at.slot >= 0) dst = (n < hk ? p.k_pool : p.v_pool) + at.slot + (long long)head * p.page_size * p.hd + j;
       }
-      if (n < hk) {
-        const float* cf = (const float*)co;
-        const float* sf = (const float*)si;
+      if (dst != nullptr) {
+        if (p.bias) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float o1 = 0.f, o2 = 0.f;
-          if (at.there) fz_rope_pair(v[i], u[i], cf[i], sf[i], o1, o2);
-          v[i] = o1;
-          u[i] = o2;
+          for (int i = 0; i < 16; ++i) { v[i] += p.bias[n + i]; u[i] += p.bias[n + half + i]; }
         }
+        if (n < hk) {
+          const float* cf = (const float*)co;
+          const float* sf = (const float*)si;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            float o1 = 0.f, o2 = 0.f;
+            if (at.there) fz_rope_pair(v[i], u[i], cf[i], sf[i], o1, o2);
+            v[i] = o1;
+            u[i] = o2;
+          }
+        }
+        store16_bf16(dst, v);
+        store16_bf16(dst + half, u);
       }
-      store16_bf16(dst, v);
-      store16_bf16(dst + half, u);
     }
     return;
   }
@@ -684,30 +687,32 @@ __device__ __forceinline__ void rows_store_tile(const Params& p, uint32_t taddr,
 #pragma unroll 1
     for (int f = part * FEATS; f < (part + 1) * FEATS; f += 16) {
       const int c = (f >> 6) * 128 + (f & 63);
+      __syncwarp();
       tmem_ld16(taddr + (uint32_t)c, v);
       tmem_ld16(taddr + (uint32_t)(c + 64), u);
       const int n = n0 + c;                       // packed index of the gate column
-      if (row >= p.rows || n >= p.feats) continue;
-      uint32_t w[8];
+      if (row < p.rows && n < p.feats) {
+        uint32_t w[8];
 #pragma unroll
-      for (int i = 0; i < 16; i += 2) {
-        const float g0 = v[i] + (p.bias ? p.bias[n + i] : 0.f), g1 = v[i + 1] + (p.bias ? p.bias[n + i + 1] : 0.f);
-        const float u0 = u[i] + (p.bias ? p.bias[n + 64 + i] : 0.f), u1 = u[i + 1] + (p.bias ? p.bias[n + 64 + i + 1] : 0.f);
-        const __nv_bfloat162 h2 = __floats2bfloat162_rn(glu_mul(g0, u0, p.swiglu), glu_mul(g1, u1, p.swiglu));
-        w[i >> 1] = *(const uint32_t*)&h2;
+        for (int i = 0; i < 16; i += 2) {
+          const float g0 = v[i] + (p.bias ? p.bias[n + i] : 0.f), g1 = v[i + 1] + (p.bias ? p.bias[n + i + 1] : 0.f);
+          const float u0 = u[i] + (p.bias ? p.bias[n + 64 + i] : 0.f), u1 = u[i + 1] + (p.bias ? p.bias[n + 64 + i + 1] : 0.f);
+          const __nv_bfloat162 h2 = __floats2bfloat162_rn(glu_mul(g0, u0, p.swiglu), glu_mul(g1, u1, p.swiglu));
+          w[i >> 1] = *(const uint32_t*)&h2;
+        }
+        uint4* dst = (uint4*)(p.c_bf16 + (size_t)row * (p.feats >> 1) + (n >> 7) * 64 + (n & 63));
+        dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
       }
-      uint4* dst = (uint4*)(p.c_bf16 + (size_t)row * (p.feats >> 1) + (n >> 7) * 64 + (n & 63));
-      dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-      dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
     return;
   }
 #pragma unroll 1
   for (int c = part * (BN / PARTS); c < (part + 1) * (BN / PARTS); c += 16) {
+    __syncwarp();
     tmem_ld16(taddr + (uint32_t)c, v);
-    if (row >= p.rows) continue;
     const int n = n0 + c;
-    if (p.vec_ok && n + 16 <= p.feats) {
+    if (row < p.rows && p.vec_ok && n + 16 <= p.feats) {
       if (p.bias) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] += p.bias[n + i];
@@ -731,7 +736,7 @@ __device__ __forceinline__ void rows_store_tile(const Params& p, uint32_t taddr,
         dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
         dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
       }
-    } else {
+    } else if (row < p.rows) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         if (n + i < p.feats) {

@@ -375,6 +375,44 @@ def test_qkv_product_of_many_rows_with_rotation_and_cache_write(Hq, Hkv, hd, K, 
     assert flagged[0] == flagged[1] and bool(flagged[0]) == write
 
 
+@pytest.mark.parametrize("Hq,Hkv,hd,K,M", [(32, 8, 128, 512, 300), (32, 8, 128, 512, 1100), (14, 2, 64, 896, 2101)])
+@pytest.mark.parametrize("stride", [1, 2, 3, 32])
+def test_rows_of_a_warp_that_store_nothing(Hq, Hkv, hd, K, M, stride):
+    """Many rows: padding rows and rows without a page next to others in every warp (each `stride`-th row one of them, in turn; stride
+    1: no row stores), so that a warp's lanes part in every step through a tile and meet again for the next load."""
+    from fusezap_core_b200.kernels import cuda_ops
+    from fusezap_core_b200.kernels.table import KernelError
+    from test_kernels_gpu import Meta, make_cache
+    ops, bs, N = cuda_ops("bfloat16"), 16, (Hq + 2 * Hkv) * hd
+    assert ops.tc.fz_gemm_tc_qkv_rope_rows(M, N, K, hd) == 1
+    g = torch.Generator(device="cuda").manual_seed(M + stride)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(torch.bfloat16)
+    b = torch.randn(N, generator=g, device="cuda")
+    ang = torch.rand(1500, hd // 2, generator=g, device="cuda") * 6.28
+    # request 0 has its pages, request 1 none
+    table = [list(range(-(-1500 // bs))), [-1] * -(-1500 // bs)]
+    pos = [i % 1500 if i < 1500 else 0 for i in range(M)]
+    seq = [0 if i < 1500 else -1 for i in range(M)]
+    for i in range(0, M, stride):
+        seq[i] = -1 if i // stride % 2 else 1
+    meta, res = Meta(pos, seq, table, "cuda"), []
+    for fused in (True, False):
+        cache = make_cache(len(table[0]), Hkv, bs, hd, torch.bfloat16, "cuda")
+        q = torch.full((M, Hq * hd), float("nan"), dtype=torch.bfloat16, device="cuda")
+        if fused:
+            assert ops.linear_rope_kv_write(a, w, b, ang.cos(), ang.sin(), meta, cache, q, Hq, Hkv, hd)
+        else:
+            qkv = torch.empty(M, N, device="cuda")
+            ops.linear(a, w, b, qkv)
+            ops.rope_kv_write(qkv, ang.cos(), ang.sin(), meta, cache, q, Hq, Hkv, hd)
+        with pytest.raises(KernelError):      # (rows without a page are reported)
+            ops.check_errors()
+        res.append((q, cache.pool.clone()))
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    assert float(res[0][0][torch.tensor(seq) < 0].float().abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 20000, 256), (8, 33333, 128), (37, 17000, 64), (128, 16512, 72)])
 def test_product_that_keeps_only_the_largest_of_each_row(M, N, K):
     """`linear_argmax` gives the ids that `argmax` finds in the logits `linear` writes, with the numpy rule for ties (the
