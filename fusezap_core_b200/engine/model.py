@@ -13,6 +13,7 @@ import torch
 from ..cache import KVNeed
 from ..config import ModelSpec, describe, read_config_json
 from ..parts import BLOCKS, EMBED_EXTRAS, FEED_FORWARDS, LOGIT_TRANSFORMS, MIXERS, NORMS, POSITIONS, build
+from ..parts.base import can_take_products
 from ..weights import ParamSpec, load_weights
 from ..weights.loader import TORCH_DTYPE
 
@@ -85,14 +86,6 @@ class DecoderModel:
             pn = self.layers[e.layer].mixer.position_name()
             if pn is not None and pn not in self.positions:
                 raise ValueError(f"layer {e.layer} names position encoding {pn!r}, the model has {sorted(self.positions)}")
-        # a block whose every successor's first norm takes products leaves its last one to it
-        behind: dict[int, list[bool]] = {}
-        for e, then in zip(spec.schedule, [*spec.schedule[1:], None]):
-            behind.setdefault(e.layer, []).append(getattr(self.final_norm, "takes_products", False) if then is None else
-                                                  not then.add_embedding and getattr(self.layers[then.layer], "scaled1", False))
-        for layer, takes in behind.items():
-            if hasattr(self.layers[layer], "product_left"):
-                self.layers[layer].product_left = all(takes)
         self.embed: torch.Tensor | None = None
         self.lm_head: torch.Tensor | None = None
         self.dtype: str | None = None
@@ -160,6 +153,16 @@ class DecoderModel:
             block.bind({k[len(ls.prefix):]: v for k, v in tensors.items() if k.startswith(ls.prefix)}, ops)
         stem = spec.final_norm_name.rsplit(".", 1)[0] + "."
         self.final_norm.bind({k[len(stem):]: v for k, v in tensors.items() if k.startswith(stem)}, ops)
+        # a block whose every successor's first norm takes products leaves its last one to it
+        behind: dict[int, list[bool]] = {}
+        for e, then in zip(spec.schedule, [*spec.schedule[1:], None]):
+            block = None if then is None else self.layers[then.layer]
+            behind.setdefault(e.layer, []).append(can_take_products(self.final_norm) if then is None else
+                                                  not then.add_embedding and can_take_products(block) and block.scaled1)
+        for layer, takes in behind.items():
+            block = self.layers[layer]
+            if can_take_products(block):      # (such a block leaves products, too)
+                block.product_left = all(takes)
         for p in self.positions.values():
             p.prepare(max_len, self.device)
         return self

@@ -13,7 +13,8 @@ import torch
 
 from ..cache import KVNeed
 from ..weights import ParamSpec
-from .base import LayerCache, Mixer, PendingProduct, register_mixer
+from .base import LayerCache, Mixer, PendingProduct, can_take_scaled, leaves_product, register_mixer, takes_scaled
+from ..kernels.interface import ScaledRows
 
 
 @register_mixer("gqa_attention")
@@ -57,18 +58,19 @@ class GQAttention(Mixer):
     def step_needs(self) -> tuple[str, ...]:
         return ("attention",)
 
-    takes_scaled = True      # h may be `ScaledRows`
-
+    @takes_scaled
     def forward(self, ctx, h: torch.Tensor, cache: LayerCache) -> torch.Tensor:
         return self.forward_pending(ctx, h, cache).resolve(ctx, None)
 
+    @leaves_product(forward)
     def forward_pending(self, ctx, h, cache: LayerCache) -> PendingProduct:
         """`forward` with the output product left to the norm behind it."""
         n, ops, ws = h.shape[0], ctx.ops, ctx.ws
         Hq, Hkv, hd = self.Hq, self.Hkv, self.hd
         q = ws.get("q", (n, Hq * hd), ops.dtype)
         position = ctx.positions[self.position]
-        if not position.project_rotate_store(ctx, h, self.wqkv, self.bqkv, q, cache, Hq, Hkv, hd):
+        fused = not isinstance(h, ScaledRows) or can_take_scaled(position, "project_rotate_store")
+        if not fused or not position.project_rotate_store(ctx, h, self.wqkv, self.bqkv, q, cache, Hq, Hkv, hd):
             qkv = ws.get("qkv", (n, (Hq + 2 * Hkv) * hd), torch.float32)
             ops.linear(h, self.wqkv, self.bqkv, qkv)
             position.rotate_and_store(ctx, qkv, q, cache, Hq, Hkv, hd)

@@ -111,10 +111,55 @@ class PendingNorm:
         return out
 
 
+# What a part's method can do beyond the interfaces above. Marked on the function itself, so that a class that brings its own method
+# is asked for nothing that the function it replaces could do.
+_TAKES_SCALED: set[Callable] = set()
+_TAKES_PRODUCTS: set[Callable] = set()
+_LEAVES_PRODUCT: dict[Callable, Callable] = {}
+
+
+def takes_scaled(method: Callable) -> Callable:
+    """Marks a method whose rows may be `ScaledRows`."""
+    _TAKES_SCALED.add(method)
+    return method
+
+
+def takes_products(method: Callable) -> Callable:
+    """Marks a `forward` whose pending term may be a `PendingProduct`."""
+    _TAKES_PRODUCTS.add(method)
+    return method
+
+
+def leaves_product(forward: Callable) -> Callable[[Callable], Callable]:
+    """Marks a method that does what `forward` does but for the last product, which it hands back as a `PendingProduct`."""
+    def put(method: Callable) -> Callable:
+        _LEAVES_PRODUCT[forward] = method
+        return method
+    return put
+
+
+def can_take_scaled(part: Any, method: str = "forward") -> bool:
+    return getattr(type(part), method, None) in _TAKES_SCALED
+
+
+def can_take_products(part: Any) -> bool:
+    return getattr(type(part), "forward", None) in _TAKES_PRODUCTS
+
+
+def can_leave_product(part: Any) -> Callable | None:
+    """The method that stands in for the part's `forward`, or None."""
+    return _LEAVES_PRODUCT.get(getattr(type(part), "forward", None))
+
+
+def replaced(part: Any) -> bool:
+    """Whether the object itself has a `forward` in place of its class's (one that watches it, for instance)."""
+    return "forward" in getattr(part, "__dict__", ())
+
+
 @dataclass
 class PendingProduct:
     """A pending residual term that is still to be computed, rows . weight^T + bias, with nothing read or written in between: what a
-    sublayer hands to a norm with `takes_products`, which can have the product end in the stream and the norm."""
+    sublayer hands to a norm whose `forward` takes products, which can have the product end in the stream and the norm."""
     rows: torch.Tensor
     weight: torch.Tensor
     bias: torch.Tensor | None

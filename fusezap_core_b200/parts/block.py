@@ -9,11 +9,18 @@ Sandwich block: `x += post1(mixer(norm1(x))); x += post2(ffn(norm2(x)))`; the pe
 from __future__ import annotations
 from dataclasses import replace
 from ..weights import ParamSpec
-from .base import Block, FeedForward, LayerCache, Mixer, Norm, PendingNorm, register_block
+from .base import (Block, FeedForward, LayerCache, Mixer, Norm, PendingNorm, can_leave_product, can_take_products, can_take_scaled, register_block,
+                   replaced, takes_products)
 
 
 @register_block("pre_norm")
 class PreNormBlock(Block):
+    # Which of its norms may hand `ScaledRows` on (see `Ops.linear_add_norm`), and so take a sublayer's last product unlaunched, and what
+    # leaves that product: asked of the parts when they are bound.
+    scaled1 = scaled2 = False
+    mixer_pending = ffn_pending = None
+    product_left = False      # the model says whether the norm behind the block takes the feed-forward's
+
     def __init__(self, mixer: Mixer, ffn: FeedForward | None, make_norm,
                  names: tuple[str, str, str, str] = ("input_layernorm", "self_attn", "post_attention_layernorm", "mlp"),
                  norms: tuple = (None, None)):
@@ -25,10 +32,6 @@ class PreNormBlock(Block):
         self.norm2 = None
         if ffn is not None:
             self.norm2 = make_norm(norms[1]) if norms[1] is not None else make_norm()
-        # Which of its norms may hand `ScaledRows` on (see `Ops.linear_add_norm`), and so take a sublayer's last product unlaunched.
-        self.scaled1, self.scaled2 = (getattr(norm, "takes_products", False) and getattr(part, "takes_scaled", False)
-                                      for norm, part in ((self.norm1, mixer), (self.norm2, ffn)))
-        self.product_left = False      # the model says whether the norm behind the block takes the feed-forward's
 
     def children(self):
         n1, mx, n2, ff = self.names
@@ -49,18 +52,28 @@ class PreNormBlock(Block):
         for prefix, part in self.children():
             own = {k[len(prefix) + 1:]: v for k, v in tensors.items() if k == prefix or k.startswith(prefix + ".")}
             part.bind(own, ops)
+        self.scaled1 = can_take_products(self.norm1) and can_take_scaled(self.mixer)
+        self.scaled2 = self.ffn is not None and can_take_products(self.norm2) and can_take_scaled(self.ffn)
+        self.mixer_pending, self.ffn_pending = can_leave_product(self.mixer), can_leave_product(self.ffn)
 
+    @takes_products
     def forward(self, ctx, x, delta, cache: LayerCache):
-        h = self.norm1.forward(ctx, x, delta, scaled=True) if self.scaled1 else self.norm1.forward(ctx, x, delta)
-        if self.ffn is None:
-            return x, self.mixer.forward(ctx, h, cache)
-        if self.scaled2 and hasattr(self.mixer, "forward_pending"):
-            h = self.norm2.forward(ctx, x, self.mixer.forward_pending(ctx, h, cache), scaled=True)
+        mixer, ffn = self.mixer, self.ffn
+        own_mixer = replaced(mixer)      # (an object's own `forward` is run, on plain rows)
+        if self.scaled1 and not own_mixer and not replaced(self.norm1):
+            h = self.norm1.forward(ctx, x, delta, scaled=True)
         else:
-            h = self.norm2.forward(ctx, x, self.mixer.forward(ctx, h, cache))
-        if self.product_left and hasattr(self.ffn, "forward_pending"):
-            return x, self.ffn.forward_pending(ctx, h)
-        return x, self.ffn.forward(ctx, h)
+            h = self.norm1.forward(ctx, x, delta)
+        if ffn is None:
+            return x, mixer.forward(ctx, h, cache)
+        own_ffn = replaced(ffn)
+        if self.scaled2 and self.mixer_pending is not None and not own_mixer and not own_ffn and not replaced(self.norm2):
+            h = self.norm2.forward(ctx, x, self.mixer_pending(mixer, ctx, h, cache), scaled=True)
+        else:
+            h = self.norm2.forward(ctx, x, mixer.forward(ctx, h, cache))
+        if self.product_left and self.ffn_pending is not None and not own_ffn and not replaced(self):
+            return x, self.ffn_pending(ffn, ctx, h)
+        return x, ffn.forward(ctx, h)
 
 
 @register_block("sandwich_norm")

@@ -11,7 +11,7 @@ from __future__ import annotations
 import torch
 
 from ..weights import ParamSpec
-from .base import FeedForward, PendingProduct, register_feed_forward
+from .base import FeedForward, PendingProduct, leaves_product, register_feed_forward, takes_scaled
 
 
 @register_feed_forward("swiglu")
@@ -50,8 +50,6 @@ class SwiGLU(FeedForward):
         self.wd = tensors[f"{d}{sx}"]
         self.bd = tensors[f"{d}.bias"].float() if f"{d}.bias" in tensors else None
 
-    takes_scaled = True      # h may be `ScaledRows`
-
     def _act(self, ctx, h, tag: str = "") -> torch.Tensor:
         n, ops, ws = h.shape[0], ctx.ops, ctx.ws
         a = ws.get(tag + "act", (n, self.I), ops.dtype)
@@ -64,6 +62,7 @@ class SwiGLU(FeedForward):
             ops.swiglu(gu, a, **other)
         return a
 
+    @takes_scaled
     def forward(self, ctx, h: torch.Tensor, tag: str = "") -> torch.Tensor:
         """tag: a prefix for the names of its scratch buffers (a feed-forward that runs inside another one)."""
         a = self._act(ctx, h, tag)
@@ -71,6 +70,7 @@ class SwiGLU(FeedForward):
         ctx.ops.linear(a, self.wd, self.bd, delta)
         return delta
 
+    @leaves_product(forward)
     def forward_pending(self, ctx, h) -> PendingProduct:
         """`forward` with the down product left to the norm behind it."""
         return PendingProduct(self._act(ctx, h), self.wd, self.bd)

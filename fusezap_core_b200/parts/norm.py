@@ -16,7 +16,7 @@ import torch
 
 from ..weights import ParamSpec
 from ..kernels.interface import ScaledRows
-from .base import Norm, PendingNorm, PendingProduct, PendingSum, register_norm
+from .base import Norm, PendingNorm, PendingProduct, PendingSum, register_norm, takes_products
 
 
 @register_norm("rmsnorm")
@@ -34,11 +34,6 @@ class RMSNorm(Norm):
         self.weight: torch.Tensor | None = None
         self.weight32: torch.Tensor | None = None
 
-    @property
-    def takes_products(self) -> bool:
-        """Whether the pending term may be a `PendingProduct`."""
-        return True
-
     def tensors(self) -> dict[str, ParamSpec]:
         return {self.name: ParamSpec(() if self.scalar else (self.size,), role="vector", init="normal" if self.offset else "ones")}
 
@@ -50,6 +45,7 @@ class RMSNorm(Norm):
             self.weight = self.weight.float().reshape(1).expand(self.size).contiguous()
         self.weight32 = self.weight.float()      # (the product that ends in the norm takes float32)
 
+    @takes_products
     def forward(self, ctx, x, delta, rows=None, n_rows=None, scaled: bool = False):
         """scaled: the caller's next part takes `ScaledRows`; it gets them where the pending term is a product whose kernel can
         end in the norm."""

@@ -14,7 +14,7 @@ import math
 import numpy as np
 import torch
 
-from .base import LayerCache, PositionEncoding, register_position
+from .base import LayerCache, PositionEncoding, register_position, takes_scaled
 
 
 def inverse_frequencies(head_dim: int, theta: float, kind: str = "default", factor: float = 1.0,
@@ -100,6 +100,7 @@ class RotaryEncoding(PositionEncoding):
             raise ValueError(f"rope was built for head_dim {self.head_dim}, the mixer has {head_dim}")
         ctx.ops.rope_kv_write(qkv, self.cos, self.sin, ctx.meta, cache, q_out, num_heads, num_kv_heads, head_dim)
 
+    @takes_scaled
     def project_rotate_store(self, ctx, h, w, bias, q_out, cache, num_heads, num_kv_heads, head_dim) -> bool:
         if head_dim != self.head_dim:
             raise ValueError(f"rope was built for head_dim {self.head_dim}, the mixer has {head_dim}")
