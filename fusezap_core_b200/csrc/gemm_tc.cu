@@ -148,7 +148,8 @@ struct Params {
   // Llama-3.1-8B sizes, 1, 8 and 64 rows of 4,096 keys: 2,957 -> 2,847 us, 3,455 -> 3,392, 7,643 -> 7,631; at Qwen2.5-0.5B sizes,
   // 1 row of 300 and 32 of 1,280: 592 -> 545, 879 -> 843.)
   float* x;
-  const float* norm_w;
+  const void* norm_w;      // [feats], float32 or bfloat16 (norm_bf16)
+  int norm_bf16;
   __nv_bfloat16* h;
   float* ss_out;           // [rows][ss_parts]
   // ss set: the rows of X are such an h; each output is the product times its row's factor, plus the bias
@@ -293,7 +294,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       if constexpr (PAIRS) b2 = p.bias[feat + half];
     }
     if constexpr (EP == EP_NORM)
-      if (own) nw = p.norm_w[feat];
+      if (own) nw = p.norm_bf16 ? __bfloat162float(((const __nv_bfloat16*)p.norm_w)[feat]) : ((const float*)p.norm_w)[feat];
     if constexpr (EP == EP_ROPE) {
 #pragma unroll
       for (int e = 0; e < CV; ++e)
@@ -1551,15 +1552,16 @@ FZ_API int fz_gemm_tc_norm_parts(int M, int N, int K) {
   return (N + BM - 1) / BM * 4;
 }
 
-// stream [M, N] float32 += x . w^T + bias; h [M, N] bf16 = the new stream * norm_w; ss [M, fz_gemm_tc_norm_parts(M, N, K)]: partial
+// stream [M, N] float32 += x . w^T + bias; h [M, N] bf16 = the new stream * norm_w (float32 or bf16); ss [M, fz_gemm_tc_norm_parts(M, N, K)]: partial
 // sums of the new stream's squares.
-FZ_API int fz_gemm_tc_add_norm(const void* x, const void* w, const float* bias, float* stream_x, const float* norm_w, void* h, float* ss,
+FZ_API int fz_gemm_tc_add_norm(const void* x, const void* w, const float* bias, float* stream_x, const void* norm_w, int norm_dtype, void* h, float* ss,
                                int M, int N, int K, int* err, cudaStream_t stream) {
   Params f{};
   f.ss_parts = fz_gemm_tc_norm_parts(M, N, K);
   if (f.ss_parts == 0) return FZ_BAD_SHAPE;
+  if (norm_dtype != FZ_F32 && norm_dtype != FZ_BF16) return FZ_BAD_DTYPE;
   if ((uintptr_t)h & 15) return FZ_BAD_ALIGNMENT;      // (the next product reads it)
-  f.x = stream_x; f.norm_w = norm_w; f.h = (__nv_bfloat16*)h; f.ss_out = ss;
+  f.x = stream_x; f.norm_w = norm_w; f.norm_bf16 = norm_dtype == FZ_BF16; f.h = (__nv_bfloat16*)h; f.ss_out = ss;
   return gemm_tc_impl(x, w, bias, h, FZ_BF16, M, N, K, f, err, stream);
 }
 

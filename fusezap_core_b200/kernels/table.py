@@ -501,13 +501,12 @@ class CudaOps(Ops):
         m, k = a.shape
         n = w.shape[0]
         parts = self.norm_parts(m, n, k)
-        if parts == 0 or weight.dtype != torch.float32 or self.tc.fz_gemm_tc_check(_p(a), _p(w), c_int(m), c_int(n), c_int(k)) != 0 or \
-                h.data_ptr() % 16:
+        if parts == 0 or self.tc.fz_gemm_tc_check(_p(a), _p(w), c_int(m), c_int(n), c_int(k)) != 0 or h.data_ptr() % 16:
             return False
         self._want(a, "linear input", (torch.bfloat16,), 2)
         self._want(w, "linear weight", (torch.bfloat16,), 2)
         self._want(x, "x", (torch.float32,), 2)
-        self._want(weight, "norm weight", (torch.float32,), 1)
+        self._want(weight, "norm weight", (torch.float32, torch.bfloat16), 1)
         self._want(h, "h", (torch.bfloat16,), 2)
         self._want(squares, "sums of squares", (torch.float32,), 2)
         if bias is not None:
@@ -516,8 +515,8 @@ class CudaOps(Ops):
                 (bias is not None and bias.shape[0] != n):
             raise KernelError(f"linear_add_norm: a {tuple(a.shape)}, w {tuple(w.shape)}, x {tuple(x.shape)}, h {tuple(h.shape)}, "
                               f"squares {tuple(squares.shape)}")
-        self._check(self.tc.fz_gemm_tc_add_norm(_p(a), _p(w), _p(bias), _p(x), _p(weight), _p(h), _p(squares), c_int(m), c_int(n), c_int(k),
-                                                _p(self.err), self._stream()), "linear_add_norm (tensor cores)",
+        self._check(self.tc.fz_gemm_tc_add_norm(_p(a), _p(w), _p(bias), _p(x), _p(weight), c_int(_CODE[weight.dtype]), _p(h), _p(squares),
+                                                c_int(m), c_int(n), c_int(k), _p(self.err), self._stream()), "linear_add_norm (tensor cores)",
                     ideal_linear_bytes(m, n, k, 2, 2, 10))
         return True
 

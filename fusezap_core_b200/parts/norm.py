@@ -32,7 +32,6 @@ class RMSNorm(Norm):
         self.size, self.eps, self.groups, self.name, self.scalar = size, float(eps), int(groups), name, bool(scalar)
         self.offset = float(offset)
         self.weight: torch.Tensor | None = None
-        self.weight32: torch.Tensor | None = None
 
     def tensors(self) -> dict[str, ParamSpec]:
         return {self.name: ParamSpec(() if self.scalar else (self.size,), role="vector", init="normal" if self.offset else "ones")}
@@ -43,7 +42,6 @@ class RMSNorm(Norm):
             self.weight = (self.weight.float() + self.offset).contiguous()
         if self.scalar:      # the kernels take a weight per coordinate
             self.weight = self.weight.float().reshape(1).expand(self.size).contiguous()
-        self.weight32 = self.weight.float()      # (the product that ends in the norm takes float32)
 
     @takes_products
     def forward(self, ctx, x, delta, rows=None, n_rows=None, scaled: bool = False):
@@ -56,7 +54,7 @@ class RMSNorm(Norm):
             parts = count(n, self.size, delta.rows.shape[1]) if count is not None and scaled and rows is None and self.groups == 1 else 0
             if parts:
                 squares = ctx.ws.get("norm_squares", (n, parts), torch.float32)
-                if ctx.ops.linear_add_norm(delta.rows, delta.weight, delta.bias, x, self.weight32, h, squares):
+                if ctx.ops.linear_add_norm(delta.rows, delta.weight, delta.bias, x, self.weight, h, squares):
                     return ScaledRows(h, squares, self.eps)
             delta = delta.resolve(ctx, x)
         self._run(ctx, x, delta, h, rows)

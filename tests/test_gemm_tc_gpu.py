@@ -230,6 +230,29 @@ def test_product_that_ends_in_the_norm(D, K):
     assert ops.norm_parts(129, D, K) == 0 and ops.norm_parts(1, D, 64) == 0 and ops.norm_parts(1, 129 * 128, K) == 0 and ops.norm_parts(1, D + 4, K) == 0
 
 
+@pytest.mark.parametrize("D,K,rows", [(136, 72, 1), (896, 4864, 8), (1000, 200, 33), (4096, 4096, 128)])
+def test_norm_weight_in_either_type(D, K, rows):
+    """The product that ends in the norm reads a bfloat16 weight as it stands: the bits of the same weight in float32, also where it is
+    not aligned beyond its type."""
+    from fusezap_core_b200.kernels import cuda_ops
+    from fusezap_core_b200.kernels.table import KernelError
+    ops = cuda_ops("bfloat16")
+    g = torch.Generator(device="cuda").manual_seed(D + rows)
+    a, w = (torch.randn(n, K, generator=g, device="cuda").to(torch.bfloat16) for n in (rows, D))
+    x0 = torch.randn(rows, D, generator=g, device="cuda")
+    weight = torch.randn(D + 1, generator=g, device="cuda").to(torch.bfloat16)[1:]
+    out = []
+    for t in (weight, weight.float()):
+        x, h = x0.clone(), torch.empty(rows, D, dtype=torch.bfloat16, device="cuda")
+        squares = torch.empty(rows, ops.norm_parts(rows, D, K), device="cuda")
+        assert ops.linear_add_norm(a, w, None, x, t, h, squares)
+        out.append((x, h, squares))
+    assert all(torch.equal(i, j) for i, j in zip(*out)) and torch.equal(out[0][1], (out[0][0] * weight.float()).to(torch.bfloat16))
+    with pytest.raises(KernelError):
+        ops.linear_add_norm(a, w, None, *(out[0][0], weight.half(), *out[0][1:]))
+    ops.check_errors()
+
+
 def test_refused_shapes_fall_back_to_the_plain_kernel():
     from fusezap_core_b200.kernels import cuda_ops
     ops = cuda_ops("bfloat16")

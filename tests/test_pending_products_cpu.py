@@ -257,3 +257,24 @@ def test_a_pending_product_is_the_product():
     from fusezap_core_b200.engine.step import Workspace
     ctx.ws = Workspace(torch.device("cpu"), 4)
     assert torch.equal(PendingProduct(a, w, b).resolve(ctx, None), a @ w.T + b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("in_place", [True, False])
+def test_a_norm_weight_changed_after_loading(dtype, in_place):
+    """Folded or not, a norm multiplies by the weight it has at the call, in the type it has."""
+    out = []
+    for ops in (Plain(), FoldingOps()):
+        model = bound(model_of(), ops)
+        norms = [n for layer in model.layers for n in (layer.norm1, layer.norm2)]
+        for n in norms:
+            n.bind({"weight": n.weight.to(dtype)}, ops)
+        logits(model)
+        for i, n in enumerate(norms):
+            new = torch.linspace(0.5, 1.5 + i, D).to(dtype)
+            if in_place:
+                n.weight.copy_(new)
+            else:
+                n.weight = new
+        out.append(logits(model))
+    same(out[1], out[0])
