@@ -57,11 +57,12 @@ class Workspace:
         # what was handed out, by exactly what was asked for: a step asks for some 200 views, 2 us of Python each
         self._views: dict[tuple, torch.Tensor] = {}
 
-    def get(self, tag: str, shape: tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+    def get(self, tag: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
+        shape = tuple(shape)
         view = self._views.get((tag, shape, dtype))
         if view is not None:
             return view
-        key = (tag, tuple(shape[1:]), dtype)
+        key = (tag, shape[1:], dtype)
         buf = self._bufs.get(key)
         if buf is None or buf.shape[0] < shape[0]:
             if buf is not None:
@@ -71,7 +72,7 @@ class Workspace:
             self._views.clear()
         if len(self._views) >= 1024:      # (steps of many sizes)
             self._views.clear()
-        view = self._views[tag, tuple(shape), dtype] = buf[:shape[0]]
+        view = self._views[tag, shape, dtype] = buf[:shape[0]]
         return view
 
     def bytes(self) -> int:

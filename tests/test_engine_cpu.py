@@ -264,3 +264,15 @@ def test_engine_takes_one_config_object(models):
         LLMEngine(model, max_model_len=100000)
     with pytest.raises(TypeError):
         LLMEngine(model, no_such_option=1)
+
+
+def test_workspace_shapes():
+    """A buffer's shape may be any sequence; equal shapes get the same memory, whatever they are written as, and a buffer that
+    has grown is not handed out in its former place."""
+    from fusezap_core_b200.engine.step import Workspace
+    ws = Workspace(torch.device("cpu"), 4)
+    views = [ws.get("a", shape, torch.float32) for shape in ((3, 5), [3, 5], torch.Size((3, 5)), (3, np.int64(5)))]
+    assert all(v.shape == (3, 5) and v.data_ptr() == views[0].data_ptr() for v in views)
+    grown = ws.get("a", [9, 5], torch.float32)
+    assert grown.shape == (9, 5) and ws.get("a", (3, 5), torch.float32).data_ptr() == grown.data_ptr()
+    assert ws.get("a", [3, 5], torch.int32).dtype == torch.int32
