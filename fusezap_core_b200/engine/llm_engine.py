@@ -17,7 +17,9 @@ while requests only decode, the next step is launched (fed from the ids still on
 last one's tokens, so the device does not idle between steps.
 """
 from __future__ import annotations
+import gc
 import itertools
+from contextlib import contextmanager
 from dataclasses import dataclass
 from typing import Iterable, Sequence as Seq
 
@@ -325,7 +327,7 @@ class LLMEngine:
                 logits = self._eager(n_w)
                 g = torch.cuda.CUDAGraph()
                 before = ops.launches
-                with torch.cuda.graph(g):
+                with _no_collection(), torch.cuda.graph(g):
                     self._eager(n_w)
                 self.launches_per_graph[key] = ops.launches - before
                 ops.launches = before
@@ -418,6 +420,19 @@ class LLMEngine:
         if not self.profile:
             raise RuntimeError("the engine was made without profile=True")
         return self.ops.profile_report()
+
+
+@contextmanager
+def _no_collection():
+    """No automatic garbage collection: one that came upon an engine in a cycle of references would destroy its captured steps, which
+    the CUDA runtime does not allow while a step is being recorded, and the recording would be lost."""
+    was = gc.isenabled()
+    gc.disable()
+    try:
+        yield
+    finally:
+        if was:
+            gc.enable()
 
 
 def _sampling_views(buffer: torch.Tensor, rows: int) -> tuple[torch.Tensor, ...]:

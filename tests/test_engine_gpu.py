@@ -131,6 +131,44 @@ def test_small_steps_replay_captured_graphs(folders):
     assert only_decode.generate(P, ps) == without.generate(P, ps) and only_decode.stats["step_graph_replays"] == 0
 
 
+def test_garbage_is_not_collected_while_a_step_is_recorded(folders):
+    """Captured steps of an engine that is garbage (in a cycle of references) cannot be destroyed while another engine records one:
+    the CUDA runtime refuses, and the recording is lost. The collector runs at almost every allocation here."""
+    import gc
+    from fusezap_core_b200 import LLMEngine, SamplingParams, load_model
+    d, cfg, opts = folders["tiny_hd64"]
+    model = load_model(d, "bfloat16", "cuda:0", max_len=128)
+    make = lambda: LLMEngine(model, num_blocks=16, block_size=16, max_num_seqs=2, max_prefill_tokens=32, max_model_len=128)
+    P, sp = prompts(cfg, (9, 14), seed=4), SamplingParams(max_tokens=5, ignore_eos=True)
+    old, new = make(), make()
+    want = old.generate(P, sp)
+    left = list(old._graphs.values())
+    old._graphs.clear()
+    assert len(left) >= 1
+    recorded = []
+
+    class Held:
+        pass
+
+    def eager(n, inner=new._eager):
+        if torch.cuda.is_current_stream_capturing():
+            h = Held()
+            h.me, h.graph = h, left.pop() if left else None
+            recorded.append(len(left))
+        junk = [[[] for _ in range(100)] for _ in range(100)]      # (more than a generation's threshold)
+        return inner(n)
+
+    new._eager = eager
+    thresholds = gc.get_threshold()
+    gc.set_threshold(10, 1, 1)
+    try:
+        assert new.generate(P, sp) == want
+    finally:
+        gc.set_threshold(*thresholds)
+    assert recorded and gc.isenabled()
+    new.ops.check_errors()
+
+
 @pytest.mark.parametrize("name", ["tiny_hd64", "tiny_hd128"])
 def test_the_serving_path_at_tensor_core_head_sizes(folders, name):
     """bfloat16 at head sizes 64 and 128, where attention runs on the tensor-core kernels (portions of 8 tokens and more
