@@ -172,6 +172,105 @@ def test_tokens_dealt_out_to_the_splits(tiles, splits):
     ops.check_errors()
 
 
+def row_sizes(n):
+    """A power of two per row, another one than that of the rows it could be taken for (the tokens are dealt out by ones and fours)."""
+    return 2.0 ** ((torch.arange(n, device="cuda") % 11) - 5.0)[:, None]
+
+
+def product_bound(normed, w, bias):
+    """D exact products, each addition off by at most 2^-23 of the magnitudes' sum, and the factor's own 40 roundings."""
+    b = 0 if bias is None else bias.double()
+    return normed @ w.double().T + b, (normed.shape[1] + 48) * 2.0 ** -23 * (normed.abs() @ w.abs().double().T + abs(b))
+
+
+def check_product(out, normed, w, bias, what):
+    ref, bound = product_bound(normed, w, bias)
+    assert bool(((out.double() - ref).abs() <= bound).all()), what
+
+
+def check_gated(out, normed, gate, up, gate_bias, up_bias, activation, what):
+    """Per element: what the sums may be off by, through an activation of slope at most 1.13, the activation's own roundings (an
+    exponential of 2 + 1.2 |z| units or a hyperbolic tangent of 2, a division and three products), one rounding to bfloat16, whose 8 bits leave half a unit of at most 2^-8 of the value."""
+    (z, dz), (u, du) = product_bound(normed, gate, gate_bias), product_bound(normed, up, up_bias)
+    f = z / (1 + torch.exp(-z)) if activation == "silu" else 0.5 * z * (1 + torch.tanh((2 / torch.pi) ** 0.5 * (z + 0.044715 * z ** 3)))
+    own = (8 + 2 * z.abs()) * 2.0 ** -23 * (f.abs() if activation == "silu" else z.abs()) * u.abs()
+    sums = 1.13 * dz * (u.abs() + du) + f.abs() * du + own
+    bound = sums + 2.0 ** -8 * ((f * u).abs() + sums) + 1e-37
+    assert bool(((out.double() - f * u).abs() <= bound).all()), what
+
+
+ROWS_AROUND_GROUPS = (1, 2, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128)
+
+
+def rows_without_factors(D, parts, g):
+    """The rows of a norm of weight one without their factors, with sums of squares in `parts` pieces, and the normed rows in 64 bits."""
+    from fusezap_core_b200.kernels.interface import ScaledRows
+    h = (torch.randn(128, D, generator=g, device="cuda") * row_sizes(128)).to(torch.bfloat16)
+    squares = torch.stack([c.float().square().sum(-1) for c in h.tensor_split(parts, -1)], -1).contiguous()
+    eps = 2e-3      # (the smallest rows have a mean square of 1e-3)
+    normed = h.double() * (squares.double().sum(-1, keepdim=True) / D + eps).rsqrt()
+    return normed, lambda rows: ScaledRows(h[:rows].contiguous(), squares[:rows].contiguous(), eps)
+
+
+@pytest.mark.parametrize("D,parts", [(896, 28), (1000, 33), (2048, 64), (264, 1)])
+@pytest.mark.parametrize("tiles,splits", [(3, 8), (36, 7), (42, 6), (48, 5), (64, 4), (76, 3), (128, 2), (130, 1)])
+def test_products_of_rows_without_factors(D, parts, tiles, splits):
+    """Products that read such rows multiply every sum by its row's factor, whoever finishes it: for every number of CTAs that share a
+    tile (one: K is not cut), plain and gated, with and without a bias, the last tile ragged or whole."""
+    from fusezap_core_b200.kernels import cuda_ops
+    ops = cuda_ops("bfloat16")
+    splits = min(splits, -(-D // 64))
+    g = torch.Generator(device="cuda").manual_seed(D + tiles)
+    normed, scaled = rows_without_factors(D, parts, g)
+    N, inner = tiles * 128 - 40, tiles * 64
+    assert ops.tc.fz_gemm_tc_splits(N, D) == splits and ops.tc.fz_gemm_tc_splits(2 * inner, D) == splits
+    w, gate, up = ((torch.randn(n, D, generator=g, device="cuda") * D ** -0.5).to(torch.bfloat16) for n in (N, inner, inner))
+    b, bg, bu = (torch.randn(n, generator=g, device="cuda") for n in (N, inner, inner))
+    for bias in (False, True):
+        packed = ops.pack_gate_up(gate, up, *((bg, bu) if bias else ()))
+        for rows in ROWS_AROUND_GROUPS:
+            what, rest = f"{rows} rows, bias {bias}", normed[:rows]
+            out = torch.full((rows + 1, N), float("nan"), device="cuda")
+            ops.linear(scaled(rows), w, b if bias else None, out[:rows])
+            check_product(out[:rows], rest, w, b if bias else None, what)
+            assert bool(out[rows].isnan().all()), what
+            act = torch.full((rows + 1, inner), float("nan"), dtype=torch.bfloat16, device="cuda")
+            for activation in ("silu", "gelu_tanh"):
+                ops.linear_swiglu(scaled(rows), packed, act[:rows], activation)
+                check_gated(act[:rows], rest, gate, up, bg if bias else None, bu if bias else None, activation, f"{what}, {activation}")
+                assert bool(act[rows].isnan().all()), what
+    ops.check_errors()
+
+
+@pytest.mark.parametrize("Hq,Hkv,hd,D", [(128, 1, 128, 512), (14, 2, 64, 896), (46, 1, 128, 264)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_rotated_product_of_rows_without_factors(Hq, Hkv, hd, D, bias):
+    """The same for the product that ends in the rotation and the cache write (K not cut, cut in 8 and in 5): the bits of the plain
+    product of these rows followed by the rotation's kernel."""
+    from fusezap_core_b200.kernels import cuda_ops
+    from test_kernels_gpu import Meta, make_cache
+    ops, N = cuda_ops("bfloat16"), (Hq + 2 * Hkv) * hd
+    g = torch.Generator(device="cuda").manual_seed(D + Hq)
+    normed, scaled = rows_without_factors(D, 7, g)
+    w = (torch.randn(N, D, generator=g, device="cuda") * D ** -0.5).to(torch.bfloat16)
+    b = torch.randn(N, generator=g, device="cuda") if bias else None
+    ang = torch.rand(200, hd // 2, generator=g, device="cuda") * 6.28
+    for rows in (1, 3, 8, 9, 16, 17, 31, 32):
+        meta = Meta([3 * i % 200 for i in range(rows)], [i % 2 for i in range(rows)], [list(range(13)), list(range(13, 26))], "cuda")
+        out, res = torch.empty(rows, N, device="cuda"), []
+        ops.linear(scaled(rows), w, b, out)
+        check_product(out, normed[:rows], w, b, f"{rows} rows")
+        for fused in (True, False):
+            cache, q = make_cache(26, Hkv, 16, hd, torch.bfloat16, "cuda"), torch.empty(rows, Hq * hd, dtype=torch.bfloat16, device="cuda")
+            if fused:
+                assert ops.linear_rope_kv_write(scaled(rows), w, b, ang.cos(), ang.sin(), meta, cache, q, Hq, Hkv, hd)
+            else:
+                ops.rope_kv_write(out, ang.cos(), ang.sin(), meta, cache, q, Hq, Hkv, hd)
+            res.append((q, cache.pool.clone()))
+        assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1]), f"{rows} rows"
+    ops.check_errors()
+
+
 @pytest.mark.parametrize("D,K", [(896, 4864), (4096, 4096), (136, 72), (1000, 200), (16384, 128)])
 def test_product_that_ends_in_the_norm(D, K):
     """x += a . w^T + bias and the norm behind it in the product's kernel, then the products that read its rows: the stream has
@@ -180,10 +279,11 @@ def test_product_that_ends_in_the_norm(D, K):
     from fusezap_core_b200.kernels import cuda_ops
     from fusezap_core_b200.kernels.interface import ScaledRows
     from test_kernels_gpu import Meta, make_cache
-    ops, eps = cuda_ops("bfloat16"), 1e-5
+    ops, eps = cuda_ops("bfloat16"), 1.0
     g = torch.Generator(device="cuda").manual_seed(D + K)
     a, w = (torch.randn(n, K, generator=g, device="cuda").to(torch.bfloat16) for n in (128, D))
-    x0 = 30 * torch.randn(128, D, generator=g, device="cuda")
+    a *= row_sizes(128)      # (so that a factor of another row shows; eps matters to the smallest)
+    x0 = 30 * torch.randn(128, D, generator=g, device="cuda") * row_sizes(128)
     bias, weight = torch.randn(D, generator=g, device="cuda"), 1 + 0.1 * torch.randn(D, generator=g, device="cuda")
     Hq, Hkv, hd, inner = 3, 1, 64, 192
     wq = (torch.randn((Hq + 2 * Hkv) * hd, D, generator=g, device="cuda") * D ** -0.5).to(torch.bfloat16)
@@ -191,7 +291,7 @@ def test_product_that_ends_in_the_norm(D, K):
     gate, up = ((torch.randn(inner, D, generator=g, device="cuda") * D ** -0.5).to(torch.bfloat16) for _ in range(2))
     packed = ops.pack_gate_up(gate, up)
     ang = torch.rand(200, hd // 2, generator=g, device="cuda") * 6.28
-    for rows in (1, 2, 5, 8, 9, 16, 17, 32, 33, 64, 65, 128):
+    for rows in ROWS_AROUND_GROUPS:
         parts = ops.norm_parts(rows, D, K)
         assert parts == -(-D // 128) * 4
         x, h = x0[:rows].clone(), torch.empty(rows, D, dtype=torch.bfloat16, device="cuda")
@@ -207,14 +307,10 @@ def test_product_that_ends_in_the_norm(D, K):
         normed, scaled = factor * h.double(), ScaledRows(h, squares, eps)
         out = torch.empty(rows, wq.shape[0], device="cuda")
         ops.linear(scaled, wq, bq, out)
-        # (D exact products, each addition off by at most 2^-23 of the magnitudes' sum, and the factor's own 40 roundings)
-        bound = (D + 48) * 2.0 ** -23 * (normed.abs() @ wq.abs().double().T + bq.abs().double())
-        assert bool(((out.double() - (normed @ wq.double().T + bq.double())).abs() <= bound).all()), f"{rows} rows"
+        check_product(out, normed, wq, bq, f"{rows} rows")
         act = torch.empty(rows, inner, dtype=torch.bfloat16, device="cuda")
         ops.linear_swiglu(scaled, packed, act)
-        z = normed @ gate.double().T
-        ref = z / (1 + torch.exp(-z)) * (normed @ up.double().T)
-        assert float((act.double() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()) * 1.01, f"{rows} rows"
+        check_gated(act, normed, gate, up, None, None, "silu", f"{rows} rows")
         if rows <= 32:      # the rotated product against the plain one and the rotation's kernel
             meta = Meta([3 * i % 200 for i in range(rows)], [i % 2 for i in range(rows)], [list(range(13)), list(range(13, 26))], "cuda")
             res = []
