@@ -129,7 +129,11 @@ __device__ __forceinline__ void fz_copy16(void* dst, const void* src, bool ok) {
 // All the shared memory that a block may have, as the limit of a kernel without static shared memory whose need differs from
 // call to call: set once per kernel. (A limit raised step by step to each call's need can be lowered again by another thread's
 // smaller call between the check and the launch.)
+#ifndef FZ_TIMELINE
 constexpr int FZ_MOST_SMEM = 227 * 1024;
+#else
+constexpr int FZ_MOST_SMEM = 227 * 1024 - 16;      // (the measurement aid's own word)
+#endif
 #define FZ_RAISE_SMEM(kern)                                                                                                    \
   do {                                                                                                                         \
     static const cudaError_t raised__ = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FZ_MOST_SMEM); \

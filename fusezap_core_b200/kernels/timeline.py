@@ -11,7 +11,9 @@ import ctypes
 
 import numpy as np
 
-_FILES = (("core", ("rowwise", "gemm_simt", "attn_simt")), ("tc", ("gemm_tc", "attn_decode", "attn_prefill", "attn_prefill_tc")))
+# (library, the kernel table's attribute that holds it once it is loaded, the source files whose launches are read)
+_FILES = (("fzb200_core", "core", ("rowwise", "gemm_simt", "attn_simt")), ("fzb200_tc", "tc", ("gemm_tc",)),
+          ("fzb200_attn_tc", "_attn_tc", ("attn_decode", "attn_prefill", "attn_prefill_tc")))
 SLOTS = 4096
 
 
@@ -19,7 +21,7 @@ def read(ops) -> list[tuple[int, int, str]]:
     """(start ns, dependency met ns, source file) of every launch since the last call, in order of start; clears the
     buffers. Raises if the libraries were built without the switch."""
     out = []
-    for attr, names in _FILES:
+    for _, attr, names in _FILES:
         lib = getattr(ops, attr, None)
         if lib is None:
             continue

@@ -47,6 +47,13 @@ def test_ideal_bytes_helpers():
     assert contexts([Seg(1, 99), Seg(3, 10)]) == 100 + 36
 
 
+def test_timeline_reads_the_libraries_that_hold_the_kernels():
+    from fusezap_core_b200.kernels import timeline
+    from fusezap_core_b200.kernels.build import LIBRARIES
+    for library, _, names in timeline._FILES:
+        assert {f"{n}.cu" for n in names} <= set(LIBRARIES[library])
+
+
 def test_timeline_costs_from_timestamps():
     """`per_launch_costs`: per position in a step, the median over the steps of (next launch's dependency met - this
     launch's dependency met) and of (dependency met - first block started)."""
