@@ -258,9 +258,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // The rotation needs, of every token this thread will finish, the request's row, the position, the page and the angles:
   // loads that depend on one another and on nothing a kernel before this one writes (the host packed the step's metadata
   // before the step began). They are asked for now, and the addresses computed, by the epilogue warps that would otherwise only
-  // wait, for the first group of tokens; those of further groups in the loop at the end. (With
-  // the addresses computed and the bias waited for at the end, what follows the sums took 2.2 us of the product at one row at
-  // Qwen2.5-0.5B sizes, 0.6 now: one warp per scheduler walks two hundred dependent instructions in a microsecond.)
+  // wait, for the first group of tokens; those of further groups in the loop at the end. (What
+  // follows the sums then takes 0.1 us of the product at one row at Qwen2.5-0.5B sizes. One warp per scheduler walks two hundred
+  // dependent instructions in a microsecond.)
   Place ahead[CV];
   const int head = EP == EP_ROPE ? feat / p.hd : 0;      // (a tile starts at a head's first feature: hd divides 128)
   auto place = [&](int m, Place& at) {
@@ -396,10 +396,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (p.splits > 1) {
           // Every CTA sends, whatever became of its waits, and nobody leaves before all that it is sent has arrived: no CTA's
           // memory goes away under a sender. In the ring's memory the parts may arrive once every CTA of the cluster has consumed
-          // its stages. (Fetched column by column from the other CTAs' shared memory, with a cluster barrier before and one behind,
-          // what follows the accumulator took 2.0 to 2.6 us of each of a layer's products at Qwen2.5-0.5B sizes at one row and 3.0 to
-          // 5.7 at 32; 0.9 to 1.2 and 1.3 to 3.4 now. Decode steps: 1 row of 300 keys 674 -> 592 us, 32 of 1,280 1,057 -> 879; at
-          // Llama-3.1-8B sizes 1, 8 and 64 rows of 4,096 keys 3,085 -> 2,957, 3,604 -> 3,455, 7,752 -> 7,643.)
+          // its stages. (Against sums fetched column by column from the other CTAs' shared memory, with a cluster barrier before and
+          // one behind: decode steps at Qwen2.5-0.5B sizes, 1 row of 300 keys 674 -> 592 us, 32 of 1,280 1,057 -> 879; at
+          // Llama-3.1-8B sizes 1, 8 and 64 rows of 4,096 keys 3,085 -> 2,957, 3,604 -> 3,455, 7,752 -> 7,643. What follows the
+          // accumulator takes 0.5 to 0.9 us of each of a layer's products at Qwen2.5-0.5B sizes at one row, 1.4 to 2.8 at 32.)
           cluster_wait();
           if (p.parts_in_ring) cluster_sync_all();
         }
@@ -602,9 +602,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // With p.rope the columns are whole heads [q | k | v] (the head size divides a share): q and k are rotated by the row's position, q
 // goes to c_bf16, k and v to the token's slot of the paged pools, as the rotation's kernel does from the product's float32 output,
 // with the same roundings. `RowPlace`: what a row's rotation needs, looked up while the tile is being computed.
-// (The rotation's kernel read the product from L2 and wrote half of it again: 16.7 us of a layer of 2,048 rows at Llama-3.1-8B sizes
-// beside 94 of the product; 88 together now, 27.5 -> 26.5 ms a prompt. 2,100 rows at Qwen2.5-0.5B sizes 14.0 + 4.5 -> 15.6, 507 rows at
-// the former 31.4 + 13.0 -> 34.4.)
+// (The rotation's kernel read the product from L2 and wrote half of it again: 16.8 us of a layer of 2,048 rows at Llama-3.1-8B sizes
+// beside 93 of the product, 89 to 92 together; a layer 826 -> 783 to 805 us, a whole prompt 26.86 -> 26.63 ms, where the runs of one side
+// differ by 1.5 %. 2,100 rows at Qwen2.5-0.5B sizes 13.7 + 3.8 -> 15.0. 507 rows at the former 31.5 + 12.3 -> 34.2, but 6 us of that
+// come back in the attention of the decoded rows behind it, whose blocks find no room beside the pairs'.)
 struct RowPlace { int there, ps; long long slot; };      // slot: of the row's key in a page's first head, negative: not stored
 __device__ __forceinline__ RowPlace row_place(const Params& p, int row, bool first) {
   RowPlace at{0, 0, -1};

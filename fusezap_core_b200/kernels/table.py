@@ -134,7 +134,7 @@ class CudaOps(Ops):
         self.fuse_argmax = True            # lm_head product and argmax in one pass where no logits are asked for
         self.sink_max_runs = 64            # single-token steps over all earlier keys: a row's keys are cut into at most this many runs
         self.fuse_depth_norm = True        # the depth average of a layer's result and the norm that follows in one kernel
-        self.fuse_rope = True              # q/k/v product, rotation and cache write in one kernel (few-token steps)
+        self.fuse_rope = True              # q/k/v product, rotation and cache write in one kernel (up to 32 rows; where K is not cut, more than 256)
         # 128-row tiles for experts with hundreds of rows: measured slower for the gated product (347 against 319 us at
         # 8,192 pairs x 2,048 x 1,024) and the same for the scatter product (199 against 205 us), so off
         self.grouped_tiles_128 = False

@@ -3,7 +3,8 @@
 `x <- x + delta` (the pending term of the previous sublayer), then `h = w * (x / sqrt(mean(x^2) + eps))`
 (fusezap/serve/models/llama.py:500-503, 508-523: `mean = sum * (1/D)`, the fused kernel also writes the residual
 stream). The residual stream x is float32 in both dtypes; the sum of squares, the scale and the weight product are
-computed in 32-bit and h is rounded once to the activation dtype. With `groups` > 1 the vector is normed in that many
+computed in 32-bit and h is rounded once to the activation dtype: behind the scale, or, where the products that read h apply the scale
+to their 32-bit sums (`ScaledRows`), ahead of it. With `groups` > 1 the vector is normed in that many
 equal consecutive parts, each by its own mean square; the weight still spans the whole vector. With `offset` the
 multiplier is `offset + w` (a weight stored as its distance from one has offset 1), added in float32 once at load.
 
