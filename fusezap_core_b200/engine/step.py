@@ -58,10 +58,13 @@ class Workspace:
         self._views: dict[tuple, torch.Tensor] = {}
 
     def get(self, tag: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
-        shape = tuple(shape)
-        view = self._views.get((tag, shape, dtype))
+        try:
+            view = self._views.get((tag, shape, dtype))
+        except TypeError:      # (a list cannot be looked up)
+            view = None
         if view is not None:
             return view
+        shape = tuple(shape)
         key = (tag, shape[1:], dtype)
         buf = self._bufs.get(key)
         if buf is None or buf.shape[0] < shape[0]:

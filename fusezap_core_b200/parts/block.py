@@ -10,7 +10,7 @@ from __future__ import annotations
 from dataclasses import replace
 from ..weights import ParamSpec
 from .base import (Block, FeedForward, LayerCache, Mixer, Norm, PendingNorm, can_leave_product, can_take_products, can_take_scaled, register_block,
-                   replaced, takes_products)
+                   takes_products)
 
 
 @register_block("pre_norm")
@@ -59,19 +59,18 @@ class PreNormBlock(Block):
     @takes_products
     def forward(self, ctx, x, delta, cache: LayerCache):
         mixer, ffn = self.mixer, self.ffn
-        own_mixer = replaced(mixer)      # (an object's own `forward` is run, on plain rows)
-        if self.scaled1 and not own_mixer and not replaced(self.norm1):
+        # (an object's own `forward` is run, on plain rows and terms)
+        if self.scaled1 and not (self.norm1.own_forward or mixer.own_forward):
             h = self.norm1.forward(ctx, x, delta, scaled=True)
         else:
             h = self.norm1.forward(ctx, x, delta)
         if ffn is None:
             return x, mixer.forward(ctx, h, cache)
-        own_ffn = replaced(ffn)
-        if self.scaled2 and self.mixer_pending is not None and not own_mixer and not own_ffn and not replaced(self.norm2):
+        if self.scaled2 and self.mixer_pending is not None and not (mixer.own_forward or self.norm2.own_forward or ffn.own_forward):
             h = self.norm2.forward(ctx, x, self.mixer_pending(mixer, ctx, h, cache), scaled=True)
         else:
             h = self.norm2.forward(ctx, x, mixer.forward(ctx, h, cache))
-        if self.product_left and self.ffn_pending is not None and not own_ffn and not replaced(self):
+        if self.product_left and self.ffn_pending is not None and not (ffn.own_forward or self.own_forward):
             return x, self.ffn_pending(ffn, ctx, h)
         return x, ffn.forward(ctx, h)
 

@@ -183,6 +183,10 @@ def test_a_forward_replaced_on_the_object_is_run(part, ops):
         p.forward = wraps(inner)(watch)
     same(logits(model), want)
     assert len(seen) == 4
+    for layer in model.layers:      # and no longer, once it is taken away
+        del getattr(layer, part).forward
+    same(logits(model), want)
+    assert len(seen) == 4 and not any(getattr(layer, part).own_forward for layer in model.layers)
 
 
 @pytest.mark.parametrize("ops", [Plain, FoldingOps])
