@@ -956,9 +956,10 @@ int launch_units(const void* q, const void* k_pool, long long pool_rows, const i
   // Few blocks merge twice: once before they wait, with nothing read of the scratch and nothing stored, so that the instructions are
   // in the SMs' caches when the partial results are there. Where all blocks are resident at once and have little to read (4 MB):
   // 32 rows of 1,280 keys and 4 of 2,000 at Qwen2.5-0.5B sizes 825 -> 787 us a step, 666 -> 641, one of 4,096 at Llama-3.1-8B sizes
-  // 2,818 -> 2,793. 8 of 4,096 there have 8 MB: 3,375 -> 3,407 with a first walk that also read the scratch. Reading the scratch
-  // ahead of the wait gained nothing over the zeros in shared memory; a branch around every load of the first walk lost 9 us of the
-  // 32 rows' gain, prefetches of the scratch 12.
+  // 2,818 -> 2,793. 8 of 4,096 there have 8 MB: 3,375 -> 3,407 with a first walk that also read the scratch, which raced with the grid
+  // that writes it. Against that walk the zeros in shared memory take 620 us for 613 at 2 rows of 2,000 keys at Qwen2.5-0.5B sizes, 666
+  // for 676 at 8 of 1,200, the same at 16 of 1,100, 5 of 4,000 and 32 of 1,280. A branch around every load of the first walk lost 9 us
+  // of the 32 rows' gain, prefetches of the scratch 12.
   const bool twice = (long long)cgrid.y * Hq <= 4 * sms && (long long)cgrid.y * Hq * NPU * HD <= 1 << 20;
   fz_launch(rows_high < N ? attn_combine_units_kernel<true, false> : twice ? attn_combine_units_kernel<false, true> : attn_combine_units_kernel<false, false>, cgrid, dim3(ct),
             (size_t)(NPU + 2) * 8 + 256 * 16 + 16 * 8, stream, (const float*)part_o,
